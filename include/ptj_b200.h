@@ -190,7 +190,11 @@ int ptj_colsum(const void* x, float* out, float* scratch, size_t scratch_floats,
  *   b_kmajor != 0: B is stored [N, K] (K contiguous, leading dim ldb); else B is stored [K, N] (N contiguous)
  *   in_dtype   PTJ_BF16: tcgen05 tensor-core kernel (TMA-fed, fp32 accumulate in TMEM); pointers 16-byte aligned,
  *              leading dimensions multiples of 8 elements.
- *              PTJ_F32 : exact-fp32 SIMT kernel, any shape (the "fp32 path").
+ *              PTJ_F32 : float32 accuracy, any shape (the "fp32 path"). With a workspace of
+ *              ptj_gemm_f32_workspace_floats floats (16-byte aligned) and float32 output the product runs on the tensor
+ *              cores, every operand split exactly into three bf16 parts; without one, or where that function returns
+ *              0 (small products), on fused-multiply-add units. An operand element that is infinite turns the
+ *              outputs it reaches into NaN on the tensor-core path (inf * 0 of a split part), not into +-inf.
  *   out_dtype  PTJ_F32 or PTJ_BF16, C row-major with leading dim ldc
  *   epilogue   PTJ_EPI_*; aux / aux_out meaning depends on it (same dtype and ld as C unless noted)
  *   split_k    >1 splits K over that many work items; partial tiles go to `workspace`
@@ -213,6 +217,9 @@ int ptj_gemm(const void* a, const void* b, void* c, const float* bias, const voi
              int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int64_t ldc, int a_kmajor,
              int b_kmajor, int in_dtype, int out_dtype, int epilogue, const ptj_dropout_args* dropout,
              int split_k, float* workspace, size_t workspace_floats, void* stream);
+
+/* Workspace (floats) with which a float32 product of this shape runs on the tensor cores; 0: it does not. */
+size_t ptj_gemm_f32_workspace_floats(int64_t M, int64_t N, int64_t K, int a_kmajor, int b_kmajor);
 
 /* split_k = PTJ_SPLIT_TAIL lets ptj_gemm even out a bad last round of tiles: a bf16 product on the 256 x 256-tile
  * thread-block-pair kernel whose tile count leaves most of the GPU idle in its last round (96 tiles on 74 pairs) runs

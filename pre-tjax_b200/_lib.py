@@ -63,6 +63,7 @@ _SIGNATURES = {
     "ptj_colsum": (c_int, [_P, _P, _P, c_size_t, c_int64, c_int64, c_int64, c_int, _P]),
     "ptj_gemm": (c_int, [_P, _P, _P, _P, _P, _P, c_int64, c_int64, c_int64, c_int64, c_int64, c_int64, c_int, c_int,
                          c_int, c_int, c_int, POINTER(DropoutArgs), c_int, _P, c_size_t, _P]),
+    "ptj_gemm_f32_workspace_floats": (c_size_t, [c_int64, c_int64, c_int64, c_int, c_int]),
     "ptj_gemm_tail_split_floats": (c_size_t, [c_int64, c_int64, c_int64]),
     "ptj_gemm_tail_split_rows": (c_int64, [c_int64, c_int64, c_int64]),
     "ptj_gemm_grouped2": (c_int, [POINTER(GemmProblem), POINTER(GemmProblem), c_int64, c_int, c_int, _P]),

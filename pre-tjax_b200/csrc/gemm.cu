@@ -7,11 +7,13 @@
 // or MN-major, which covers forward (x W^T), input-gradient (dy W) and weight-gradient (dy^T x) products without
 // any transposed copy. Work items = output tiles x K splits, walked by a static persistent schedule.
 //
-// fp32 inputs: plain shared-memory tiled FMA kernel (exact fp32, any shape) for the fp32 parity path.
+// fp32 inputs: products of some size run on the tensor cores with float32 accuracy (gemm_f32.cu); the others, and callers
+// that pass no workspace, on a plain shared-memory tiled FMA kernel (any shape).
 #include <atomic>
 
 #include "common.cuh"
 #include "gemm_epilogue.cuh"
+#include "gemm_f32.h"
 #include "tc_common.cuh"
 #include "tc_runtime.h"
 
@@ -975,6 +977,12 @@ extern "C" int ptj_gemm(const void* a, const void* b, void* c, const float* bias
 
   if (in_dtype == PTJ_F32) {
     if (split_k != 1) return PTJ_ERR_UNSUPPORTED;
+    if (out_dtype == PTJ_F32 && workspace != nullptr && aligned16(workspace)) {
+      const size_t need = gemm_f32_workspace_floats(M, N, K, a_kmajor != 0, b_kmajor != 0);
+      if (need > 0 && workspace_floats >= need && ptj_device_check() == PTJ_OK)
+        return gemm_f32_tc(static_cast<const float*>(a), static_cast<const float*>(b), ep, M, N, K, lda, ldb,
+                           a_kmajor != 0, b_kmajor != 0, workspace, st);
+    }
     const int64_t sam = a_kmajor ? lda : 1, sak = a_kmajor ? 1 : lda;
     const int64_t sbn = b_kmajor ? ldb : 1, sbk = b_kmajor ? 1 : ldb;
     dim3 grid(static_cast<unsigned>(ceil_div(N, SM_BN)), static_cast<unsigned>(ceil_div(M, SM_BM)));

@@ -236,6 +236,11 @@ def gemm(a, b, *, a_kmajor=True, b_kmajor=True, M=None, N=None, K=None, lda=None
                 split_k = 1  # this shape has no bad last round
             elif workspace is None or workspace.numel() < ws_n:
                 workspace = torch.empty(ws_n, device=a.device, dtype=torch.float32)
+    if a.dtype == torch.float32 and out.dtype == torch.float32:
+        # bf16 planes of both operands (and K parts): with them the product runs on the tensor cores, at float32 accuracy
+        ws_n = _lib.lib().ptj_gemm_f32_workspace_floats(M, N, K, int(a_kmajor), int(b_kmajor))
+        if ws_n and (workspace is None or workspace.numel() < ws_n):
+            workspace = torch.empty(ws_n, device=a.device, dtype=torch.float32)
     dargs = None
     if dropout_args is not None:
         p, train, seed, sid = dropout_args
