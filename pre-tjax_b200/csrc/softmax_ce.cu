@@ -235,7 +235,7 @@ cross_entropy_kernel(const int32_t* __restrict__ labels, const T* logits, T* dlo
   }
 }
 
-// ---- bf16 cross entropy, rows that start on a 16-byte boundary ---------------------------------------------------
+// ---- bf16 cross entropy; logits and gradient rows start at the same distance from a 16-byte boundary -----------------
 // The kernel above spends about 25 instructions per logit (64-bit column arithmetic, arg-max bookkeeping and the
 // online rescale inside the inner loop, a compare per element for the label) and is issue-bound at half of the memory
 // roofline. This one walks the row three times with 16-byte vectors and does the least possible per element:
@@ -246,6 +246,9 @@ cross_entropy_kernel(const int32_t* __restrict__ labels, const T* logits, T* dlo
 // Passes 2 and 3 read the row from L2 (512-thread blocks, three per SM: the 444 rows in flight, 100 KB each at
 // GPT-2's vocabulary, stay well inside the L2). Accuracy: the label is the arg-max iff x[label] equals the maximum and no earlier column does (ties go to
 // the first index, as in torch.argmax); the second condition is only walked for rows where the first holds.
+// Rows of an odd vocabulary stored without padding start anywhere: up to seven elements before the first boundary and
+// seven after the last whole vector are walked one by one. [8192, 50257] contiguous: 507 us through the generic kernel
+// above, 399 us here, calls and all; padded rows of the same size 340 us.
 constexpr int kCeThreads = 512;
 
 __device__ __forceinline__ uint32_t bf2_max(uint32_t a, uint32_t b) {
@@ -269,10 +272,23 @@ __device__ __forceinline__ uint64_t f2_add2(uint64_t a, uint64_t b) {
 
 constexpr float kLog2e = 1.4426950408889634f;
 
-// maximum of a row (every thread gets it): packed bf16 pairs over the 16-byte vectors, the last cols & 7 elements one by one
-__device__ __forceinline__ float row_max_bf16(const __nv_bfloat16* xr, int cols, float* red) {
-  const uint4* xv = reinterpret_cast<const uint4*>(xr);
-  const int nvec = cols >> 3;
+// The elements of a row outside its 16-byte vectors: `head` before the first boundary, then what the vectors leave over.
+struct RowEnds {
+  int head, nvec, n;  // n = head + tail elements
+  __device__ __forceinline__ RowEnds(int cols, int h) : head(h < cols ? h : cols) {
+    nvec = (cols - head) >> 3;
+    n = cols - (nvec << 3);
+  }
+  __device__ __forceinline__ int col(int i) const { return i < head ? i : i + (nvec << 3); }
+};
+__device__ __forceinline__ int head_bf16(const __nv_bfloat16* xr) {
+  return static_cast<int>(((16u - (reinterpret_cast<uintptr_t>(xr) & 15u)) & 15u) >> 1);
+}
+
+// maximum of a row (every thread gets it): packed bf16 pairs over the 16-byte vectors, the other elements one by one
+__device__ __forceinline__ float row_max_bf16(const __nv_bfloat16* xr, const RowEnds& re, float* red) {
+  const uint4* xv = reinterpret_cast<const uint4*>(xr + re.head);
+  const int nvec = re.nvec;
   uint32_t pm = 0xff80ff80u;  // two packed -inf
   int i = threadIdx.x;
   for (; i + 3 * kCeThreads < nvec; i += 4 * kCeThreads) {
@@ -285,14 +301,14 @@ __device__ __forceinline__ float row_max_bf16(const __nv_bfloat16* xr, int cols,
     pm = bf2_max(pm, bf2_max(bf2_max(a.x, a.y), bf2_max(a.z, a.w)));
   }
   float m = fmaxf(__uint_as_float(pm << 16), __uint_as_float(pm & 0xffff0000u));
-  for (int c = (nvec << 3) + threadIdx.x; c < cols; c += kCeThreads) m = fmaxf(m, __bfloat162float(xr[c]));
+  for (int t = threadIdx.x; t < re.n; t += kCeThreads) m = fmaxf(m, __bfloat162float(xr[re.col(t)]));
   return block_max(m, red);
 }
 
 // sum over the row of 2^(x log2 e + nml), nml = -max log2 e (every thread gets it)
-__device__ __forceinline__ float row_expsum_bf16(const __nv_bfloat16* xr, int cols, float nml, float* red) {
-  const uint4* xv = reinterpret_cast<const uint4*>(xr);
-  const int nvec = cols >> 3;
+__device__ __forceinline__ float row_expsum_bf16(const __nv_bfloat16* xr, const RowEnds& re, float nml, float* red) {
+  const uint4* xv = reinterpret_cast<const uint4*>(xr + re.head);
+  const int nvec = re.nvec;
   const uint64_t l2e2 = f2_pack(kLog2e, kLog2e), nml2 = f2_pack(nml, nml);
   float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
   auto add8 = [&](const uint4& a) {
@@ -308,7 +324,7 @@ __device__ __forceinline__ float row_expsum_bf16(const __nv_bfloat16* xr, int co
   };
   // (four loads in flight per thread, as in the maximum pass, measured no faster here: 344 against 340 us)
   for (int i = threadIdx.x; i < nvec; i += kCeThreads) add8(xv[i]);
-  for (int c = (nvec << 3) + threadIdx.x; c < cols; c += kCeThreads) s0 += ex2_approx(fmaf(__bfloat162float(xr[c]), kLog2e, nml));
+  for (int t = threadIdx.x; t < re.n; t += kCeThreads) s0 += ex2_approx(fmaf(__bfloat162float(xr[re.col(t)]), kLog2e, nml));
   return block_sum((s0 + s1) + (s2 + s3), red);
 }
 
@@ -319,11 +335,11 @@ cross_entropy_bf16_kernel(const int32_t* __restrict__ labels, const __nv_bfloat1
   grid_dep_sync();
   __shared__ float red[33];
   const float inv_n = 1.f / *n_valid;
-  const int nvec = cols >> 3;        // whole 16-byte vectors; the last cols & 7 elements are walked one by one
-  const int tail0 = nvec << 3;
   for (int64_t row = blockIdx.x; row < rows; row += gridDim.x) {
     const __nv_bfloat16* xr = logits + row * ld;
-    const uint4* xv = reinterpret_cast<const uint4*>(xr);
+    const RowEnds re(cols, head_bf16(xr));
+    const int nvec = re.nvec;
+    const uint4* xv = reinterpret_cast<const uint4*>(xr + re.head);
     __nv_bfloat16* dr = dlogits != nullptr ? dlogits + row * ld : nullptr;
     const int label = labels[row];
     if (label <= 0 || label >= cols) {  // padding (or an id outside the vocabulary): no contribution
@@ -332,14 +348,14 @@ cross_entropy_bf16_kernel(const int32_t* __restrict__ labels, const __nv_bfloat1
         row_stats[rows + row] = 0.f;
       }
       if (dr != nullptr) {
-        for (int i = threadIdx.x; i < nvec; i += kCeThreads) reinterpret_cast<uint4*>(dr)[i] = make_uint4(0u, 0u, 0u, 0u);
-        for (int c = tail0 + threadIdx.x; c < cols; c += kCeThreads) dr[c] = __float2bfloat16_rn(0.f);
+        for (int i = threadIdx.x; i < nvec; i += kCeThreads) reinterpret_cast<uint4*>(dr + re.head)[i] = make_uint4(0u, 0u, 0u, 0u);
+        for (int t = threadIdx.x; t < re.n; t += kCeThreads) dr[re.col(t)] = __float2bfloat16_rn(0.f);
       }
       continue;
     }
     const float x_label = __bfloat162float(xr[label]);  // read before the row is overwritten in place
     // pass 1: maximum
-    const float m = row_max_bf16(xr, cols, red);
+    const float m = row_max_bf16(xr, re, red);
     // is the label the first column that attains the maximum?
     float hit = 0.f;
     if (x_label == m) {  // (uniform over the block)
@@ -350,7 +366,7 @@ cross_entropy_bf16_kernel(const int32_t* __restrict__ labels, const __nv_bfloat1
     // pass 2: sum of exponentials
     const float nml = -m * kLog2e;
     const uint64_t l2e2 = f2_pack(kLog2e, kLog2e);
-    const float s = row_expsum_bf16(xr, cols, nml, red);
+    const float s = row_expsum_bf16(xr, re, nml, red);
     if (threadIdx.x == 0) {
       row_stats[row] = -(x_label - m - logf(s));
       row_stats[rows + row] = hit;
@@ -359,7 +375,7 @@ cross_entropy_bf16_kernel(const int32_t* __restrict__ labels, const __nv_bfloat1
     // pass 3: dlogits = softmax / n_valid, the label's column minus 1 / n_valid
     const float c3 = nml + log2f(inv_n / s);
     const uint64_t c32 = f2_pack(c3, c3);
-    uint4* dv = reinterpret_cast<uint4*>(dr);
+    uint4* dv = reinterpret_cast<uint4*>(dr + re.head);
     auto grad8 = [&](const uint4& a) {
       const uint32_t w[4] = {a.x, a.y, a.z, a.w};
       uint32_t o[4];
@@ -373,8 +389,10 @@ cross_entropy_bf16_kernel(const int32_t* __restrict__ labels, const __nv_bfloat1
       return make_uint4(o[0], o[1], o[2], o[3]);
     };
     for (int i = threadIdx.x; i < nvec; i += kCeThreads) dv[i] = grad8(xv[i]);
-    for (int c = tail0 + threadIdx.x; c < cols; c += kCeThreads)
+    for (int t = threadIdx.x; t < re.n; t += kCeThreads) {
+      const int c = re.col(t);
       dr[c] = __float2bfloat16_rn(ex2_approx(fmaf(__bfloat162float(xr[c]), kLog2e, c3)));
+    }
     __syncthreads();  // the label's column has been written (by whichever thread owns it) before it is patched
     if (threadIdx.x == 0) dr[label] = __float2bfloat16_rn(ex2_approx(fmaf(x_label, kLog2e, c3)) - inv_n);
   }
@@ -390,8 +408,9 @@ log_softmax_fwd_bf16_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* 
   for (int64_t row = blockIdx.x; row < rows; row += gridDim.x) {
     const __nv_bfloat16* xr = x + row * ld_x;
     __nv_bfloat16* yr = y + row * ld_y;
-    const float m = row_max_bf16(xr, cols, red);
-    const float s = row_expsum_bf16(xr, cols, -m * kLog2e, red);
+    const RowEnds re(cols, 0);
+    const float m = row_max_bf16(xr, re, red);
+    const float s = row_expsum_bf16(xr, re, -m * kLog2e, red);
     const float nshift = -(m + logf(s));
     const uint64_t ns2 = f2_pack(nshift, nshift);
     const uint4* xv = reinterpret_cast<const uint4*>(xr);
@@ -427,9 +446,10 @@ log_softmax_bwd_bf16_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfl
     __nv_bfloat16* dr = dx + row * ld;
     const uint4* xv = reinterpret_cast<const uint4*>(xr);
     const uint4* gv = reinterpret_cast<const uint4*>(gr);
-    const float m = row_max_bf16(xr, cols, red);
+    const RowEnds re(cols, 0);
+    const float m = row_max_bf16(xr, re, red);
     const float nml = -m * kLog2e;
-    const float s = row_expsum_bf16(xr, cols, nml, red);
+    const float s = row_expsum_bf16(xr, re, nml, red);
     uint64_t g0 = 0ull, g1 = 0ull;  // two packed +0.0f each
     for (int i = threadIdx.x; i < nvec; i += kCeThreads) {
       const uint4 a = gv[i];
@@ -577,7 +597,8 @@ extern "C" int ptj_cross_entropy(const int32_t* labels, const void* logits, void
     launch_k(cross_entropy_kernel<float>, row_grid(rows), kRowThreads, 0, st, 
         labels, static_cast<const float*>(logits), static_cast<float*>(dlogits), row_stats, n_valid, rows, cols, ld,
         same_phase<float>(logits, ld, dlogits, ld));
-  } else if (aligned16(logits) && (dlogits == nullptr || aligned16(dlogits)) && ld % 8 == 0 && cols <= 0x7fffffffLL) {
+  } else if (same_phase<__nv_bfloat16>(logits, ld, dlogits, ld) && cols <= 0x7fffffffLL &&
+             reinterpret_cast<uintptr_t>(logits) % 2 == 0) {
     const int64_t cap = static_cast<int64_t>(kNumSMs) * 3;  // three resident 512-thread blocks per SM
     launch_k(cross_entropy_bf16_kernel, static_cast<int>(rows < cap ? rows : cap), kCeThreads, 0, st, labels,
              static_cast<const __nv_bfloat16*>(logits), static_cast<__nv_bfloat16*>(dlogits), row_stats, n_valid, rows,
