@@ -78,6 +78,9 @@ _SIGNATURES = {
     "ptj_sumsq": (c_int, [_P, _P, _P, c_size_t, c_int64, _P]),
     "ptj_adamw": (c_int, [_P, _P, _P, _P, _P, c_int64, _P, _P, c_int, c_float, c_float, c_float, c_float, c_float,
                           c_int64, c_float, _P, c_float, _P]),
+    "ptj_decode_workspace_floats": (c_size_t, [c_int64] * 7),
+    "ptj_decode": (c_int, [_P, _P, _P, _P, _P, _P, _P, c_int64, c_float, c_int64, c_int64, c_int64, c_int64, c_int64, c_int64,
+                           c_int64, _P, c_size_t, _P]),
     "ptj_cast_f32_to_bf16": (c_int, [_P, _P, c_int64, _P]),
 }
 

@@ -5,7 +5,7 @@ Mirrors the callers the reference's train script uses between training steps:
 * ``t_gpt2_forward``  – logits only (model_triton.py:2523-2527, the forward without saved activations)
 * ``t_loss`` / ``loss_eval`` – ``(loss, (loss, accuracy, valid fraction))`` (loss_and_optimizer_triton.py:217-232)
 * ``log_probs``       – per-sequence sum of label log-probabilities, HellaSwag-style scoring (:293-311)
-* ``predict``         – greedy decoding that re-runs the whole forward for every new token (:203-212)
+* ``predict``         – greedy decoding (:203-212)
 
 With ``train=False`` every dropout site multiplies by ``1 - DROPOUT_RATE`` (model_torch_func.py:98-102) instead of
 drawing a mask. The quirks of the reference are kept because its outputs are the contract: ``log_probs`` adds **1**
@@ -65,13 +65,22 @@ def log_probs(params, y, y_mask=None, y_indices=None):
 
 def predict(params, y_mask, y_indices, sample_len, start_tok, end_tok):
     """Greedy decoding of ``y_mask.shape[0]`` sequences (an int batch size is accepted too): int64[B, sample_len-1].
-    Every step runs the full forward over the ``sample_len`` positions (the reference has no KV cache) and takes the
-    arg-max of position ``step`` with the row arg-max kernel. ``sample_len`` must equal the model's sequence length
-    because the positional table is added without slicing."""
+    ``sample_len`` must equal the model's sequence length because the positional table is added without slicing.
+    float32 weights: one launch decodes all positions with the keys and values of earlier ones kept, as the causal mask
+    allows (operators.decode_greedy). Otherwise, bf16 weights above all, every step runs the full forward over the
+    ``sample_len`` positions, as the reference does, and takes the arg-max of position ``step``: there the activations
+    are rounded to bf16 between the launches, and which token wins depends on that."""
     B = int(y_mask) if isinstance(y_mask, int) else y_mask.shape[0]
     device = params[0][0].device
     y_sample = torch.full((B, sample_len), start_tok, device=device, dtype=torch.int64)
-    for step_i in range(sample_len - 1):
+    cfg = config_from_params(params, ops.DROPOUT_RATE)
+    assert sample_len == cfg.seq or sample_len < 2, "the positional table is added without slicing: sample_len must equal cfg.seq"
+    tokens = None
+    if params[0][0].dtype == torch.float32 and sample_len > 1:
+        tokens = ops.decode_greedy(Weights.from_pytree(params, cfg, torch.float32), cfg, B, int(start_tok))
+    if tokens is not None:
+        y_sample[:, 1:] = tokens[:, 1:]
+    for step_i in range(sample_len - 1 if tokens is None else 0):
         logits, cfg, _ = _forward_padded(params, y_sample, False, None)
         rows = logits.view(B, sample_len, -1)[:, step_i]  # [B, vocab_ld], row stride sample_len * vocab_ld
         y_sample[:, step_i + 1] = ops.argmax_rows(rows, cols=cfg.vocab).to(torch.int64)

@@ -514,6 +514,32 @@ def cross_entropy(labels, logits, cols=None, want_grad=True, in_place=False, n_v
     return out3, n_valid, dlogits
 
 
+DECODE_GROUP = 8  # sequences that ptj_decode takes in one launch
+
+
+def decode_greedy(w, cfg, batch: int, start: int, p=None):
+    """int32 [batch, cfg.seq]: greedy decoding of `batch` sequences from the token `start` (columns 1.. are written), for
+    float32 weights; None where ptj_decode does not apply (other types, sizes or alignments). w: gpt2.Weights."""
+    if any(t.dtype != torch.float32 or t.data_ptr() % 16 for t in w.t.values()) or cfg.seq < 2 or batch < 1:
+        return None
+    lib, p = _lib.lib(), DROPOUT_RATE if p is None else p
+    dims = (cfg.vocab, cfg.dim, cfg.layers, cfg.heads, cfg.ffn, cfg.seq)
+    need = int(lib.ptj_decode_workspace_floats(min(batch, DECODE_GROUP), *dims))
+    if need == 0:
+        return None
+    device = w["w_emb"].device
+    names = [n for n, _ in cfg.param_shapes() if n.startswith("l")]
+    ptrs = torch.tensor([w[n].data_ptr() for n in names], dtype=torch.int64, device=device)
+    tokens = torch.empty((batch, cfg.seq), device=device, dtype=torch.int32)
+    ws = torch.empty(need, device=device, dtype=torch.float32)
+    for b0 in range(0, batch, DECODE_GROUP):
+        n = min(batch - b0, DECODE_GROUP)
+        _lib.check(lib.ptj_decode(_ptr(w["w_emb"]), _ptr(w["b_head"]), _ptr(w["w_pos"]), _ptr(ptrs), _ptr(w["g_f"]),
+                                  _ptr(w["b_f"]), _ptr(tokens[b0:]), start, p, n, *dims, _ptr(ws), ws.numel(), _stream()),
+                   "ptj_decode")
+    return tokens
+
+
 def argmax_rows(x: torch.Tensor, cols=None) -> torch.Tensor:
     """int32[rows] = index of the largest of the first `cols` elements of every row of x [rows, ld] (first index on
     ties): the torch.argmax of the reference's greedy decoding loop (loss_and_optimizer_triton.py:207)."""
