@@ -259,25 +259,24 @@ class Gpt2Step:
             seeds = [0] * (1 + 3 * cfg.layers)
         x = ops.embed_fwd(ids_in, w["w_emb"], w["w_pos"], train, seeds[0], out_dtype=self.dtype, p=p).view(T, D)
         acts = {"layers": [], "row_kstart": row_kstart}
+        tail = tail_split_for(T, D, cfg.ffn) if (self.tail_split and self.dtype == torch.bfloat16) else None
         for l in range(cfg.layers):
             s_attn, s_res1, s_res2 = seeds[1 + 3 * l: 4 + 3 * l]
-            g = lambda n: w[f"l{l}.{n}"]
+            g = lambda n: w.t[f"l{l}.{n}"]
             a = {"x": x}
             a["ln1"] = ops.t_layernorm_fwd_t((g("g1"), g("b1")), x)
             a["qkv"] = ops.gemm(a["ln1"], g("w_qkv").view(3 * D, D))  # columns ordered (head, q/k/v, d_head)
-            qkv5 = a["qkv"].view(B, S, H, 3, dh)
-            q, k, v = (qkv5[:, :, :, c, :].permute(0, 2, 1, 3) for c in range(3))
-            a["attn"] = torch.empty((T, D), device=x.device, dtype=self.dtype)
-            o4 = a["attn"].view(B, S, H, dh).permute(0, 2, 1, 3)
+            q, k, v = a["qkv"].view(B, S, H, 3, dh).permute(3, 0, 2, 1, 4).unbind(0)
+            a["attn"] = x.new_empty((T, D))
+            o4 = a["attn"].view(B, S, H, dh).transpose(1, 2)
             # the layer's attention-dropout keep flags are drawn once and shared by the forward and backward kernels
             a["keep"] = ops.attn_keep_bits(q, k, v, o4, s_attn, p=p) if (train and p > 0.0) else None
             a["m"], a["l"] = ops.attn_fwd(q, k, v, o4, train, s_attn, p=p, keep_bits=a["keep"], row_kstart=row_kstart)
             a["x_mid"] = ops.gemm(a["attn"], g("w_o"), epilogue=_lib.EPI_DROPOUT_RESID, aux=x,
                                   dropout_args=(p, train, s_res1, 0))
             a["ln2"] = ops.t_layernorm_fwd_t((g("g2"), g("b2")), a["x_mid"])
-            a["h_pre"] = torch.empty((T, cfg.ffn), device=x.device, dtype=self.dtype)
+            a["h_pre"] = x.new_empty((T, cfg.ffn))
             a["h_act"] = ops.gemm(a["ln2"], g("w1"), bias=g("b1f"), epilogue=_lib.EPI_GELU, aux_out=a["h_pre"])
-            tail = tail_split_for(T, D, cfg.ffn) if (self.tail_split and self.dtype == torch.bfloat16) else None
             x = ops.gemm(a["h_act"], g("w2"), bias=g("b2f"), epilogue=_lib.EPI_DROPOUT_RESID, aux=a["x_mid"],
                          dropout_args=(p, train, s_res2, 0), split_k=ops.SPLIT_TAIL if tail else 1,
                          workspace=self._workspace(tail[1]) if tail else None)
@@ -340,12 +339,11 @@ class Gpt2Step:
                 dy = ops.dropout(dx, train, s_res1, p=p)
             dy_attn = dy
             d_attn = self._dgrad(dy, g("w_o"))
-            dqkv = torch.empty((T, 3 * D), device=dy.device, dtype=self.dtype)
-            qkv5, dqkv5 = a["qkv"].view(B, S, H, 3, dh), dqkv.view(B, S, H, 3, dh)
-            q, k, v = (qkv5[:, :, :, c, :].permute(0, 2, 1, 3) for c in range(3))
-            dq, dk, dv = (dqkv5[:, :, :, c, :].permute(0, 2, 1, 3) for c in range(3))
-            o4 = a["attn"].view(B, S, H, dh).permute(0, 2, 1, 3)
-            do4 = d_attn.view(B, S, H, dh).permute(0, 2, 1, 3)
+            dqkv = dy.new_empty((T, 3 * D))
+            q, k, v = a["qkv"].view(B, S, H, 3, dh).permute(3, 0, 2, 1, 4).unbind(0)
+            dq, dk, dv = dqkv.view(B, S, H, 3, dh).permute(3, 0, 2, 1, 4).unbind(0)
+            o4 = a["attn"].view(B, S, H, dh).transpose(1, 2)
+            do4 = d_attn.view(B, S, H, dh).transpose(1, 2)
             ops.attn_bwd(do4, q, k, v, o4, a["m"], a["l"], dq, dk, dv, train, s_attn, p=p, keep_bits=a.get("keep"),
                          row_kstart=acts.get("row_kstart"))
             self._wgrad2((dqkv, a["ln1"], G("w_qkv").view(3 * D, D)), (dy_attn, a["attn"], G("w_o")))
