@@ -8,9 +8,10 @@
 // output tile, in registers: two or three 16-byte shared loads per 32 multiply-adds. Score products pack neighbouring
 // d into the two-wide FMA straight from those loads. Bound by the FP32 pipe (a warp per row with scalar global loads
 // was bound by the load/store unit instead). Measured, float32, forward / backward: [8, 12, 512, 64] with dropout and
-// document masks 98 / 314 us (33 / 36 TFLOP/s of the causal half), where a warp per row with a Philox call per probability
-// took 2526 / 16152 us; [4, 12, 512, 64] without dropout 90 / 298 us, forward 1900 us before. R = 8 keeps most operands in registers; head sizes above 64 take R = 4
-// with twice the threads, because R = 8 would need more than 255 registers.
+// document masks 88 / 317 us (36 / 36 TFLOP/s of the causal half), where a warp per row with a Philox call per probability
+// took 2526 / 16152 us; [4, 12, 512, 64] without dropout 84 / 268 us, forward 1900 us before. R = 4: twice the warps of
+// R = 8, which needs 255 registers and measured 98 / 314 and 90 / 294 us there, 23 / 75 us against 17 / 55 us at
+// [2, 12, 128, 64].
 #include "attn_common.cuh"
 
 namespace ptj {
@@ -593,8 +594,8 @@ int fwd_typed(const void* q, const void* k, const void* v, void* o, float* row_m
   const FwdArgs<T> a{static_cast<const T*>(q), static_cast<const T*>(k), static_cast<const T*>(v), static_cast<T*>(o),
                      row_max, row_sum, row_kstart, sh, 1.f / sqrtf(static_cast<float>(sh.d_head)),
                      static_cast<int>(ceil_div(sh.seq, kB)), rows_vectorise<T>(sh, ptrs, 4), dr};
-  if (sh.d_head <= 32) return run_fwd<T, 32, 8>(a, st);
-  if (sh.d_head <= 64) return run_fwd<T, 64, 8>(a, st);
+  if (sh.d_head <= 32) return run_fwd<T, 32, 4>(a, st);
+  if (sh.d_head <= 64) return run_fwd<T, 64, 4>(a, st);
   return run_fwd<T, 128, 4>(a, st);
 }
 
@@ -608,8 +609,8 @@ int bwd_typed(const void* d_o, const void* q, const void* k, const void* v, cons
                      static_cast<T*>(dk), static_cast<T*>(dv), row_kstart, sh, dsh,
                      1.f / sqrtf(static_cast<float>(sh.d_head)), static_cast<int>(ceil_div(sh.seq, kB)),
                      rows_vectorise<T>(sh, ptrs, 8) && rows_vectorise<T>(dsh, ptrs, 0), dr};
-  if (sh.d_head <= 32) return run_bwd<T, 32, 8>(a, st);
-  if (sh.d_head <= 64) return run_bwd<T, 64, 8>(a, st);
+  if (sh.d_head <= 32) return run_bwd<T, 32, 4>(a, st);
+  if (sh.d_head <= 64) return run_bwd<T, 64, 4>(a, st);
   return run_bwd<T, 128, 4>(a, st);
 }
 
