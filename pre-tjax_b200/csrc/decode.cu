@@ -10,9 +10,11 @@
 // through rows, steps, layers and tokens: memory stays busy while the block waits at a barrier, normalises or attends.
 // A lane reads only bytes that it copied itself, so the ring needs no barrier.
 //
-// Measured, 12 layers x 768, vocabulary 35374, two sequences of 128: 46.8 ms, 369 us a token; the weights alone take 69 us,
+// Measured, 12 layers x 768, vocabulary 35374, two sequences of 128: 38.4 ms, 302 us a token; the weights alone take 69 us,
 // the rest is the chain of 61 steps (barrier, activations, normalisation, reduction). A whole forward pass per token on
-// the tensor cores took 374 ms.
+// the tensor cores took 374 ms. 46.8 ms before these: the ring's next address kept in registers, layer pointers in shared
+// memory (their loads stood in front of every unit), attention without block-wide scores, a barrier of one release and
+// acquire without fences.
 #include "common.cuh"
 #include "tc_common.cuh"
 #include "tc_runtime.h"
@@ -62,21 +64,17 @@ struct Share {
   int first, n;
 };
 
-// The order in which a warp meets the weights: (token, layer, step, unit, chunk).
+// The order in which a warp meets the weights: (token, layer, step, unit, chunk). Between units a lane only moves a pointer:
+// the ring is refilled in the multiplying loop, whose length is what the steps wait for.
 struct Cursor {
-  int t, l, s, u, c, c1;
-  int nunits;
-  const float* w;   // the pair's first row
-  const Share* share;
+  int t, l, s, u;
+  int left, col, K;   // chunks of the unit still to fetch, this lane's column, row length
+  const float* w;     // this lane's position in the pair's first row
   bool two, valid;
-  __device__ __forceinline__ const float* matrix(const DecodeParams& p) const {
-    if (s == 4) return p.w_emb;
-    const int idx = s == 0 ? 2 : (s == 1 ? 3 : (s == 2 ? 6 : 8));
-    return p.layers[l * kLayerTensors + idx];
-  }
-  __device__ __forceinline__ void enter(const DecodeParams& p) { nunits = share[s].n * p.step[s].parts; }
+  const Share* share;
+  const float* const* layers;  // in shared memory
   __device__ __forceinline__ void locate(const DecodeParams& p) {  // unit u of the current step, or the next step that has one
-    while (u >= nunits) {
+    while (u >= share[s].n * p.step[s].parts) {
       u = threadIdx.x >> 5;
       if (s == 4) {
         if (++t >= p.S - 1) {
@@ -94,39 +92,38 @@ struct Cursor {
       } else {
         ++s;
       }
-      enter(p);
     }
     const Step& st = p.step[s];
-    const int pair = share[s].first + u / st.parts, part = u % st.parts;
-    w = matrix(p) + static_cast<int64_t>(pair) * 2 * st.K;
+    const int pair = share[s].first + u / st.parts, c = u % st.parts * st.cpp;
+    const int idx = s == 0 ? 2 : (s == 1 ? 3 : (s == 2 ? 6 : 8));
+    K = st.K;
+    col = c * kChunk + (threadIdx.x & 31) * 4;
+    w = (s == 4 ? p.w_emb : layers[l * kLayerTensors + idx]) + static_cast<int64_t>(pair) * 2 * K + col;
     two = 2 * pair + 1 < st.R;
-    c = part * st.cpp;
-    c1 = min(st.nch, c + st.cpp);
+    left = min(st.nch - c, st.cpp);
   }
-  __device__ __forceinline__ void init(const DecodeParams& p, const Share* sh) {
+  __device__ __forceinline__ void init(const DecodeParams& p, const Share* sh, const float* const* lt) {
     share = sh;
+    layers = lt;
     t = l = s = 0;
     u = threadIdx.x >> 5;
     valid = true;
-    enter(p);
     locate(p);
-  }
-  __device__ __forceinline__ void advance(const DecodeParams& p) {
-    if (++c == c1) {
-      u += kWarps;
-      locate(p);
-    }
   }
 };
 
-// One ring slot: [2 rows][32 lanes] x 16 bytes.
-__device__ __forceinline__ void fetch(Cursor& cur, const DecodeParams& p, uint32_t slot, int lane) {
+// One ring slot: [2 rows][32 lanes] x 16 bytes. dst: this lane's place in the first row.
+__device__ __forceinline__ void fetch(Cursor& cur, const DecodeParams& p, uint32_t dst) {
   if (cur.valid) {
-    const int K = p.step[cur.s].K, col = cur.c * kChunk + lane * 4;
-    const bool in = col < K;
-    cp_async16(slot + lane * 16, cur.w + (in ? col : 0), in);
-    cp_async16(slot + 512 + lane * 16, cur.w + (in && cur.two ? K + col : 0), in && cur.two);
-    cur.advance(p);
+    const bool in = cur.col < cur.K, in2 = in && cur.two;
+    cp_async16(dst, in ? cur.w : p.w_emb, in);
+    cp_async16(dst + 512, in2 ? cur.w + cur.K : p.w_emb, in2);
+    cur.w += kChunk;
+    cur.col += kChunk;
+    if (--cur.left == 0) {
+      cur.u += kWarps;
+      cur.locate(p);
+    }
   }
   cp_async_commit();  // one group per chunk, empty ones at the end: the wait below counts groups
 }
@@ -136,8 +133,7 @@ __device__ __forceinline__ bool grid_barrier(const DecodeParams& p, unsigned int
   __syncthreads();
   target += gridDim.x;
   if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(p.barrier, 1u);
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p.barrier) : "memory");
     const long long t0 = clock64();
     int ok = 1;
     unsigned int seen;
@@ -150,7 +146,6 @@ __device__ __forceinline__ bool grid_barrier(const DecodeParams& p, unsigned int
         break;
       }
     }
-    __threadfence();
     *ok_s = ok;
   }
   __syncthreads();
@@ -189,14 +184,15 @@ __global__ void __launch_bounds__(kThreads, 1)
 decode_kernel(const __grid_constant__ DecodeParams p) {
   extern __shared__ __align__(16) uint8_t smem[];
   float* act = reinterpret_cast<float*>(smem + kWarps * DEPTH * 1024);  // [NB][act_ld], zero beyond the row
-  float* part = act + NB * p.act_ld;                                     // [units][2][NB]
+  const float** layers = reinterpret_cast<const float**>(act + NB * p.act_ld);  // [L][kLayerTensors]
+  float* part = reinterpret_cast<float*>(layers + p.L * kLayerTensors);  // [units][2][NB]
   __shared__ int ok_s;
   __shared__ Share share[kSteps];
   __shared__ Best best_s[kWarps][NB];
   __shared__ int token_s[NB];
   __shared__ float2 stats_s[NB];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t ring = tc::smem_u32(smem + warp * DEPTH * 1024);
+  const uint32_t ring = tc::smem_u32(smem + warp * DEPTH * 1024) + lane * 16;
   const uint8_t* ring_p = smem + warp * DEPTH * 1024;
 
   if (tid < kSteps) {
@@ -205,11 +201,12 @@ decode_kernel(const __grid_constant__ DecodeParams p) {
     share[tid].n = static_cast<int>(pairs * (blockIdx.x + 1) / gridDim.x) - share[tid].first;
   }
   if (tid < p.B) token_s[tid] = p.start;
+  for (int i = tid; i < p.L * kLayerTensors; i += kThreads) layers[i] = p.layers[i];
   __syncthreads();
   Cursor cur;
-  cur.init(p, share);
+  cur.init(p, share, layers);
 #pragma unroll 1
-  for (int i = 0; i < DEPTH - 1; ++i) fetch(cur, p, ring + i * 1024, lane);
+  for (int i = 0; i < DEPTH - 1; ++i) fetch(cur, p, ring + i * 1024);
   int slot = 0;                     // next chunk to consume
   int free_slot = DEPTH - 1;        // next slot to fill
   unsigned int target = 0;
@@ -236,7 +233,7 @@ decode_kernel(const __grid_constant__ DecodeParams p) {
           acc[0][b] = fmaf(w0.w, a.w, fmaf(w0.z, a.z, fmaf(w0.y, a.y, fmaf(w0.x, a.x, acc[0][b]))));
           acc[1][b] = fmaf(w1.w, a.w, fmaf(w1.z, a.z, fmaf(w1.y, a.y, fmaf(w1.x, a.x, acc[1][b]))));
         }
-        fetch(cur, p, ring + free_slot * 1024, lane);
+        fetch(cur, p, ring + free_slot * 1024);
         slot = slot + 1 == DEPTH ? 0 : slot + 1;
         free_slot = free_slot + 1 == DEPTH ? 0 : free_slot + 1;
       }
@@ -250,13 +247,13 @@ decode_kernel(const __grid_constant__ DecodeParams p) {
     }
     __syncthreads();
   };
-  // The products of a step and finish(row, b, sum, side(row, b)) for every output of this block's rows. side (a bias, the
+  // The products of a step and finish(row, b, sum, side(row, b)) for every output of this block's rows. side (a bias and the
   // residual) is read from memory before the products for the first output of a thread, which is the only one as a rule.
   auto run_step = [&](int s, auto&& side, auto&& finish) {
     const Step& st = p.step[s];
     const int row0 = 2 * share[s].first, n = share[s].n * 2 * NB;
     auto real = [&](int i) { return i < n && i % NB < p.B && row0 + i / NB < st.R; };
-    const float side0 = real(tid) ? side(row0 + tid / NB, tid % NB) : 0.f;
+    const float2 side0 = real(tid) ? side(row0 + tid / NB, tid % NB) : make_float2(0.f, 0.f);
     multiply(s);
     for (int i = tid; i < n; i += kThreads) {
       if (!real(i)) continue;
@@ -308,7 +305,7 @@ decode_kernel(const __grid_constant__ DecodeParams p) {
     }
     __syncthreads();
   };
-  const auto none = [](int, int) { return 0.f; };
+  const auto none = [](int, int) { return make_float2(0.f, 0.f); };
 
   for (int pos = 0; pos < p.S - 1; ++pos) {
     // embedding of the token at `pos`: every block forms the whole row, and keeps its own rows of the residual stream
@@ -321,13 +318,13 @@ decode_kernel(const __grid_constant__ DecodeParams p) {
       if (d >= x0 && d < x1) p.x[i] = e;
     }
     for (int l = 0; l < p.L; ++l) {
-      const float* const* w = p.layers + l * kLayerTensors;
+      const float* const* w = layers + l * kLayerTensors;
       float* kv = p.kv + static_cast<int64_t>(l) * p.B * p.H * 2 * kv_plane;
       // QKV: rows ordered (head, q/k/v, d)
       if (l > 0) load_act(p.x, p.D);
       clear_tail(p.step[0]);
       normalise(w[0], w[1]);
-      run_step(0, none, [&](int row, int b, float v, float) {
+      run_step(0, none, [&](int row, int b, float v, float2) {
         const int hd = row / (3 * dh), c = row / dh % 3, d = row % dh;
         if (c == 0) p.q[(b * p.H + hd) * dh + d] = v;
         else kv[((static_cast<int64_t>(b) * p.H + hd) * 2 + (c - 1)) * kv_plane + static_cast<int64_t>(pos) * dh + d] = v;
@@ -336,52 +333,74 @@ decode_kernel(const __grid_constant__ DecodeParams p) {
 
       // attention of one position over the cached keys: a block per (sequence, head)
       {
+        // A group of lanes takes every groups-th key with a running maximum, sum and output of its own, so that no thread
+        // waits for another before the groups are merged.
         int lpk = 1;  // lanes per key
         while (lpk * 4 < dh) lpk *= 2;
         const int sub = lane % lpk, group = tid / lpk, groups = kThreads / lpk;
         const bool on = sub * 4 < dh;
-        float* sc = part;             // [S] scores, then probabilities
-        float* red = act;             // [groups][dh] partial outputs
+        float* red = act;        // [groups][dh] outputs
+        float* ml = part;        // [groups][2] maxima, sums
         const float scale = 1.f / sqrtf(static_cast<float>(dh));
         for (int bh = blockIdx.x; bh < p.B * p.H; bh += gridDim.x) {
-          const float* kb = kv + static_cast<int64_t>(bh) * 2 * kv_plane;
+          const float* kb = kv + static_cast<int64_t>(bh) * 2 * kv_plane + sub * 4;
           const float* vb = kb + kv_plane;
           const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
           const float4 q = on ? __ldcg(reinterpret_cast<const float4*>(p.q + bh * dh + sub * 4)) : zero;
-#pragma unroll 4
-          for (int j = group; j < (pos / groups + 1) * groups; j += groups) {
-            const float4 k = on && j <= pos ? __ldcg(reinterpret_cast<const float4*>(kb + static_cast<int64_t>(j) * dh + sub * 4)) : zero;
-            float s = fmaf(q.x, k.x, fmaf(q.y, k.y, fmaf(q.z, k.z, q.w * k.w)));
-            for (int o = lpk / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (sub == 0 && j <= pos) sc[j] = s * scale;
-          }
-          __syncthreads();
-          float m = -INFINITY;
-          for (int j = lane; j <= pos; j += 32) m = fmaxf(m, sc[j]);
-          m = warp_max(m);
-          __syncthreads();
-          for (int j = tid; j <= pos; j += kThreads) sc[j] = expf(sc[j] - m);
-          __syncthreads();
-          float sum = 0.f;
-          for (int j = lane; j <= pos; j += 32) sum += sc[j];
-          sum = warp_sum(sum);
+          float m = -INFINITY, sum = 0.f;
           float4 o = zero;
-          if (on) {
-#pragma unroll 4
-            for (int j = group; j <= pos; j += groups) {
-              const float4 v = __ldcg(reinterpret_cast<const float4*>(vb + static_cast<int64_t>(j) * dh + sub * 4));
-              const float pj = sc[j];
-              o.x = fmaf(pj, v.x, o.x); o.y = fmaf(pj, v.y, o.y); o.z = fmaf(pj, v.z, o.z); o.w = fmaf(pj, v.w, o.w);
+          for (int j0 = 0; j0 <= pos; j0 += 4 * groups) {
+            float4 k[4], v[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const int j = j0 + e * groups + group;
+              const bool in = on && j <= pos;
+              k[e] = in ? __ldcg(reinterpret_cast<const float4*>(kb + static_cast<int64_t>(j) * dh)) : zero;
+              v[e] = in ? __ldcg(reinterpret_cast<const float4*>(vb + static_cast<int64_t>(j) * dh)) : zero;
             }
-            *reinterpret_cast<float4*>(red + group * dh + sub * 4) = o;
+            float s[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[e] = fmaf(q.x, k[e].x, fmaf(q.y, k[e].y, fmaf(q.z, k[e].z, q.w * k[e].w)));
+            for (int x = lpk / 2; x > 0; x >>= 1) {
+#pragma unroll
+              for (int e = 0; e < 4; ++e) s[e] += __shfl_xor_sync(0xffffffffu, s[e], x);
+            }
+            float mnew = m;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              s[e] = j0 + e * groups + group <= pos ? s[e] * scale : -INFINITY;
+              mnew = fmaxf(mnew, s[e]);
+            }
+            const float ref = mnew == -INFINITY ? 0.f : mnew;
+            const float corr = expf(m - ref);
+            sum *= corr;
+            o.x *= corr; o.y *= corr; o.z *= corr; o.w *= corr;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float pe = expf(s[e] - ref);
+              sum += pe;
+              o.x = fmaf(pe, v[e].x, o.x); o.y = fmaf(pe, v[e].y, o.y); o.z = fmaf(pe, v[e].z, o.z); o.w = fmaf(pe, v[e].w, o.w);
+            }
+            m = mnew;
+          }
+          if (on) *reinterpret_cast<float4*>(red + group * dh + sub * 4) = o;
+          if (sub == 0) {
+            ml[2 * group] = m;
+            ml[2 * group + 1] = sum;
           }
           __syncthreads();
           if (tid < dh) {
-            float v = 0.f;
-            const int n = min(groups, pos + 1);
+            const int n = min(groups, pos + 1);  // the groups that hold keys
+            float mm = -INFINITY, l = 0.f, v = 0.f;
 #pragma unroll 8
-            for (int g = 0; g < n; ++g) v += red[g * dh + tid];
-            p.attn[bh * dh + tid] = v * (p.keep / sum);  // heads are consecutive: [B][D]
+            for (int g = 0; g < n; ++g) mm = fmaxf(mm, ml[2 * g]);
+#pragma unroll 8
+            for (int g = 0; g < n; ++g) {
+              const float f = expf(ml[2 * g] - mm);
+              l = fmaf(f, ml[2 * g + 1], l);
+              v = fmaf(f, red[g * dh + tid], v);
+            }
+            p.attn[bh * dh + tid] = v * (p.keep / l);  // heads are consecutive: [B][D]
           }
           __syncthreads();
         }
@@ -391,23 +410,22 @@ decode_kernel(const __grid_constant__ DecodeParams p) {
       load_act(p.attn, p.D);
       clear_tail(p.step[1]);
       __syncthreads();
-      run_step(1, [&](int row, int b) { return p.x[b * p.D + row]; },
-               [&](int row, int b, float v, float x) { p.x[b * p.D + row] = fmaf(v, p.keep, x); });
+      run_step(1, [&](int row, int b) { return make_float2(0.f, p.x[b * p.D + row]); },
+               [&](int row, int b, float v, float2 e) { p.x[b * p.D + row] = fmaf(v, p.keep, e.y); });
       if (!grid_barrier(p, target, &ok_s)) goto out;
 
       load_act(p.x, p.D);
       clear_tail(p.step[2]);
       normalise(w[4], w[5]);
-      run_step(2, [&](int row, int) { return __ldg(w[7] + row); },
-               [&](int row, int b, float v, float bias) { p.h[b * p.F + row] = gelu_tanh(v + bias); });
+      run_step(2, [&](int row, int) { return make_float2(__ldg(w[7] + row), 0.f); },
+               [&](int row, int b, float v, float2 e) { p.h[b * p.F + row] = gelu_tanh(v + e.x); });
       if (!grid_barrier(p, target, &ok_s)) goto out;
 
       load_act(p.h, p.F);
       clear_tail(p.step[3]);
       __syncthreads();
-      const float* b2f = w[9];
-      run_step(3, [&](int row, int b) { return p.x[b * p.D + row]; },
-               [&](int row, int b, float v, float x) { p.x[b * p.D + row] = fmaf(v + __ldg(b2f + row), p.keep, x); });
+      run_step(3, [&](int row, int b) { return make_float2(__ldg(w[9] + row), p.x[b * p.D + row]); },
+               [&](int row, int b, float v, float2 e) { p.x[b * p.D + row] = fmaf(v + e.x, p.keep, e.y); });
       if (!grid_barrier(p, target, &ok_s)) goto out;
     }
 
@@ -418,8 +436,8 @@ decode_kernel(const __grid_constant__ DecodeParams p) {
     Best mine[NB];
 #pragma unroll
     for (int b = 0; b < NB; ++b) mine[b] = Best{-INFINITY, 0x7fffffff};
-    run_step(4, [&](int row, int) { return __ldg(p.b_head + row); }, [&](int row, int b, float v, float bias) {
-      const Best c{v + bias, row};
+    run_step(4, [&](int row, int) { return make_float2(__ldg(p.b_head + row), 0.f); }, [&](int row, int b, float v, float2 e) {
+      const Best c{v + e.x, row};
 #pragma unroll
       for (int k = 0; k < NB; ++k)
         if (k == b) mine[k] = better(mine[k], c);
@@ -504,17 +522,17 @@ bool make_plan(int64_t B, int64_t V, int64_t D, int64_t L, int64_t H, int64_t F,
     units = u > units ? u : units;
     ld = s.nch * kChunk > ld ? s.nch * kChunk : ld;
   }
-  // the attention step keeps its scores where the partial sums go and its partial outputs (16 floats per group of lanes at
-  // most: 512 / lanes-per-key groups of a head) where the activations go
+  // the attention step keeps its groups' maxima and sums where the partial sums go, and their outputs where the
+  // activations go
   int lpk = 1;
   while (lpk * 4 < p.D / p.H) lpk *= 2;
   const int red = kThreads / lpk * (p.D / p.H);
   size_t part = static_cast<size_t>(units) * 2 * out.nb;
-  if (part < static_cast<size_t>(S)) part = S;
+  if (part < static_cast<size_t>(2 * kThreads / lpk)) part = 2 * kThreads / lpk;
   if (ld * out.nb < red) ld = static_cast<int>(ceil_div(ceil_div(red, out.nb), 4) * 4);
   p.act_ld = ld;
   p.max_units = units;
-  const size_t fixed = (static_cast<size_t>(ld) * out.nb + part) * 4;
+  const size_t fixed = (static_cast<size_t>(ld) * out.nb + part) * 4 + static_cast<size_t>(L) * kLayerTensors * 8;
   out.depth = 0;
   for (int d : kDepths) {
     out.smem = static_cast<size_t>(kWarps) * d * 1024 + fixed;
