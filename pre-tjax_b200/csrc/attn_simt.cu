@@ -8,10 +8,11 @@
 // output tile, in registers: two or three 16-byte shared loads per 32 multiply-adds. Score products pack neighbouring
 // d into the two-wide FMA straight from those loads. Bound by the FP32 pipe (a warp per row with scalar global loads
 // was bound by the load/store unit instead). Measured, float32, forward / backward: [8, 12, 512, 64] with dropout and
-// document masks 88 / 317 us (36 / 36 TFLOP/s of the causal half), where a warp per row with a Philox call per probability
-// took 2526 / 16152 us; [4, 12, 512, 64] without dropout 84 / 268 us, forward 1900 us before. R = 4: twice the warps of
-// R = 8, which needs 255 registers and measured 98 / 314 and 90 / 294 us there, 23 / 75 us against 17 / 55 us at
-// [2, 12, 128, 64].
+// document masks 88 / 262 us (36 / 43 TFLOP/s of the causal half), where a warp per row with a Philox call per probability
+// took 2526 / 16152 us; [4, 12, 512, 64] without dropout 84 / 261 us, forward 1900 us before. R = 4: twice the warps of
+// R = 8, which needs 255 registers and measured 98 / 314 and 90 / 294 us there, 23 / 75 us against 17 / 58 us at
+// [2, 12, 128, 64]. The dK/dV kernel is held to two blocks per SM: left alone it took 234 registers and one block, 317 us
+// at the first of these sizes.
 #include "attn_common.cuh"
 
 namespace ptj {
@@ -479,7 +480,7 @@ attn_dq_simt_kernel(const BwdArgs<T> a) {
 
 // dK and dV: block = one key tile, the ones with the most query tiles first; sweeps the query tiles.
 template <typename T, int DP, int R>
-__global__ void __launch_bounds__(Tile<DP, R>::kThreads)
+__global__ void __launch_bounds__(Tile<DP, R>::kThreads, DP <= 64 ? 2 : 1)  // (wide heads: shared memory takes one block)
 attn_dkv_simt_kernel(const BwdArgs<T> a) {
   grid_dep_sync();
   using TT = Tile<DP, R>;
