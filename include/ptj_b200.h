@@ -264,8 +264,9 @@ int ptj_gemm_grouped2(const ptj_gemm_problem* p0, const ptj_gemm_problem* p1, in
  * (d_head contiguous), so both the reference's [B,H,3,N,D] tensor and a fused [B*N, H*3*D] projection
  * output are addressed without copies. row_max / row_sum are float[batch*heads*seq] (the reference's acts0 /
  * acts1: running maximum of the scaled scores and sum of exp(score - max)).
- *   dtype PTJ_BF16 with d_head a multiple of 8 up to 64 (16-byte aligned rows) runs the tcgen05 kernels; everything else runs the
- *   exact-fp32 SIMT kernels.
+ *   dtype PTJ_BF16 with d_head == 64 and seq % 128 == 0 (16-byte aligned rows) runs the tcgen05 kernels, which round
+ *   probabilities and score gradients to bf16 before they are multiplied; everything else runs the SIMT kernels, float32
+ *   from the operands to the stored result.
  * Backward recomputes the probabilities; it is deterministic (no atomics).
  *
  * row_kstart (optional, int32[batch, seq]): the first key each query row may attend to, so that row i attends keys

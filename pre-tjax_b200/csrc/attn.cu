@@ -1,4 +1,4 @@
-// C entry points of causal attention: validate, then route to the tcgen05 kernels (bf16, d_head a multiple of 8 up to 64)
+// C entry points of causal attention: validate, then route to the tcgen05 kernels (bf16, d_head 64, seq % 128 == 0)
 // or to the exact-fp32 CUDA-core kernels (everything else).
 #include "attn_common.cuh"
 

@@ -1,5 +1,4 @@
-// Causal flash attention backward on tcgen05 tensor cores (bf16 in, fp32 accumulate), d_head a multiple of 8 up to 64,
-// any seq (query rows beyond the sequence arrive as zeros in Q and dO, so they add exact zeros to dK and dV).
+// Causal flash attention backward on tcgen05 tensor cores (bf16 in, fp32 accumulate), d_head = 64, seq % 128 == 0.
 // Semantics: model_triton.py:801-811 / 550-577: with P = softmax(causal(Q K^T / sqrt(d))) recomputed from the saved row
 // statistics and Pd = dropout(P):  dV = Pd^T dO,  dP = dO V^T,  dS = P o (dP o keep - delta) / sqrt(d) with
 // delta = rowsum(dO o O),  dK = dS^T Q,  dQ = dS K.
@@ -91,12 +90,12 @@ struct Cursor {
 __global__ void __launch_bounds__(256)
 attn_bwd_prep_kernel(const RowView d_o, const RowView o_view, const float* __restrict__ row_max,
                      const float* __restrict__ row_sum, float* __restrict__ delta, float* __restrict__ lse2, int S, int H,
-                     int D, int64_t rows) {
+                     int64_t rows) {
   grid_dep_sync();
   const int64_t r = (static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x) >> 3;
   const int part = threadIdx.x & 7;
   float acc = 0.f;
-  if (r < rows && part * 8 < D) {
+  if (r < rows) {
     const int64_t bh = r / S, q = r % S;
     const __nv_bfloat16* g = d_o.row(bh / H, bh % H, q) + part * 8;
     const __nv_bfloat16* o = o_view.row(bh / H, bh % H, q) + part * 8;
@@ -121,7 +120,7 @@ attn_bwd_prep_kernel(const RowView d_o, const RowView o_view, const float* __res
 // float4 over kt; consecutive threads take consecutive rows.
 __global__ void __launch_bounds__(256)
 attn_dq_reduce_kernel(const float* __restrict__ part, const RowView dq, const int32_t* __restrict__ kstart, int S, int H,
-                      int D, int nq, int64_t total_vec) {
+                      int nq, int64_t total_vec) {
   grid_dep_sync();
   const int64_t v = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
   if (v >= total_vec) return;
@@ -131,7 +130,6 @@ attn_dq_reduce_kernel(const float* __restrict__ part, const RowView dq, const in
   const int64_t bh = tile_id / nq;
   const int qt = static_cast<int>(tile_id % nq);
   const int64_t q = static_cast<int64_t>(qt) * T + row;
-  if (q >= S || c4 * 4 >= D) return;
   const int64_t ntri = static_cast<int64_t>(nq) * (nq + 1) / 2;
   const float4* src = reinterpret_cast<const float4*>(part) +
                       ((bh * ntri + static_cast<int64_t>(qt) * (qt + 1) / 2) * (DH / 4) + c4) * T + row;
@@ -159,7 +157,7 @@ attn_dq_reduce_kernel(const float* __restrict__ part, const RowView dq, const in
 // P phase of one 32-column chunk: s holds the raw scores on entry (-inf where the causal mask applies) and Pd (what
 // goes to shared memory) on exit;
 // pk receives P as packed bf16 pairs whose sign bit marks a dropped element. rw: the four Philox calls of the chunk.
-// MODE 0: no mask; 1: raw Philox words in rw; 2, 3: keep flags of the chunk in keepw (bit i = column i).
+// MODE 0: no mask; 1: raw Philox words in rw; 2: precomputed keep flags of the chunk in keepw (bit i = column i).
 template <int MODE>
 __device__ __forceinline__ void p_chunk(float (&s)[32], uint32_t* pk, const uint32_t (&rw)[4][4], uint32_t keepw,
                                         uint64_t sc2, uint64_t nl2, uint32_t thr_hi, float f_keep) {
@@ -214,8 +212,8 @@ struct BwdViews {
 };
 
 // VARLEN: query row i attends keys [p.kstart[b, i], i] only (see the forward kernel); masked scores are -inf, so their
-// probabilities, and with them every product they enter, are exact zeros. MODE, RAGGED: see the forward kernel.
-template <int MODE, bool VARLEN, bool RAGGED>
+// probabilities, and with them every product they enter, are exact zeros.
+template <int MODE, bool VARLEN>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_g,
@@ -276,7 +274,7 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   tc_fence_after_sync();
   grid_dep_sync();  // set-up above touches no global memory; everything below may
   const uint32_t tmem = *tmem_slot;
-  if (MODE == 1 || MODE == 3) {  // the kernel draws its own keep flags: round keys of the (possibly device-resident) seed
+  if (MODE == 1) {  // the kernel draws its own keep flags: round keys of the (possibly device-resident) seed
     if (tid == 0) philox_round_keys(p.dr.seed, rk_s);
     __syncthreads();
   }
@@ -296,7 +294,7 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         last = kt;
         for (int i = kt + 1; i < sched.nq; ++i) {
           bool reach = false;
-          for (int r = lane; r < T && (!RAGGED || i * T + r < p.S); r += 32) {
+          for (int r = lane; r < T; r += 32) {
             const int row = i * T + r, k = __ldg(ks + row);
             reach = reach || (k <= row && k < kv_end);  // the row has keys and its first one is in or before the tile
           }
@@ -509,9 +507,8 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         const uint32_t ph = (c.g >> 1) & 1;
         const int64_t q_row = static_cast<int64_t>(c.i) * T + row;
         const int64_t ri = static_cast<int64_t>(c.bh) * p.S + q_row;
-        const bool real = !RAGGED || q_row < p.S;  // rows beyond the sequence: P = 1, multiplied by zero rows of Q and dO
-        const float lse = real ? lse2[ri] : 0.f;
-        const float dsc = real ? delta[ri] * p.scale : 0.f;  // delta / sqrt(d)
+        const float lse = lse2[ri];
+        const float dsc = delta[ri] * p.scale;  // delta / sqrt(d)
         // dropout random words of this thread's row, one 32-column chunk ahead of their use
         uint32_t rw[2][4][4];
         const uint64_t call0 = ((static_cast<uint64_t>(c.bh) * p.S + q_row) * p.S + static_cast<uint64_t>(c.kt) * T) >> 3;
@@ -519,10 +516,7 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         uint4 kb = make_uint4(0u, 0u, 0u, 0u);
         if (MODE == 2)
           kb = __ldg(p.keep_bits + (static_cast<int64_t>(c.bh) * ntri + c.i * (c.i + 1) / 2 + c.kt) * T + row);
-        uint32_t keepw[4] = {kb.x, kb.y, kb.z, kb.w};
-        if (MODE == 3)
-          keep_words_unaligned(rk_s, (static_cast<uint64_t>(c.bh) * p.S + q_row) * p.S + static_cast<uint64_t>(c.kt) * T,
-                               p.dr.stream_id, thr_hi, keepw);
+        const uint32_t keepw[4] = {kb.x, kb.y, kb.z, kb.w};
         // ---- P from the scores; Pd to shared memory; P kept as packed bf16, sign bit set where dropped ----
         ok = mbar_wait(&s_full[grp], ph, ctx, 0x2502u);
         ok = __all_sync(0xffffffffu, ok);
@@ -547,7 +541,7 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
               if (cc * 32 + i > row) s[cc][i] = -INFINITY;
         }
         if (VARLEN) {  // keys before the row's document
-          const int rel = real ? __ldg(p.kstart + static_cast<int64_t>(c.bh / p.H) * p.S + q_row) - c.kt * T : 0;
+          const int rel = __ldg(p.kstart + static_cast<int64_t>(c.bh / p.H) * p.S + q_row) - c.kt * T;
           if (__any_sync(0xffffffffu, rel > 0)) {  // (most tiles hold no document boundary for any row of the warp)
 #pragma unroll
             for (int cc = 0; cc < 4; ++cc)
@@ -619,7 +613,6 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
               tmem_ld_wait();
 #pragma unroll
               for (int c8 = 0; c8 < 4; ++c8) {
-                if (RAGGED && (kv_row >= p.S || cc * 32 + c8 * 8 >= p.D)) continue;
                 float t8[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) t8[i] = t[c8 * 8 + i];
@@ -654,24 +647,21 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 }  // namespace
 
 bool attn_tc_supported(const ptj_attn_shape& sh, const void* const* ptrs, int nptrs) {
-  if (sh.d_head > DH || sh.d_head % 8 != 0 || sh.seq > (1 << 20)) return false;
-  const int64_t bh = sh.batch * sh.heads, items = bh * ((sh.seq + T - 1) / T);
-  // rows that fill no tile may also take the general kernels, which need no workspace: a backward workspace (it grows
-  // with seq^2) that could exhaust the device is not asked for on their behalf
-  if ((sh.seq % T != 0 || sh.d_head != DH) && attn_bwd_tc_workspace_bytes(sh) > (4ull << 30)) return false;
+  if (sh.d_head != DH || sh.seq % T != 0 || sh.seq < T || sh.seq > (1 << 20)) return false;
+  const int64_t bh = sh.batch * sh.heads, items = bh * (sh.seq / T);
   if (items * bh >= (1LL << 32)) return false;  // exactness bound of the kernels' reciprocal division by bh
   for (int i = 0; i < nptrs; ++i)
     if (!aligned16(ptrs[i])) return false;
   const int64_t* sts[4] = {sh.q_strides, sh.k_strides, sh.v_strides, sh.o_strides};
   for (const int64_t* st : sts) {
-    if (st[0] % 8 != 0 || st[1] % 8 != 0 || st[2] % 8 != 0 || st[2] < sh.d_head) return false;
+    if (st[0] % 8 != 0 || st[1] % 8 != 0 || st[2] % 8 != 0 || st[2] < DH) return false;
     if ((sh.batch > 1 && st[0] <= 0) || (sh.heads > 1 && st[1] <= 0)) return false;
   }
   return ptj_device_check() == PTJ_OK;
 }
 
 size_t attn_bwd_tc_workspace_bytes(const ptj_attn_shape& sh) {
-  const int64_t nq = (sh.seq + T - 1) / T, bh = sh.batch * sh.heads;
+  const int64_t nq = sh.seq / T, bh = sh.batch * sh.heads;
   const int64_t part = bh * (nq * (nq + 1) / 2) * T * DH;  // dQ shares
   const int64_t rows = bh * sh.seq;                        // delta, lse2
   return static_cast<size_t>(part + 2 * rows) * sizeof(float);
@@ -691,16 +681,14 @@ int attn_bwd_tc(const void* d_o, const void* q, const void* k, const void* v, co
   if (p.fault == nullptr) return PTJ_ERR_DEVICE;
   p.keep_bits = reinterpret_cast<const uint4*>(keep_bits);
   p.kstart = row_kstart;
-  const bool masked = dr.train && dr.thr16 != 0u, ragged = p.S % T != 0 || p.D != DH;
-  const int mode = !masked ? 0 : (p.keep_bits != nullptr ? 2 : (ragged ? 3 : 1));
+  const bool masked = dr.train && dr.thr16 != 0u;
+  const int mode = !masked ? 0 : (p.keep_bits != nullptr ? 2 : 1);
   using Kern = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const float*,
                         const float*, float*, const BwdViews, const AttnParams, const Sched);
-  static const Kern kerns[2][2][4] = {
-      {{attn_bwd_ws_kernel<0, false, false>, attn_bwd_ws_kernel<1, false, false>, attn_bwd_ws_kernel<2, false, false>, nullptr},
-       {attn_bwd_ws_kernel<0, true, false>, attn_bwd_ws_kernel<1, true, false>, attn_bwd_ws_kernel<2, true, false>, nullptr}},
-      {{attn_bwd_ws_kernel<0, false, true>, nullptr, attn_bwd_ws_kernel<2, false, true>, attn_bwd_ws_kernel<3, false, true>},
-       {attn_bwd_ws_kernel<0, true, true>, nullptr, attn_bwd_ws_kernel<2, true, true>, attn_bwd_ws_kernel<3, true, true>}}};
-  const Kern kern = kerns[ragged][row_kstart != nullptr][mode];
+  static const Kern kerns[2][3] = {
+      {attn_bwd_ws_kernel<0, false>, attn_bwd_ws_kernel<1, false>, attn_bwd_ws_kernel<2, false>},
+      {attn_bwd_ws_kernel<0, true>, attn_bwd_ws_kernel<1, true>, attn_bwd_ws_kernel<2, true>}};
+  const Kern kern = kerns[row_kstart != nullptr ? 1 : 0][mode];
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess) {
     (void)cudaGetLastError();
     return PTJ_ERR_LAUNCH;
@@ -711,7 +699,7 @@ int attn_bwd_tc(const void* d_o, const void* q, const void* k, const void* v, co
   float* lse2 = delta + rows;
   const RowView g_view = make_view(d_o, sh.o_strides), o_view = make_view(o, sh.o_strides);
   launch_k(attn_bwd_prep_kernel, static_cast<unsigned>((rows * 8 + 255) / 256), 256, 0, st, g_view, o_view, row_max, row_sum,
-                                                                                     delta, lse2, p.S, p.H, p.D, rows);
+                                                                                     delta, lse2, p.S, p.H, rows);
   PTJ_CHECK_LAUNCH();
   Sched s;
   s.nq = p.nq;
@@ -723,9 +711,9 @@ int attn_bwd_tc(const void* d_o, const void* q, const void* k, const void* v, co
   BwdViews views{make_view(dk, dsh.k_strides), make_view(dv, dsh.v_strides)};
   launch_k(kern, grid, kThreads, kSmemBytes, st, tq, tk, tv, tg, delta, lse2, part, views, p, s);
   PTJ_CHECK_LAUNCH();
-  const int64_t total_vec = static_cast<int64_t>(p.BH) * p.nq * T * (DH / 4);
+  const int64_t total_vec = rows * (DH / 4);
   launch_k(attn_dq_reduce_kernel, static_cast<unsigned>((total_vec + 255) / 256), 256, 0, st, part, make_view(dq, dsh.q_strides),
-                                                                                        row_kstart, p.S, p.H, p.D, p.nq, total_vec);
+                                                                                        row_kstart, p.S, p.H, p.nq, total_vec);
   PTJ_CHECK_LAUNCH();
   return PTJ_OK;
 }

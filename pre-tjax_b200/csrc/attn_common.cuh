@@ -28,9 +28,7 @@ int attn_bwd_simt(const void* d_o, const void* q, const void* k, const void* v, 
                   const float* row_sum, void* dq, void* dk, void* dv, const int32_t* row_kstart,
                   const ptj_attn_shape& sh, const ptj_attn_shape& dsh, const AttnDropout& dr, int dtype, cudaStream_t st);
 
-// tcgen05 kernels: bf16, d_head a multiple of 8 up to 64, any seq, 16-byte aligned strides (what a tensor map takes). Row
-// lengths and heads that fill no tile cost the padding of the last tile: [4, 12, 500, 64] forward + backward with dropout
-// takes 96 us here and took 10.2 ms on the general kernels of the time.
+// tcgen05 kernels: bf16, d_head == 64, seq % 128 == 0, 16-byte aligned strides.
 bool attn_tc_supported(const ptj_attn_shape& sh, const void* const* ptrs, int nptrs);
 // keep_bits (optional, both directions): the call's dropout keep flags from attn_keep_bits_tc; NULL = the kernels draw
 // the same flags themselves.

@@ -1,5 +1,4 @@
-// Causal flash attention forward on tcgen05 tensor cores (bf16 in, fp32 accumulate), d_head a multiple of 8 up to 64,
-// any seq (rows beyond the sequence arrive as zeros, are computed and not stored).
+// Causal flash attention forward on tcgen05 tensor cores (bf16 in, fp32 accumulate), d_head = 64, seq % 128 == 0.
 // Semantics: model_triton.py:608-611 / 510-517: softmax of the causally masked scaled scores, dropout on the
 // probabilities (no rescale), times V; the row maximum and row sum of exponentials are saved (acts0 / acts1, :699-700).
 //
@@ -77,15 +76,12 @@ struct Cursor {
   }
 };
 
-// MODE 0: no dropout mask; 1: Philox drawn in the kernel; 2: precomputed keep flags (p.keep_bits); 3: Philox drawn in
-// the kernel for rows that start anywhere in a call's eight elements (RAGGED).
-// RAGGED: the last tile holds rows beyond the sequence or the head is narrower than the tile; a kernel of its own because
-// the store conditions cost the full-tile kernels 4 % ([8, 12, 1024, 64] forward + backward: 257 -> 268 us).
+// MODE 0: no dropout mask; 1: Philox drawn in the kernel; 2: precomputed keep flags (p.keep_bits).
 // VARLEN: query row i attends keys [p.kstart[b, i], i] only (packed documents / padding, the block-diagonal x causal x
 // padding masks of the reference's collator, tokenized_dataset.py:110-131); a row whose range is empty gets a zero
 // output row and the statistics (row_max, row_sum) = (0, 1). The tile stream is the causal one: keys outside a row's
 // range are masked, whole tiles outside it contribute exact zeros.
-template <int MODE, bool VARLEN, bool RAGGED>
+template <int MODE, bool VARLEN>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const RowView out, float* __restrict__ row_max,
@@ -144,7 +140,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   tc_fence_after_sync();
   grid_dep_sync();  // set-up above touches no global memory; everything below may
   const uint32_t tmem = *tmem_slot;
-  if (MODE == 1 || MODE == 3) {  // the kernel draws its own keep flags: round keys of the (possibly device-resident) seed
+  if (MODE == 1) {  // the kernel draws its own keep flags: round keys of the (possibly device-resident) seed
     if (tid == 0) philox_round_keys(p.dr.seed, rk_s);
     __syncthreads();
   }
@@ -162,7 +158,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         const int qt = sched.nq - 1 - t, bh = sp - t * sched.BH;
         const int32_t* ks = p.kstart + static_cast<int64_t>(bh / p.H) * p.S + static_cast<int64_t>(qt) * T;
         int lo = 0x7fffffff;
-        for (int r = lane; r < T && (!RAGGED || qt * T + r < p.S); r += 32) {
+        for (int r = lane; r < T; r += 32) {
           const int k = __ldg(ks + r);
           if (k <= qt * T + r) lo = min(lo, k);  // (k > row: the row has no keys)
         }
@@ -344,10 +340,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         uint4 kb = make_uint4(0u, 0u, 0u, 0u);
         if (MODE == 2)
           kb = __ldg(p.keep_bits + (static_cast<int64_t>(c.bh) * (p.nq * (p.nq + 1) / 2) + c.qt * (c.qt + 1) / 2 + c.j) * T + row);
-        uint32_t keepw[4] = {kb.x, kb.y, kb.z, kb.w};
-        if (MODE == 3)
-          keep_words_unaligned(rk_s, (static_cast<uint64_t>(c.bh) * p.S + q_row) * p.S + static_cast<uint64_t>(c.j) * T,
-                               p.dr.stream_id, thr_hi, keepw);
+        const uint32_t keepw[4] = {kb.x, kb.y, kb.z, kb.w};
         ok = mbar_wait(&s_full[sb], (c.g / kSBufs) & 1, ctx, 0x1303u);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
@@ -368,7 +361,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
               if (cc * 32 + i > row) s[cc][i] = -INFINITY;
         }
         if (VARLEN) {  // keys before the row's document: columns below rel (any tile may hold a boundary)
-          const int rel = !RAGGED || q_row < p.S ? __ldg(p.kstart + static_cast<int64_t>(c.bh / p.H) * p.S + q_row) - c.j * T : 0;
+          const int rel = __ldg(p.kstart + static_cast<int64_t>(c.bh / p.H) * p.S + q_row) - c.j * T;
           if (__any_sync(0xffffffffu, rel > 0)) {  // (most tiles hold no document boundary for any row of the warp)
 #pragma unroll
             for (int cc = 0; cc < 4; ++cc)
@@ -427,7 +420,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
               const uint32_t w = rw[cc & 1][i >> 3][(i & 7) >> 1];
               if ((w << 16) < thr_hi) a = 0.f;
               if (w < thr_hi) b = 0.f;
-            } else if (MODE >= 2) {
+            } else if (MODE == 2) {
               if ((keepw[cc] & (1u << i)) == 0u) a = 0.f;
               if ((keepw[cc] & (2u << i)) == 0u) b = 0.f;
             }
@@ -510,7 +503,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           }
           ++nd;
         }
-        if (mine && (!RAGGED || q_row < p.S)) {
+        if (mine) {
           const bool empty = VARLEN && !(l > 0.f);  // the row attends nothing: zero output, neutral statistics
           const float inv = empty ? 0.f : f_eval / l;
           __nv_bfloat16* dst = out.row(c.bh / p.H, c.bh % p.H, q_row);
@@ -519,7 +512,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             float t[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) t[i] = o[c8 * 8 + i] * inv;
-            if (!RAGGED || c8 * 8 < p.D) Elem<__nv_bfloat16>::store_vec(dst + c8 * 8, t);
+            Elem<__nv_bfloat16>::store_vec(dst + c8 * 8, t);
           }
           const int64_t ri = static_cast<int64_t>(c.bh) * p.S + q_row;
           row_max[ri] = empty ? 0.f : m_true * kLn2;                   // acts0: row maximum of the scaled scores
@@ -547,9 +540,8 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 // Keep flags of the attention-probability dropout for one call, computed once and shared by the forward and the
 // backward kernel: word c of the uint4 at ((bh * ntri + qt (qt + 1) / 2 + kt) * 128 + row) holds the flags of
 // columns 32 c .. 32 c + 31 of row `row` of tile (qt, kt); ntri = nq (nq + 1) / 2. One thread per word.
-template <bool ALIGNED>
 __global__ void __launch_bounds__(512)
-attn_keep_bits_kernel(uint32_t* __restrict__ bits, const AttnDropout dr, int S, int nq) {  // ALIGNED: S % 8 == 0
+attn_keep_bits_kernel(uint32_t* __restrict__ bits, const AttnDropout dr, int S, int nq) {
   grid_dep_sync();
   __shared__ uint32_t rk_s[20];
   if (threadIdx.x == 0) philox_round_keys(dr.seed, rk_s);
@@ -569,19 +561,19 @@ attn_keep_bits_kernel(uint32_t* __restrict__ bits, const AttnDropout dr, int S, 
   const int cc = threadIdx.x & 3, row = threadIdx.x >> 2;
   const uint64_t idx0 = (static_cast<uint64_t>(bh) * S + static_cast<uint64_t>(qt) * T + row) * S +
                         static_cast<uint64_t>(kt) * T + cc * 32;
-  // four Philox calls (five when the row does not start on a call boundary), eight flags each
+  // four Philox calls (round keys from the kernel parameters), eight 16-bit lanes each: bit e of a call's byte is set
+  // when lane e (low half of word e / 2 for even e, high half for odd e) is >= the threshold
   const uint32_t thr_hi = dr.thr16 << 16;
   uint32_t word = 0;
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     uint32_t w[4];
     philox_rk(rk, (idx0 >> 3) + q, dr.stream_id, w);
-    word |= keep_flags8(w, thr_hi) << (8 * q);
-  }
-  if (!ALIGNED) {
-    uint32_t w[4];
-    philox_rk(rk, (idx0 >> 3) + 4, dr.stream_id, w);
-    word = __funnelshift_r(word, keep_flags8(w, thr_hi), static_cast<uint32_t>(idx0) & 7u);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      word |= ((w[e] << 16) >= thr_hi ? 1u : 0u) << (8 * q + 2 * e);
+      word |= (w[e] >= thr_hi ? 1u : 0u) << (8 * q + 2 * e + 1);
+    }
   }
   bits[tile * 512 + threadIdx.x] = word;
 }
@@ -589,15 +581,14 @@ attn_keep_bits_kernel(uint32_t* __restrict__ bits, const AttnDropout dr, int S, 
 }  // namespace
 
 size_t attn_keep_bits_bytes(const ptj_attn_shape& sh) {
-  const int64_t nq = (sh.seq + T - 1) / T;
+  const int64_t nq = sh.seq / T;
   return static_cast<size_t>(sh.batch * sh.heads * (nq * (nq + 1) / 2) * T) * 16;
 }
 
 int attn_keep_bits_tc(uint32_t* bits, const ptj_attn_shape& sh, const AttnDropout& dr, cudaStream_t st) {
   const int64_t tiles = static_cast<int64_t>(attn_keep_bits_bytes(sh) / 2048);
-  const int seq = static_cast<int>(sh.seq), nq = (seq + T - 1) / T;
-  launch_k(seq % 8 == 0 ? attn_keep_bits_kernel<true> : attn_keep_bits_kernel<false>, static_cast<unsigned>(tiles), 512, 0,
-           st, bits, dr, seq, nq);
+  launch_k(attn_keep_bits_kernel, static_cast<unsigned>(tiles), 512, 0, st, bits, dr, static_cast<int>(sh.seq),
+                                                                      static_cast<int>(sh.seq / T));
   PTJ_CHECK_LAUNCH();
   return PTJ_OK;
 }
@@ -612,16 +603,14 @@ int attn_fwd_tc(const void* q, const void* k, const void* v, void* o, float* row
   if (p.fault == nullptr) return PTJ_ERR_DEVICE;
   p.keep_bits = reinterpret_cast<const uint4*>(keep_bits);
   p.kstart = row_kstart;
-  const bool masked = dr.train && dr.thr16 != 0u, ragged = p.S % T != 0 || p.D != DH;
-  const int mode = !masked ? 0 : (keep_bits != nullptr ? 2 : (ragged ? 3 : 1));
+  const bool masked = dr.train && dr.thr16 != 0u;
+  const int mode = !masked ? 0 : (keep_bits != nullptr ? 2 : 1);
   using Kern = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const RowView, float*, float*,
                         const AttnParams, const Sched);
-  static const Kern kerns[2][2][4] = {
-      {{attn_fwd_ws_kernel<0, false, false>, attn_fwd_ws_kernel<1, false, false>, attn_fwd_ws_kernel<2, false, false>, nullptr},
-       {attn_fwd_ws_kernel<0, true, false>, attn_fwd_ws_kernel<1, true, false>, attn_fwd_ws_kernel<2, true, false>, nullptr}},
-      {{attn_fwd_ws_kernel<0, false, true>, nullptr, attn_fwd_ws_kernel<2, false, true>, attn_fwd_ws_kernel<3, false, true>},
-       {attn_fwd_ws_kernel<0, true, true>, nullptr, attn_fwd_ws_kernel<2, true, true>, attn_fwd_ws_kernel<3, true, true>}}};
-  const Kern kern = kerns[ragged][row_kstart != nullptr][mode];
+  static const Kern kerns[2][3] = {
+      {attn_fwd_ws_kernel<0, false>, attn_fwd_ws_kernel<1, false>, attn_fwd_ws_kernel<2, false>},
+      {attn_fwd_ws_kernel<0, true>, attn_fwd_ws_kernel<1, true>, attn_fwd_ws_kernel<2, true>}};
+  const Kern kern = kerns[row_kstart != nullptr ? 1 : 0][mode];
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess) {
     (void)cudaGetLastError();
     return PTJ_ERR_LAUNCH;

@@ -10,12 +10,12 @@ namespace attn_tc {
 using namespace tc;
 
 constexpr int T = 128;            // tile edge along queries and keys
-constexpr int DH = 64;            // head size of the tiles; smaller heads are zero-filled up to it by the TMA copies
+constexpr int DH = 64;            // head size
 constexpr int kTileBytes = T * DH * 2;  // one [128][64] bf16 tile
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 
-struct RowView {  // a [batch, heads, seq, d_head] view with d_head contiguous
+struct RowView {  // a [batch, heads, seq, 64] view with 64 contiguous
   __nv_bfloat16* base;
   int64_t sb, sh, sr;
   __device__ __forceinline__ __nv_bfloat16* row(int64_t b, int64_t h, int64_t r) const {
@@ -24,8 +24,7 @@ struct RowView {  // a [batch, heads, seq, d_head] view with d_head contiguous
 };
 
 struct AttnParams {
-  int S, H, BH, nq;  // nq = ceil(S / T): rows and keys beyond S are zero-filled by the TMA copies and never stored
-  int D;             // head size, a multiple of 8 up to DH
+  int S, H, BH, nq;
   float scale_log2;  // log2(e) / sqrt(d_head)
   float scale;       // 1 / sqrt(d_head)
   AttnDropout dr;
@@ -100,17 +99,6 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return y;
 }
 
-// flags of the eight 16-bit lanes of one call (low half of word e / 2 for even e, high half for odd): set when >= threshold
-__device__ __forceinline__ uint32_t keep_flags8(const uint32_t (&w)[4], uint32_t thr_hi) {
-  uint32_t bits = 0u;
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    bits |= ((w[e] << 16) >= thr_hi ? 1u : 0u) << (2 * e);
-    bits |= (w[e] >= thr_hi ? 1u : 0u) << (2 * e + 1);
-  }
-  return bits;
-}
-
 // NCALL consecutive counters at once, rounds in a rolled loop (small code, the calls give the instruction-level
 // parallelism), round keys read from shared memory (rk_s[2r], rk_s[2r+1]).
 template <int NCALL>
@@ -143,28 +131,6 @@ __device__ __forceinline__ void philox_rolled(const uint32_t* rk_s, uint64_t ctr
   for (int q = 0; q < NCALL; ++q) {
     out[q][0] = c0[q]; out[q][1] = c1[q]; out[q][2] = c2[q]; out[q][3] = c3[q];
   }
-}
-
-// Keep flags of a tile row (128 consecutive elements from flat index idx0, any alignment): a call yields the flags of
-// eight elements from a multiple of eight, so 17 calls cover the row and the words are shifted into place. Rows of a
-// sequence that is a multiple of eight start on a call boundary and take the cheaper 16 calls drawn chunk by chunk.
-__device__ __forceinline__ void keep_words_unaligned(const uint32_t* rk_s, uint64_t idx0, uint32_t stream_id,
-                                                     uint32_t thr_hi, uint32_t (&keepw)[4]) {
-  const uint32_t shift = static_cast<uint32_t>(idx0) & 7u;
-  uint32_t w[5];
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    uint32_t r[4][4];
-    philox_rolled<4>(rk_s, (idx0 >> 3) + 4 * c, stream_id, r);
-    w[c] = 0u;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) w[c] |= keep_flags8(r[q], thr_hi) << (8 * q);
-  }
-  uint32_t r[1][4];
-  philox_rolled<1>(rk_s, (idx0 >> 3) + 16, stream_id, r);
-  w[4] = keep_flags8(r[0], thr_hi);
-#pragma unroll
-  for (int c = 0; c < 4; ++c) keepw[c] = __funnelshift_r(w[c], w[c + 1], shift);
 }
 
 // packed pairs of floats for the two-wide fp32 instructions of sm_100 (fma.rn.f32x2, add.f32x2)
@@ -217,7 +183,7 @@ __device__ __forceinline__ uint8_t* align1024(uint8_t* raw) {
 
 // ---- host side -------------------------------------------------------------------------------------------------
 inline bool make_map(CUtensorMap* m, const void* base, const ptj_attn_shape& sh, const int64_t (&st)[3]) {
-  const uint64_t dims[4] = {static_cast<uint64_t>(sh.d_head), static_cast<uint64_t>(sh.seq), static_cast<uint64_t>(sh.heads),
+  const uint64_t dims[4] = {static_cast<uint64_t>(DH), static_cast<uint64_t>(sh.seq), static_cast<uint64_t>(sh.heads),
                             static_cast<uint64_t>(sh.batch)};
   // a size-1 dimension may come with a zero stride; the encoder wants positive multiples of 16 bytes
   auto fix = [&](int64_t s) { return static_cast<uint64_t>(s > 0 ? s : DH) * 2; };
@@ -235,9 +201,8 @@ inline AttnParams make_params(const ptj_attn_shape& sh, const AttnDropout& dr) {
   p.S = static_cast<int>(sh.seq);
   p.H = static_cast<int>(sh.heads);
   p.BH = static_cast<int>(sh.batch * sh.heads);
-  p.nq = (p.S + T - 1) / T;
-  p.D = static_cast<int>(sh.d_head);
-  p.scale = 1.f / sqrtf(static_cast<float>(p.D));
+  p.nq = p.S / T;
+  p.scale = 1.f / sqrtf(static_cast<float>(DH));
   p.scale_log2 = p.scale * kLog2e;
   p.dr = dr;
   p.fault = tc::fault_word();
