@@ -246,9 +246,12 @@ cross_entropy_kernel(const int32_t* __restrict__ labels, const T* logits, T* dlo
 // Passes 2 and 3 read the row from L2 (512-thread blocks, three per SM: the 444 rows in flight, 100 KB each at
 // GPT-2's vocabulary, stay well inside the L2). Accuracy: the label is the arg-max iff x[label] equals the maximum and no earlier column does (ties go to
 // the first index, as in torch.argmax); the second condition is only walked for rows where the first holds.
-// Rows of an odd vocabulary stored without padding start anywhere: up to seven elements before the first boundary and
-// seven after the last whole vector are walked one by one. [8192, 50257] contiguous: 507 us through the generic kernel
-// above, 399 us here, calls and all; padded rows of the same size 340 us.
+// Rows of an odd vocabulary stored without padding (PHASED) start anywhere: up to seven elements before the first boundary
+// and seven after the last whole vector are walked one by one. They also keep the arithmetic of the generic kernel above:
+// the maximum is subtracted, exactly, before the product with log2 e, and the scale multiplies the exponential. (Folding
+// both into the exponent, as the aligned rows do, rounds max log2 e: an error of 2^-24 |max log2 e| in the loss, and an
+// overflow in rows that hold nothing but the type's lowest value.) [8192, 50257] contiguous: 507 us through the generic
+// kernel, 394 us here, calls and all; padded rows of the same size 340 us.
 constexpr int kCeThreads = 512;
 
 __device__ __forceinline__ uint32_t bf2_max(uint32_t a, uint32_t b) {
@@ -305,18 +308,32 @@ __device__ __forceinline__ float row_max_bf16(const __nv_bfloat16* xr, const Row
   return block_max(m, red);
 }
 
-// sum over the row of 2^(x log2 e + nml), nml = -max log2 e (every thread gets it)
-__device__ __forceinline__ float row_expsum_bf16(const __nv_bfloat16* xr, const RowEnds& re, float nml, float* red) {
+// The exponent of x relative to the row's maximum m: x log2 e + nml with nml = -m log2 e; EXACT: (x - m) log2 e, nm = -m.
+template <bool EXACT>
+struct Shifted {
+  float c;
+  uint64_t c2, l2e2;
+  __device__ __forceinline__ explicit Shifted(float m)
+      : c(EXACT ? -m : -m * kLog2e), c2(f2_pack(c, c)), l2e2(f2_pack(kLog2e, kLog2e)) {}
+  __device__ __forceinline__ uint64_t operator()(uint64_t x2) const {
+    return EXACT ? f2_mul(f2_add2(x2, c2), l2e2) : f2_fma(x2, l2e2, c2);
+  }
+  __device__ __forceinline__ float operator()(float x) const { return EXACT ? (x + c) * kLog2e : fmaf(x, kLog2e, c); }
+};
+
+// sum over the row of 2^arg(x) (every thread gets it)
+template <bool EXACT>
+__device__ __forceinline__ float row_expsum_bf16(const __nv_bfloat16* xr, const RowEnds& re, const Shifted<EXACT>& arg,
+                                                 float* red) {
   const uint4* xv = reinterpret_cast<const uint4*>(xr + re.head);
   const int nvec = re.nvec;
-  const uint64_t l2e2 = f2_pack(kLog2e, kLog2e), nml2 = f2_pack(nml, nml);
   float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
   auto add8 = [&](const uint4& a) {
     float e0, e1, e2, e3, e4, e5, e6, e7;
-    f2_unpack(f2_fma(bf2_as_f2(a.x), l2e2, nml2), e0, e1);
-    f2_unpack(f2_fma(bf2_as_f2(a.y), l2e2, nml2), e2, e3);
-    f2_unpack(f2_fma(bf2_as_f2(a.z), l2e2, nml2), e4, e5);
-    f2_unpack(f2_fma(bf2_as_f2(a.w), l2e2, nml2), e6, e7);
+    f2_unpack(arg(bf2_as_f2(a.x)), e0, e1);
+    f2_unpack(arg(bf2_as_f2(a.y)), e2, e3);
+    f2_unpack(arg(bf2_as_f2(a.z)), e4, e5);
+    f2_unpack(arg(bf2_as_f2(a.w)), e6, e7);
     s0 += ex2_approx(e0) + ex2_approx(e1);
     s1 += ex2_approx(e2) + ex2_approx(e3);
     s2 += ex2_approx(e4) + ex2_approx(e5);
@@ -324,10 +341,11 @@ __device__ __forceinline__ float row_expsum_bf16(const __nv_bfloat16* xr, const 
   };
   // (four loads in flight per thread, as in the maximum pass, measured no faster here: 344 against 340 us)
   for (int i = threadIdx.x; i < nvec; i += kCeThreads) add8(xv[i]);
-  for (int t = threadIdx.x; t < re.n; t += kCeThreads) s0 += ex2_approx(fmaf(__bfloat162float(xr[re.col(t)]), kLog2e, nml));
+  for (int t = threadIdx.x; t < re.n; t += kCeThreads) s0 += ex2_approx(arg(__bfloat162float(xr[re.col(t)])));
   return block_sum((s0 + s1) + (s2 + s3), red);
 }
 
+template <bool PHASED>
 __global__ void __launch_bounds__(kCeThreads, 3)
 cross_entropy_bf16_kernel(const int32_t* __restrict__ labels, const __nv_bfloat16* logits, __nv_bfloat16* dlogits,
                           float* __restrict__ row_stats, const float* __restrict__ n_valid, int64_t rows, int cols,
@@ -337,7 +355,7 @@ cross_entropy_bf16_kernel(const int32_t* __restrict__ labels, const __nv_bfloat1
   const float inv_n = 1.f / *n_valid;
   for (int64_t row = blockIdx.x; row < rows; row += gridDim.x) {
     const __nv_bfloat16* xr = logits + row * ld;
-    const RowEnds re(cols, head_bf16(xr));
+    const RowEnds re(cols, PHASED ? head_bf16(xr) : 0);
     const int nvec = re.nvec;
     const uint4* xv = reinterpret_cast<const uint4*>(xr + re.head);
     __nv_bfloat16* dr = dlogits != nullptr ? dlogits + row * ld : nullptr;
@@ -364,17 +382,17 @@ cross_entropy_bf16_kernel(const int32_t* __restrict__ labels, const __nv_bfloat1
       hit = __syncthreads_or(earlier) ? 0.f : 1.f;
     }
     // pass 2: sum of exponentials
-    const float nml = -m * kLog2e;
-    const uint64_t l2e2 = f2_pack(kLog2e, kLog2e);
-    const float s = row_expsum_bf16(xr, re, nml, red);
+    const Shifted<PHASED> arg(m);
+    const float s = row_expsum_bf16(xr, re, arg, red);
     if (threadIdx.x == 0) {
       row_stats[row] = -(x_label - m - logf(s));
       row_stats[rows + row] = hit;
     }
     if (dr == nullptr) continue;
     // pass 3: dlogits = softmax / n_valid, the label's column minus 1 / n_valid
-    const float c3 = nml + log2f(inv_n / s);
-    const uint64_t c32 = f2_pack(c3, c3);
+    const float k = inv_n / s;
+    const float c3 = PHASED ? arg.c : arg.c + log2f(k);
+    const uint64_t c32 = f2_pack(c3, c3), k2 = f2_pack(k, k);
     uint4* dv = reinterpret_cast<uint4*>(dr + re.head);
     auto grad8 = [&](const uint4& a) {
       const uint32_t w[4] = {a.x, a.y, a.z, a.w};
@@ -382,19 +400,23 @@ cross_entropy_bf16_kernel(const int32_t* __restrict__ labels, const __nv_bfloat1
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         float y0, y1;
-        f2_unpack(f2_fma(bf2_as_f2(w[q]), l2e2, c32), y0, y1);
-        __nv_bfloat162 h = __floats2bfloat162_rn(ex2_approx(y0), ex2_approx(y1));
+        f2_unpack(PHASED ? arg(bf2_as_f2(w[q])) : f2_fma(bf2_as_f2(w[q]), arg.l2e2, c32), y0, y1);
+        y0 = ex2_approx(y0);
+        y1 = ex2_approx(y1);
+        if (PHASED) f2_unpack(f2_mul(f2_pack(y0, y1), k2), y0, y1);
+        __nv_bfloat162 h = __floats2bfloat162_rn(y0, y1);
         o[q] = *reinterpret_cast<uint32_t*>(&h);
       }
       return make_uint4(o[0], o[1], o[2], o[3]);
     };
+    auto grad1 = [&](float x) { return PHASED ? ex2_approx(arg(x)) * k : ex2_approx(fmaf(x, kLog2e, c3)); };
     for (int i = threadIdx.x; i < nvec; i += kCeThreads) dv[i] = grad8(xv[i]);
     for (int t = threadIdx.x; t < re.n; t += kCeThreads) {
       const int c = re.col(t);
-      dr[c] = __float2bfloat16_rn(ex2_approx(fmaf(__bfloat162float(xr[c]), kLog2e, c3)));
+      dr[c] = __float2bfloat16_rn(grad1(__bfloat162float(xr[c])));
     }
     __syncthreads();  // the label's column has been written (by whichever thread owns it) before it is patched
-    if (threadIdx.x == 0) dr[label] = __float2bfloat16_rn(ex2_approx(fmaf(x_label, kLog2e, c3)) - inv_n);
+    if (threadIdx.x == 0) dr[label] = __float2bfloat16_rn(grad1(x_label) - inv_n);
   }
 }
 
@@ -410,7 +432,7 @@ log_softmax_fwd_bf16_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* 
     __nv_bfloat16* yr = y + row * ld_y;
     const RowEnds re(cols, 0);
     const float m = row_max_bf16(xr, re, red);
-    const float s = row_expsum_bf16(xr, re, -m * kLog2e, red);
+    const float s = row_expsum_bf16(xr, re, Shifted<false>(m), red);
     const float nshift = -(m + logf(s));
     const uint64_t ns2 = f2_pack(nshift, nshift);
     const uint4* xv = reinterpret_cast<const uint4*>(xr);
@@ -449,7 +471,7 @@ log_softmax_bwd_bf16_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfl
     const RowEnds re(cols, 0);
     const float m = row_max_bf16(xr, re, red);
     const float nml = -m * kLog2e;
-    const float s = row_expsum_bf16(xr, re, nml, red);
+    const float s = row_expsum_bf16(xr, re, Shifted<false>(m), red);
     uint64_t g0 = 0ull, g1 = 0ull;  // two packed +0.0f each
     for (int i = threadIdx.x; i < nvec; i += kCeThreads) {
       const uint4 a = gv[i];
@@ -600,7 +622,8 @@ extern "C" int ptj_cross_entropy(const int32_t* labels, const void* logits, void
   } else if (same_phase<__nv_bfloat16>(logits, ld, dlogits, ld) && cols <= 0x7fffffffLL &&
              reinterpret_cast<uintptr_t>(logits) % 2 == 0) {
     const int64_t cap = static_cast<int64_t>(kNumSMs) * 3;  // three resident 512-thread blocks per SM
-    launch_k(cross_entropy_bf16_kernel, static_cast<int>(rows < cap ? rows : cap), kCeThreads, 0, st, labels,
+    const bool aligned = aligned16(logits) && ld % 8 == 0;  // (the gradient is in the same phase)
+    launch_k(aligned ? cross_entropy_bf16_kernel<false> : cross_entropy_bf16_kernel<true>, static_cast<int>(rows < cap ? rows : cap), kCeThreads, 0, st, labels,
              static_cast<const __nv_bfloat16*>(logits), static_cast<__nv_bfloat16*>(dlogits), row_stats, n_valid, rows,
              static_cast<int>(cols), ld);
   } else {
