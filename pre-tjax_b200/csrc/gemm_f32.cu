@@ -48,8 +48,19 @@ struct F32Params {
   int64_t M, N;
   int num_m, num_n, num_kb, split_k;
   float* workspace;  // [split_k, M, N] partial sums when split_k > 1
+  // the operands themselves, for products with elements that the parts cannot carry
+  const float *a, *b;
+  int64_t lda, ldb, K;
+  const int* flags;  // [num_flags] one per block of the splitting pass: it met such an element
+  int num_flags;
+  int* any_flag;     // whether any is set, for the finishing kernel
   unsigned int* fault;
 };
+
+// Operands with an infinity, or with a finite magnitude of 2^48 or more, are multiplied by fused multiply-adds instead, as if
+// there were no tensor-core path: an infinity times the parts of a number gives NaNs (their signs differ, or they are zero),
+// and products of parts may overflow where the sum does not. Below 2^48 neither can happen: |sum| < 2^30 2^96.
+constexpr float kBig = 281474976710656.f;  // 2^48
 
 // ---- splitting pass -------------------------------------------------------------------------------------------------
 struct SplitSrc {
@@ -59,19 +70,8 @@ struct SplitSrc {
 };
 
 __device__ __forceinline__ void split3(float a, uint16_t& p1, uint16_t& p2, uint16_t& p3) {
-  __nv_bfloat16 h1 = __float2bfloat16_rn(a);
-  float f1 = __bfloat162float(h1);
-  if (isinf(f1)) {
-    // a finite value above the largest bf16 must not round up to infinity; infinities and NaNs go through alone
-    if (isinf(a)) {
-      p1 = __bfloat16_as_ushort(h1);
-      p2 = p3 = 0;
-      return;
-    }
-    h1 = __ushort_as_bfloat16(static_cast<uint16_t>(a > 0.f ? 0x7f7fu : 0xff7fu));
-    f1 = __bfloat162float(h1);
-  }
-  const float r1 = isnan(a) ? 0.f : a - f1;  // exact
+  const __nv_bfloat16 h1 = __float2bfloat16_rn(a);
+  const float r1 = isnan(a) ? 0.f : a - __bfloat162float(h1);  // exact; a NaN goes through alone
   const __nv_bfloat16 h2 = __float2bfloat16_rn(r1);
   const float r2 = r1 - __bfloat162float(h2);  // exact, at most eight significant bits
   p1 = __bfloat16_as_ushort(h1);
@@ -81,8 +81,9 @@ __device__ __forceinline__ void split3(float a, uint16_t& p1, uint16_t& p2, uint
 
 // Memory-bound: 4 bytes read and 6 written per element, eight elements per thread.
 __global__ void __launch_bounds__(256)
-split_planes_kernel(const SplitSrc s0, const SplitSrc s1) {
+split_planes_kernel(const SplitSrc s0, const SplitSrc s1, int* __restrict__ flags) {
   grid_dep_sync();
+  float top = 0.f;  // largest magnitude, NaNs aside
   const int64_t g0 = s0.rows * (s0.ldp / 8), total = g0 + s1.rows * (s1.ldp / 8);
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -99,6 +100,8 @@ split_planes_kernel(const SplitSrc s0, const SplitSrc s1) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) v[j] = c + j < s.cols ? src[j] : 0.f;
     }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) top = fmaxf(top, fabsf(v[j]));
     uint32_t w[3][4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -113,6 +116,8 @@ split_planes_kernel(const SplitSrc s0, const SplitSrc s1) {
     for (int p = 0; p < 3; ++p)
       *reinterpret_cast<uint4*>(s.dst + p * plane + r * s.ldp + c) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
   }
+  const int any = __syncthreads_or(top >= kBig);
+  if (threadIdx.x == 0) flags[blockIdx.x] = any;
 }
 
 // ---- product --------------------------------------------------------------------------------------------------------
@@ -120,6 +125,78 @@ __device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
   uint64_t r;
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
+}
+
+__device__ __forceinline__ void epilogue_warps_sync() { asm volatile("barrier.sync 1, %0;" ::"n"(kEpilogueWarps * 32) : "memory"); }
+
+// The whole product by fused multiply-adds, in the order of the kernel in gemm.cu (one sum per output, along K): the same
+// bits. Run by the epilogue warps in their store strips: 64 x 128 outputs a block, 4 x 8 a thread; the next 16 of K are on
+// their way while a tile of them is multiplied. Not inlined: as part of the
+// kernel it took registers from the epilogue ([4096, 2304] x 768: 77 us in place of 72).
+constexpr int kFmaM = 64, kFmaN = 128, kFmaK = 16;
+constexpr int kFmaLdA = kFmaM + 4, kFmaLdB = kFmaN + 4;
+static_assert(kEpilogueWarps * 32 == (kFmaM / 4) * (kFmaN / 8), "a thread per 4 x 8 outputs");
+static_assert(kFmaK * (kFmaLdA + kFmaLdB) * 4 <= kEpilogueWarps * kStripBytes, "operand tiles fit the strips");
+template <bool A_KMAJOR, bool B_KMAJOR>
+__device__ __noinline__ void product_by_fma(const F32Params& p, float* smem, uint64_t seed, int tid) {
+  constexpr int kN = kEpilogueWarps * 32, kA = kFmaM * kFmaK / kN, kB = kFmaN * kFmaK / kN;
+  float* a_s = smem;                     // [kFmaK][kFmaLdA]
+  float* b_s = smem + kFmaK * kFmaLdA;   // [kFmaK][kFmaLdB]: columns 8 x + 4 h + e at 64 h + 4 x + e, read without conflicts
+  const int tx = tid % (kFmaN / 8), ty = tid / (kFmaN / 8);
+  const int64_t M = p.M, N = p.N, K = p.K, lda = p.lda, ldb = p.ldb;
+  const float *A = p.a, *B = p.b;
+  const int64_t cols = (N + kFmaN - 1) / kFmaN, tiles = (M + kFmaM - 1) / kFmaM * cols;
+  for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int64_t m0 = tile / cols * kFmaM, n0 = tile % cols * kFmaN;
+    float ra[kA], rb[kB], acc[4][8];
+    auto fetch = [&](int64_t k0) {
+#pragma unroll
+      for (int e = 0; e < kA; ++e) {
+        const int i = tid + e * kN, r = A_KMAJOR ? i / kFmaK : i % kFmaM, k = A_KMAJOR ? i % kFmaK : i / kFmaM;
+        const int64_t m = m0 + r, kk = k0 + k;
+        ra[e] = m < M && kk < K ? A[A_KMAJOR ? m * lda + kk : kk * lda + m] : 0.f;
+      }
+#pragma unroll
+      for (int e = 0; e < kB; ++e) {
+        const int i = tid + e * kN, r = B_KMAJOR ? i / kFmaK : i % kFmaN, k = B_KMAJOR ? i % kFmaK : i / kFmaN;
+        const int64_t n = n0 + r, kk = k0 + k;
+        rb[e] = n < N && kk < K ? B[B_KMAJOR ? n * ldb + kk : kk * ldb + n] : 0.f;
+      }
+    };
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+    fetch(0);
+    for (int64_t k0 = 0; k0 < K; k0 += kFmaK) {
+      epilogue_warps_sync();  // the tile before has been read
+#pragma unroll
+      for (int e = 0; e < kA; ++e) {
+        const int i = tid + e * kN, r = A_KMAJOR ? i / kFmaK : i % kFmaM, k = A_KMAJOR ? i % kFmaK : i / kFmaM;
+        a_s[k * kFmaLdA + r] = ra[e];
+      }
+#pragma unroll
+      for (int e = 0; e < kB; ++e) {
+        const int i = tid + e * kN, r = B_KMAJOR ? i / kFmaK : i % kFmaN, k = B_KMAJOR ? i % kFmaK : i / kFmaN;
+        b_s[k * kFmaLdB + (r % 8 / 4) * (kFmaN / 2) + r / 8 * 4 + r % 4] = rb[e];
+      }
+      epilogue_warps_sync();
+      if (k0 + kFmaK < K) fetch(k0 + kFmaK);
+#pragma unroll 4
+      for (int k = 0; k < kFmaK; ++k) {
+        const float4 a = *reinterpret_cast<const float4*>(a_s + k * kFmaLdA + ty * 4);
+        const float4 b0 = *reinterpret_cast<const float4*>(b_s + k * kFmaLdB + tx * 4);
+        const float4 b1 = *reinterpret_cast<const float4*>(b_s + k * kFmaLdB + kFmaN / 2 + tx * 4);
+        const float av[4] = {a.x, a.y, a.z, a.w}, bv[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) epilogue_row_segment<float, 8>(p.ep, m0 + ty * 4 + i, n0 + tx * 8, acc[i], seed);
+  }
 }
 
 template <bool A_KMAJOR, bool B_KMAJOR>
@@ -135,6 +212,7 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   uint64_t* tmem_empty = tmem_full + 2;   // used in the leader only: 8 local + 8 remote epilogue warps
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  int* epi_state = reinterpret_cast<int*>(tmem_slot + 2);  // written by the epilogue warps: 1 multiply by FMA, 2 a wait ran out
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
@@ -150,6 +228,7 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       mbar_init(&tmem_empty[b], 2 * kEpilogueWarps);
     }
     *abort_flag = 0;
+    *epi_state = 0;
     fence_barrier_init();
     prefetch_tensormap(&tmap_a);
     prefetch_tensormap(&tmap_b);
@@ -253,6 +332,31 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     const uint64_t seed = p.ep.mode == PTJ_EPI_DROPOUT_RESID ? resolve_seed(p.ep.seed) : 0ull;
     int it = 0;
     bool ok = true;
+    // the splitting pass's findings are read while the first tile is fetched and multiplied
+    const int etid = threadIdx.x - kFirstEpilogueWarp * 32;
+    int big = 0;
+    for (int i = etid; i < p.num_flags; i += kEpilogueWarps * 32) big |= __ldcg(p.flags + i);
+    if (big) atomicOr(epi_state, 1);
+    epilogue_warps_sync();
+    big = *epi_state & 1;  // the same in every block
+    if (blockIdx.x == 0 && etid == 0) *p.any_flag = big;
+    if (big) {  // let the issuing warps run through, unread, then multiply here
+      for (int item = pair; item < total && ok; item += npairs) {
+        const int split = item / tiles;
+        const int nkb = static_cast<int>(static_cast<int64_t>(split + 1) * p.num_kb / p.split_k) -
+                        static_cast<int>(static_cast<int64_t>(split) * p.num_kb / p.split_k);
+        for (int kb = 0; kb < nkb; ++kb, ++it) {
+          ok = mbar_wait(&tmem_full[it & 1], (it >> 1) & 1u, ctx, 0x0901u);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          if (lane == 0) mbar_arrive_cluster((it & 1) == 0 ? leader_empty0 : leader_empty1);
+        }
+      }
+      if (!ok) atomicOr(epi_state, 2);
+      epilogue_warps_sync();  // (reached by every warp: the waits above are bounded)
+      if (*epi_state == 1) product_by_fma<A_KMAJOR, B_KMAJOR>(p, reinterpret_cast<float*>(strips), seed, etid);
+      ok = false;
+    }
     for (int item = pair; item < total && ok; item += npairs) {
       const int split = item / tiles, tile = item - split * tiles;
       const int m_blk = tile % p.num_m, n_blk = tile / p.num_m;
@@ -337,8 +441,9 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
 
 // Sum of the K parts (fixed order) followed by the full epilogue: one thread per row and group of eight columns.
 __global__ void __launch_bounds__(256)
-f32_finish_kernel(const float* __restrict__ ws, const EpilogueParams ep, int split_k) {
+f32_finish_kernel(const float* __restrict__ ws, const int* __restrict__ any_flag, const EpilogueParams ep, int split_k) {
   grid_dep_sync();
+  const int stored = *any_flag;  // the product kernel has stored the result itself
   const uint64_t seed = ep.mode == PTJ_EPI_DROPOUT_RESID ? resolve_seed(ep.seed) : 0ull;
   const int64_t groups = (ep.N + 7) / 8, total = ep.M * groups;
   const bool vec = (ep.N & 3) == 0;
@@ -360,6 +465,7 @@ f32_finish_kernel(const float* __restrict__ ws, const EpilogueParams ep, int spl
           if (n0 + j < ep.N) acc[j] += src[j];
       }
     }
+    if (stored) return;
     epilogue_row_segment<float, 8>(ep, m, n0, acc, seed);
   }
 }
@@ -391,6 +497,9 @@ int f32_split_k(int64_t M, int64_t N, int64_t K) {
   }
   return best;
 }
+
+constexpr int kMaxSplitBlocks = kNumSMs * 16;
+constexpr size_t kFlagBytes = (static_cast<size_t>(kMaxSplitBlocks + 1) * 4 + 255) / 256 * 256;
 
 size_t plane_bytes(int64_t rows, int64_t cols) {  // multiple of 256
   return (static_cast<size_t>(3) * rows * ((cols + 7) / 8 * 8) * 2 + 255) / 256 * 256;
@@ -445,6 +554,7 @@ int launch_product(const CUtensorMap& ta, const CUtensorMap& tb, const F32Params
 size_t gemm_f32_workspace_floats(int64_t M, int64_t N, int64_t K, bool a_kmajor, bool b_kmajor) {
   if (!use_f32_tc(M, N, K)) return 0;
   size_t bytes = plane_bytes(a_kmajor ? M : K, a_kmajor ? K : M) + plane_bytes(b_kmajor ? N : K, b_kmajor ? K : N);
+  bytes += kFlagBytes;
   const int s = f32_split_k(M, N, K);
   if (s > 1) bytes += static_cast<size_t>(s) * M * N * 4;
   return bytes / 4;
@@ -458,6 +568,8 @@ int gemm_f32_tc(const float* a, const float* b, const EpilogueParams& ep, int64_
   ws += plane_bytes(ar, ac);
   SplitSrc sb{b, reinterpret_cast<__nv_bfloat16*>(ws), ldb, br, bc, (bc + 7) / 8 * 8};
   ws += plane_bytes(br, bc);
+  int* flags = reinterpret_cast<int*>(ws);
+  ws += kFlagBytes;
   F32Params p{};
   p.ep = ep;
   p.M = M;
@@ -467,6 +579,13 @@ int gemm_f32_tc(const float* a, const float* b, const EpilogueParams& ep, int64_
   p.num_kb = static_cast<int>(ceil_div(K, BK));
   p.split_k = f32_split_k(M, N, K);
   p.workspace = reinterpret_cast<float*>(ws);
+  p.a = a;
+  p.b = b;
+  p.lda = lda;
+  p.ldb = ldb;
+  p.K = K;
+  p.flags = flags;
+  p.any_flag = flags + kMaxSplitBlocks;
   p.fault = fault_word();
   if (p.fault == nullptr) return PTJ_ERR_DEVICE;
   if (static_cast<int64_t>(p.num_m) * p.num_n * p.split_k > 0x3fffffffLL) return PTJ_ERR_BAD_SHAPE;
@@ -475,15 +594,16 @@ int gemm_f32_tc(const float* a, const float* b, const EpilogueParams& ep, int64_
 
   const int64_t groups = ar * (sa.ldp / 8) + br * (sb.ldp / 8);
   int64_t blocks = ceil_div(groups, 256);
-  if (blocks > kNumSMs * 16) blocks = kNumSMs * 16;
-  launch_k(split_planes_kernel, static_cast<int>(blocks), 256, 0, st, sa, sb);
+  if (blocks > kMaxSplitBlocks) blocks = kMaxSplitBlocks;
+  p.num_flags = static_cast<int>(blocks);
+  launch_k(split_planes_kernel, static_cast<int>(blocks), 256, 0, st, sa, sb, flags);
   PTJ_CHECK_LAUNCH();
   const int rc = a_kmajor ? (b_kmajor ? launch_product<true, true>(ta, tb, p, st) : launch_product<true, false>(ta, tb, p, st))
                           : (b_kmajor ? launch_product<false, true>(ta, tb, p, st) : launch_product<false, false>(ta, tb, p, st));
   if (rc != PTJ_OK || p.split_k == 1) return rc;
   blocks = ceil_div(M * ceil_div(N, 8), 256);
   if (blocks > kNumSMs * 8) blocks = kNumSMs * 8;
-  launch_k(f32_finish_kernel, static_cast<int>(blocks), 256, 0, st, p.workspace, ep, p.split_k);
+  launch_k(f32_finish_kernel, static_cast<int>(blocks), 256, 0, st, p.workspace, p.any_flag, ep, p.split_k);
   PTJ_CHECK_LAUNCH();
   return PTJ_OK;
 }

@@ -102,3 +102,48 @@ def test_extreme_values(ops):
     assert float(out[0, 0]) == torch.finfo(torch.float32).max
     assert abs(float(out[1, 1]) / 1e-30 - 1.0) < 3e-7
     assert bool(torch.isnan(out[2]).all()) and not bool(torch.isnan(out[[0, 1, 3]]).any())
+
+
+def fma_product(ops, sa, sb, M, N, K, a_k, b_k):
+    """The same product on the fused-multiply-add kernel: no workspace."""
+    lib, out = pkg("_lib"), torch.empty(M, N, device="cuda")
+    lib.check(lib.lib().ptj_gemm(sa.data_ptr(), sb.data_ptr(), out.data_ptr(), 0, 0, 0, M, N, K, sa.shape[1], sb.shape[1],
+                                 N, int(a_k), int(b_k), 0, 0, 0, None, 1, 0, 0, torch.cuda.current_stream().cuda_stream), "ptj_gemm")
+    return out
+
+
+@pytest.mark.parametrize("a_k,b_k,M,N,K", [(True, True, 300, 520, 256), (True, False, 257, 333, 700), (False, True, 64, 130, 4200),
+                                           (False, False, 520, 776, 768)])
+def test_infinite_and_huge_operands_match_the_fma_kernel(ops, a_k, b_k, M, N, K):
+    """An infinity gives the infinities (and the NaNs of inf - inf and inf * 0) that it gives in a float32 sum, and products
+    that overflow do so where a float32 sum does; both bit for bit as on the fused-multiply-add kernel."""
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    base = [torch.randn(r, K, generator=g, device="cuda") for r in (M, N)]
+    for case in ("inf in A", "-inf in B", "both", "huge", "overflow"):
+        A, B = (t.clone() for t in base)
+        if case in ("inf in A", "both"):
+            A[3, 5] = A[M - 1, K - 1] = float("inf")
+            B[7, 5] = 0.0
+        if case in ("-inf in B", "both"):
+            B[N - 1, 5] = -float("inf")
+        if case == "huge":
+            A[2] *= 2.0 ** 100
+            B[4] *= 2.0 ** -100
+        if case == "overflow":
+            A[1] *= 2.0 ** 120
+            B[9] *= 2.0 ** 30
+        sa, sb = A if a_k else A.t().contiguous(), B if b_k else B.t().contiguous()
+        kw = dict(a_kmajor=a_k, b_kmajor=b_k, M=M, N=N, K=K, lda=sa.shape[1], ldb=sb.shape[1])
+        got, want = ops.gemm(sa, sb, **kw), fma_product(ops, sa, sb, M, N, K, a_k, b_k)
+        assert torch.equal(torch.isnan(got), torch.isnan(want)), case
+        assert torch.equal(torch.nan_to_num(got, nan=0.0), torch.nan_to_num(want, nan=0.0)), case
+        if case == "inf in A":
+            assert bool(torch.isinf(got[3]).sum() == N - 1) and bool(torch.isnan(got[3, 7]))
+        # the epilogue runs on what the sum gave: accumulation, bias and GELU
+        lib, bias = pkg("_lib"), torch.randn(N, generator=g, device="cuda")
+        acc, pre = torch.ones(M, N, device="cuda"), torch.empty(M, N, device="cuda")
+        ops.gemm(sa, sb, **kw, out=acc, epilogue=lib.EPI_ACCUM)
+        assert torch.equal(torch.nan_to_num(acc, nan=0.0), torch.nan_to_num(want + 1.0, nan=0.0)), case
+        ops.gemm(sa, sb, **kw, bias=bias, epilogue=lib.EPI_GELU, aux_out=pre)
+        assert torch.equal(torch.nan_to_num(pre, nan=0.0), torch.nan_to_num(want + bias, nan=0.0)), case
+    assert ops.last_kernel_fault() == 0
