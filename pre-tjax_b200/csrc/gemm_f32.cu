@@ -7,7 +7,8 @@
 // accumulation chain, which over a long K would bias the result. So a chain is only 64 elements of K long, runs from the
 // smallest partial products to the largest (four truncations at full magnitude), and the epilogue warps add each
 // finished chain into float32 REGISTERS with round-to-nearest. Measured against float64 the result is as accurate as a
-// sequential fused-multiply-add loop or better (tests/test_gemm_f32_gpu.py compares the two).
+// sequential fused-multiply-add loop or better (tests/test_gemm_f32_gpu.py compares the two). Operands with infinities, or
+// so large that a partial product could overflow, are found by the splitting pass and take the fused-multiply-add loop.
 //
 // Two launches: a splitting pass writes the three bf16 planes of both operands ([3][rows][ld], same storage order as the
 // operand, so K-major and MN-major operands need no transposition), then a persistent thread-block-pair kernel like the
@@ -131,8 +132,9 @@ __device__ __forceinline__ void epilogue_warps_sync() { asm volatile("barrier.sy
 
 // The whole product by fused multiply-adds, in the order of the kernel in gemm.cu (one sum per output, along K): the same
 // bits. Run by the epilogue warps in their store strips: 64 x 128 outputs a block, 4 x 8 a thread; the next 16 of K are on
-// their way while a tile of them is multiplied. Not inlined: as part of the
-// kernel it took registers from the epilogue ([4096, 2304] x 768: 77 us in place of 72).
+// their way while a tile of them is multiplied. [4096, 2304] x 768 with one infinity: 591 us (72 without, 593 on the kernel in
+// gemm.cu); [256, 256] x 256: 110 us (20, 20), as the launch has the few blocks that the tensor-core tiles need. Not inlined:
+// as part of the kernel it took registers from the epilogue ([4096, 2304] x 768 without an infinity: 76 us).
 constexpr int kFmaM = 64, kFmaN = 128, kFmaK = 16;
 constexpr int kFmaLdA = kFmaM + 4, kFmaLdB = kFmaN + 4;
 static_assert(kEpilogueWarps * 32 == (kFmaM / 4) * (kFmaN / 8), "a thread per 4 x 8 outputs");
