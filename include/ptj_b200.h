@@ -194,7 +194,7 @@ int ptj_colsum(const void* x, float* out, float* scratch, size_t scratch_floats,
  *              ptj_gemm_f32_workspace_floats floats (16-byte aligned) and float32 output the product runs on the tensor
  *              cores, every operand split exactly into three bf16 parts; without one, or where that function returns
  *              0 (small products), on fused-multiply-add units, as does (inside the same launches) a product with an
- *              operand element that is infinite or of magnitude 2^48 or more: its outputs are those of a float32 sum.
+ *              operand element that is infinite or of magnitude 2^24 or more: its outputs are those of a float32 sum.
  *   out_dtype  PTJ_F32 or PTJ_BF16, C row-major with leading dim ldc
  *   epilogue   PTJ_EPI_*; aux / aux_out meaning depends on it (same dtype and ld as C unless noted)
  *   split_k    >1 splits K over that many work items; partial tiles go to `workspace`

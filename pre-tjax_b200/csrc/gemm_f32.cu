@@ -1,8 +1,10 @@
 // float32 GEMM on the tensor cores.
 //
-// Every float32 operand element a is split exactly into three bf16 values, a = a1 + a2 + a3 (8 + 8 + 8 mantissa bits,
-// round to nearest), and the product is the sum of the six partial products whose magnitude can matter in float32:
+// Every float32 operand element a, times 2^24, is split exactly into three bf16 values, 2^24 a = a1 + a2 + a3 (8 + 8 + 8
+// mantissa bits, round to nearest), and the product is the sum of the six partial products whose magnitude can matter in float32:
 //   a1 b1 + (a1 b2 + a2 b1) + (a2 b2 + a1 b3 + a3 b1);   what is left out is below 2^-26 of |a b|.
+// The factor keeps the last bits of the smallest numbers (multiples of 2^-149) above bf16's smallest normal value, 2^-126;
+// without it parts of elements below 2^-110 were lost. 2^-48 times the sum undoes it, exactly down to float32's subnormals.
 // bf16 products are exact in the tensor core; its float32 accumulator, however, truncates at every step of an
 // accumulation chain, which over a long K would bias the result. So a chain is only 64 elements of K long, runs from the
 // smallest partial products to the largest (four truncations at full magnitude), and the epilogue warps add each
@@ -58,10 +60,12 @@ struct F32Params {
   unsigned int* fault;
 };
 
-// Operands with an infinity, or with a finite magnitude of 2^48 or more, are multiplied by fused multiply-adds instead, as if
+// Operands with an infinity, or with a finite magnitude of 2^24 or more, are multiplied by fused multiply-adds instead, as if
 // there were no tensor-core path: an infinity times the parts of a number gives NaNs (their signs differ, or they are zero),
-// and products of parts may overflow where the sum does not. Below 2^48 neither can happen: |sum| < 2^30 2^96.
-constexpr float kBig = 281474976710656.f;  // 2^48
+// and products of parts may overflow where the sum does not. Below 2^24 neither can happen: the sum of products of scaled
+// elements, each below 2^48, stays below 2^30 2^96.
+constexpr float kBig = 16777216.f, kScale = 16777216.f;  // 2^24 both
+constexpr float kUnscale = 1.f / (kScale * kScale);
 
 // ---- splitting pass -------------------------------------------------------------------------------------------------
 struct SplitSrc {
@@ -70,7 +74,8 @@ struct SplitSrc {
   int64_t ld, rows, cols, ldp;
 };
 
-__device__ __forceinline__ void split3(float a, uint16_t& p1, uint16_t& p2, uint16_t& p3) {
+__device__ __forceinline__ void split3(float x, uint16_t& p1, uint16_t& p2, uint16_t& p3) {
+  const float a = x * kScale;
   const __nv_bfloat16 h1 = __float2bfloat16_rn(a);
   const float r1 = isnan(a) ? 0.f : a - __bfloat162float(h1);  // exact; a NaN goes through alone
   const __nv_bfloat16 h2 = __float2bfloat16_rn(r1);
@@ -395,7 +400,7 @@ gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         const int64_t n0 = static_cast<int64_t>(n_blk) * BN + half * 128 + c * 32;
         float v[32];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) f2_unpack(acc[c * 16 + j], v[2 * j], v[2 * j + 1]);
+        for (int j = 0; j < 16; ++j) f2_unpack(f2_mul(acc[c * 16 + j], f2_pack(kUnscale, kUnscale)), v[2 * j], v[2 * j + 1]);
         if (p.split_k > 1) {
           float* w = p.workspace + static_cast<int64_t>(split) * p.M * p.N;
           if ((p.N & 3) == 0 && n0 + 32 <= p.N) {

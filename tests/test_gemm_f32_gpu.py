@@ -147,3 +147,18 @@ def test_infinite_and_huge_operands_match_the_fma_kernel(ops, a_k, b_k, M, N, K)
         ops.gemm(sa, sb, **kw, bias=bias, epilogue=lib.EPI_GELU, aux_out=pre)
         assert torch.equal(torch.nan_to_num(pre, nan=0.0), torch.nan_to_num(want + bias, nan=0.0)), case
     assert ops.last_kernel_fault() == 0
+
+
+@pytest.mark.parametrize("ea,eb", [(-120, 0), (-140, 10), (-126, 20), (0, -133), (-70, -60)])
+@pytest.mark.parametrize("a_k,b_k,K", [(True, True, 300), (False, False, 2100)])
+def test_small_magnitudes_keep_all_their_bits(ops, a_k, b_k, K, ea, eb):
+    """Operands down to float32's subnormals: their last bits lie far below bf16's smallest value."""
+    M, N = 264, 300
+    g = torch.Generator(device="cuda").manual_seed(K)
+    A, B = (torch.ldexp(1.0 + torch.rand(r, K, generator=g, device="cuda"), torch.tensor(e, device="cuda"))
+            * (torch.randint(0, 2, (r, K), generator=g, device="cuda") * 2 - 1) for r, e in ((M, ea), (N, eb)))
+    sa, sb = A if a_k else A.t().contiguous(), B if b_k else B.t().contiguous()
+    out = ops.gemm(sa, sb, a_kmajor=a_k, b_kmajor=b_k, M=M, N=N, K=K, lda=sa.shape[1], ldb=sb.shape[1])
+    ref, absum = A.double() @ B.double().t(), A.double().abs() @ B.double().abs().t()
+    # results below 2^-126 are rounded to multiples of 2^-149, once per chain and part of K at most
+    assert bool(((out.double() - ref).abs() <= bound(K, absum) + (K / 64 + 8) * 2.0 ** -149).all())
