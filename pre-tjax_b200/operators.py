@@ -244,7 +244,10 @@ def gemm(a, b, *, a_kmajor=True, b_kmajor=True, M=None, N=None, K=None, lda=None
         # bf16 planes of both operands (and K parts): with them the product runs on the tensor cores, at float32 accuracy
         ws_n = lib.ptj_gemm_f32_workspace_floats(M, N, K, int(a_kmajor), int(b_kmajor))
         if ws_n and (workspace is None or workspace.numel() < ws_n):
-            workspace = torch.empty(ws_n, device=a.device, dtype=torch.float32)
+            try:
+                workspace = torch.empty(ws_n, device=a.device, dtype=torch.float32)
+            except torch.OutOfMemoryError:  # 6 bytes per operand element: a product that fits without them still runs
+                workspace = None
     dargs = None
     if dropout_args is not None:
         p, train, seed, sid = dropout_args

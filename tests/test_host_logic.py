@@ -304,3 +304,27 @@ def test_checkpoint_step_index_follows_the_reference(tmp_path):
         i2, rows2, p2, _ = pickle.load(f)
     assert (i2, rows2) == (N, rows)
     assert all(torch.equal(a, b) for ga, gb in zip(p2, prm) for a, b in zip(ga, gb))
+
+
+def test_float32_product_without_room_for_its_workspace(monkeypatch):
+    """A float32 product whose workspace does not fit on the device runs without one (on the kernel that needs none)."""
+    ops, calls = pkg("operators"), []
+
+    class Library:
+        def ptj_gemm_f32_workspace_floats(self, *a):
+            return 1 << 40
+
+        def ptj_gemm(self, *a):
+            calls.append(a)
+            return 0
+
+    def empty(*a, **kw):
+        raise torch.OutOfMemoryError("no room")
+
+    a, b, out = torch.ones(4, 3), torch.ones(5, 3), torch.zeros(4, 5)
+    monkeypatch.setattr(ops._lib, "lib", Library)
+    monkeypatch.setattr(ops, "_stream", lambda: 0)
+    monkeypatch.setattr(ops.torch, "empty", empty)
+    for ws in (None, torch.zeros(8)):  # none given; one given that is too small
+        ops.gemm(a, b, out=out, workspace=ws)
+    assert [c[-3:] for c in calls] == [(None, 0, 0)] * 2
