@@ -275,6 +275,10 @@ int ptj_gemm_grouped2(const ptj_gemm_problem* p0, const ptj_gemm_problem* p1, in
  * the kernels without a dense [B,N,N] tensor: a row of a packed document starts at its document's first token, a
  * padding row gets row_kstart > i and attends nothing (zero output row, row_max 0, row_sum 1, zero gradients).
  * NULL = plain causal attention. Forward and backward of one call must be given the same array.
+ *
+ * A row reads only the keys it attends: on the SIMT kernels an infinity or a NaN in a row of Q, K, V or d_o reaches no
+ * output that does not attend that row. The tcgen05 kernels multiply masked entries by exact zeros, so there it also
+ * reaches the other rows of its 128-row tile.
  */
 typedef struct {
   int64_t batch, heads, seq, d_head;

@@ -8,8 +8,8 @@
 // output tile, in registers: two or three 16-byte shared loads per 32 multiply-adds. Score products pack neighbouring
 // d into the two-wide FMA straight from those loads. Bound by the FP32 pipe (a warp per row with scalar global loads
 // was bound by the load/store unit instead). Measured, float32, forward / backward: [8, 12, 512, 64] with dropout and
-// document masks 88 / 262 us (36 / 43 TFLOP/s of the causal half), where a warp per row with a Philox call per probability
-// took 2526 / 16152 us; [4, 12, 512, 64] without dropout 84 / 261 us, forward 1900 us before. R = 4: twice the warps of
+// document masks 88 / 265 us (36 / 43 TFLOP/s of the causal half), where a warp per row with a Philox call per probability
+// took 2526 / 16152 us; [4, 12, 512, 64] without dropout 84 / 264 us, forward 1900 us before. R = 4: twice the warps of
 // R = 8, which needs 255 registers and measured 98 / 314 and 90 / 294 us there, 23 / 75 us against 17 / 58 us at
 // [2, 12, 128, 64]. The dK/dV kernel is held to two blocks per SM: left alone it took 234 registers and one block, 317 us
 // at the first of these sizes.
@@ -56,34 +56,49 @@ __device__ __forceinline__ float4 load4(const T* p, int n, bool vec) {
   return v;
 }
 
-// rows [r0, r0 + 64) of a [seq][D] view, zero-filled to [64][DP]
+// A masked probability is an exact zero, but zero times an infinity or a NaN is a NaN: a tile that holds one is multiplied
+// with the masked entries left out (mul_*_masked), so that a row reads only what it attends. The loads form this sum of
+// zeros on the side; it is a NaN where an element is not finite. Cost: 262 -> 265 us in the backward kernels at
+// [8, 12, 512, 64], none in the forward kernel.
+__device__ __forceinline__ float zero_sum(float z, const float4& v) {
+  return fmaf(v.x, 0.f, fmaf(v.y, 0.f, fmaf(v.z, 0.f, fmaf(v.w, 0.f, z))));
+}
+
+// rows [r0, r0 + 64) of a [seq][D] view, zero-filled to [64][DP]; true when this thread met an element that is not finite
 template <typename T, int DP, int R>
-__device__ __forceinline__ void load_tile(float* dst, const T* base, int64_t rs, int64_t r0, int64_t S, int D, bool vec) {
+__device__ __forceinline__ bool load_tile(float* dst, const T* base, int64_t rs, int64_t r0, int64_t S, int D, bool vec) {
   constexpr int kC4 = DP / 4;
+  float z = 0.f;
 #pragma unroll 4
   for (int idx = threadIdx.x; idx < kB * kC4; idx += Tile<DP, R>::kThreads) {
     const int row = idx / kC4, c = idx % kC4 * 4;
     const int n = r0 + row < S ? D - c : 0;
-    *reinterpret_cast<float4*>(dst + row * Tile<DP, R>::kLd + c) = load4(base + (r0 + row) * rs + c, n, vec);
+    const float4 v = load4(base + (r0 + row) * rs + c, n, vec);
+    *reinterpret_cast<float4*>(dst + row * Tile<DP, R>::kLd + c) = v;
+    z = zero_sum(z, v);
   }
+  return z != 0.f;  // (a NaN is unequal to everything)
 }
 
 // the same for dO, with delta[row] = sum_d dO O on the side
 template <typename T, int DP, int R>
-__device__ __forceinline__ void load_tile_delta(float* dst, float* delta, const T* g, const T* o, int64_t rs, int64_t r0,
+__device__ __forceinline__ bool load_tile_delta(float* dst, float* delta, const T* g, const T* o, int64_t rs, int64_t r0,
                                                 int64_t S, int D, bool vec) {
   constexpr int kC4 = DP / 4;  // 8, 16 or 32 consecutive lanes hold a row
+  float z = 0.f;
 #pragma unroll 4
   for (int idx = threadIdx.x; idx < kB * kC4; idx += Tile<DP, R>::kThreads) {
     const int row = idx / kC4, c = idx % kC4 * 4;
     const int n = r0 + row < S ? D - c : 0;
     const float4 a = load4(g + (r0 + row) * rs + c, n, vec), b = load4(o + (r0 + row) * rs + c, n, vec);
     *reinterpret_cast<float4*>(dst + row * Tile<DP, R>::kLd + c) = a;
+    z = zero_sum(z, a);
     float s = fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, a.w * b.w)));
 #pragma unroll
     for (int off = kC4 / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
     if (idx % kC4 == 0) delta[row] = s;
   }
+  return z != 0.f;
 }
 
 // keep flags of the 64 x 64 tile at (r0, j0): nine bytes per row from the Philox call that holds the row's first element
@@ -185,6 +200,42 @@ __device__ __forceinline__ void mul_tn(float (&acc)[R][Tile<DP, R>::kCols], cons
     for (int r = 0; r < R; ++r)
 #pragma unroll
       for (int c = 0; c < kCols; ++c) acc[r][c] = fmaf(p[r], v[c], acc[r][c]);
+  }
+}
+
+// The two sums over unmasked entries alone, on(r, k) and on(q, r): for tiles with elements that are not finite.
+template <int DP, int R, typename On>
+__device__ __forceinline__ void mul_nn_masked(float (&acc)[R][Tile<DP, R>::kCols], const float* w, const float* x, int tx, int ty,
+                                              On&& on) {
+  constexpr int kCols = Tile<DP, R>::kCols;
+#pragma unroll 1
+  for (int k = 0; k < kB; ++k) {
+    float v[kCols];
+    load_cols<DP, R>(v, x + k * Tile<DP, R>::kLd, tx);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (!on(r, k)) continue;
+      const float p = w[(ty * R + r) * kPS + k];
+#pragma unroll
+      for (int c = 0; c < kCols; ++c) acc[r][c] = fmaf(p, v[c], acc[r][c]);
+    }
+  }
+}
+template <int DP, int R, typename On>
+__device__ __forceinline__ void mul_tn_masked(float (&acc)[R][Tile<DP, R>::kCols], const float* w, const float* x, int tx, int ty,
+                                              On&& on) {
+  constexpr int kCols = Tile<DP, R>::kCols;
+#pragma unroll 1
+  for (int q = 0; q < kB; ++q) {
+    float v[kCols];
+    load_cols<DP, R>(v, x + q * Tile<DP, R>::kLd, tx);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (!on(q, r)) continue;
+      const float p = w[q * kPS + ty * R + r];
+#pragma unroll
+      for (int c = 0; c < kCols; ++c) acc[r][c] = fmaf(p, v[c], acc[r][c]);
+    }
   }
 }
 
@@ -297,9 +348,9 @@ attn_fwd_simt_kernel(const FwdArgs<T> a) {
     const int64_t j0 = static_cast<int64_t>(kt) * kB;
     __syncthreads();
     load_tile<T, DP, R>(k_s, kb, a.sh.k_strides[2], j0, S, D, a.vec);
-    load_tile<T, DP, R>(v_s, vb, a.sh.v_strides[2], j0, S, D, a.vec);
+    const bool odd_v = load_tile<T, DP, R>(v_s, vb, a.sh.v_strides[2], j0, S, D, a.vec);
     if (drop) draw_flags(flags, dr, bh, S, r0, j0, TT::kThreads);
-    __syncthreads();
+    const bool masked = __syncthreads_or(odd_v);
     float s[R][4];
     mul_nt<DP, R>(s, q_s, k_s, tx, ty);
     __syncthreads();  // the key tile is free
@@ -335,7 +386,8 @@ attn_fwd_simt_kernel(const FwdArgs<T> a) {
       m[r] = mnew;
     }
     __syncwarp();  // a row's probabilities are written and read by the same half-warp
-    mul_nn<DP, R>(acc, p_s, v_s, tx, ty);
+    if (!masked) mul_nn<DP, R>(acc, p_s, v_s, tx, ty);
+    else mul_nn_masked<DP, R>(acc, p_s, v_s, tx, ty, [&](int r, int k) { return j0 + k <= r0 + ty * R + r && j0 + k >= ks[r]; });
   }
   float inv[R];
 #pragma unroll
@@ -458,10 +510,11 @@ attn_dq_simt_kernel(const BwdArgs<T> a) {
   for (int kt = kt0; kt <= qt; ++kt) {
     const int64_t j0 = static_cast<int64_t>(kt) * kB;
     __syncthreads();
-    load_tile<T, DP, R>(k_s, a.k + b * a.sh.k_strides[0] + h * a.sh.k_strides[1], a.sh.k_strides[2], j0, S, D, a.vec);
+    const bool odd_k =
+        load_tile<T, DP, R>(k_s, a.k + b * a.sh.k_strides[0] + h * a.sh.k_strides[1], a.sh.k_strides[2], j0, S, D, a.vec);
     load_tile<T, DP, R>(v_s, a.v + b * a.sh.v_strides[0] + h * a.sh.v_strides[1], a.sh.v_strides[2], j0, S, D, a.vec);
     if (drop) draw_flags(flags, dr, bh, S, r0, j0, TT::kThreads);
-    __syncthreads();
+    const bool masked = __syncthreads_or(odd_k);
     float s[R][4], dp[R][4];
     mul_nt<DP, R>(s, q_s, k_s, tx, ty);
     mul_nt<DP, R>(dp, g_s, v_s, tx, ty);
@@ -471,7 +524,10 @@ attn_dq_simt_kernel(const BwdArgs<T> a) {
 #pragma unroll
       for (int c = 0; c < 4; ++c) ds_s[(ty * R + r) * kPS + tx + 16 * c] = dp[r][c];
     __syncwarp();  // a row is written and read by the same half-warp
-    mul_nn<DP, R>(acc, ds_s, k_s, tx, ty);
+    if (!masked) mul_nn<DP, R>(acc, ds_s, k_s, tx, ty);
+    else mul_nn_masked<DP, R>(acc, ds_s, k_s, tx, ty, [&](int r, int k) {
+      return j0 + k <= r0 + ty * R + r && j0 + k >= rc.ks[ty * R + r];
+    });
     __syncwarp();
   }
   store_rows<T, DP, R>(a.dq + b * a.dsh.q_strides[0] + h * a.dsh.q_strides[1], a.dsh.q_strides[2], r0, S, D, a.vec, acc,
@@ -520,10 +576,12 @@ attn_dkv_simt_kernel(const BwdArgs<T> a) {
       const bool reach = threadIdx.x < kB && rc.ks[threadIdx.x] <= r0 + threadIdx.x && rc.ks[threadIdx.x] < j0 + kB;
       if (!__syncthreads_or(reach)) continue;
     }
-    load_tile<T, DP, R>(q_s, a.q + b * a.sh.q_strides[0] + h * a.sh.q_strides[1], a.sh.q_strides[2], r0, S, D, a.vec);
-    load_tile_delta<T, DP, R>(g_s, rc.delta, a.d_o + o_off, a.o + o_off, a.sh.o_strides[2], r0, S, D, a.vec);
+    const bool odd_q =
+        load_tile<T, DP, R>(q_s, a.q + b * a.sh.q_strides[0] + h * a.sh.q_strides[1], a.sh.q_strides[2], r0, S, D, a.vec);
+    const bool odd_g =
+        load_tile_delta<T, DP, R>(g_s, rc.delta, a.d_o + o_off, a.o + o_off, a.sh.o_strides[2], r0, S, D, a.vec);
     if (drop) draw_flags(flags, dr, bh, S, r0, j0, TT::kThreads);
-    __syncthreads();
+    const bool masked = __syncthreads_or(odd_q || odd_g);
     float s[R][4], dp[R][4];
     mul_nt<DP, R>(s, q_s, k_s, tx, ty);
     mul_nt<DP, R>(dp, g_s, v_s, tx, ty);
@@ -536,8 +594,14 @@ attn_dkv_simt_kernel(const BwdArgs<T> a) {
         ds_s[(ty * R + r) * kPS + tx + 16 * c] = dp[r][c];
       }
     __syncthreads();
-    mul_tn<DP, R>(dv, p_s, g_s, tx, ty);
-    mul_tn<DP, R>(dk, ds_s, q_s, tx, ty);
+    if (!masked) {
+      mul_tn<DP, R>(dv, p_s, g_s, tx, ty);
+      mul_tn<DP, R>(dk, ds_s, q_s, tx, ty);
+    } else {
+      const auto on = [&](int q, int r) { return j0 + ty * R + r <= r0 + q && j0 + ty * R + r >= rc.ks[q]; };
+      mul_tn_masked<DP, R>(dv, p_s, g_s, tx, ty, on);
+      mul_tn_masked<DP, R>(dk, ds_s, q_s, tx, ty, on);
+    }
   }
   store_rows<T, DP, R>(a.dv + b * a.dsh.v_strides[0] + h * a.dsh.v_strides[1], a.dsh.v_strides[2], j0, S, D, a.vec, dv,
                        one, tx, ty);

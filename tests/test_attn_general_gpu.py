@@ -101,3 +101,40 @@ def test_against_float64(dtype, B, H, S, D, p, train, packed, pad):
     for name, got, (ref, mag) in zip(("O", "dQ", "dK", "dV"), (o, dq, dk, dv), refs):
         worst = ((got.double() - ref).abs() - u * ref.abs() - 2.0 ** -17 * mag).max()
         assert bool(torch.isfinite(got.float()).all()) and float(worst) <= 1e-30, f"{name} {float(worst):.3e}"
+
+
+@pytest.mark.parametrize("bad", [math.nan, math.inf, -math.inf])
+@pytest.mark.parametrize("dtype,S,D,p,packed", [(F32, 200, 64, 0.0, False), (F32, 200, 32, 0.2, True), (F32, 130, 80, 0.0, True),
+                                                (BF16, 150, 64, 0.1, True)])
+def test_nonfinite_rows_reach_only_what_attends_them(dtype, S, D, p, packed, bad):
+    """A NaN or an infinity in one row of V, K, Q or dO must not reach an output whose mask leaves that row out, although
+    both lie in the same tile: those outputs are bit for bit what they are without it."""
+    ops = pkg("operators")
+    B, H, row = 1, 2, S - 40  # inside the last tile but one of the sequence, and of a document
+    lens = [[max(1, S // 3), S - S // 3 - 20]] if packed else None
+    ks = ops.row_kstart_from_lengths(lens, S) if packed else None
+    g = torch.Generator(device="cuda").manual_seed(S)
+    clean = [torch.randn(B, H, S, D, generator=g, device="cuda").to(dtype) for _ in range(4)]
+    first = ks[0].long() if packed else torch.zeros(S, dtype=torch.long, device="cuda")
+    i = torch.arange(S, device="cuda")
+    attends = (row >= first) & (row <= i)        # query rows that read key `row`
+    attended = (i >= first[row]) & (i <= row)    # keys that query row `row` reads
+    want, _ = run(ops, *clean, p, True, 7, ks, 0)
+    for which in range(4):
+        x = [t.clone() for t in clean]
+        x[which][0, 1, row, D // 2] = bad
+        (o, m, l, dq, dk, dv), _ = run(ops, *x, p, True, 7, ks, 0)
+        own = i == row
+        queries = {0: own, 1: attends, 2: attends, 3: own}[which]  # rows of O and dQ that may change
+        keys = attended
+        if which in (1, 2):  # every key of a row that attends `row` shares its normalisation and its delta
+            keys = torch.zeros_like(own)
+            for r in i[attends].tolist():
+                keys |= (i >= first[r]) & (i <= r)
+        for name, got, ref, may in (("O", o, want[0], queries if which != 3 else ~own & own), ("dQ", dq, want[3], queries),
+                                    ("dK", dk, want[4], keys), ("dV", dv, want[5], keys)):
+            assert torch.equal(got[:, 0], ref[:, 0]), (which, name, "another head")
+            same = got[0, 1][~may] == ref[0, 1][~may]
+            assert bool(same.all()), (which, name, int((~same).any(dim=1).sum()))
+        if which == 2:  # and it does reach the rows that attend it
+            assert not bool(torch.isfinite(o[0, 1, row]).all())
