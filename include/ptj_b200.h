@@ -332,8 +332,9 @@ int ptj_cast_f32_to_bf16(const float* src, void* dst_bf16, int64_t n, void* stre
 /* Greedy decoding with train=False (loss_and_optimizer_triton.py:203-212) of `batch` (1..8) sequences that start with the
  * token `start`, float32 weights, keys and values of earlier positions kept: tokens[batch, seq] gets the arg-max tokens of
  * positions 0 .. seq-2 in columns 1 .. seq-1 (column 0 is not written). layer_tensors: DEVICE array of layers x 10 pointers
- * (g1, b1, w_qkv, w_o, g2, b2, w1, b1f, w2, b2f), matrices 16-byte aligned and contiguous. dim, ffn and dim / heads are
- * multiples of 4. workspace: ptj_decode_workspace_floats(...) floats, 16-byte aligned; 0 = shape not supported. The launch
+ * (g1, b1, w_qkv, w_o, g2, b2, w1, b1f, w2, b2f), matrices 16-byte aligned and contiguous, vectors on any float. The
+ * kernel checks the matrices of the array: with a misaligned one it decodes nothing and ptj_last_kernel_fault reports
+ * 0x3102. dim, ffn and dim / heads are multiples of 4. workspace: ptj_decode_workspace_floats(...) floats, 16-byte aligned; 0 = shape not supported. The launch
  * is cooperative (one block per SM). */
 size_t ptj_decode_workspace_floats(int64_t batch, int64_t vocab, int64_t dim, int64_t layers, int64_t heads, int64_t ffn,
                                    int64_t seq);

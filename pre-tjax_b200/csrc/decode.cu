@@ -28,6 +28,7 @@ constexpr int kSteps = 5;    // QKV, out-projection, FFN-1, FFN-2, LM head
 constexpr int kMaxHead = 128;
 constexpr int kLayerTensors = 10;  // g1, b1, w_qkv, w_o, g2, b2, w1, b1f, w2, b2f
 constexpr int kSmemLimit = 227 * 1024;
+constexpr unsigned int kFaultBarrier = 0x3101u, kFaultMisaligned = 0x3102u;
 
 struct Step {
   int R, K;         // rows and row length of the matrix
@@ -141,7 +142,7 @@ __device__ __forceinline__ bool grid_barrier(const DecodeParams& p, unsigned int
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(p.barrier) : "memory");
       if (static_cast<int>(seen - target) >= 0) break;
       if (clock64() - t0 > tc::kWaitLimitCycles) {
-        tc::record_fault(p.fault, 0x3101u);
+        tc::record_fault(p.fault, kFaultBarrier);
         ok = 0;
         break;
       }
@@ -169,6 +170,12 @@ __device__ __forceinline__ float2 warp_row_stats(const float* row, int D, int la
     ss += fmaf(a, a, b * b) + fmaf(c, c, d * d);
   }
   return make_float2(mean, 1.f / sqrtf(warp_sum(ss) / static_cast<float>(D - 1)));
+}
+
+// elements 4 i .. 4 i + 3 of a scale or shift; aligned: it starts on a 16-byte boundary
+__device__ __forceinline__ float4 load_vector4(const float* v, int i, bool aligned) {
+  if (aligned) return __ldg(reinterpret_cast<const float4*>(v) + i);
+  return make_float4(__ldg(v + 4 * i), __ldg(v + 4 * i + 1), __ldg(v + 4 * i + 2), __ldg(v + 4 * i + 3));
 }
 
 struct Best {
@@ -201,8 +208,19 @@ decode_kernel(const __grid_constant__ DecodeParams p) {
     share[tid].n = static_cast<int>(pairs * (blockIdx.x + 1) / gridDim.x) - share[tid].first;
   }
   if (tid < p.B) token_s[tid] = p.start;
-  for (int i = tid; i < p.L * kLayerTensors; i += kThreads) layers[i] = p.layers[i];
-  __syncthreads();
+  // The host cannot see these pointers. Matrices are copied in 16-byte pieces; scales and shifts may lie on any float.
+  auto off16 = [](const float* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) != 0; };
+  bool bad = false, odd = off16(p.g_f) || off16(p.b_f);
+  for (int i = tid; i < p.L * kLayerTensors; i += kThreads) {
+    layers[i] = p.layers[i];
+    const int k = i % kLayerTensors;
+    (k == 2 || k == 3 || k == 6 || k == 8 ? bad : odd) |= off16(layers[i]);
+  }
+  if (__syncthreads_or(bad)) {  // the same in every block: none waits for another yet
+    if (blockIdx.x == 0 && tid == 0) tc::record_fault(p.fault, kFaultMisaligned);
+    return;
+  }
+  const bool aligned = !__syncthreads_or(odd);
   Cursor cur;
   cur.init(p, share, layers);
 #pragma unroll 1
@@ -280,8 +298,8 @@ decode_kernel(const __grid_constant__ DecodeParams p) {
     const int nd = p.D / 4, n = p.B * nd;
     float4 g0, b0;
     if (tid < n) {
-      g0 = __ldg(reinterpret_cast<const float4*>(g) + tid % nd);
-      b0 = __ldg(reinterpret_cast<const float4*>(b) + tid % nd);
+      g0 = load_vector4(g, tid % nd, aligned);
+      b0 = load_vector4(b, tid % nd, aligned);
     }
     __syncthreads();
     if (warp < p.B) {
@@ -291,8 +309,8 @@ decode_kernel(const __grid_constant__ DecodeParams p) {
     __syncthreads();
     for (int i = tid; i < n; i += kThreads) {
       if (i != tid) {
-        g0 = __ldg(reinterpret_cast<const float4*>(g) + i % nd);
-        b0 = __ldg(reinterpret_cast<const float4*>(b) + i % nd);
+        g0 = load_vector4(g, i % nd, aligned);
+        b0 = load_vector4(b, i % nd, aligned);
       }
       const float2 st = stats_s[i / nd];
       float4* x = reinterpret_cast<float4*>(act + i / nd * p.act_ld) + i % nd;

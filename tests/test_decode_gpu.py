@@ -55,3 +55,44 @@ def test_other_weights_take_the_whole_forward():
         dtype = torch.float32 if D == 24 else torch.bfloat16
         cfg = gpt2.config_from_params(params, 0.1)
         assert ops.decode_greedy(gpt2.Weights.from_pytree(params, cfg, dtype), cfg, 2, 1) is None
+
+
+def decode_from(params, cfg, B, start, vectors, w_qkv_offset=0):
+    """ptj_decode with every vector `vectors` floats and the first layer's W_QKV `w_qkv_offset` floats off a 16-byte boundary."""
+    lib, ops, gpt2 = pkg("_lib"), pkg("operators"), pkg("gpt2")
+    w = gpt2.Weights.from_pytree(params, cfg, torch.float32)
+    moved = {}
+    for n, t in w.t.items():
+        off = vectors if t.dim() == 1 else (w_qkv_offset if n == "l0.w_qkv" else 0)
+        buf = torch.zeros(t.numel() + 4, device="cuda")
+        buf[off:off + t.numel()] = t.reshape(-1)
+        moved[n] = buf[off:off + t.numel()]
+        assert moved[n].data_ptr() % 16 == 4 * off
+    ptrs = torch.tensor([moved[n].data_ptr() for n, _ in cfg.param_shapes() if n.startswith("l")], dtype=torch.int64, device="cuda")
+    dims = (cfg.vocab, cfg.dim, cfg.layers, cfg.heads, cfg.ffn, cfg.seq)
+    ws = torch.empty(lib.lib().ptj_decode_workspace_floats(B, *dims), device="cuda")
+    tokens = torch.full((B, cfg.seq), -7, device="cuda", dtype=torch.int32)
+    m = {n: t.data_ptr() for n, t in moved.items()}
+    rc = lib.lib().ptj_decode(m["w_emb"], m["b_head"], m["w_pos"], ptrs.data_ptr(), m["g_f"], m["b_f"], tokens.data_ptr(), start,
+                              ops.DROPOUT_RATE, B, *dims, ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
+    return rc, ops.last_kernel_fault(), tokens
+
+
+@pytest.mark.parametrize("offset", [1, 2, 3])
+def test_vectors_on_any_float(offset):
+    ops, gpt2 = pkg("operators"), pkg("gpt2")
+    params = weights(1001, 96, 2, 3, 388, 33, 5)
+    cfg = gpt2.config_from_params(params, ops.DROPOUT_RATE)
+    rc, fault, tokens = decode_from(params, cfg, 2, 1000, offset)
+    assert (rc, fault) == (0, 0)
+    want = ops.decode_greedy(gpt2.Weights.from_pytree(params, cfg, torch.float32), cfg, 2, 1000)
+    assert torch.equal(tokens[:, 1:], want[:, 1:]) and want[0, 1:].unique().numel() > 2
+
+
+def test_a_misaligned_matrix_is_reported():
+    ops, gpt2 = pkg("operators"), pkg("gpt2")
+    params = weights(64, 32, 1, 2, 64, 8, 3)
+    cfg = gpt2.config_from_params(params, ops.DROPOUT_RATE)
+    rc, fault, tokens = decode_from(params, cfg, 1, 1, 0, w_qkv_offset=1)
+    assert (rc, fault) == (0, 0x3102) and bool((tokens == -7).all())
+    assert decode_from(params, cfg, 1, 1, 0)[:2] == (0, 0)
