@@ -10,6 +10,7 @@ set ``operators.DROPOUT_RATE`` before calling.
 from __future__ import annotations
 
 import ctypes
+import math
 import weakref
 
 import torch
@@ -524,15 +525,17 @@ DECODE_GROUP = 8  # sequences that ptj_decode takes in one launch
 
 def decode_greedy(w, cfg, batch: int, start: int, p=None):
     """int32 [batch, cfg.seq]: greedy decoding of `batch` sequences from the token `start` (columns 1.. are written), for
-    float32 weights; None where ptj_decode does not apply (other types, sizes or alignments). w: gpt2.Weights."""
-    if any(t.dtype != torch.float32 or t.data_ptr() % 16 for t in w.t.values()) or cfg.seq < 2 or batch < 1:
+    float32 weights; None where ptj_decode does not apply (other types, sizes or alignments, or tensors that are not what
+    the configuration says: the kernel reads them by the configuration's sizes). w: gpt2.Weights."""
+    device = w["w_emb"].device
+    if any(w[n].dtype != torch.float32 or w[n].data_ptr() % 16 or w[n].device != device or not w[n].is_contiguous()
+           or w[n].numel() != math.prod(shape) for n, shape in cfg.param_shapes()) or cfg.seq < 2 or batch < 1:
         return None
     lib, p = _lib.lib(), DROPOUT_RATE if p is None else p
     dims = (cfg.vocab, cfg.dim, cfg.layers, cfg.heads, cfg.ffn, cfg.seq)
     need = int(lib.ptj_decode_workspace_floats(min(batch, DECODE_GROUP), *dims))
     if need == 0:
         return None
-    device = w["w_emb"].device
     names = [n for n, _ in cfg.param_shapes() if n.startswith("l")]
     ptrs = torch.tensor([w[n].data_ptr() for n in names], dtype=torch.int64, device=device)
     tokens = torch.empty((batch, cfg.seq), device=device, dtype=torch.int32)

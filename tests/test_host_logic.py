@@ -328,3 +328,24 @@ def test_float32_product_without_room_for_its_workspace(monkeypatch):
     for ws in (None, torch.zeros(8)):  # none given; one given that is too small
         ops.gemm(a, b, out=out, workspace=ws)
     assert [c[-3:] for c in calls] == [(None, 0, 0)] * 2
+
+
+def test_decoding_refuses_tensors_that_are_not_the_configurations(monkeypatch):
+    """The decoding kernel reads every tensor by the sizes of the first layer: a pytree whose layers differ, or whose tensors
+    are views with gaps, is left to the whole forward pass and its checks."""
+    ops, g = pkg("operators"), pkg("gpt2")
+    cfg = g.GPT2Config(vocab=64, dim=16, layers=2, heads=2, ffn=32, seq=8)
+    asked = []
+
+    class Library:
+        def ptj_decode_workspace_floats(self, *a):
+            asked.append(a)
+            return 0  # sizes not supported: nothing is launched
+
+    monkeypatch.setattr(ops._lib, "lib", Library)
+    whole = {n: torch.empty(s) for n, s in cfg.param_shapes()}
+    cases = [{}, {"l1.w1": torch.empty(24, 16)}, {"l1.w2": torch.empty(16, 64)[:, :32]}, {"b_head": torch.empty(63)},
+             {"l0.w_o": torch.empty(16, 16, device="meta")}]
+    for i, other in enumerate(cases):
+        assert ops.decode_greedy(g.Weights(cfg, {**whole, **other}), cfg, 2, 1) is None
+        assert len(asked) == 1, f"case {i}: only the fitting tensors get as far as the kernel's own sizes"
