@@ -520,7 +520,7 @@ def cross_entropy(labels, logits, cols=None, want_grad=True, in_place=False, n_v
     return out3, n_valid, dlogits
 
 
-DECODE_GROUP = 8  # sequences that ptj_decode takes in one launch
+DECODE_GROUPS = (8, 4, 2, 1)  # sequences in one launch of ptj_decode: the first that its shared memory holds
 
 
 def decode_greedy(w, cfg, batch: int, start: int, p=None):
@@ -533,15 +533,18 @@ def decode_greedy(w, cfg, batch: int, start: int, p=None):
         return None
     lib, p = _lib.lib(), DROPOUT_RATE if p is None else p
     dims = (cfg.vocab, cfg.dim, cfg.layers, cfg.heads, cfg.ffn, cfg.seq)
-    need = int(lib.ptj_decode_workspace_floats(min(batch, DECODE_GROUP), *dims))
-    if need == 0:
+    for group in (min(batch, g) for g in DECODE_GROUPS):
+        need = int(lib.ptj_decode_workspace_floats(group, *dims))
+        if need:
+            break
+    else:
         return None
     names = [n for n, _ in cfg.param_shapes() if n.startswith("l")]
     ptrs = torch.tensor([w[n].data_ptr() for n in names], dtype=torch.int64, device=device)
     tokens = torch.empty((batch, cfg.seq), device=device, dtype=torch.int32)
     ws = torch.empty(need, device=device, dtype=torch.float32)
-    for b0 in range(0, batch, DECODE_GROUP):
-        n = min(batch - b0, DECODE_GROUP)
+    for b0 in range(0, batch, group):
+        n = min(batch - b0, group)
         _lib.check(lib.ptj_decode(_ptr(w["w_emb"]), _ptr(w["b_head"]), _ptr(w["w_pos"]), _ptr(ptrs), _ptr(w["g_f"]),
                                   _ptr(w["b_f"]), _ptr(tokens[b0:]), start, p, n, *dims, _ptr(ws), ws.numel(), _stream()),
                    "ptj_decode")

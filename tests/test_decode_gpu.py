@@ -25,6 +25,7 @@ def weights(V, D, L, H, F, S, seed):
     (5, 1024, 256, 1, 4, 1024, 9),    # five sequences in the kernel for eight
     (8, 300, 1024, 1, 8, 4096, 40),   # largest activations: the shallow ring
     (11, 513, 128, 3, 2, 512, 20),    # two groups of sequences
+    (5, 300, 1280, 3, 20, 5120, 10),  # rows of which shared memory holds four: groups of four and one
 ])
 def test_decode_matches_whole_forward(B, V, D, L, H, F, S):
     ops, ev, gpt2 = pkg("operators"), pkg("evaluate"), pkg("gpt2")

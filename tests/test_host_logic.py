@@ -347,5 +347,6 @@ def test_decoding_refuses_tensors_that_are_not_the_configurations(monkeypatch):
     cases = [{}, {"l1.w1": torch.empty(24, 16)}, {"l1.w2": torch.empty(16, 64)[:, :32]}, {"b_head": torch.empty(63)},
              {"l0.w_o": torch.empty(16, 16, device="meta")}]
     for i, other in enumerate(cases):
+        asked.clear()
         assert ops.decode_greedy(g.Weights(cfg, {**whole, **other}), cfg, 2, 1) is None
-        assert len(asked) == 1, f"case {i}: only the fitting tensors get as far as the kernel's own sizes"
+        assert bool(asked) == (i == 0), f"case {i}: only the fitting tensors get as far as the kernel's own sizes"
