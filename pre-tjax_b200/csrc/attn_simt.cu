@@ -4,13 +4,13 @@
 // both recompute the probabilities from the saved row maximum and row sum.
 //
 // A thread block owns a tile of 64 query (dK/dV pass: key) rows and sweeps 64-row tiles of the other side through shared
-// memory. 16 x (64 / R) threads each form an R x 4 block of the 64 x 64 scores, and an R x (DP / 16) block of every
+// memory. 16 x (64 / kR) threads each form a kR x 4 block of the 64 x 64 scores, and a kR x (DP / 16) block of every
 // output tile, in registers: two or three 16-byte shared loads per 32 multiply-adds. Score products pack neighbouring
 // d into the two-wide FMA straight from those loads. Bound by the FP32 pipe (a warp per row with scalar global loads
 // was bound by the load/store unit instead). Measured, float32, forward / backward: [8, 12, 512, 64] with dropout and
 // document masks 88 / 265 us (36 / 43 TFLOP/s of the causal half), where a warp per row with a Philox call per probability
-// took 2526 / 16152 us; [4, 12, 512, 64] without dropout 84 / 264 us, forward 1900 us before. R = 4: twice the warps of
-// R = 8, which needs 255 registers and measured 98 / 314 and 90 / 294 us there, 23 / 75 us against 17 / 58 us at
+// took 2526 / 16152 us; [4, 12, 512, 64] without dropout 84 / 264 us, forward 1900 us before. kR = 4: twice the warps of
+// kR = 8, which needs 255 registers and measured 98 / 314 and 90 / 294 us there, 23 / 75 us against 17 / 58 us at
 // [2, 12, 128, 64]. The dK/dV kernel is held to two blocks per SM: left alone it took 234 registers and one block, 317 us
 // at the first of these sizes.
 #include "attn_common.cuh"
@@ -21,11 +21,12 @@ namespace {
 constexpr int kMaxD = 128;
 constexpr int kB = 64;         // tile edge along queries and keys
 constexpr int kPS = kB + 4;    // row stride of a [64][64] tile in shared memory
+constexpr int kR = 4;          // rows of a tile per thread
 constexpr int kFlagStride = 12;  // bytes per row of keep flags: 64 flags that may start anywhere in a byte
 
-template <int DP, int R>
+template <int DP>
 struct Tile {
-  static constexpr int kThreads = 16 * kB / R;
+  static constexpr int kThreads = 16 * kB / kR;
   static constexpr int kLd = DP + 4;             // row stride (words): 16-byte reads of 8 consecutive rows hit 32 banks
   static constexpr int kWords = kB * kLd;
   static constexpr int kCols = DP / 16;          // output columns of a thread
@@ -65,33 +66,33 @@ __device__ __forceinline__ float zero_sum(float z, const float4& v) {
 }
 
 // rows [r0, r0 + 64) of a [seq][D] view, zero-filled to [64][DP]; true when this thread met an element that is not finite
-template <typename T, int DP, int R>
+template <typename T, int DP>
 __device__ __forceinline__ bool load_tile(float* dst, const T* base, int64_t rs, int64_t r0, int64_t S, int D, bool vec) {
   constexpr int kC4 = DP / 4;
   float z = 0.f;
 #pragma unroll 4
-  for (int idx = threadIdx.x; idx < kB * kC4; idx += Tile<DP, R>::kThreads) {
+  for (int idx = threadIdx.x; idx < kB * kC4; idx += Tile<DP>::kThreads) {
     const int row = idx / kC4, c = idx % kC4 * 4;
     const int n = r0 + row < S ? D - c : 0;
     const float4 v = load4(base + (r0 + row) * rs + c, n, vec);
-    *reinterpret_cast<float4*>(dst + row * Tile<DP, R>::kLd + c) = v;
+    *reinterpret_cast<float4*>(dst + row * Tile<DP>::kLd + c) = v;
     z = zero_sum(z, v);
   }
   return z != 0.f;  // (a NaN is unequal to everything)
 }
 
 // the same for dO, with delta[row] = sum_d dO O on the side
-template <typename T, int DP, int R>
+template <typename T, int DP>
 __device__ __forceinline__ bool load_tile_delta(float* dst, float* delta, const T* g, const T* o, int64_t rs, int64_t r0,
                                                 int64_t S, int D, bool vec) {
   constexpr int kC4 = DP / 4;  // 8, 16 or 32 consecutive lanes hold a row
   float z = 0.f;
 #pragma unroll 4
-  for (int idx = threadIdx.x; idx < kB * kC4; idx += Tile<DP, R>::kThreads) {
+  for (int idx = threadIdx.x; idx < kB * kC4; idx += Tile<DP>::kThreads) {
     const int row = idx / kC4, c = idx % kC4 * 4;
     const int n = r0 + row < S ? D - c : 0;
     const float4 a = load4(g + (r0 + row) * rs + c, n, vec), b = load4(o + (r0 + row) * rs + c, n, vec);
-    *reinterpret_cast<float4*>(dst + row * Tile<DP, R>::kLd + c) = a;
+    *reinterpret_cast<float4*>(dst + row * Tile<DP>::kLd + c) = a;
     z = zero_sum(z, a);
     float s = fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, a.w * b.w)));
 #pragma unroll
@@ -113,13 +114,13 @@ __device__ __forceinline__ void draw_flags(uint8_t* flags, const AttnDropout& dr
 }
 __device__ __forceinline__ bool flag_at(const uint8_t* row_flags, int bit) { return (row_flags[bit >> 3] >> (bit & 7)) & 1; }
 
-// acc[r][c] = sum_d a[ty * R + r][d] * b[tx + 16 c][d]
-template <int DP, int R>
-__device__ __forceinline__ void mul_nt(float (&out)[R][4], const float* a, const float* b, int tx, int ty) {
-  constexpr int ld = Tile<DP, R>::kLd;
-  uint64_t acc[R][4];
+// acc[r][c] = sum_d a[ty * kR + r][d] * b[tx + 16 c][d]
+template <int DP>
+__device__ __forceinline__ void mul_nt(float (&out)[kR][4], const float* a, const float* b, int tx, int ty) {
+  constexpr int ld = Tile<DP>::kLd;
+  uint64_t acc[kR][4];
 #pragma unroll
-  for (int r = 0; r < R; ++r)
+  for (int r = 0; r < kR; ++r)
 #pragma unroll
     for (int c = 0; c < 4; ++c) acc[r][c] = 0ull;
 #pragma unroll 2
@@ -128,14 +129,14 @@ __device__ __forceinline__ void mul_nt(float (&out)[R][4], const float* a, const
 #pragma unroll
     for (int c = 0; c < 4; ++c) y[c] = *reinterpret_cast<const ulonglong2*>(b + (tx + 16 * c) * ld + d);
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(a + (ty * R + r) * ld + d);
+    for (int r = 0; r < kR; ++r) {
+      const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(a + (ty * kR + r) * ld + d);
 #pragma unroll
       for (int c = 0; c < 4; ++c) acc[r][c] = f2_fma(x.y, y[c].y, f2_fma(x.x, y[c].x, acc[r][c]));
     }
   }
 #pragma unroll
-  for (int r = 0; r < R; ++r)
+  for (int r = 0; r < kR; ++r)
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       float lo, hi;
@@ -145,9 +146,9 @@ __device__ __forceinline__ void mul_nt(float (&out)[R][4], const float* a, const
 }
 
 // one row of an output tile's operand: this thread's columns
-template <int DP, int R>
-__device__ __forceinline__ void load_cols(float (&v)[Tile<DP, R>::kCols], const float* row, int tx) {
-  using TT = Tile<DP, R>;
+template <int DP>
+__device__ __forceinline__ void load_cols(float (&v)[Tile<DP>::kCols], const float* row, int tx) {
+  using TT = Tile<DP>;
 #pragma unroll
   for (int c = 0; c < TT::kCols; c += TT::kVec) {
     if constexpr (TT::kVec == 4) {
@@ -160,21 +161,21 @@ __device__ __forceinline__ void load_cols(float (&v)[Tile<DP, R>::kCols], const 
   }
 }
 
-// acc[r][.] += sum_k w[ty * R + r][k] * x[k][cols]   (rows of w written by the same half-warp)
-template <int DP, int R>
-__device__ __forceinline__ void mul_nn(float (&acc)[R][Tile<DP, R>::kCols], const float* w, const float* x, int tx, int ty) {
-  constexpr int kCols = Tile<DP, R>::kCols;
+// acc[r][.] += sum_k w[ty * kR + r][k] * x[k][cols]   (rows of w written by the same half-warp)
+template <int DP>
+__device__ __forceinline__ void mul_nn(float (&acc)[kR][Tile<DP>::kCols], const float* w, const float* x, int tx, int ty) {
+  constexpr int kCols = Tile<DP>::kCols;
 #pragma unroll 1
   for (int k = 0; k < kB; k += 4) {
-    float4 p[R];
+    float4 p[kR];
 #pragma unroll
-    for (int r = 0; r < R; ++r) p[r] = *reinterpret_cast<const float4*>(w + (ty * R + r) * kPS + k);
+    for (int r = 0; r < kR; ++r) p[r] = *reinterpret_cast<const float4*>(w + (ty * kR + r) * kPS + k);
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk) {
       float v[kCols];
-      load_cols<DP, R>(v, x + (k + kk) * Tile<DP, R>::kLd, tx);
+      load_cols<DP>(v, x + (k + kk) * Tile<DP>::kLd, tx);
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
+      for (int r = 0; r < kR; ++r) {
         const float pr = kk == 0 ? p[r].x : (kk == 1 ? p[r].y : (kk == 2 ? p[r].z : p[r].w));
 #pragma unroll
         for (int c = 0; c < kCols; ++c) acc[r][c] = fmaf(pr, v[c], acc[r][c]);
@@ -183,56 +184,56 @@ __device__ __forceinline__ void mul_nn(float (&acc)[R][Tile<DP, R>::kCols], cons
   }
 }
 
-// acc[r][.] += sum_q w[q][ty * R + r] * x[q][cols]
-template <int DP, int R>
-__device__ __forceinline__ void mul_tn(float (&acc)[R][Tile<DP, R>::kCols], const float* w, const float* x, int tx, int ty) {
-  constexpr int kCols = Tile<DP, R>::kCols;
+// acc[r][.] += sum_q w[q][ty * kR + r] * x[q][cols]
+template <int DP>
+__device__ __forceinline__ void mul_tn(float (&acc)[kR][Tile<DP>::kCols], const float* w, const float* x, int tx, int ty) {
+  constexpr int kCols = Tile<DP>::kCols;
 #pragma unroll 2
   for (int q = 0; q < kB; ++q) {
-    float p[R], v[kCols];
+    float p[kR], v[kCols];
 #pragma unroll
-    for (int r = 0; r < R; r += 4) {
-      const float4 t = *reinterpret_cast<const float4*>(w + q * kPS + ty * R + r);
+    for (int r = 0; r < kR; r += 4) {
+      const float4 t = *reinterpret_cast<const float4*>(w + q * kPS + ty * kR + r);
       p[r] = t.x; p[r + 1] = t.y; p[r + 2] = t.z; p[r + 3] = t.w;
     }
-    load_cols<DP, R>(v, x + q * Tile<DP, R>::kLd, tx);
+    load_cols<DP>(v, x + q * Tile<DP>::kLd, tx);
 #pragma unroll
-    for (int r = 0; r < R; ++r)
+    for (int r = 0; r < kR; ++r)
 #pragma unroll
       for (int c = 0; c < kCols; ++c) acc[r][c] = fmaf(p[r], v[c], acc[r][c]);
   }
 }
 
 // The two sums over unmasked entries alone, on(r, k) and on(q, r): for tiles with elements that are not finite.
-template <int DP, int R, typename On>
-__device__ __forceinline__ void mul_nn_masked(float (&acc)[R][Tile<DP, R>::kCols], const float* w, const float* x, int tx, int ty,
+template <int DP, typename On>
+__device__ __forceinline__ void mul_nn_masked(float (&acc)[kR][Tile<DP>::kCols], const float* w, const float* x, int tx, int ty,
                                               On&& on) {
-  constexpr int kCols = Tile<DP, R>::kCols;
+  constexpr int kCols = Tile<DP>::kCols;
 #pragma unroll 1
   for (int k = 0; k < kB; ++k) {
     float v[kCols];
-    load_cols<DP, R>(v, x + k * Tile<DP, R>::kLd, tx);
+    load_cols<DP>(v, x + k * Tile<DP>::kLd, tx);
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
+    for (int r = 0; r < kR; ++r) {
       if (!on(r, k)) continue;
-      const float p = w[(ty * R + r) * kPS + k];
+      const float p = w[(ty * kR + r) * kPS + k];
 #pragma unroll
       for (int c = 0; c < kCols; ++c) acc[r][c] = fmaf(p, v[c], acc[r][c]);
     }
   }
 }
-template <int DP, int R, typename On>
-__device__ __forceinline__ void mul_tn_masked(float (&acc)[R][Tile<DP, R>::kCols], const float* w, const float* x, int tx, int ty,
+template <int DP, typename On>
+__device__ __forceinline__ void mul_tn_masked(float (&acc)[kR][Tile<DP>::kCols], const float* w, const float* x, int tx, int ty,
                                               On&& on) {
-  constexpr int kCols = Tile<DP, R>::kCols;
+  constexpr int kCols = Tile<DP>::kCols;
 #pragma unroll 1
   for (int q = 0; q < kB; ++q) {
     float v[kCols];
-    load_cols<DP, R>(v, x + q * Tile<DP, R>::kLd, tx);
+    load_cols<DP>(v, x + q * Tile<DP>::kLd, tx);
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
+    for (int r = 0; r < kR; ++r) {
       if (!on(q, r)) continue;
-      const float p = w[q * kPS + ty * R + r];
+      const float p = w[q * kPS + ty * kR + r];
 #pragma unroll
       for (int c = 0; c < kCols; ++c) acc[r][c] = fmaf(p, v[c], acc[r][c]);
     }
@@ -240,13 +241,13 @@ __device__ __forceinline__ void mul_tn_masked(float (&acc)[R][Tile<DP, R>::kCols
 }
 
 // this thread's block of an output tile; mul[r] scales a row
-template <typename T, int DP, int R>
+template <typename T, int DP>
 __device__ __forceinline__ void store_rows(T* base, int64_t rs, int64_t r0, int64_t S, int D, bool vec,
-                                           const float (&acc)[R][Tile<DP, R>::kCols], const float (&mul)[R], int tx, int ty) {
-  using TT = Tile<DP, R>;
+                                           const float (&acc)[kR][Tile<DP>::kCols], const float (&mul)[kR], int tx, int ty) {
+  using TT = Tile<DP>;
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int64_t i = r0 + ty * R + r;
+  for (int r = 0; r < kR; ++r) {
+    const int64_t i = r0 + ty * kR + r;
     if (i >= S) continue;
     T* row = base + i * rs;
 #pragma unroll
@@ -291,11 +292,11 @@ struct FwdArgs {
 };
 
 // Block = one query tile of one (batch, head), the longest rows first. Online softmax over the key tiles.
-template <typename T, int DP, int R>
-__global__ void __launch_bounds__(Tile<DP, R>::kThreads)
+template <typename T, int DP>
+__global__ void __launch_bounds__(Tile<DP>::kThreads)
 attn_fwd_simt_kernel(const FwdArgs<T> a) {
   grid_dep_sync();
-  using TT = Tile<DP, R>;
+  using TT = Tile<DP>;
   extern __shared__ __align__(16) float smem[];
   float* q_s = smem;
   float* v_s = q_s + TT::kWords;
@@ -316,13 +317,13 @@ attn_fwd_simt_kernel(const FwdArgs<T> a) {
   const int64_t r0 = static_cast<int64_t>(qt) * kB;
   const T* kb = a.k + b * a.sh.k_strides[0] + h * a.sh.k_strides[1];
   const T* vb = a.v + b * a.sh.v_strides[0] + h * a.sh.v_strides[1];
-  load_tile<T, DP, R>(q_s, a.q + b * a.sh.q_strides[0] + h * a.sh.q_strides[1], a.sh.q_strides[2], r0, S, D, a.vec);
+  load_tile<T, DP>(q_s, a.q + b * a.sh.q_strides[0] + h * a.sh.q_strides[1], a.sh.q_strides[2], r0, S, D, a.vec);
 
   // row i attends keys [ks, i]; ks > i (padding, rows beyond the sequence): nothing
-  int64_t ks[R];
+  int64_t ks[kR];
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int64_t i = r0 + ty * R + r;
+  for (int r = 0; r < kR; ++r) {
+    const int64_t i = r0 + ty * kR + r;
     ks[r] = i >= S ? i + 1 : (a.kstart != nullptr ? a.kstart[b * S + i] : 0);
   }
   int kt0 = 0;
@@ -330,15 +331,15 @@ attn_fwd_simt_kernel(const FwdArgs<T> a) {
     if (threadIdx.x == 0) first_key = 0x7fffffff;
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < R; ++r)
-      if (tx == 0 && ks[r] <= r0 + ty * R + r) atomicMin(&first_key, static_cast<int>(ks[r] > 0 ? ks[r] : 0));
+    for (int r = 0; r < kR; ++r)
+      if (tx == 0 && ks[r] <= r0 + ty * kR + r) atomicMin(&first_key, static_cast<int>(ks[r] > 0 ? ks[r] : 0));
     __syncthreads();
     kt0 = first_key / kB;
   }
 
-  float m[R], l[R], acc[R][TT::kCols];
+  float m[kR], l[kR], acc[kR][TT::kCols];
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
+  for (int r = 0; r < kR; ++r) {
     m[r] = -INFINITY;
     l[r] = 0.f;
 #pragma unroll
@@ -347,16 +348,16 @@ attn_fwd_simt_kernel(const FwdArgs<T> a) {
   for (int kt = kt0; kt <= qt; ++kt) {
     const int64_t j0 = static_cast<int64_t>(kt) * kB;
     __syncthreads();
-    load_tile<T, DP, R>(k_s, kb, a.sh.k_strides[2], j0, S, D, a.vec);
-    const bool odd_v = load_tile<T, DP, R>(v_s, vb, a.sh.v_strides[2], j0, S, D, a.vec);
+    load_tile<T, DP>(k_s, kb, a.sh.k_strides[2], j0, S, D, a.vec);
+    const bool odd_v = load_tile<T, DP>(v_s, vb, a.sh.v_strides[2], j0, S, D, a.vec);
     if (drop) draw_flags(flags, dr, bh, S, r0, j0, TT::kThreads);
     const bool masked = __syncthreads_or(odd_v);
-    float s[R][4];
-    mul_nt<DP, R>(s, q_s, k_s, tx, ty);
+    float s[kR][4];
+    mul_nt<DP>(s, q_s, k_s, tx, ty);
     __syncthreads();  // the key tile is free
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int64_t i = r0 + ty * R + r;
+    for (int r = 0; r < kR; ++r) {
+      const int64_t i = r0 + ty * kR + r;
       float mx = -INFINITY;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
@@ -374,11 +375,11 @@ attn_fwd_simt_kernel(const FwdArgs<T> a) {
         float p = expf(s[r][c] - ref);
         sum += p;
         if (drop) {
-          if (!flag_at(flags + (ty * R + r) * kFlagStride, tx + 16 * c + shift)) p = 0.f;
+          if (!flag_at(flags + (ty * kR + r) * kFlagStride, tx + 16 * c + shift)) p = 0.f;
         } else if (!dr.train) {
           p *= dr.eval_scale;
         }
-        p_s[(ty * R + r) * kPS + tx + 16 * c] = p;
+        p_s[(ty * kR + r) * kPS + tx + 16 * c] = p;
       }
       l[r] = l[r] * corr + half_warp_sum(sum);
 #pragma unroll
@@ -386,13 +387,13 @@ attn_fwd_simt_kernel(const FwdArgs<T> a) {
       m[r] = mnew;
     }
     __syncwarp();  // a row's probabilities are written and read by the same half-warp
-    if (!masked) mul_nn<DP, R>(acc, p_s, v_s, tx, ty);
-    else mul_nn_masked<DP, R>(acc, p_s, v_s, tx, ty, [&](int r, int k) { return j0 + k <= r0 + ty * R + r && j0 + k >= ks[r]; });
+    if (!masked) mul_nn<DP>(acc, p_s, v_s, tx, ty);
+    else mul_nn_masked<DP>(acc, p_s, v_s, tx, ty, [&](int r, int k) { return j0 + k <= r0 + ty * kR + r && j0 + k >= ks[r]; });
   }
-  float inv[R];
+  float inv[kR];
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int64_t i = r0 + ty * R + r;
+  for (int r = 0; r < kR; ++r) {
+    const int64_t i = r0 + ty * kR + r;
     const bool empty = ks[r] > i;  // zero output, neutral statistics
     inv[r] = empty ? 0.f : 1.f / l[r];
     if (empty) {
@@ -404,7 +405,7 @@ attn_fwd_simt_kernel(const FwdArgs<T> a) {
       a.row_sum[bh * S + i] = empty ? 1.f : l[r];
     }
   }
-  store_rows<T, DP, R>(a.o + b * a.sh.o_strides[0] + h * a.sh.o_strides[1], a.sh.o_strides[2], r0, S, D, a.vec, acc, inv,
+  store_rows<T, DP>(a.o + b * a.sh.o_strides[0] + h * a.sh.o_strides[1], a.sh.o_strides[2], r0, S, D, a.vec, acc, inv,
                        tx, ty);
 }
 
@@ -437,15 +438,15 @@ __device__ __forceinline__ void load_row_const(RowConst& rc, const BwdArgs<T>& a
   }
 }
 
-// Probabilities and score gradients of this thread's R x 4 block: s holds Q K^T on entry and dropout(P) on exit, dp holds
+// Probabilities and score gradients of this thread's kR x 4 block: s holds Q K^T on entry and dropout(P) on exit, dp holds
 // dO V^T on entry and dS = P o (dP o keep - delta) * scale on exit.
-template <typename T, int R>
-__device__ __forceinline__ void p_and_ds(float (&s)[R][4], float (&dp)[R][4], const RowConst& rc, const uint8_t* flags,
+template <typename T>
+__device__ __forceinline__ void p_and_ds(float (&s)[kR][4], float (&dp)[kR][4], const RowConst& rc, const uint8_t* flags,
                                          bool drop, const BwdArgs<T>& a, int64_t bh, int64_t r0, int64_t j0, int tx, int ty) {
   const int64_t S = a.sh.seq;
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int row = ty * R + r;
+  for (int r = 0; r < kR; ++r) {
+    const int row = ty * kR + r;
     const int64_t i = r0 + row;
     const float m = rc.m[row], inv_l = rc.inv_l[row], delta = rc.delta[row];
     const int64_t ks = rc.ks[row];
@@ -464,11 +465,11 @@ __device__ __forceinline__ void p_and_ds(float (&s)[R][4], float (&dp)[R][4], co
 }
 
 // dQ: block = one query tile, the longest rows first; sweeps the key tiles.
-template <typename T, int DP, int R>
-__global__ void __launch_bounds__(Tile<DP, R>::kThreads)
+template <typename T, int DP>
+__global__ void __launch_bounds__(Tile<DP>::kThreads)
 attn_dq_simt_kernel(const BwdArgs<T> a) {
   grid_dep_sync();
-  using TT = Tile<DP, R>;
+  using TT = Tile<DP>;
   extern __shared__ __align__(16) float smem[];
   float* q_s = smem;
   float* g_s = q_s + TT::kWords;
@@ -490,8 +491,8 @@ attn_dq_simt_kernel(const BwdArgs<T> a) {
   const int64_t r0 = static_cast<int64_t>(qt) * kB, o_off = b * a.sh.o_strides[0] + h * a.sh.o_strides[1];
   if (threadIdx.x == 0) first_key = 0x7fffffff;
   load_row_const(rc, a, b, bh, r0);
-  load_tile<T, DP, R>(q_s, a.q + b * a.sh.q_strides[0] + h * a.sh.q_strides[1], a.sh.q_strides[2], r0, S, D, a.vec);
-  load_tile_delta<T, DP, R>(g_s, rc.delta, a.d_o + o_off, a.o + o_off, a.sh.o_strides[2], r0, S, D, a.vec);
+  load_tile<T, DP>(q_s, a.q + b * a.sh.q_strides[0] + h * a.sh.q_strides[1], a.sh.q_strides[2], r0, S, D, a.vec);
+  load_tile_delta<T, DP>(g_s, rc.delta, a.d_o + o_off, a.o + o_off, a.sh.o_strides[2], r0, S, D, a.vec);
   __syncthreads();
   int kt0 = 0;
   if (a.kstart != nullptr) {
@@ -500,9 +501,9 @@ attn_dq_simt_kernel(const BwdArgs<T> a) {
     __syncthreads();
     kt0 = first_key / kB;
   }
-  float acc[R][TT::kCols], one[R];
+  float acc[kR][TT::kCols], one[kR];
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
+  for (int r = 0; r < kR; ++r) {
     one[r] = 1.f;
 #pragma unroll
     for (int c = 0; c < TT::kCols; ++c) acc[r][c] = 0.f;
@@ -511,35 +512,35 @@ attn_dq_simt_kernel(const BwdArgs<T> a) {
     const int64_t j0 = static_cast<int64_t>(kt) * kB;
     __syncthreads();
     const bool odd_k =
-        load_tile<T, DP, R>(k_s, a.k + b * a.sh.k_strides[0] + h * a.sh.k_strides[1], a.sh.k_strides[2], j0, S, D, a.vec);
-    load_tile<T, DP, R>(v_s, a.v + b * a.sh.v_strides[0] + h * a.sh.v_strides[1], a.sh.v_strides[2], j0, S, D, a.vec);
+        load_tile<T, DP>(k_s, a.k + b * a.sh.k_strides[0] + h * a.sh.k_strides[1], a.sh.k_strides[2], j0, S, D, a.vec);
+    load_tile<T, DP>(v_s, a.v + b * a.sh.v_strides[0] + h * a.sh.v_strides[1], a.sh.v_strides[2], j0, S, D, a.vec);
     if (drop) draw_flags(flags, dr, bh, S, r0, j0, TT::kThreads);
     const bool masked = __syncthreads_or(odd_k);
-    float s[R][4], dp[R][4];
-    mul_nt<DP, R>(s, q_s, k_s, tx, ty);
-    mul_nt<DP, R>(dp, g_s, v_s, tx, ty);
-    p_and_ds<T, R>(s, dp, rc, flags, drop, a, bh, r0, j0, tx, ty);
+    float s[kR][4], dp[kR][4];
+    mul_nt<DP>(s, q_s, k_s, tx, ty);
+    mul_nt<DP>(dp, g_s, v_s, tx, ty);
+    p_and_ds<T>(s, dp, rc, flags, drop, a, bh, r0, j0, tx, ty);
 #pragma unroll
-    for (int r = 0; r < R; ++r)
+    for (int r = 0; r < kR; ++r)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) ds_s[(ty * R + r) * kPS + tx + 16 * c] = dp[r][c];
+      for (int c = 0; c < 4; ++c) ds_s[(ty * kR + r) * kPS + tx + 16 * c] = dp[r][c];
     __syncwarp();  // a row is written and read by the same half-warp
-    if (!masked) mul_nn<DP, R>(acc, ds_s, k_s, tx, ty);
-    else mul_nn_masked<DP, R>(acc, ds_s, k_s, tx, ty, [&](int r, int k) {
-      return j0 + k <= r0 + ty * R + r && j0 + k >= rc.ks[ty * R + r];
+    if (!masked) mul_nn<DP>(acc, ds_s, k_s, tx, ty);
+    else mul_nn_masked<DP>(acc, ds_s, k_s, tx, ty, [&](int r, int k) {
+      return j0 + k <= r0 + ty * kR + r && j0 + k >= rc.ks[ty * kR + r];
     });
     __syncwarp();
   }
-  store_rows<T, DP, R>(a.dq + b * a.dsh.q_strides[0] + h * a.dsh.q_strides[1], a.dsh.q_strides[2], r0, S, D, a.vec, acc,
+  store_rows<T, DP>(a.dq + b * a.dsh.q_strides[0] + h * a.dsh.q_strides[1], a.dsh.q_strides[2], r0, S, D, a.vec, acc,
                        one, tx, ty);
 }
 
 // dK and dV: block = one key tile, the ones with the most query tiles first; sweeps the query tiles.
-template <typename T, int DP, int R>
-__global__ void __launch_bounds__(Tile<DP, R>::kThreads, DP <= 64 ? 2 : 1)  // (wide heads: shared memory takes one block)
+template <typename T, int DP>
+__global__ void __launch_bounds__(Tile<DP>::kThreads, DP <= 64 ? 2 : 1)  // (wide heads: shared memory takes one block)
 attn_dkv_simt_kernel(const BwdArgs<T> a) {
   grid_dep_sync();
-  using TT = Tile<DP, R>;
+  using TT = Tile<DP>;
   extern __shared__ __align__(16) float smem[];
   float* q_s = smem;
   float* g_s = q_s + TT::kWords;
@@ -559,11 +560,11 @@ attn_dkv_simt_kernel(const BwdArgs<T> a) {
   const int kt = static_cast<int>(blockIdx.x / nbh);
   const int64_t bh = blockIdx.x % nbh, b = bh / a.sh.heads, h = bh % a.sh.heads;
   const int64_t j0 = static_cast<int64_t>(kt) * kB, o_off = b * a.sh.o_strides[0] + h * a.sh.o_strides[1];
-  load_tile<T, DP, R>(k_s, a.k + b * a.sh.k_strides[0] + h * a.sh.k_strides[1], a.sh.k_strides[2], j0, S, D, a.vec);
-  load_tile<T, DP, R>(v_s, a.v + b * a.sh.v_strides[0] + h * a.sh.v_strides[1], a.sh.v_strides[2], j0, S, D, a.vec);
-  float dk[R][TT::kCols], dv[R][TT::kCols], one[R];
+  load_tile<T, DP>(k_s, a.k + b * a.sh.k_strides[0] + h * a.sh.k_strides[1], a.sh.k_strides[2], j0, S, D, a.vec);
+  load_tile<T, DP>(v_s, a.v + b * a.sh.v_strides[0] + h * a.sh.v_strides[1], a.sh.v_strides[2], j0, S, D, a.vec);
+  float dk[kR][TT::kCols], dv[kR][TT::kCols], one[kR];
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
+  for (int r = 0; r < kR; ++r) {
     one[r] = 1.f;
 #pragma unroll
     for (int c = 0; c < TT::kCols; ++c) dk[r][c] = dv[r][c] = 0.f;
@@ -577,35 +578,35 @@ attn_dkv_simt_kernel(const BwdArgs<T> a) {
       if (!__syncthreads_or(reach)) continue;
     }
     const bool odd_q =
-        load_tile<T, DP, R>(q_s, a.q + b * a.sh.q_strides[0] + h * a.sh.q_strides[1], a.sh.q_strides[2], r0, S, D, a.vec);
+        load_tile<T, DP>(q_s, a.q + b * a.sh.q_strides[0] + h * a.sh.q_strides[1], a.sh.q_strides[2], r0, S, D, a.vec);
     const bool odd_g =
-        load_tile_delta<T, DP, R>(g_s, rc.delta, a.d_o + o_off, a.o + o_off, a.sh.o_strides[2], r0, S, D, a.vec);
+        load_tile_delta<T, DP>(g_s, rc.delta, a.d_o + o_off, a.o + o_off, a.sh.o_strides[2], r0, S, D, a.vec);
     if (drop) draw_flags(flags, dr, bh, S, r0, j0, TT::kThreads);
     const bool masked = __syncthreads_or(odd_q || odd_g);
-    float s[R][4], dp[R][4];
-    mul_nt<DP, R>(s, q_s, k_s, tx, ty);
-    mul_nt<DP, R>(dp, g_s, v_s, tx, ty);
-    p_and_ds<T, R>(s, dp, rc, flags, drop, a, bh, r0, j0, tx, ty);
+    float s[kR][4], dp[kR][4];
+    mul_nt<DP>(s, q_s, k_s, tx, ty);
+    mul_nt<DP>(dp, g_s, v_s, tx, ty);
+    p_and_ds<T>(s, dp, rc, flags, drop, a, bh, r0, j0, tx, ty);
 #pragma unroll
-    for (int r = 0; r < R; ++r)
+    for (int r = 0; r < kR; ++r)
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        p_s[(ty * R + r) * kPS + tx + 16 * c] = s[r][c];
-        ds_s[(ty * R + r) * kPS + tx + 16 * c] = dp[r][c];
+        p_s[(ty * kR + r) * kPS + tx + 16 * c] = s[r][c];
+        ds_s[(ty * kR + r) * kPS + tx + 16 * c] = dp[r][c];
       }
     __syncthreads();
     if (!masked) {
-      mul_tn<DP, R>(dv, p_s, g_s, tx, ty);
-      mul_tn<DP, R>(dk, ds_s, q_s, tx, ty);
+      mul_tn<DP>(dv, p_s, g_s, tx, ty);
+      mul_tn<DP>(dk, ds_s, q_s, tx, ty);
     } else {
-      const auto on = [&](int q, int r) { return j0 + ty * R + r <= r0 + q && j0 + ty * R + r >= rc.ks[q]; };
-      mul_tn_masked<DP, R>(dv, p_s, g_s, tx, ty, on);
-      mul_tn_masked<DP, R>(dk, ds_s, q_s, tx, ty, on);
+      const auto on = [&](int q, int r) { return j0 + ty * kR + r <= r0 + q && j0 + ty * kR + r >= rc.ks[q]; };
+      mul_tn_masked<DP>(dv, p_s, g_s, tx, ty, on);
+      mul_tn_masked<DP>(dk, ds_s, q_s, tx, ty, on);
     }
   }
-  store_rows<T, DP, R>(a.dv + b * a.dsh.v_strides[0] + h * a.dsh.v_strides[1], a.dsh.v_strides[2], j0, S, D, a.vec, dv,
+  store_rows<T, DP>(a.dv + b * a.dsh.v_strides[0] + h * a.dsh.v_strides[1], a.dsh.v_strides[2], j0, S, D, a.vec, dv,
                        one, tx, ty);
-  store_rows<T, DP, R>(a.dk + b * a.dsh.k_strides[0] + h * a.dsh.k_strides[1], a.dsh.k_strides[2], j0, S, D, a.vec, dk,
+  store_rows<T, DP>(a.dk + b * a.dsh.k_strides[0] + h * a.dsh.k_strides[1], a.dsh.k_strides[2], j0, S, D, a.vec, dk,
                        one, tx, ty);
 }
 
@@ -636,20 +637,20 @@ int launch_tiles(void (*kern)(const Args), int threads, size_t smem, const Args&
 
 constexpr size_t kFlagBytes = kB * kFlagStride;
 
-template <typename T, int DP, int R>
+template <typename T, int DP>
 int run_fwd(const FwdArgs<T>& a, cudaStream_t st) {
-  using TT = Tile<DP, R>;
+  using TT = Tile<DP>;
   const size_t k_words = TT::kWords > kB * kPS ? TT::kWords : kB * kPS;
-  return launch_tiles(attn_fwd_simt_kernel<T, DP, R>, TT::kThreads, (2 * TT::kWords + k_words) * 4 + kFlagBytes, a, st);
+  return launch_tiles(attn_fwd_simt_kernel<T, DP>, TT::kThreads, (2 * TT::kWords + k_words) * 4 + kFlagBytes, a, st);
 }
 
-template <typename T, int DP, int R>
+template <typename T, int DP>
 int run_bwd(const BwdArgs<T>& a, cudaStream_t st) {
-  using TT = Tile<DP, R>;
+  using TT = Tile<DP>;
   const size_t tiles = 4 * TT::kWords * 4 + kFlagBytes, p = kB * kPS * 4;
-  const int rc = launch_tiles(attn_dq_simt_kernel<T, DP, R>, TT::kThreads, tiles + p, a, st);
+  const int rc = launch_tiles(attn_dq_simt_kernel<T, DP>, TT::kThreads, tiles + p, a, st);
   if (rc != PTJ_OK) return rc;
-  return launch_tiles(attn_dkv_simt_kernel<T, DP, R>, TT::kThreads, tiles + 2 * p, a, st);
+  return launch_tiles(attn_dkv_simt_kernel<T, DP>, TT::kThreads, tiles + 2 * p, a, st);
 }
 
 template <typename T>
@@ -659,9 +660,9 @@ int fwd_typed(const void* q, const void* k, const void* v, void* o, float* row_m
   const FwdArgs<T> a{static_cast<const T*>(q), static_cast<const T*>(k), static_cast<const T*>(v), static_cast<T*>(o),
                      row_max, row_sum, row_kstart, sh, 1.f / sqrtf(static_cast<float>(sh.d_head)),
                      static_cast<int>(ceil_div(sh.seq, kB)), rows_vectorise<T>(sh, ptrs, 4), dr};
-  if (sh.d_head <= 32) return run_fwd<T, 32, 4>(a, st);
-  if (sh.d_head <= 64) return run_fwd<T, 64, 4>(a, st);
-  return run_fwd<T, 128, 4>(a, st);
+  if (sh.d_head <= 32) return run_fwd<T, 32>(a, st);
+  if (sh.d_head <= 64) return run_fwd<T, 64>(a, st);
+  return run_fwd<T, 128>(a, st);
 }
 
 template <typename T>
@@ -674,9 +675,9 @@ int bwd_typed(const void* d_o, const void* q, const void* k, const void* v, cons
                      static_cast<T*>(dk), static_cast<T*>(dv), row_kstart, sh, dsh,
                      1.f / sqrtf(static_cast<float>(sh.d_head)), static_cast<int>(ceil_div(sh.seq, kB)),
                      rows_vectorise<T>(sh, ptrs, 8) && rows_vectorise<T>(dsh, ptrs, 0), dr};
-  if (sh.d_head <= 32) return run_bwd<T, 32, 4>(a, st);
-  if (sh.d_head <= 64) return run_bwd<T, 64, 4>(a, st);
-  return run_bwd<T, 128, 4>(a, st);
+  if (sh.d_head <= 32) return run_bwd<T, 32>(a, st);
+  if (sh.d_head <= 64) return run_bwd<T, 64>(a, st);
+  return run_bwd<T, 128>(a, st);
 }
 
 }  // namespace

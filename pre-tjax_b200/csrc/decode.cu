@@ -43,7 +43,6 @@ struct DecodeParams {
   float emb_scale, keep;       // sqrt(D); what evaluation multiplies every dropout site by
   Step step[kSteps];
   int act_ld;                  // floats of one sequence's activations in shared memory
-  int max_units;
   float *x, *q, *attn, *h, *kv;
   float* best;                 // [blocks][B] block maxima
   int* best_arg;
@@ -56,9 +55,6 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool v
   const int n = valid ? 16 : 0;  // 0: the destination is filled with zeros
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // row pairs [first, first + n) of a step that this block owns
 struct Share {
@@ -460,7 +456,7 @@ decode_kernel(const __grid_constant__ DecodeParams p) {
       for (int k = 0; k < NB; ++k)
         if (k == b) mine[k] = better(mine[k], c);
     });
-    // (a row without any value above -inf keeps the index 0, as the row arg-max kernel does)
+    // (a row without any value above -inf takes the index 0, as torch.argmax does)
     auto warp_best = [&](Best v) {
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1)
@@ -549,7 +545,6 @@ bool make_plan(int64_t B, int64_t V, int64_t D, int64_t L, int64_t H, int64_t F,
   if (part < static_cast<size_t>(2 * kThreads / lpk)) part = 2 * kThreads / lpk;
   if (ld * out.nb < red) ld = static_cast<int>(ceil_div(ceil_div(red, out.nb), 4) * 4);
   p.act_ld = ld;
-  p.max_units = units;
   const size_t fixed = (static_cast<size_t>(ld) * out.nb + part) * 4 + static_cast<size_t>(L) * kLayerTensors * 8;
   out.depth = 0;
   for (int d : kDepths) {

@@ -127,11 +127,6 @@ split_planes_kernel(const SplitSrc s0, const SplitSrc s1, int* __restrict__ flag
 }
 
 // ---- product --------------------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
 
 __device__ __forceinline__ void epilogue_warps_sync() { asm volatile("barrier.sync 1, %0;" ::"n"(kEpilogueWarps * 32) : "memory"); }
 

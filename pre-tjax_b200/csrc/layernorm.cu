@@ -292,11 +292,6 @@ ln_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const float* __
 constexpr int kRing = 4;
 __host__ __device__ constexpr int ln_rows_groups(int W) { return W >= 7 ? 1 : 12 / W; }
 
-__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
 __device__ __forceinline__ uint64_t bf2_to_f2(uint32_t w) {  // two packed bf16 -> two floats
   return f2_pack(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
 }
@@ -310,9 +305,6 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) {
                "l"(gsrc)
                : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // Sum of one value per warp over the W warps of a row group (every thread gets the total; fixed order). `slot` is this
 // exchange's own W floats; a slot is reused one row later, with two other exchanges' barriers in between.

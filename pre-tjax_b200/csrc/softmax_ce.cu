@@ -267,11 +267,6 @@ __device__ __forceinline__ float ex2_approx(float x) {
 __device__ __forceinline__ uint64_t bf2_as_f2(uint32_t w) {
   return f2_pack(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
 }
-__device__ __forceinline__ uint64_t f2_add2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
 
 constexpr float kLog2e = 1.4426950408889634f;
 
@@ -316,7 +311,7 @@ struct Shifted {
   __device__ __forceinline__ explicit Shifted(float m)
       : c(EXACT ? -m : -m * kLog2e), c2(f2_pack(c, c)), l2e2(f2_pack(kLog2e, kLog2e)) {}
   __device__ __forceinline__ uint64_t operator()(uint64_t x2) const {
-    return EXACT ? f2_mul(f2_add2(x2, c2), l2e2) : f2_fma(x2, l2e2, c2);
+    return EXACT ? f2_mul(f2_add(x2, c2), l2e2) : f2_fma(x2, l2e2, c2);
   }
   __device__ __forceinline__ float operator()(float x) const { return EXACT ? (x + c) * kLog2e : fmaf(x, kLog2e, c); }
 };
@@ -444,7 +439,7 @@ log_softmax_fwd_bf16_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* 
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         float y0, y1;
-        f2_unpack(f2_add2(bf2_as_f2(w[q]), ns2), y0, y1);
+        f2_unpack(f2_add(bf2_as_f2(w[q]), ns2), y0, y1);
         __nv_bfloat162 h = __floats2bfloat162_rn(y0, y1);
         o[q] = *reinterpret_cast<uint32_t*>(&h);
       }
@@ -475,11 +470,11 @@ log_softmax_bwd_bf16_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfl
     uint64_t g0 = 0ull, g1 = 0ull;  // two packed +0.0f each
     for (int i = threadIdx.x; i < nvec; i += kCeThreads) {
       const uint4 a = gv[i];
-      g0 = f2_add2(g0, f2_add2(bf2_as_f2(a.x), bf2_as_f2(a.y)));
-      g1 = f2_add2(g1, f2_add2(bf2_as_f2(a.z), bf2_as_f2(a.w)));
+      g0 = f2_add(g0, f2_add(bf2_as_f2(a.x), bf2_as_f2(a.y)));
+      g1 = f2_add(g1, f2_add(bf2_as_f2(a.z), bf2_as_f2(a.w)));
     }
     float ga, gb;
-    f2_unpack(f2_add2(g0, g1), ga, gb);
+    f2_unpack(f2_add(g0, g1), ga, gb);
     float gs = ga + gb;
     for (int c = tail0 + threadIdx.x; c < cols; c += kCeThreads) gs += __bfloat162float(gr[c]);
     const float nk = -block_sum(gs, red) / s;

@@ -1,5 +1,5 @@
 """Greedy decoding with kept keys and values against the same loop over whole forward passes, at sizes that fill no chunk,
-part, block share or lane group of the kernel."""
+part, block share or lane group of the kernel, and the alignments that its entry point takes."""
 import pytest
 import torch
 
@@ -39,7 +39,8 @@ def test_decode_matches_whole_forward(B, V, D, L, H, F, S):
     # terms in another order differ by about 1e-6 of the logits' scale; a token may win only within ten times that.
     ids = got.long()
     ids[:, 0] = start
-    assert torch.equal(ids, ids[:1].expand_as(ids))  # every sequence starts alike
+    # every sequence starts alike, so all are equal: a mix-up between sequences could not show, to a caller neither
+    assert torch.equal(ids, ids[:1].expand_as(ids))
     logits = ev.t_gpt2_forward(params, ids[:2], None, None, False).double()
     top = logits[:, :-1].max(dim=-1).values
     mine = logits[:, :-1].gather(2, ids[:2, 1:, None]).squeeze(2)

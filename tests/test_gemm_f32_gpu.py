@@ -58,8 +58,7 @@ def test_layouts_edges_and_k_split(ops, a_k, b_k, M, N, K, pad):
                                  N, int(a_k), int(b_k), 0, 0, 0, None, 1, 0, 0, torch.cuda.current_stream().cuda_stream), "ptj_gemm")
     rms = lambda x: float((x.double() - ref).pow(2).mean().sqrt())
     print("rms error / rms value: tensor cores %.2e, FMA %.2e" % (rms(out) / float(ref.pow(2).mean().sqrt()), rms(fma) / float(ref.pow(2).mean().sqrt())))
-    # short sums: both errors are a few roundings of the result, hence the half-ulp term
-    assert rms(out) <= 1.5 * rms(fma) + 2.0 ** -24 * float(ref.pow(2).mean().sqrt())
+    assert rms(out) <= rms(fma)  # measured: 0.7 of it at K = 72, 0.1 at K = 4096
     again = torch.empty_like(out)
     ops.gemm(sa, sb, a_kmajor=a_k, b_kmajor=b_k, M=M, N=N, K=K, lda=sa.shape[1], ldb=sb.shape[1], out=again)
     assert torch.equal(out, again)
@@ -92,7 +91,8 @@ def test_epilogues_match_the_fma_kernel(ops, M, N, K):
 
 
 def test_extreme_values(ops):
-    """The largest finite float32, subnormal parts and zeros survive the split; a NaN stays where it belongs."""
+    """The largest finite float32 (by fused multiply-adds), a small number's last bit and zeros come through; a NaN stays where
+    it belongs."""
     M = N = 256
     A, B = torch.zeros(M, 256, device="cuda"), torch.zeros(N, 256, device="cuda")
     A[0, 0], B[0, 0] = torch.finfo(torch.float32).max, 1.0
