@@ -66,8 +66,8 @@ def log_probs(params, y, y_mask=None, y_indices=None):
 def predict(params, y_mask, y_indices, sample_len, start_tok, end_tok):
     """Greedy decoding of ``y_mask.shape[0]`` sequences (an int batch size is accepted too): int64[B, sample_len-1].
     ``sample_len`` must equal the model's sequence length because the positional table is added without slicing.
-    float32 weights: one launch decodes all positions with the keys and values of earlier ones kept, as the causal mask
-    allows (operators.decode_greedy). Otherwise, bf16 weights above all, every step runs the full forward over the
+    float32 weights: one launch per group of up to eight sequences decodes all positions with the keys and values of
+    earlier ones kept, as the causal mask allows (operators.decode_greedy). Otherwise, bf16 weights above all, every step runs the full forward over the
     ``sample_len`` positions, as the reference does, and takes the arg-max of position ``step``: there the activations
     are rounded to bf16 between the launches, and which token wins depends on that."""
     B = int(y_mask) if isinstance(y_mask, int) else y_mask.shape[0]
