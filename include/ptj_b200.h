@@ -264,9 +264,10 @@ int ptj_gemm_grouped2(const ptj_gemm_problem* p0, const ptj_gemm_problem* p1, in
  * (d_head contiguous), so both the reference's [B,H,3,N,D] tensor and a fused [B*N, H*3*D] projection
  * output are addressed without copies. row_max / row_sum are float[batch*heads*seq] (the reference's acts0 /
  * acts1: running maximum of the scaled scores and sum of exp(score - max)).
- *   dtype PTJ_BF16 with d_head == 64 and seq % 128 == 0 (16-byte aligned rows) runs the tcgen05 kernels, which round
- *   probabilities and score gradients to bf16 before they are multiplied; everything else runs the SIMT kernels, float32
- *   from the operands to the stored result.
+ *   dtype PTJ_BF16 with d_head a multiple of 8 from 16 to 128 and 16-byte aligned rows runs the tcgen05 kernels. With
+ *   d_head == 64 and seq % 128 == 0 they round probabilities and score gradients to bf16 before they are multiplied;
+ *   otherwise they multiply them in three bf16 parts that hold all 24 bits of a float32. Everything else runs the SIMT
+ *   kernels, float32 from the operands to the stored result.
  * Backward recomputes the probabilities; it is deterministic (no atomics).
  *
  * row_kstart (optional, int32[batch, seq]): the first key each query row may attend to, so that row i attends keys
@@ -276,9 +277,9 @@ int ptj_gemm_grouped2(const ptj_gemm_problem* p0, const ptj_gemm_problem* p1, in
  * padding row gets row_kstart > i and attends nothing (zero output row, row_max 0, row_sum 1, zero gradients).
  * NULL = plain causal attention. Forward and backward of one call must be given the same array.
  *
- * A row reads only the keys it attends: on the SIMT kernels an infinity or a NaN in a row of Q, K, V or d_o reaches no
- * output that does not attend that row. The tcgen05 kernels multiply masked entries by exact zeros, so there it also
- * reaches the other rows of its 128-row tile.
+ * A row reads only the keys it attends: an infinity or a NaN in a row of Q, K, V or d_o reaches no output that does not
+ * attend that row, except with bf16 probabilities (d_head == 64 and seq % 128 == 0), where masked entries are multiplied by
+ * exact zeros and it also reaches the other rows of its 128-row tile.
  */
 typedef struct {
   int64_t batch, heads, seq, d_head;
@@ -300,7 +301,8 @@ int ptj_attn_fwd(const void* q, const void* k, const void* v, void* o, float* ro
  * workspace: ptj_attn_bwd_workspace_bytes(shape, dtype) bytes of device memory, 16-byte aligned, contents
  * irrelevant before and after the call (the tensor-core path keeps each KV tile's share of dQ there in fp32 and sums
  * the shares in a fixed order instead of the reference's tl.atomic_add, model_triton.py:938; 0 bytes = not needed,
- * NULL allowed). Too small a workspace returns PTJ_ERR_WORKSPACE. */
+ * NULL allowed). Without one, or with too small a one, a shape with bf16 probabilities returns PTJ_ERR_WORKSPACE and any
+ * other runs on the SIMT kernels. */
 size_t ptj_attn_bwd_workspace_bytes(const ptj_attn_shape* shape, int dtype);
 int ptj_attn_bwd(const void* d_o, const void* q, const void* k, const void* v, const void* o,
                  const float* row_max, const float* row_sum, void* dq, void* dk, void* dv,

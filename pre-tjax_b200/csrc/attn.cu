@@ -1,5 +1,5 @@
-// C entry points of causal attention: validate, then route to the tcgen05 kernels (bf16, d_head 64, seq % 128 == 0)
-// or to the exact-fp32 CUDA-core kernels (everything else).
+// C entry points of causal attention: validate, then route to the tcgen05 kernels (bf16, d_head a multiple of 8 from 16 to
+// 128, rows on 16-byte boundaries) or to the float32 CUDA-core kernels (everything else).
 #include "attn_common.cuh"
 
 using namespace ptj;
@@ -48,9 +48,11 @@ extern "C" int ptj_attn_fwd(const void* q, const void* k, const void* v, void* o
   return attn_fwd_simt(q, k, v, o, row_max, row_sum, row_kstart, *shape, dr, dtype, st);
 }
 
+// Beyond 4 GiB of dQ shares the shapes that the general kernels can take (no workspace) stay there.
 static bool bwd_uses_tc(const ptj_attn_shape* shape, int dtype) {
   const void* none[1] = {nullptr};
-  return dtype == PTJ_BF16 && attn_tc_supported(*shape, none, 0);
+  return dtype == PTJ_BF16 && attn_tc_supported(*shape, none, 0) &&
+         (attn_bf16_probabilities(*shape) || attn_bwd_tc_workspace_bytes(*shape) <= (1ull << 32));
 }
 
 extern "C" size_t ptj_attn_bwd_workspace_bytes(const ptj_attn_shape* shape, int dtype) {
@@ -73,8 +75,11 @@ extern "C" int ptj_attn_bwd(const void* d_o, const void* q, const void* k, const
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const AttnDropout dr = make_dropout(p, train, seed, stream_id);
   const void* ptrs[8] = {d_o, q, k, v, o, dq, dk, dv};
-  if (dtype == PTJ_BF16 && attn_tc_supported(*shape, ptrs, 8) && attn_tc_supported(*dshape, ptrs, 0))
+  // (without a workspace the float32-probability shapes run on the general kernels)
+  if (bwd_uses_tc(shape, dtype) && attn_tc_supported(*shape, ptrs, 8) && attn_tc_supported(*dshape, ptrs, 0) &&
+      (attn_bf16_probabilities(*shape) ||
+       (aligned16(workspace) && workspace != nullptr && workspace_bytes >= attn_bwd_tc_workspace_bytes(*shape))))
     return attn_bwd_tc(d_o, q, k, v, o, row_max, row_sum, dq, dk, dv, *shape, *dshape, dr, keep_bits, row_kstart,
                        workspace, workspace_bytes, st);
-  return attn_bwd_simt(d_o, q, k, v, o, row_max, row_sum, dq, dk, dv, row_kstart, *shape, *dshape, dr, dtype, st);
+  return attn_bwd_simt(d_o, q, k, v, o, row_max, row_sum, dq, dk, dv, row_kstart, *shape, *dshape, dr, dtype, nullptr, st);
 }

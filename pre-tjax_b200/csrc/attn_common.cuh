@@ -24,11 +24,17 @@ struct AttnDropout {
 // attends keys [row_kstart[b, i], i] (empty when row_kstart > i: zero output row, statistics (0, 1)). NULL = 0.
 int attn_fwd_simt(const void* q, const void* k, const void* v, void* o, float* row_max, float* row_sum,
                   const int32_t* row_kstart, const ptj_attn_shape& sh, const AttnDropout& dr, int dtype, cudaStream_t st);
+// patch (optional, device word): the results are in place already; nothing is done unless the word is not zero, and then
+// only elements that are not finite (computed, or in place) are stored.
 int attn_bwd_simt(const void* d_o, const void* q, const void* k, const void* v, const void* o, const float* row_max,
                   const float* row_sum, void* dq, void* dk, void* dv, const int32_t* row_kstart,
-                  const ptj_attn_shape& sh, const ptj_attn_shape& dsh, const AttnDropout& dr, int dtype, cudaStream_t st);
+                  const ptj_attn_shape& sh, const ptj_attn_shape& dsh, const AttnDropout& dr, int dtype,
+                  const unsigned int* patch, cudaStream_t st);
 
-// tcgen05 kernels: bf16, d_head == 64, seq % 128 == 0, 16-byte aligned strides.
+// tcgen05 kernels: bf16, d_head a multiple of 8 from 16 to 128, any seq, 16-byte aligned strides.
+// attn_bf16_probabilities: d_head == 64 and seq % 128 == 0: probabilities and score gradients are rounded to bf16 before they
+// are multiplied; the other shapes multiply them in three bf16 parts (24 bits), as the general kernels do in float32.
+inline bool attn_bf16_probabilities(const ptj_attn_shape& sh) { return sh.d_head == 64 && sh.seq % 128 == 0; }
 bool attn_tc_supported(const ptj_attn_shape& sh, const void* const* ptrs, int nptrs);
 // keep_bits (optional, both directions): the call's dropout keep flags from attn_keep_bits_tc; NULL = the kernels draw
 // the same flags themselves.

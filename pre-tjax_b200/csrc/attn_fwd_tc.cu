@@ -1,22 +1,26 @@
-// Causal flash attention forward on tcgen05 tensor cores (bf16 in, fp32 accumulate), d_head = 64, seq % 128 == 0.
+// Causal flash attention forward on tcgen05 tensor cores (bf16 in, fp32 accumulate), heads up to 128 wide, any seq.
 // Semantics: model_triton.py:608-611 / 510-517: softmax of the causally masked scaled scores, dropout on the
 // probabilities (no rescale), times V; the row maximum and row sum of exponentials are saved (acts0 / acts1, :699-700).
 //
-// Persistent, warp-specialised thread block (one per SM, 384 threads):
-//   warp 0      one thread issues the TMA copies: Q of a work item (2 buffers), K tiles (3-deep ring), V tiles (2-deep
-//               ring), K and V as independent sequences
-//   warp 1      issues the score MMAs S_g = Q K_g^T, up to three tiles ahead of the softmax
-//   warps 2, 3  issue the output MMAs O += P_g V_g, one warp per softmax group
-//   warps 4..7 / 8..11  two softmax groups; group x takes the tiles g of the block's tile stream with g % 2 == x, so
-//               one group's exponentials overlap the other group's tensor-memory loads, barriers and bookkeeping.
-//               Thread t of a group owns row t of the 128 x 128 score tile (tensor-memory lane t): no shuffles. Each
-//               group accumulates its own output rows in tensor memory (the P V product adds onto them) with its
-//               own reference exponent and row sums; when the item ends, the group that did not get the last tile
-//               hands its state over through shared memory and the other one merges the two (log-sum-exp merge in
-//               a fixed order) and writes the rows out.
+// Persistent, warp-specialised thread block (one per SM; 16 softmax warps for heads up to 64, 8 beyond):
+//   warp 0      one thread issues the TMA copies: Q of a work item, K tiles, V tiles, as independent sequences
+//   warp 1      issues the score MMAs S = Q K^T, up to two tiles ahead of the softmax
+//   warp 2      issues the output MMAs O_x += P[:, block c] V[block c, :] for the NC column blocks of a tile
+//   warps 4..   softmax, in G groups that take the tiles of the block's stream in turn, so that one group's exponentials
+//               overlap the other's loads, stores and barriers. Warp (quarter, c) of a group owns rows 32 quarter .. + 31
+//               (tensor-memory lane = row, one row per thread) and the 128 / NC columns of block c of the group's tiles. Every
+//               (group, block) has its own reference exponent, row sums and output accumulator, so the warps of a row never
+//               meet before the item ends; then the group that got the last tile merges the G NC states of each row
+//               (log-sum-exp merge in a fixed order) and writes it.
+// PARTS: what a probability is multiplied as. 1: rounded to bf16. 3: split exactly into three bf16 parts, three products
+// each, which keeps float32 probabilities; the operands of S are bf16 as they are.
 // Work items = (query tile, batch*head), heaviest first, dealt to the blocks in boustrophedon order; all tiles of a
 // block's items form one stream, so the next item's first tiles overlap the tail of the current one.
-// Tensor memory: three S buffers at columns [0,384), one output accumulator per group at [384,512).
+// Tensor memory: two S buffers at columns [0,256), the G NC accumulators at [256,512).
+// Bound by the latencies a softmax warp meets in a row on its tile (tensor-memory loads, barriers, exponentials), not by a
+// pipe. Measured, dropout 0.1, flags drawn here: [4, 12, 500, 64] 22 us (the float32 FMA kernels 95), [8, 12, 1024, 32] 111
+// (338), [8, 12, 1024, 128] 136 (837); whole tiles of 64-wide heads, [8, 12, 1024, 64], flags given: 42 us, as a thread per
+// row of 128 columns took before (41); all 16 warps on one tile, 32 columns a thread: 65.
 #include "attn_tc_dev.cuh"
 
 namespace ptj {
@@ -24,16 +28,35 @@ namespace {
 
 using namespace attn_tc;
 
-constexpr int kThreads = 384;  // warps 0-3: TMA and MMA issue; warps 4-7 and 8-11: the softmax groups
-constexpr int kKStages = 3, kVStages = 2, kSBufs = 3;
-constexpr int kOffK = 2 * kTileBytes;                     // after Q[2]
-constexpr int kOffV = kOffK + kKStages * kTileBytes;
-constexpr int kOffP = kOffV + kVStages * kTileBytes;     // P[2 groups][2 sub-tiles]
-constexpr int kOffDump = kOffP + 4 * kTileBytes;          // float[64 + 3][128]: hand-over of one group's state
-constexpr int kOffBars = kOffDump + (DH + 3) * T * 4;
-constexpr int kNumBars = 4 + 2 * kKStages + 2 * kVStages + 2 * kSBufs + 6 + 2;
-constexpr int kSmemBytes = kOffBars + kNumBars * 8 + 16 + 80 + 4 * 32 + 1024;  // (+ 32 first-tile entries, VARLEN)
+template <int DHP, int PARTS>
+struct Cfg {
+  static constexpr int kG = DHP == 64 ? 2 : 1;     // groups
+  static constexpr int kNC = 2;                    // column blocks of a tile
+  static constexpr int kCW = T / kNC;              // columns of a block
+  static constexpr int kGroupWarps = 4 * kNC;
+  static constexpr int kWarps = kG * kGroupWarps;  // softmax warps
+  static constexpr int kAcc = kG * kNC;            // accumulators
+  static constexpr int kThreads = 128 + 32 * kWarps;
+  static constexpr int kTB = T * DHP * 2;          // one operand tile
+  // shared memory, in tiles: what fits beside the probabilities
+  static constexpr int kQ = DHP == 64 ? 2 : 1;
+  static constexpr int kK = DHP == 64 ? (PARTS == 1 ? 3 : 2) : 1;
+  static constexpr int kV = DHP == 64 ? (PARTS == 1 ? 4 : 3) : 1;
+  static constexpr int kP = PARTS == 1 ? 2 : 1;    // probability buffers, PARTS tiles each
+  static constexpr int kOffK = kQ * kTB;
+  static constexpr int kOffV = kOffK + kK * kTB;
+  static constexpr int kOffP = kOffV + kV * kTB;
+  static constexpr int kOffStats = kOffP + kP * PARTS * kPBytes;  // float [kAcc][3][128]
+  static constexpr int kOffBars = kOffStats + kAcc * 3 * T * 4;
+  static constexpr int kNumBars = 2 * (kQ + kK + kV) + 4 + kG + kP + 2;
+  static constexpr int kSmemBytes = kOffBars + kNumBars * 8 + 16 + 80 + 4 * 32 + 1024;  // (+ 32 first-tile entries)
+  static_assert(kSmemBytes <= 227 * 1024, "shared memory of a block");
+  // of 96 (640 threads) or 168 (384 threads) a thread at launch
+  static constexpr int kRegsIO = DHP == 64 ? 56 : 40, kRegsSoftmax = DHP == 64 ? 104 : 232;
+};
+constexpr int kSBufs = 2;
 constexpr int kTmemCols = 512;
+constexpr uint32_t kColO = kSBufs * T;
 
 struct Sched {
   int total, rounds, nq, BH;
@@ -41,7 +64,7 @@ struct Sched {
 };
 
 // Position in the stream of (item, kv tile) pairs of one thread block; every role walks the same stream.
-// first_tile (VARLEN): per round of this block, the first KV tile its item needs (keys before the first key of every
+// first_tile (row_kstart): per round of this block, the first KV tile its item needs (keys before the first key of every
 // row of the query tile are masked anyway: those tiles are skipped); nullptr = every item starts at tile 0.
 constexpr int kMaxRoundsTabled = 32;
 struct Cursor {
@@ -76,56 +99,92 @@ struct Cursor {
   }
 };
 
+// An item one of whose V tiles held an infinity or a NaN (replaced by zero before it was multiplied): the products of a
+// row's attended probabilities with those elements, columns [col0, col0 + 16). Slow and rare.
+__device__ __noinline__ void add_nonfinite_v(float (&o)[16], const RowView& q, const RowView& k, const RowView& v, const AttnParams& p,
+                                             const uint32_t* rk_s, int mode, int bh, int q_row, int first_key, int col0,
+                                             float m_true) {
+  const int b = bh / p.H, h = bh % p.H;
+  const __nv_bfloat16* qr = q.row(b, h, q_row);
+  for (int j = max(first_key, 0); j <= q_row; ++j) {
+    const __nv_bfloat16* vr = v.row(b, h, j);
+    uint32_t bad = 0u;
+    for (int i = 0; i < 16 && col0 + i < p.D; ++i)
+      if (!isfinite(__bfloat162float(vr[col0 + i]))) bad |= 1u << i;
+    if (bad == 0u) continue;
+    const __nv_bfloat16* kr = k.row(b, h, j);
+    float s = 0.f;
+    for (int d = 0; d < p.D; ++d) s = fmaf(__bfloat162float(qr[d]), __bfloat162float(kr[d]), s);
+    float w = ex2_approx((s - m_true) * p.scale_log2);
+    if (mode != 0) {
+      const uint64_t idx = (static_cast<uint64_t>(bh) * p.S + q_row) * p.S + j;
+      uint32_t keep;
+      if (mode == 1) {
+        keep = keep_word(rk_s, idx, p.dr.stream_id, p.dr.thr16 << 16) & 1u;
+      } else {
+        const int qt = q_row / T, kt = j / T;
+        const uint32_t* words = reinterpret_cast<const uint32_t*>(p.keep_bits);
+        const int64_t tile = static_cast<int64_t>(bh) * (p.nq * (p.nq + 1) / 2) + qt * (qt + 1) / 2 + kt;
+        keep = (__ldg(words + (tile * T + q_row % T) * 4 + (j % T) / 32) >> (j & 31)) & 1u;
+      }
+      if (keep == 0u) w = 0.f;
+    }
+    for (int i = 0; i < 16; ++i)
+      if ((bad >> i) & 1u) o[i] += w * __bfloat162float(vr[col0 + i]);
+  }
+}
+
+struct FwdViews {
+  RowView q, k, v, o;
+};
+
 // MODE 0: no dropout mask; 1: Philox drawn in the kernel; 2: precomputed keep flags (p.keep_bits).
-// VARLEN: query row i attends keys [p.kstart[b, i], i] only (packed documents / padding, the block-diagonal x causal x
-// padding masks of the reference's collator, tokenized_dataset.py:110-131); a row whose range is empty gets a zero
-// output row and the statistics (row_max, row_sum) = (0, 1). The tile stream is the causal one: keys outside a row's
-// range are masked, whole tiles outside it contribute exact zeros.
-template <int MODE, bool VARLEN>
-__global__ void __launch_bounds__(kThreads, 1)
+// p.kstart (optional): query row i attends keys [p.kstart[b, i], i] only (packed documents / padding, the block-diagonal x
+// causal x padding masks of the reference's collator, tokenized_dataset.py:110-131); a row whose range is empty gets a
+// zero output row and the statistics (row_max, row_sum) = (0, 1).
+template <int DHP, int PARTS, int MODE>
+__global__ void __launch_bounds__(Cfg<DHP, PARTS>::kThreads, 1)
 attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                   const __grid_constant__ CUtensorMap tm_v, const RowView out, float* __restrict__ row_max,
-                   float* __restrict__ row_sum, const AttnParams p, const Sched sched) {
+                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ FwdViews views,
+                   float* __restrict__ row_max, float* __restrict__ row_sum, const __grid_constant__ AttnParams p,
+                   const Sched sched) {
+  using C = Cfg<DHP, PARTS>;
+  constexpr int kTB = C::kTB;
+  constexpr bool kExact = PARTS > 1;  // float32 probabilities, and an element that is not finite reaches what attends it only
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sm = align1024(smem_raw);
   uint8_t* q_s = sm;
-  uint8_t* k_s = sm + kOffK;
-  uint8_t* v_s = sm + kOffV;
-  uint8_t* p_s = sm + kOffP;
-  float* dump = reinterpret_cast<float*>(sm + kOffDump);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sm + kOffBars);
-  uint64_t* q_full = bars;                  // [2]
-  uint64_t* q_empty = bars + 2;             // [2]
-  uint64_t* k_full = bars + 4;              // [kKStages]
-  uint64_t* k_empty = k_full + kKStages;
-  uint64_t* v_full = k_empty + kKStages;    // [kVStages]
-  uint64_t* v_empty = v_full + kVStages;
-  uint64_t* s_full = v_empty + kVStages;    // [kSBufs]
-  uint64_t* s_free = s_full + kSBufs;       // [kSBufs] one arrival per warp of the group that read the tile
-  uint64_t* p_ready = s_free + kSBufs;      // [2] per group, one arrival per warp
-  uint64_t* o_full = p_ready + 2;           // [2] per group
-  uint64_t* o_free = o_full + 2;            // [2] per group, one arrival per warp
-  uint64_t* dump_full = o_free + 2;         // one arrival per warp of the group that hands over
-  uint64_t* dump_free = dump_full + 1;      // one arrival per warp of the group that merges
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(dump_free + 1);
+  uint8_t* k_s = sm + C::kOffK;
+  uint8_t* v_s = sm + C::kOffV;
+  uint8_t* p_s = sm + C::kOffP;
+  float* stats = reinterpret_cast<float*>(sm + C::kOffStats);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sm + C::kOffBars);
+  uint64_t* q_full = bars;                  // [kQ]
+  uint64_t* q_empty = q_full + C::kQ;
+  uint64_t* k_full = q_empty + C::kQ;       // [kK]
+  uint64_t* k_empty = k_full + C::kK;
+  uint64_t* v_full = k_empty + C::kK;       // [kV]
+  uint64_t* v_empty = v_full + C::kV;
+  uint64_t* s_full = v_empty + C::kV;       // [2]
+  uint64_t* o_full = s_full + kSBufs;       // [kG] per group: its tile's output MMAs, and all before, are done
+  uint64_t* s_free = o_full + C::kG;        // [2] one arrival per warp of the tile's group from here on
+  uint64_t* p_ready = s_free + kSBufs;      // [kP]
+  uint64_t* stats_full = p_ready + C::kP;   // the item's row states are in shared memory (all softmax warps)
+  uint64_t* o_free = stats_full + 1;        // the item's accumulators and states have been read
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_free + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  uint32_t* rk_s = tmem_slot + 2;  // Philox round keys (MODE 1)
-  int* first_tab = reinterpret_cast<int*>(rk_s + 20);  // [kMaxRoundsTabled] first KV tile of this block's items (VARLEN)
+  volatile int* bad_v = abort_flag + 1;  // a V tile of this block held an element that is not finite
+  uint32_t* rk_s = tmem_slot + 4;        // Philox round keys (MODE 1)
+  int* first_tab = reinterpret_cast<int*>(rk_s + 20);  // [kMaxRoundsTabled] first KV tile of this block's items
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const AbortCtx ctx{abort_flag, p.fault};
 
   if (tid == 0) {
-    for (int i = 0; i < 4 + 2 * kKStages + 2 * kVStages + kSBufs; ++i) mbar_init(&bars[i], 1);  // TMA / MMA completions
-    for (int i = 0; i < kSBufs; ++i) mbar_init(&s_free[i], 4);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&p_ready[i], 4);
-      mbar_init(&o_full[i], 1);
-      mbar_init(&o_free[i], 4);
-    }
-    mbar_init(dump_full, 4);
-    mbar_init(dump_free, 4);
+    for (uint64_t* b = bars; b < s_free; ++b) mbar_init(b, 1);  // TMA / MMA completions
+    for (uint64_t* b = s_free; b < o_free + 1; ++b) mbar_init(b, b == stats_full ? C::kWarps : C::kGroupWarps);
     *abort_flag = 0;
+    *bad_v = 0;
     fence_barrier_init();
     prefetch_tensormap(&tm_q);
     prefetch_tensormap(&tm_k);
@@ -144,12 +203,12 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     if (tid == 0) philox_round_keys(p.dr.seed, rk_s);
     __syncthreads();
   }
-  // VARLEN: whole KV tiles before the first key of every row of a query tile are skipped. Warp w looks at the item of
-  // round w, w + 12, ...: the smallest first key over the tile's rows that have keys at all (none: only the diagonal
+  // Whole KV tiles before the first key of every row of a query tile are skipped. Warp w looks at the item of round
+  // w, w + warps, ...: the smallest first key over the tile's rows that have keys at all (none: only the diagonal
   // tile is visited, it masks everything).
   const int* first_tile = nullptr;
-  if (VARLEN && sched.rounds <= kMaxRoundsTabled) {
-    for (int n = warp; n < sched.rounds; n += kThreads / 32) {
+  if (p.kstart != nullptr && sched.rounds <= kMaxRoundsTabled) {
+    for (int n = warp; n < sched.rounds; n += C::kThreads / 32) {
       const int pos = (n & 1) ? static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x);
       const int sp = n * static_cast<int>(gridDim.x) + pos;
       int first = 0;
@@ -158,7 +217,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         const int qt = sched.nq - 1 - t, bh = sp - t * sched.BH;
         const int32_t* ks = p.kstart + static_cast<int64_t>(bh / p.H) * p.S + static_cast<int64_t>(qt) * T;
         int lo = 0x7fffffff;
-        for (int r = lane; r < T; r += 32) {
+        for (int r = lane; r < T && qt * T + r < p.S; r += 32) {
           const int k = __ldg(ks + r);
           if (k <= qt * T + r) lo = min(lo, k);  // (k > row: the row has no keys)
         }
@@ -171,8 +230,8 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     first_tile = first_tab;
   }
 
-  // the copy / MMA warps hand most of their registers to the softmax warps (whole groups of four warps switch together)
-  if (warp < 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+  // the copy / MMA warps hand registers to the softmax warps (whole groups of four warps switch together)
+  if (warp < 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kRegsIO));
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer
     // K (with Q at an item's first tile) and V are two independent sequences over the same stream: whichever has a
@@ -187,27 +246,27 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         bool progress = false;
         if (ck.valid) {
           const int b = ck.bh / p.H, h = ck.bh % p.H;
-          const int qb = ck.ord & 1;
-          if (ck.j == ck.j0 && !q_done && mbar_try_wait(&q_empty[qb], ((ck.ord >> 1) & 1) ^ 1u)) {
-            mbar_expect_tx(&q_full[qb], kTileBytes);
-            tma_load_4d(q_s + qb * kTileBytes, &tm_q, &q_full[qb], 0, ck.qt * T, h, b);
+          const int qb = ck.ord % C::kQ;
+          if (ck.j == ck.j0 && !q_done && mbar_try_wait(&q_empty[qb], ((ck.ord / C::kQ) & 1) ^ 1u)) {
+            mbar_expect_tx(&q_full[qb], kTB);
+            load_rows<DHP>(q_s + qb * kTB, &tm_q, &q_full[qb], ck.qt * T, h, b);
             q_done = true;
             progress = true;
           }
-          const int st = ck.g % kKStages;
-          if ((ck.j > ck.j0 || q_done) && mbar_try_wait(&k_empty[st], ((ck.g / kKStages) & 1) ^ 1u)) {
-            mbar_expect_tx(&k_full[st], kTileBytes);
-            tma_load_4d(k_s + st * kTileBytes, &tm_k, &k_full[st], 0, ck.j * T, h, b);
+          const int st = ck.g % C::kK;
+          if ((ck.j > ck.j0 || q_done) && mbar_try_wait(&k_empty[st], ((ck.g / C::kK) & 1) ^ 1u)) {
+            mbar_expect_tx(&k_full[st], kTB);
+            load_rows<DHP>(k_s + st * kTB, &tm_k, &k_full[st], ck.j * T, h, b);
             ck.advance(sched);
             q_done = false;
             progress = true;
           }
         }
         if (cv.valid) {
-          const int st = cv.g % kVStages;
-          if (mbar_try_wait(&v_empty[st], ((cv.g / kVStages) & 1) ^ 1u)) {
-            mbar_expect_tx(&v_full[st], kTileBytes);
-            tma_load_4d(v_s + st * kTileBytes, &tm_v, &v_full[st], 0, cv.j * T, cv.bh % p.H, cv.bh / p.H);
+          const int st = cv.g % C::kV;
+          if (mbar_try_wait(&v_empty[st], ((cv.g / C::kV) & 1) ^ 1u)) {
+            mbar_expect_tx(&v_full[st], kTB);
+            load_rows<DHP>(v_s + st * kTB, &tm_v, &v_full[st], cv.j * T, cv.bh % p.H, cv.bh / p.H);
             cv.advance(sched);
             progress = true;
           }
@@ -225,300 +284,323 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       }
     }
   } else if (warp == 1) {
-    // ---------------------------------------------------------------- MMA issuer, scores: S_g = Q K_g^T
+    // ---------------------------------------------------------------- MMA issuer, scores: S = Q K^T
     // every lane walks the stream and waits (addresses and descriptors stay warp-uniform); an elected lane issues
     constexpr uint32_t idesc_s = idesc_bf16_f32(T, T, false, false);
     Cursor a;
     a.init(sched, first_tile);
     bool ok = true;
     while (a.valid && ok) {
-      const int st = a.g % kKStages;
-      const int qb = a.ord & 1;
+      const int st = a.g % C::kK;
+      const int qb = a.ord % C::kQ;
       const int sb = a.g % kSBufs;
       bool w = true;
-      if (a.j == a.j0) w = mbar_wait(&q_full[qb], (a.ord >> 1) & 1, ctx, 0x1201u);
-      if (w) w = mbar_wait(&k_full[st], (a.g / kKStages) & 1, ctx, 0x1202u);
-      if (w) w = mbar_wait(&s_free[sb], ((a.g / kSBufs) & 1) ^ 1u, ctx, 0x1203u);  // tile g - 3 has been read out
+      if (a.j == a.j0) w = mbar_wait(&q_full[qb], (a.ord / C::kQ) & 1, ctx, 0x1201u);
+      if (w) w = mbar_wait(&k_full[st], (a.g / C::kK) & 1, ctx, 0x1202u);
+      if (w) w = mbar_wait(&s_free[sb], ((a.g / kSBufs) & 1) ^ 1u, ctx, 0x1203u);  // tile g - 2 has been read out
       ok = __all_sync(0xffffffffu, w);
       if (!ok) break;
       tc_fence_after_sync();
-      const uint32_t qa = smem_u32(q_s + qb * kTileBytes), ka = smem_u32(k_s + st * kTileBytes);
-      uint64_t da[DH / 16], db[DH / 16];  // built by every lane: warp-uniform values
-#pragma unroll
-      for (int k16 = 0; k16 < DH / 16; ++k16) {
-        da[k16] = desc_kmajor_d(qa, k16);
-        db[k16] = desc_kmajor_d(ka, k16);
-      }
+      const uint32_t qa = smem_u32(q_s + qb * kTB), ka = smem_u32(k_s + st * kTB);
       const uint32_t dst = tmem + sb * T;
 #pragma unroll
-      for (int k16 = 0; k16 < DH / 16; ++k16) mma_bf16_ss_elect(dst, da[k16], db[k16], idesc_s, k16 > 0);
+      for (int k16 = 0; k16 < DHP / 16; ++k16)
+        mma_bf16_ss_elect(dst, desc_kmajor(qa, k16), desc_kmajor(ka, k16), idesc_s, k16 > 0);
       mma_commit_elect(&s_full[sb]);
       mma_commit_elect(&k_empty[st]);
       if (a.j == a.qt) mma_commit_elect(&q_empty[qb]);
       a.advance(sched);
     }
-  } else if (warp < 4) {
-    // ---------------------------------------------------------------- MMA issuers, output: O += P_g V_g, one warp
-    // per softmax group (warp 2: even tiles of the stream, warp 3: odd tiles)
-    constexpr uint32_t idesc_o = idesc_bf16_f32(T, DH, false, true);
-    const int grp = warp - 2;
+  } else if (warp == 2) {
+    // ---------------------------------------------------------------- MMA issuer, output: O_x += P[:, c] V[c, :]
+    constexpr uint32_t idesc_o = idesc_bf16_f32(T, DHP, false, true);
+    constexpr int kPerBlock = T / 16 / C::kNC;  // K steps of a column block
     Cursor b;
     b.init(sched, first_tile);
     bool ok = true;
-    uint32_t items = 0;  // items this group has taken part in
     while (b.valid && ok) {
-      if ((b.g & 1) == grp) {
-        const int st = b.g % kVStages;
-        const bool first = b.j - b.j0 <= 1;  // the group's first tile of this item: start a fresh accumulator ...
-        bool w = mbar_wait(&p_ready[grp], (b.g >> 1) & 1, ctx, 0x1204u) &&
-                 mbar_wait(&v_full[st], (b.g / kVStages) & 1, ctx, 0x1205u);
-        if (first) {  // ... once the group has read the previous item's result out of it
-          if (w) w = mbar_wait(&o_free[grp], (items & 1) ^ 1u, ctx, 0x1206u);
-          ++items;
-        }
-        ok = __all_sync(0xffffffffu, w);
-        if (!ok) break;
-        tc_fence_after_sync();
-        const uint32_t pa = smem_u32(p_s + grp * 2 * kTileBytes), va = smem_u32(v_s + st * kTileBytes);
-        uint64_t da[T / 16], db[T / 16];  // built by every lane: warp-uniform values
+      const int st = b.g % C::kV, pb = b.g % C::kP;
+      const bool first = b.j - b.j0 < C::kG;  // the group's first tile of the item: fresh accumulators ...
+      bool w = mbar_wait(&p_ready[pb], (b.g / C::kP) & 1, ctx, 0x1204u) &&
+               mbar_wait(&v_full[st], (b.g / C::kV) & 1, ctx, 0x1205u);
+      if (w && first) w = mbar_wait(o_free, (b.ord & 1) ^ 1u, ctx, 0x1206u);  // ... once the previous item has been read out
+      ok = __all_sync(0xffffffffu, w);
+      if (!ok) break;
+      tc_fence_after_sync();
+      const uint32_t pa = smem_u32(p_s + pb * PARTS * kPBytes), va = smem_u32(v_s + st * kTB);
 #pragma unroll
-        for (int k16 = 0; k16 < T / 16; ++k16) {
-          da[k16] = desc_p_kmajor(pa, k16);
-          db[k16] = desc_rows_as_k(va, k16);
-        }
-        const uint32_t dst = tmem + kSBufs * T + grp * DH;
+      for (int part = 0; part < PARTS; ++part)
 #pragma unroll
         for (int k16 = 0; k16 < T / 16; ++k16)
-          mma_bf16_ss_elect(dst, da[k16], db[k16], idesc_o, (k16 > 0 || !first) ? 1u : 0u);
-        mma_commit_elect(&o_full[grp]);
-        mma_commit_elect(&v_empty[st]);
-      }
+          mma_bf16_ss_elect(tmem + kColO + ((b.g % C::kG) * C::kNC + k16 / kPerBlock) * DHP,
+                            desc_kmajor(pa + part * kPBytes, k16), desc_rows_as_k(va, k16), idesc_o,
+                            (part > 0 || k16 % kPerBlock > 0 || !first) ? 1u : 0u);
+      mma_commit_elect(&o_full[b.g % C::kG]);
+      mma_commit_elect(&v_empty[st]);
       b.advance(sched);
     }
   } else if (warp >= 4) {
     // ---------------------------------------------------------------- softmax warps
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
-    const int quarter = warp & 3;            // tensor-memory lane quarter this warp may read
-    const int grp = (warp - 4) >> 2;         // this group handles the stream's tiles with (g & 1) == grp
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::kRegsSoftmax));
+    constexpr int kCW = C::kCW, kWords = kCW / 32;
+    const int quarter = warp & 3;                  // tensor-memory lane quarter this warp may read
+    const int grp = (warp - 4) / C::kGroupWarps;   // this group handles the stream's tiles with g % kG == grp
+    const int cb = ((warp - 4) >> 2) % C::kNC;     // its column block
     const int row = quarter * 32 + lane;
     const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
-    const uint32_t t_o = tmem + lane_base + kSBufs * T + grp * DH;  // this group's output accumulator
-    uint8_t* p_tile = p_s + grp * 2 * kTileBytes;
+    const uint32_t t_o = tmem + lane_base + kColO;
+    const uint32_t t_own = t_o + (grp * C::kNC + cb) * DHP;
     const float f_eval = p.dr.train ? 1.f : p.dr.eval_scale;  // evaluation: P * (1 - p), applied to the final rows
     const uint32_t thr_hi = p.dr.thr16 << 16;
+    const float sc = p.scale_log2;
+    const int ntri = p.nq * (p.nq + 1) / 2;
+    // float32 probabilities are kept at most 1 (the reference exponent is exceeded by less than 2^8, see below), so that a
+    // sum with V overflows no earlier than one of the exact probabilities would
+    constexpr float kShift = kExact ? -8.f : 0.f;
 
     Cursor c;
     c.init(sched, first_tile);
     bool ok = true;
-    float m_ref = 0.f, l = 0.f;  // reference exponent (log2 domain) and sum of 2^(s - m_ref) of this group's tiles
-    float m_true = 0.f;          // true running row maximum (log2 domain), only reported
-    bool have = false;           // the group holds tiles of the current item
-    int pend_g = -1;             // own tile whose P V product may still be running
-    uint32_t nd = 0;             // hand-overs (items with at least two tiles) seen so far
-    auto wait_pv = [&]() {       // the group's last P V product is complete: accumulator and P buffer are quiet
-      if (pend_g < 0) return;
-      ok = mbar_wait(&o_full[grp], (pend_g >> 1) & 1, ctx, 0x1302u);
-      ok = __all_sync(0xffffffffu, ok);
-      tc_fence_after_sync();
-      pend_g = -1;
-    };
+    // reference (score units) and sum of 2^((s - m_ref) sc + shift) of this group's tiles of the item, this column block; its
+    // true row maximum
+    float m_ref = -INFINITY, l = 0.f, m_true = -INFINITY;
 
     while (c.valid && ok) {
-      const bool mine = (c.g & 1) == grp;
-      const int64_t q_row = static_cast<int64_t>(c.qt) * T + row;
-      if (c.j == c.j0) have = false;
+      const int q_row = c.qt * T + row;
+      const bool last = c.j == c.qt;
+      const bool mine = c.g % C::kG == grp;
+      if (!mine && !last) {
+        c.advance(sched);
+        continue;
+      }
+      const int first_key = p.kstart != nullptr && q_row < p.S
+                                ? __ldg(p.kstart + static_cast<int64_t>(c.bh / p.H) * p.S + q_row) : 0;
       if (mine) {
-        const int sb = c.g % kSBufs;
-        // dropout random words of this thread's row of the tile: independent of the scores, so they are drawn one
-        // 32-column chunk ahead of their use (the first chunk while the score MMA may still be running)
-        uint32_t rw[2][4][4];  // raw words of the four Philox calls of a 32-column chunk, drawn one chunk ahead
-        const uint64_t call0 = ((static_cast<uint64_t>(c.bh) * p.S + q_row) * p.S + static_cast<uint64_t>(c.j) * T) >> 3;
-        if (MODE == 1) {
+        const int sb = c.g % kSBufs, pb = c.g % C::kP;
+        const bool fresh = c.j - c.j0 < C::kG;
+        uint8_t* p_tile = p_s + pb * PARTS * kPBytes;
+        // what does not wait for the scores: the keep flags of this thread's columns
+        uint32_t keepw[kWords];
 #pragma unroll
-          for (int q = 0; q < 4; ++q) philox_rk(rk_s, call0 + q, p.dr.stream_id, rw[0][q]);
+        for (int w = 0; w < kWords; ++w)
+          if (MODE == 1)
+            keepw[w] = keep_word(rk_s, (static_cast<uint64_t>(c.bh) * p.S + q_row) * p.S + static_cast<uint64_t>(c.j * T + cb * kCW + 32 * w),
+                                 p.dr.stream_id, thr_hi);
+        if (MODE == 2) {
+          const uint2 kb = __ldg(reinterpret_cast<const uint2*>(p.keep_bits) +
+                                 ((static_cast<int64_t>(c.bh) * ntri + c.qt * (c.qt + 1) / 2 + c.j) * T + row) * 2 + cb);
+          keepw[0] = kb.x;
+          keepw[1] = kb.y;
         }
-        uint4 kb = make_uint4(0u, 0u, 0u, 0u);
-        if (MODE == 2)
-          kb = __ldg(p.keep_bits + (static_cast<int64_t>(c.bh) * (p.nq * (p.nq + 1) / 2) + c.qt * (c.qt + 1) / 2 + c.j) * T + row);
-        const uint32_t keepw[4] = {kb.x, kb.y, kb.z, kb.w};
         ok = mbar_wait(&s_full[sb], (c.g / kSBufs) & 1, ctx, 0x1303u);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after_sync();
-        float s[4][32];
-#pragma unroll
-        for (int cc = 0; cc < 4; ++cc) tmem_ld_32x32f(tmem + lane_base + sb * T + cc * 32, s[cc]);
-        tmem_ld_wait();
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&s_free[sb]);  // the scores are in registers: the buffer may take tile g + 3
-        const bool diag = c.j == c.qt;
-        if (diag) {  // causal mask: only the diagonal tile has columns beyond the row
-#pragma unroll
-          for (int cc = 0; cc < 4; ++cc)
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (cc * 32 + i > row) s[cc][i] = -INFINITY;
-        }
-        if (VARLEN) {  // keys before the row's document: columns below rel (any tile may hold a boundary)
-          const int rel = __ldg(p.kstart + static_cast<int64_t>(c.bh / p.H) * p.S + q_row) - c.j * T;
-          if (__any_sync(0xffffffffu, rel > 0)) {  // (most tiles hold no document boundary for any row of the warp)
-#pragma unroll
-            for (int cc = 0; cc < 4; ++cc)
+        // The scores are read twice, 32 columns at a time, for the maximum and for the exponentials: 64 live scores a thread
+        // do not fit the 104 registers of four warps a scheduler.
+        const uint32_t t_s = tmem + lane_base + sb * T + cb * kCW;
+        const bool edge = last || p.kstart != nullptr;
+        auto load_scores = [&](int w, float (&s)[32]) {
+          tmem_ld_32x32f(t_s + 32 * w, s);
+          tmem_ld_wait();
+          if (edge) {  // keys after the row (diagonal tile) and before its document
+            const int k0 = c.j * T + cb * kCW + 32 * w;  // first key of the word
+            const uint32_t valid = range_bits(first_key - k0, q_row - k0);
+            if (__any_sync(0xffffffffu, valid != 0xffffffffu)) {
 #pragma unroll
               for (int i = 0; i < 32; ++i)
-                if (cc * 32 + i < rel) s[cc][i] = -INFINITY;
+                if (((valid >> i) & 1u) == 0u) s[i] = -INFINITY;
+            }
           }
-        }
+        };
         float mp[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};  // four independent chains of three-input maxima
 #pragma unroll
-        for (int cc = 0; cc < 4; ++cc)
+        for (int w = 0; w < kWords; ++w) {
+          float s[32];
+          load_scores(w, s);
 #pragma unroll
-          for (int i = 0; i < 32; i += 8) {
+          for (int i = 0; i < 32; i += 8)
 #pragma unroll
-            for (int k = 0; k < 4; ++k) mp[k] = max3(mp[k], s[cc][i + 2 * k], s[cc][i + 2 * k + 1]);
-          }
-        const float mloc = fmaxf(fmaxf(mp[0], mp[1]), fmaxf(mp[2], mp[3])) * p.scale_log2;
-        // The reference exponent only moves when the row maximum outgrows it by more than 2^8: probabilities then
-        // stay below 256 (exact in fp32, same relative precision in bf16) and the accumulator in tensor memory is
-        // rescaled rarely. Any reference gives the same quotient sum(P V) / sum(P).
+            for (int k = 0; k < 4; ++k) mp[k] = max3(mp[k], s[i + 2 * k], s[i + 2 * k + 1]);
+        }
+        const float mloc = fmaxf(fmaxf(mp[0], mp[1]), fmaxf(mp[2], mp[3]));
+        // The reference only moves when the row maximum outgrows it by more than 2^8: probabilities then stay below 256
+        // times the shift (same relative precision in any scale) and the accumulator in tensor memory is rescaled rarely.
+        // Any reference gives the same quotient sum(P V) / sum(P).
         bool grow = false;
-        if (!have) {
+        if (fresh) {
           m_ref = mloc;
           m_true = mloc;
           l = 0.f;
-          have = true;
         } else {
-          grow = mloc > m_ref + 8.f;
+          grow = (mloc - m_ref) * sc > 8.f;  // (both -inf: not a number, no growth)
           m_true = fmaxf(m_true, mloc);
         }
-        wait_pv();
+        // The P buffer is free once the output MMAs of tile g - kP are done. (A wait can only tell a phase from the one before
+        // it: the group waits for every tile of its own, and with one buffer for two groups for every tile of the other.)
+        ok = mbar_wait(&o_full[grp], ((c.g / C::kG) & 1) ^ 1u, ctx, 0x1302u);
+        if (C::kP < C::kG && ok && c.g > 0)
+          ok = mbar_wait(&o_full[(c.g - 1) % C::kG], ((c.g - 1) / C::kG) & 1, ctx, 0x1302u);
+        ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
-        const float alpha = grow ? ex2_approx(m_ref - mloc) : 1.f;
-        if (grow) {
-          m_ref = mloc;
-          l *= alpha;
-        }
-        // (VARLEN: a row that has met no key yet carries m_ref = -inf; its scores are all -inf too and must give 0)
-        const float nm = (VARLEN && m_ref == -INFINITY) ? 0.f : -m_ref;
-        const uint64_t sc2 = pack2(p.scale_log2, p.scale_log2), nm2 = pack2(nm, nm);
-        uint64_t rp[2] = {0ull, 0ull};  // two packed running sums (four chains)
-#pragma unroll
-        for (int cc = 0; cc < 4; ++cc) {
-          if (MODE == 1 && cc + 1 < 4) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) philox_rk(rk_s, call0 + (cc + 1) * 4 + q, p.dr.stream_id, rw[(cc + 1) & 1][q]);
+        if (__any_sync(0xffffffffu, grow)) {  // rare: bring the accumulated rows to the new reference
+          tc_fence_after_sync();
+          const float alpha = grow ? ex2_approx((m_ref - mloc) * sc) : 1.f;
+          if (grow) {
+            m_ref = mloc;
+            l *= alpha;
           }
 #pragma unroll
-          for (int i = 0; i < 32; i += 2) {  // exp2(-inf) = 0 takes care of the masked columns
-            float a, b;
-            unpack2(fma2(pack2(s[cc][i], s[cc][i + 1]), sc2, nm2), a, b);
-            a = ex2_approx(a);
-            b = ex2_approx(b);
-            rp[(i >> 1) & 1] = add2(rp[(i >> 1) & 1], pack2(a, b));
-            if (MODE == 1) {  // 16-bit lanes of word (i % 8) / 2 of call i / 8: low half = even element, high half = odd
-              const uint32_t w = rw[cc & 1][i >> 3][(i & 7) >> 1];
-              if ((w << 16) < thr_hi) a = 0.f;
-              if (w < thr_hi) b = 0.f;
-            } else if (MODE == 2) {
-              if ((keepw[cc] & (1u << i)) == 0u) a = 0.f;
-              if ((keepw[cc] & (2u << i)) == 0u) b = 0.f;
-            }
-            s[cc][i] = a;
-            s[cc][i + 1] = b;
-          }
-          store_row32_sw128(p_tile, row, cc * 32, s[cc]);
-        }
-        float rsum;
-        {
-          float a, b;
-          unpack2(add2(rp[0], rp[1]), a, b);
-          rsum = a + b;
-        }
-        if (__any_sync(0xffffffffu, grow)) {  // rare: bring the accumulated rows to the new reference exponent
-#pragma unroll
-          for (int cc = 0; cc < 2; ++cc) {
+          for (int x = 0; x < DHP; x += 32) {
             uint32_t t[32];
-            tmem_ld_32x32(t_o + cc * 32, t);
+            tmem_ld_32x32(t_own + x, t);
             tmem_ld_wait();
 #pragma unroll
             for (int i = 0; i < 32; ++i) t[i] = __float_as_uint(__uint_as_float(t[i]) * alpha);
-            tmem_st_32x32(t_o + cc * 32, t);
+            tmem_st_32x32(t_own + x, t);
           }
           tmem_st_wait();
+        }
+        // (a row that has met no key of its own yet carries m_ref = -inf; its scores are all -inf too and must give 0)
+        const float ref = m_ref == -INFINITY ? 0.f : m_ref;
+        const uint64_t sc2 = pack2(sc, sc), sh2 = pack2(kShift, kShift);
+        const uint64_t nm2 = kExact ? pack2(-ref, -ref) : pack2(-ref * sc, -ref * sc);
+        uint64_t rp[2] = {0ull, 0ull};  // two packed running sums (four chains)
+#pragma unroll
+        for (int w = 0; w < kWords; ++w) {
+          float s[32];
+          load_scores(w, s);
+          if (w == kWords - 1) {  // the scores are in registers: the buffer may take tile g + 2
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&s_free[sb]);
+          }
+#pragma unroll
+          for (int i8 = 0; i8 < 32; i8 += 8) {
+#pragma unroll
+            for (int i = i8; i < i8 + 8; i += 2) {  // exp2(-inf) = 0 takes care of the masked columns
+              const uint64_t x = pack2(s[i], s[i + 1]);
+              float a, b;
+              unpack2(kExact ? fma2(add2(x, nm2), sc2, sh2) : fma2(x, sc2, nm2), a, b);
+              a = ex2_approx(a);
+              b = ex2_approx(b);
+              rp[(i >> 1) & 1] = add2(rp[(i >> 1) & 1], pack2(a, b));
+              s[i] = a;
+              s[i + 1] = b;
+            }
+            uint32_t pw[PARTS][4];
+            split8<PARTS>(s + i8, pw);
+            if (MODE != 0) {
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const uint32_t m = pair_mask(keepw[w], (i8 >> 1) + i);
+#pragma unroll
+                for (int part = 0; part < PARTS; ++part) pw[part][i] &= m;
+              }
+            }
+            store8<PARTS>(p_tile, row, (cb * kCW + 32 * w + i8) >> 3, pw);
+          }
+        }
+        {
+          float a, b;
+          unpack2(add2(rp[0], rp[1]), a, b);
+          l += a + b;
+        }
+        if (kExact) {  // this warp's share of the V tile: elements that are not finite must not meet masked probabilities
+          const int st = c.g % C::kV;
+          ok = mbar_wait(&v_full[st], (c.g / C::kV) & 1, ctx, 0x1307u);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          uint8_t* vt = v_s + st * kTB + (warp - 4) % C::kGroupWarps * (kTB / C::kGroupWarps) + lane * 16;
+          bool bad = false;
+#pragma unroll
+          for (int x = 0; x < kTB / C::kGroupWarps; x += 512) bad = zero_nonfinite(vt + x) || bad;
+          if (bad) *bad_v = 1;
         }
         fence_proxy_async_smem();
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&p_ready[grp]);
-        l += rsum;
-        pend_g = c.g;
+        if (lane == 0) mbar_arrive(&p_ready[pb]);
       }
-      if (c.j == c.qt) {  // the item ends with this tile: its owner finishes the rows, the other group hands over
-        float o[DH];
-        if (have) {
-          wait_pv();
-          if (!ok) break;
+      if (last) {  // the item ends with this tile: its group merges the states of all and writes the rows
+        ok = mbar_wait(o_free, (c.ord & 1) ^ 1u, ctx, 0x1306u);  // the previous item's states have been read
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        float* own = stats + (grp * C::kNC + cb) * 3 * T + row;
+        own[0] = m_ref;
+        own[T] = l;
+        own[2 * T] = m_true;
+        m_ref = m_true = -INFINITY;
+        l = 0.f;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(stats_full);
+      }
+      if (last && mine) {
+        ok = mbar_wait(stats_full, c.ord & 1, ctx, 0x1304u) &&
+             mbar_wait(&o_full[grp], (c.g / C::kG) & 1, ctx, 0x1305u);  // (of the last tile, and so of all before it)
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after_sync();
+        const bool single = c.j == c.j0;  // the other group had no tile of this item: its accumulators hold anything
+        float mx = -INFINITY, mt = -INFINITY, f[C::kAcc], lsum = 0.f;
 #pragma unroll
-          for (int cc = 0; cc < 2; ++cc) {
-            float t[32];
-            tmem_ld_row32(t_o + cc * 32, t);
-#pragma unroll
-            for (int i = 0; i < 32; ++i) o[cc * 32 + i] = t[i];
-          }
-          tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&o_free[grp]);  // the next item may overwrite the accumulator
+        for (int x = 0; x < C::kAcc; ++x) {
+          f[x] = stats[(x * 3 + 0) * T + row];
+          mx = fmaxf(mx, f[x]);
+          mt = fmaxf(mt, stats[(x * 3 + 2) * T + row]);
         }
-        if (c.qt > c.j0) {  // (an item of a single tile has nothing to merge)
-          if (!mine) {
-            ok = mbar_wait(dump_free, (nd & 1) ^ 1u, ctx, 0x1304u);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
 #pragma unroll
-            for (int i = 0; i < DH; ++i) dump[i * T + row] = o[i];
-            dump[DH * T + row] = m_ref;
-            dump[(DH + 1) * T + row] = l;
-            dump[(DH + 2) * T + row] = m_true;
+        for (int x = 0; x < C::kAcc; ++x) {  // (a block that met no key of this row: -inf - -inf is not a number)
+          f[x] = f[x] == -INFINITY ? 0.f : ex2_approx((f[x] - mx) * sc);
+          lsum = fmaf(stats[(x * 3 + 1) * T + row], f[x], lsum);
+        }
+        const bool none = first_key > q_row;  // the row attends nothing: zero output, neutral statistics
+        const float inv = none ? 0.f : f_eval / lsum;
+        constexpr int kOut = DHP / C::kNC;  // columns of the rows that this warp writes
+        __nv_bfloat16* dst = views.o.row(c.bh / p.H, c.bh % p.H, q_row);
+#pragma unroll
+        for (int x0 = 0; x0 < kOut; x0 += 16) {
+          const int col = cb * kOut + x0;
+          float o[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) o[i] = 0.f;
+#pragma unroll
+          for (int x = 0; x < C::kAcc; ++x) {
+            if (single && x / C::kNC != grp) continue;
+            uint32_t t[16];
+            tmem_ld_32x16(t_o + x * DHP + col, t);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) o[i] = fmaf(__uint_as_float(t[i]), f[x], o[i]);
+          }
+          if (x0 + 16 == kOut) {
+            tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(dump_full);
-          } else {
-            ok = mbar_wait(dump_full, nd & 1, ctx, 0x1305u);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
-            const float m_o = dump[DH * T + row], l_o = dump[(DH + 1) * T + row];
-            const float mm = fmaxf(m_ref, m_o);
-            float fa = ex2_approx(m_ref - mm), fb = ex2_approx(m_o - mm);
-            if (VARLEN) {  // a group that met no key of this row (-inf - -inf is not a number)
-              if (m_ref == -INFINITY) fa = 0.f;
-              if (m_o == -INFINITY) fb = 0.f;
+            if (lane == 0) mbar_arrive(o_free);  // the next item may overwrite the accumulators
+          }
+          if (q_row < p.S) {
+            if (kExact && *bad_v != 0 && !none) {
+              float t[16];
+#pragma unroll
+              for (int i = 0; i < 16; ++i) t[i] = 0.f;
+              add_nonfinite_v(t, views.q, views.k, views.v, p, rk_s, MODE, c.bh, q_row, first_key, col, mt);
+#pragma unroll
+              for (int i = 0; i < 16; ++i) o[i] += t[i];
             }
 #pragma unroll
-            for (int i = 0; i < DH; ++i) o[i] = o[i] * fa + dump[i * T + row] * fb;
-            l = l * fa + l_o * fb;
-            m_ref = mm;
-            m_true = fmaxf(m_true, dump[(DH + 2) * T + row]);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(dump_free);
+            for (int c8 = 0; c8 < 2; ++c8) {
+              float t[8];
+#pragma unroll
+              for (int i = 0; i < 8; ++i) t[i] = none ? 0.f : o[c8 * 8 + i] * inv;
+              if (col + c8 * 8 < p.D) Elem<__nv_bfloat16>::store_vec(dst + col + c8 * 8, t);
+            }
           }
-          ++nd;
         }
-        if (mine) {
-          const bool empty = VARLEN && !(l > 0.f);  // the row attends nothing: zero output, neutral statistics
-          const float inv = empty ? 0.f : f_eval / l;
-          __nv_bfloat16* dst = out.row(c.bh / p.H, c.bh % p.H, q_row);
-#pragma unroll
-          for (int c8 = 0; c8 < DH / 8; ++c8) {
-            float t[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) t[i] = o[c8 * 8 + i] * inv;
-            Elem<__nv_bfloat16>::store_vec(dst + c8 * 8, t);
-          }
+        if (cb == 0 && q_row < p.S) {
           const int64_t ri = static_cast<int64_t>(c.bh) * p.S + q_row;
-          row_max[ri] = empty ? 0.f : m_true * kLn2;                   // acts0: row maximum of the scaled scores
-          row_sum[ri] = empty ? 1.f : l * ex2_approx(m_ref - m_true);  // acts1: sum of exp(score - maximum)
+          row_max[ri] = none ? 0.f : mt * p.scale;  // acts0: row maximum of the scaled scores
+          row_sum[ri] = none ? 1.f : lsum * ex2_approx((mx - mt) * sc - kShift);  // acts1: sum of exp(score - maximum)
         }
-        have = false;
       }
       c.advance(sched);
     }
@@ -569,26 +651,52 @@ attn_keep_bits_kernel(uint32_t* __restrict__ bits, const AttnDropout dr, int S, 
   for (int q = 0; q < 4; ++q) {
     uint32_t w[4];
     philox_rk(rk, (idx0 >> 3) + q, dr.stream_id, w);
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      word |= ((w[e] << 16) >= thr_hi ? 1u : 0u) << (8 * q + 2 * e);
-      word |= (w[e] >= thr_hi ? 1u : 0u) << (8 * q + 2 * e + 1);
-    }
+    word |= keep_flags8(w, thr_hi) << (8 * q);
+  }
+  if (const uint32_t shift = static_cast<uint32_t>(idx0) & 7u; shift != 0u) {  // rows that start inside a call
+    uint32_t w[4];
+    philox_rk(rk, (idx0 >> 3) + 4, dr.stream_id, w);
+    word = __funnelshift_r(word, keep_flags8(w, thr_hi), shift);
   }
   bits[tile * 512 + threadIdx.x] = word;
+}
+
+template <int DHP, int PARTS>
+int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdViews& views, float* row_max,
+               float* row_sum, const AttnParams& p, int mode, cudaStream_t st) {
+  using C = Cfg<DHP, PARTS>;
+  using Kern = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const FwdViews, float*, float*,
+                        const AttnParams, const Sched);
+  static const Kern kerns[3] = {attn_fwd_ws_kernel<DHP, PARTS, 0>, attn_fwd_ws_kernel<DHP, PARTS, 1>,
+                                attn_fwd_ws_kernel<DHP, PARTS, 2>};
+  const Kern kern = kerns[mode];
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return PTJ_ERR_LAUNCH;
+  }
+  Sched s;
+  s.nq = p.nq;
+  s.BH = p.BH;
+  s.total = p.nq * p.BH;
+  const int grid = s.total < kNumSMs ? s.total : kNumSMs;
+  s.rounds = (s.total + grid - 1) / grid;
+  s.bh_magic = static_cast<uint32_t>(((1ull << 32) + s.BH - 1) / s.BH);
+  launch_k(kern, grid, C::kThreads, C::kSmemBytes, st, tq, tk, tv, views, row_max, row_sum, p, s);
+  PTJ_CHECK_LAUNCH();
+  return PTJ_OK;
 }
 
 }  // namespace
 
 size_t attn_keep_bits_bytes(const ptj_attn_shape& sh) {
-  const int64_t nq = sh.seq / T;
+  const int64_t nq = ceil_div(sh.seq, T);
   return static_cast<size_t>(sh.batch * sh.heads * (nq * (nq + 1) / 2) * T) * 16;
 }
 
 int attn_keep_bits_tc(uint32_t* bits, const ptj_attn_shape& sh, const AttnDropout& dr, cudaStream_t st) {
   const int64_t tiles = static_cast<int64_t>(attn_keep_bits_bytes(sh) / 2048);
   launch_k(attn_keep_bits_kernel, static_cast<unsigned>(tiles), 512, 0, st, bits, dr, static_cast<int>(sh.seq),
-                                                                      static_cast<int>(sh.seq / T));
+           static_cast<int>(ceil_div(sh.seq, T)));
   PTJ_CHECK_LAUNCH();
   return PTJ_OK;
 }
@@ -605,26 +713,11 @@ int attn_fwd_tc(const void* q, const void* k, const void* v, void* o, float* row
   p.kstart = row_kstart;
   const bool masked = dr.train && dr.thr16 != 0u;
   const int mode = !masked ? 0 : (keep_bits != nullptr ? 2 : 1);
-  using Kern = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const RowView, float*, float*,
-                        const AttnParams, const Sched);
-  static const Kern kerns[2][3] = {
-      {attn_fwd_ws_kernel<0, false>, attn_fwd_ws_kernel<1, false>, attn_fwd_ws_kernel<2, false>},
-      {attn_fwd_ws_kernel<0, true>, attn_fwd_ws_kernel<1, true>, attn_fwd_ws_kernel<2, true>}};
-  const Kern kern = kerns[row_kstart != nullptr ? 1 : 0][mode];
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return PTJ_ERR_LAUNCH;
-  }
-  Sched s;
-  s.nq = p.nq;
-  s.BH = p.BH;
-  s.total = p.nq * p.BH;
-  const int grid = s.total < kNumSMs ? s.total : kNumSMs;
-  s.rounds = (s.total + grid - 1) / grid;
-  s.bh_magic = static_cast<uint32_t>(((1ull << 32) + s.BH - 1) / s.BH);
-  launch_k(kern, grid, kThreads, kSmemBytes, st, tq, tk, tv, make_view(o, sh.o_strides), row_max, row_sum, p, s);
-  PTJ_CHECK_LAUNCH();
-  return PTJ_OK;
+  const FwdViews views{make_view(q, sh.q_strides), make_view(k, sh.k_strides), make_view(v, sh.v_strides),
+                       make_view(o, sh.o_strides)};
+  if (sh.d_head > 64) return launch_fwd<128, 3>(tq, tk, tv, views, row_max, row_sum, p, mode, st);
+  if (attn_bf16_probabilities(sh)) return launch_fwd<64, 1>(tq, tk, tv, views, row_max, row_sum, p, mode, st);
+  return launch_fwd<64, 3>(tq, tk, tv, views, row_max, row_sum, p, mode, st);
 }
 
 }  // namespace ptj

@@ -240,10 +240,11 @@ __device__ __forceinline__ void mul_tn_masked(float (&acc)[kR][Tile<DP>::kCols],
   }
 }
 
-// this thread's block of an output tile; mul[r] scales a row
+// this thread's block of an output tile; mul[r] scales a row. patch: only elements that are not finite, here or in memory
 template <typename T, int DP>
 __device__ __forceinline__ void store_rows(T* base, int64_t rs, int64_t r0, int64_t S, int D, bool vec,
-                                           const float (&acc)[kR][Tile<DP>::kCols], const float (&mul)[kR], int tx, int ty) {
+                                           const float (&acc)[kR][Tile<DP>::kCols], const float (&mul)[kR], int tx, int ty,
+                                           bool patch = false) {
   using TT = Tile<DP>;
 #pragma unroll
   for (int r = 0; r < kR; ++r) {
@@ -253,7 +254,12 @@ __device__ __forceinline__ void store_rows(T* base, int64_t rs, int64_t r0, int6
 #pragma unroll
     for (int c = 0; c < TT::kCols; c += TT::kVec) {
       const int col = TT::col(c, tx);
-      if (sizeof(T) == 4 && TT::kVec == 4 && vec) {
+      if (patch) {
+        for (int e = 0; e < TT::kVec; ++e) {
+          const float x = acc[r][c + e] * mul[r];
+          if (col + e < D && !(isfinite(x) && isfinite(Elem<T>::load(row + col + e)))) Elem<T>::store(row + col + e, x);
+        }
+      } else if (sizeof(T) == 4 && TT::kVec == 4 && vec) {
         if (col < D)
           *reinterpret_cast<float4*>(row + col) =
               make_float4(acc[r][c] * mul[r], acc[r][c + 1] * mul[r], acc[r][c + 2 < TT::kCols ? c + 2 : c] * mul[r],
@@ -415,6 +421,7 @@ struct BwdArgs {
   const float *row_max, *row_sum;
   T *dq, *dk, *dv;
   const int32_t* kstart;
+  const unsigned int* patch;  // optional: the results are there; when this word is set, put in what is not finite
   ptj_attn_shape sh, dsh;
   float scale;
   int nq;
@@ -469,6 +476,7 @@ template <typename T, int DP>
 __global__ void __launch_bounds__(Tile<DP>::kThreads)
 attn_dq_simt_kernel(const BwdArgs<T> a) {
   grid_dep_sync();
+  if (a.patch != nullptr && *a.patch == 0u) return;
   using TT = Tile<DP>;
   extern __shared__ __align__(16) float smem[];
   float* q_s = smem;
@@ -532,7 +540,7 @@ attn_dq_simt_kernel(const BwdArgs<T> a) {
     __syncwarp();
   }
   store_rows<T, DP>(a.dq + b * a.dsh.q_strides[0] + h * a.dsh.q_strides[1], a.dsh.q_strides[2], r0, S, D, a.vec, acc,
-                       one, tx, ty);
+                       one, tx, ty, a.patch != nullptr);
 }
 
 // dK and dV: block = one key tile, the ones with the most query tiles first; sweeps the query tiles.
@@ -540,6 +548,7 @@ template <typename T, int DP>
 __global__ void __launch_bounds__(Tile<DP>::kThreads, DP <= 64 ? 2 : 1)  // (wide heads: shared memory takes one block)
 attn_dkv_simt_kernel(const BwdArgs<T> a) {
   grid_dep_sync();
+  if (a.patch != nullptr && *a.patch == 0u) return;
   using TT = Tile<DP>;
   extern __shared__ __align__(16) float smem[];
   float* q_s = smem;
@@ -605,9 +614,9 @@ attn_dkv_simt_kernel(const BwdArgs<T> a) {
     }
   }
   store_rows<T, DP>(a.dv + b * a.dsh.v_strides[0] + h * a.dsh.v_strides[1], a.dsh.v_strides[2], j0, S, D, a.vec, dv,
-                       one, tx, ty);
+                       one, tx, ty, a.patch != nullptr);
   store_rows<T, DP>(a.dk + b * a.dsh.k_strides[0] + h * a.dsh.k_strides[1], a.dsh.k_strides[2], j0, S, D, a.vec, dk,
-                       one, tx, ty);
+                       one, tx, ty, a.patch != nullptr);
 }
 
 // every row starts on a multiple of four elements: rows are read as vectors
@@ -668,11 +677,11 @@ int fwd_typed(const void* q, const void* k, const void* v, void* o, float* row_m
 template <typename T>
 int bwd_typed(const void* d_o, const void* q, const void* k, const void* v, const void* o, const float* row_max,
               const float* row_sum, void* dq, void* dk, void* dv, const int32_t* row_kstart, const ptj_attn_shape& sh,
-              const ptj_attn_shape& dsh, const AttnDropout& dr, cudaStream_t st) {
+              const ptj_attn_shape& dsh, const AttnDropout& dr, const unsigned int* patch, cudaStream_t st) {
   const void* ptrs[8] = {d_o, q, k, v, o, dq, dk, dv};
   const BwdArgs<T> a{static_cast<const T*>(d_o), static_cast<const T*>(q), static_cast<const T*>(k),
                      static_cast<const T*>(v), static_cast<const T*>(o), row_max, row_sum, static_cast<T*>(dq),
-                     static_cast<T*>(dk), static_cast<T*>(dv), row_kstart, sh, dsh,
+                     static_cast<T*>(dk), static_cast<T*>(dv), row_kstart, patch, sh, dsh,
                      1.f / sqrtf(static_cast<float>(sh.d_head)), static_cast<int>(ceil_div(sh.seq, kB)),
                      rows_vectorise<T>(sh, ptrs, 8) && rows_vectorise<T>(dsh, ptrs, 0), dr};
   if (sh.d_head <= 32) return run_bwd<T, 32>(a, st);
@@ -691,11 +700,12 @@ int attn_fwd_simt(const void* q, const void* k, const void* v, void* o, float* r
 
 int attn_bwd_simt(const void* d_o, const void* q, const void* k, const void* v, const void* o, const float* row_max,
                   const float* row_sum, void* dq, void* dk, void* dv, const int32_t* row_kstart,
-                  const ptj_attn_shape& sh, const ptj_attn_shape& dsh, const AttnDropout& dr, int dtype, cudaStream_t st) {
+                  const ptj_attn_shape& sh, const ptj_attn_shape& dsh, const AttnDropout& dr, int dtype,
+                  const unsigned int* patch, cudaStream_t st) {
   if (sh.d_head > kMaxD) return PTJ_ERR_UNSUPPORTED;
   return dtype == PTJ_F32
-             ? bwd_typed<float>(d_o, q, k, v, o, row_max, row_sum, dq, dk, dv, row_kstart, sh, dsh, dr, st)
-             : bwd_typed<__nv_bfloat16>(d_o, q, k, v, o, row_max, row_sum, dq, dk, dv, row_kstart, sh, dsh, dr, st);
+             ? bwd_typed<float>(d_o, q, k, v, o, row_max, row_sum, dq, dk, dv, row_kstart, sh, dsh, dr, patch, st)
+             : bwd_typed<__nv_bfloat16>(d_o, q, k, v, o, row_max, row_sum, dq, dk, dv, row_kstart, sh, dsh, dr, patch, st);
 }
 
 }  // namespace ptj

@@ -396,7 +396,10 @@ def attn_bwd(d_o, q, k, v, o, m, l, dq, dk, dv, train, seed, stream_id=0, p=None
     p = DROPOUT_RATE if p is None else p
     need = int(_lib.lib().ptj_attn_bwd_workspace_bytes(ctypes.byref(sh), _dt(q)))
     if workspace is None and need > 0:
-        workspace = attn_bwd_workspace(need, q.device)
+        try:
+            workspace = attn_bwd_workspace(need, q.device)
+        except torch.OutOfMemoryError:  # most shapes run without (bf16 ones of 64-wide heads and whole tiles do not)
+            workspace = None
     wptr = _ptr(workspace) if workspace is not None else None
     wbytes = workspace.numel() * workspace.element_size() if workspace is not None else 0
     _lib.check(

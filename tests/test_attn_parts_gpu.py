@@ -1,0 +1,63 @@
+"""Attention on the tensor cores with float32 probabilities in three bf16 parts (bf16 operands; every row length and head size
+but whole tiles of 64-wide heads) against float64: edges of tiles, narrow and wide heads, one to several tiles and items."""
+import pytest
+import torch
+
+from conftest import pkg
+from oracle import philox
+from test_attn_general_gpu import documents, reference, run
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("B,H,S,D,p,train,packed", [
+    (1, 1, 1, 16, 0.1, True, False),       # one row, the narrowest head
+    (2, 1, 128, 32, 0.1, True, False),     # one whole tile of half a sub-tile
+    (1, 2, 255, 24, 0.1, True, True),
+    (1, 1, 257, 64, 0.0, True, False),     # one row in the last tile
+    (2, 2, 256, 72, 0.1, True, False),     # eight columns in the second sub-tile
+    (1, 2, 385, 96, 0.1, False, False),    # evaluation: probabilities times 1 - p
+    (1, 3, 511, 128, 0.1, True, True),     # 511 % 8 == 7: keep flags start inside a call
+    (5, 32, 130, 64, 0.1, True, False),    # more items than blocks: several a block, single tiles among them
+    (3, 50, 192, 128, 0.1, True, True),
+])
+def test_against_float64(B, H, S, D, p, train, packed):
+    ops = pkg("operators")
+    g = torch.Generator(device="cuda").manual_seed(S + D)
+    q, k, v, do = (torch.randn(B, H, S, D, generator=g, device="cuda").bfloat16() for _ in range(4))
+    ks = ops.row_kstart_from_lengths(documents(B, S, packed), S) if packed else None
+    (o, m, l, dq, dk, dv), bufs = run(ops, q, k, v, do, p, train, 99, ks, 0)
+    assert all(bool((flat[-512:] == 7.0).all()) for flat in bufs), "a store went beyond the tensor"
+    keep = torch.ones((), device="cuda", dtype=torch.float64)
+    if train and p > 0:
+        keep = torch.from_numpy(philox.keep_mask(99, 0, B * H * S * S, p)).view(B, H, S, S).cuda().double()
+    # the bound of the general kernels: one rounding of the result, and 2^-17 of the sum of magnitudes for scores and sums
+    refs = reference(q, k, v, do, o, keep, 1.0 if train else 1.0 - p, ks)
+    for name, got, (ref, mag) in zip(("O", "dQ", "dK", "dV"), (o, dq, dk, dv), refs):
+        worst = ((got.double() - ref).abs() - 2.0 ** -8 * ref.abs() - 2.0 ** -17 * mag).max()
+        assert bool(torch.isfinite(got.float()).all()) and float(worst) <= 1e-30, f"{name} {float(worst):.3e}"
+
+
+@pytest.mark.parametrize("S,D", [(500, 64), (131, 32), (256, 128)])
+def test_keep_flags_and_a_missing_workspace(S, D):
+    """Flags drawn beforehand give what the kernels draw themselves; a backward call without a workspace (the general
+    kernels then) gives the same up to one rounding of the result."""
+    ops = pkg("operators")
+    B, H, p, seed = 2, 3, 0.2, 11
+    g = torch.Generator(device="cuda").manual_seed(S)
+    q, k, v, do = (torch.randn(B, H, S, D, generator=g, device="cuda").bfloat16() for _ in range(4))
+    res = []
+    for how in ("kernel", "flags", "no workspace"):
+        o, dq, dk, dv = (torch.empty_like(q) for _ in range(4))
+        bits = ops.attn_keep_bits(q, k, v, o, seed, p=p) if how == "flags" else None
+        assert (bits is not None) == (how == "flags")
+        m, l = ops.attn_fwd(q, k, v, o, True, seed, p=p, keep_bits=bits)
+        ops.attn_bwd(do, q, k, v, o, m, l, dq, dk, dv, True, seed, p=p, keep_bits=bits,
+                     workspace=torch.empty(0, device="cuda", dtype=torch.uint8) if how == "no workspace" else None)
+        res.append((o, m, l, dq, dk, dv))
+    torch.cuda.synchronize()
+    assert ops.last_kernel_fault() == 0
+    assert all(torch.equal(a, b) for a, b in zip(res[0], res[1]))
+    # two roundings to bf16 of values that differ by float32 errors: at most one unit in the last place (2^-7 of the value)
+    for a, b in zip(res[0], res[2]):
+        assert bool(((a.double() - b.double()).abs() <= 2.0 ** -7 * b.double().abs() + 1e-5).all())
