@@ -310,6 +310,56 @@ int ptj_attn_bwd(const void* d_o, const void* q, const void* k, const void* v, c
                  uint64_t seed, uint32_t stream_id, const uint32_t* keep_bits, const int32_t* row_kstart,
                  void* workspace, size_t workspace_bytes, int dtype, void* stream);
 
+/* ---- one transformer layer ---------------------------------------------------------------------------- */
+/* The launches of a layer, issued by one call: forward (model_triton.py:2343-2410) and, in two halves so that a caller can
+ * start exchanging the gradients of one while the other runs, backward (:2545-2581). Each is exactly a sequence of this
+ * library's other entry points on contiguous tensors [batch * seq, .] (the projection's columns ordered (head, q/k/v,
+ * d_head)); a status other than PTJ_OK comes from the first of them that fails. Matrices and activations are `dtype`.
+ * workspace: ptj_layer_workspace_bytes bytes, 16-byte aligned, contents irrelevant before and after; with `products` zero
+ * the size without what K splits and float32 tensor-core products use (they then run without). */
+typedef struct {
+  int64_t batch, seq, dim, heads, ffn;
+  int dtype, train;
+  float p;                                    /* dropout probability of all four sites */
+  uint64_t seed_attn, seed_res1, seed_res2;   /* attention probabilities, both residual branches */
+} ptj_layer_shape;
+typedef struct {
+  const float *g1, *b1;      /* [dim] */
+  const void *w_qkv, *w_o;   /* [3 dim, dim], [dim, dim] */
+  const float *g2, *b2;
+  const void* w1;            /* [ffn, dim] */
+  const float* b1f;
+  const void* w2;            /* [dim, ffn] */
+  const float* b2f;
+} ptj_layer_weights;
+typedef struct {             /* x is the layer's input; the rest is written by the forward call and read by backward */
+  const void* x;
+  void *ln1, *qkv, *attn;
+  float *row_max, *row_sum;  /* [batch, heads, seq] */
+  uint32_t* keep_bits;       /* ptj_layer_keep_bits_bytes bytes; NULL where that is 0 */
+  void *x_mid, *ln2, *h_pre, *h_act;
+} ptj_layer_acts;
+typedef struct {
+  float *g1, *b1, *w_qkv, *w_o, *g2, *b2, *w1, *b1f, *w2, *b2f;
+} ptj_layer_grads;
+size_t ptj_layer_workspace_bytes(const ptj_layer_shape* shape, int backward, int products);
+size_t ptj_layer_keep_bits_bytes(const ptj_layer_shape* shape);
+int ptj_layer_fwd(const ptj_layer_shape* shape, const ptj_layer_weights* w, const ptj_layer_acts* acts, void* x_out,
+                  const int32_t* row_kstart, void* workspace, size_t workspace_bytes, void* stream);
+/* dx: gradient of x_out; dy: dropout(dx) of the second residual branch, whose column sums (grads->b2f) the caller has (see
+ * dy_sums below). Writes the gradients of w2, b1f, w1, g2, b2, dx_out (gradient of x_mid) and dy_out (dropout(dx_out) of the
+ * first residual branch). dh_pre [T, ffn] and d_ln [T, dim] are scratch. */
+int ptj_layer_bwd_ffn(const ptj_layer_shape* shape, const ptj_layer_weights* w, const ptj_layer_acts* acts,
+                      const ptj_layer_grads* grads, const void* dx, const void* dy, void* dh_pre, void* d_ln, void* dx_out,
+                      void* dy_out, void* workspace, size_t workspace_bytes, void* stream);
+/* The rest, from what the other half wrote: gradients of w_o, w_qkv, g1, b1 and dx_out (gradient of x). With dy_out (NULL in
+ * the lowest layer) also dropout(dx_out) for the second residual branch of the layer below (seed_below) and its column sums
+ * dy_sums, that layer's b2f gradient. d_attn [T, dim], dqkv [T, 3 dim] and d_ln [T, dim] are scratch. */
+int ptj_layer_bwd_attn(const ptj_layer_shape* shape, const ptj_layer_weights* w, const ptj_layer_acts* acts,
+                       const ptj_layer_grads* grads, const void* dx, const void* dy, void* d_attn, void* dqkv, void* d_ln,
+                       void* dx_out, void* dy_out, float* dy_sums, uint64_t seed_below, const int32_t* row_kstart,
+                       void* workspace, size_t workspace_bytes, void* stream);
+
 /* ---- optimizer -------------------------------------------------------------------------------------- */
 /* sum of squares of a float vector -> out[0] (deterministic two-stage). Replaces grads_l2norm
  * (loss_and_optimizer_triton.py:411-416) on a flat buffer. scratch: ptj_sumsq_scratch_floats(n). */

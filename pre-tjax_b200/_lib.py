@@ -33,6 +33,25 @@ class AttnShape(ctypes.Structure):
     ]
 
 
+class LayerShape(ctypes.Structure):
+    _fields_ = [("batch", c_int64), ("seq", c_int64), ("dim", c_int64), ("heads", c_int64), ("ffn", c_int64),
+                ("dtype", c_int), ("train", c_int), ("p", c_float), ("seed_attn", c_uint64), ("seed_res1", c_uint64),
+                ("seed_res2", c_uint64)]
+
+
+class LayerWeights(ctypes.Structure):
+    _fields_ = [(n, c_void_p) for n in ("g1", "b1", "w_qkv", "w_o", "g2", "b2", "w1", "b1f", "w2", "b2f")]
+
+
+class LayerGrads(ctypes.Structure):
+    _fields_ = LayerWeights._fields_
+
+
+class LayerActs(ctypes.Structure):
+    _fields_ = [(n, c_void_p) for n in ("x", "ln1", "qkv", "attn", "row_max", "row_sum", "keep_bits", "x_mid", "ln2", "h_pre",
+                                        "h_act")]
+
+
 _P = c_void_p
 _SIGNATURES = {
     "ptj_version": (c_int, []),
@@ -74,6 +93,13 @@ _SIGNATURES = {
     "ptj_attn_bwd_workspace_bytes": (c_size_t, [POINTER(AttnShape), c_int]),
     "ptj_attn_bwd": (c_int, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, POINTER(AttnShape), POINTER(AttnShape), c_float,
                              c_int, c_uint64, c_uint32, _P, _P, _P, c_size_t, c_int, _P]),
+    "ptj_layer_workspace_bytes": (c_size_t, [POINTER(LayerShape), c_int, c_int]),
+    "ptj_layer_keep_bits_bytes": (c_size_t, [POINTER(LayerShape)]),
+    "ptj_layer_fwd": (c_int, [POINTER(LayerShape), POINTER(LayerWeights), POINTER(LayerActs), _P, _P, _P, c_size_t, _P]),
+    "ptj_layer_bwd_ffn": (c_int, [POINTER(LayerShape), POINTER(LayerWeights), POINTER(LayerActs), POINTER(LayerGrads), _P, _P,
+                                  _P, _P, _P, _P, _P, c_size_t, _P]),
+    "ptj_layer_bwd_attn": (c_int, [POINTER(LayerShape), POINTER(LayerWeights), POINTER(LayerActs), POINTER(LayerGrads), _P,
+                                   _P, _P, _P, _P, _P, _P, _P, c_uint64, _P, _P, c_size_t, _P]),
     "ptj_sumsq_scratch_floats": (c_size_t, [c_int64]),
     "ptj_sumsq": (c_int, [_P, _P, _P, c_size_t, c_int64, _P]),
     "ptj_adamw": (c_int, [_P, _P, _P, _P, _P, c_int64, _P, _P, c_int, c_float, c_float, c_float, c_float, c_float,

@@ -16,6 +16,7 @@ the logits with their gradient; nothing uses atomics, so results are bit-reprodu
 """
 from __future__ import annotations
 
+import ctypes
 import math
 from dataclasses import dataclass
 from typing import Callable, List, Optional, Sequence
@@ -151,6 +152,39 @@ def tail_split_for(M: int, N: int, K: int):
     return (int(lib.ptj_gemm_tail_split_rows(M, N, K)), int(n)) if n else None
 
 
+class _LayerPlan:
+    """Sizes of one layer's launches for a batch shape: where the saved activations lie in one allocation and the gradients in
+    another (each on a 256-byte boundary), and the workspace."""
+
+    def __init__(self, cfg: GPT2Config, dtype: torch.dtype, B: int, S: int, train: bool):
+        lib = _lib.lib()
+        T, D, F, es = B * S, cfg.dim, cfg.ffn, 2 if dtype == torch.bfloat16 else 4
+        self.shape = _lib.LayerShape(B, S, D, cfg.heads, F, _lib.PTJ_BF16 if es == 2 else _lib.PTJ_F32, int(train), cfg.dropout,
+                                     0, 0, 0)
+        ref = ctypes.byref(self.shape)
+        keep = int(lib.ptj_layer_keep_bits_bytes(ref))
+        stats = 4 * B * cfg.heads * S
+        # ln1, qkv, attn, row_max, row_sum, keep_bits, x_mid, ln2, h_pre, h_act (LayerActs after x), then the output
+        self.act_offsets, self.act_bytes = self._place(
+            [T * D * es, 3 * T * D * es, T * D * es, stats, stats, keep, T * D * es, T * D * es, T * F * es, T * F * es, T * D * es])
+        self.out_offset, self.out_bytes = self.act_offsets.pop(), T * D * es
+        # dh_pre, d_ln, d_attn, dqkv, then dx and dropout(dx) between the halves of a layer and between layers
+        self.grad_offsets, self.grad_bytes = self._place(
+            [T * F * es, T * D * es, T * D * es, 3 * T * D * es] + 4 * [T * D * es])
+        self.ws_floats, self.ws_least = ([int(lib.ptj_layer_workspace_bytes(ref, b, products)) // 4 for b in (0, 1)]
+                                         for products in (1, 0))
+        # the LayerNorm backward that also writes the dropped gradient and its column sums takes these widths
+        self.fused = D % 8 == 0 and D <= (2048 if es == 2 else 1024)
+
+    @staticmethod
+    def _place(sizes):
+        offsets, end = [], 0
+        for n in sizes:
+            offsets.append(end if n else -1)
+            end += -(-n // 256) * 256
+        return offsets, max(end, 1)
+
+
 class Gpt2Step:
     """One forward + backward pass. Gradients are written into caller-provided float32 tensors (``grads[name]``),
     so a trainer can hand in views of one flat buffer and overlap their reduction with the rest of backward."""
@@ -170,6 +204,9 @@ class Gpt2Step:
         # input gradients whose last round of tiles is mostly empty: that round's rows split over K, same launch
         self.tail_split = True
         self._ws2 = [None, None]
+        self._layer_names = [[f"l{l}.{n}" for n in LAYER_TENSORS] for l in range(cfg.layers)]
+        self._plans = {}    # (batch, seq, train) -> _LayerPlan
+        self._held = []     # workspaces that a recorded graph may still use
 
     # -- helpers --
     def _wgrad(self, dy2d, x2d, out, accumulate=False):
@@ -189,7 +226,40 @@ class Gpt2Step:
     def _workspace(self, floats: int):
         if self._ws is None or self._ws.numel() < floats:
             self._ws = torch.empty(floats, device="cuda", dtype=torch.float32)
+        self._hold_recorded()
         return self._ws
+
+    def _hold_recorded(self):
+        """A recorded graph keeps the address of the workspace: it stays allocated when a larger one takes its place."""
+        if torch.cuda.is_current_stream_capturing() and not any(h is self._ws for h in self._held):
+            self._held.append(self._ws)
+
+    def _layer_workspace(self, plan, backward: bool):
+        """(address, bytes) of the workspace of a layer's launches; without the part that only makes products faster where
+        that does not fit (as for a single product, operators.gemm)."""
+        need = plan.ws_floats[backward]
+        if self._ws is None or self._ws.numel() < need:
+            try:
+                self._ws = torch.empty(need, device="cuda", dtype=torch.float32)
+            except torch.OutOfMemoryError:
+                least = plan.ws_least[backward]
+                if self._ws is None or self._ws.numel() < least:
+                    self._ws = torch.empty(least, device="cuda", dtype=torch.float32)
+        self._hold_recorded()
+        return self._ws.data_ptr(), self._ws.numel() * 4
+
+    def _plan(self, B: int, S: int, train: bool):
+        key = (B, S, train)
+        plan = self._plans.get(key)
+        if plan is None:
+            plan = self._plans[key] = _LayerPlan(self.cfg, self.dtype, B, S, train)
+        return plan
+
+    def _native(self, plan) -> bool:
+        """A layer's launches come from one library call (ptj_layer_fwd, ptj_layer_bwd_*) unless a caller brackets every
+        product with events or has switched one of the variants above, which are sequences of their own."""
+        return (ops.GEMM_PROFILE is None and not self.split_gelu_bwd and self.pair_wgrads and self.tail_split
+                and plan.fused)
 
     def _wgrad2(self, first, second):
         """Two weight gradients (dy, x, out) in ONE launch of the thread-block-pair kernel when both qualify: their
@@ -259,8 +329,13 @@ class Gpt2Step:
             seeds = [0] * (1 + 3 * cfg.layers)
         x = ops.embed_fwd(ids_in, w["w_emb"], w["w_pos"], train, seeds[0], out_dtype=self.dtype, p=p).view(T, D)
         acts = {"layers": [], "row_kstart": row_kstart}
+        plan = self._plan(B, S, bool(train))
+        native = self._native(plan)
+        if native:
+            row_kstart = ops._check_kstart(row_kstart, B, S, x.device)
+            x = self._layers_fwd(plan, w, x, seeds, row_kstart, acts)
         tail = tail_split_for(T, D, cfg.ffn) if (self.tail_split and self.dtype == torch.bfloat16) else None
-        for l in range(cfg.layers):
+        for l in range(0 if native else cfg.layers):
             s_attn, s_res1, s_res2 = seeds[1 + 3 * l: 4 + 3 * l]
             g = lambda n: w.t[f"l{l}.{n}"]
             a = {"x": x}
@@ -286,6 +361,59 @@ class Gpt2Step:
         logits = torch.empty((T, self.vocab_ld), device=x.device, dtype=self.dtype)
         ops.gemm(acts["x_f"], w["w_emb"], bias=w["b_head"], out=logits, N=cfg.vocab, ldc=self.vocab_ld)
         return logits, acts
+
+    def _layers_fwd(self, plan, w: Weights, x, seeds, row_kstart, acts):
+        """All layers through ptj_layer_fwd: the saved activations of each are one allocation."""
+        lib, stream = _lib.lib(), ops._stream()
+        ws, ws_bytes = self._layer_workspace(plan, False)
+        ks = 0 if row_kstart is None else row_kstart.data_ptr()
+        t, seeds = w.t, [ops._seed(s_) for s_ in seeds]
+        at, shape, slab = x.data_ptr(), plan.shape, None
+        acts["row_kstart"] = row_kstart
+        for l, names in enumerate(self._layer_names):
+            slab = torch.empty(plan.act_bytes, device=x.device, dtype=torch.uint8)
+            base = slab.data_ptr()
+            weights = _lib.LayerWeights(*[t[n].data_ptr() for n in names])
+            saved = _lib.LayerActs(at, *[base + o if o >= 0 else 0 for o in plan.act_offsets])
+            shape.seed_attn, shape.seed_res1, shape.seed_res2 = seeds[1 + 3 * l: 4 + 3 * l]
+            out = base + plan.out_offset
+            _lib.check(lib.ptj_layer_fwd(shape, weights, saved, out, ks, ws, ws_bytes, stream), "ptj_layer_fwd")
+            acts["layers"].append((saved, slab, x))  # (the first layer's input is a tensor of its own)
+            at = out
+        if slab is None:
+            return x
+        return slab[plan.out_offset:plan.out_offset + plan.out_bytes].view(self.dtype).view(x.shape)
+
+    def _layers_bwd(self, plan, w: Weights, grads, acts, dx, dy, seeds, ready):
+        """All layers through ptj_layer_bwd_ffn and ptj_layer_bwd_attn; returns the gradient of the first one's input."""
+        lib, stream = _lib.lib(), ops._stream()
+        ws, ws_bytes = self._layer_workspace(plan, True)
+        ks = acts.get("row_kstart")
+        ks = 0 if ks is None else ks.data_ptr()
+        t, seeds = w.t, [ops._seed(s_) for s_ in seeds]
+        shape = plan.shape
+        # scratch shared by all layers, and the gradients of the residual stream in turn
+        slab = torch.empty(plan.grad_bytes, device=dx.device, dtype=torch.uint8)
+        base = slab.data_ptr()
+        dh_pre, d_ln, d_attn, dqkv, dx_a, dy_a, dx_b, dy_b = [base + o for o in plan.grad_offsets]
+        dx_p, dy_p = dx.data_ptr(), dy.data_ptr()
+        for l in range(len(self._layer_names) - 1, -1, -1):
+            names = self._layer_names[l]
+            saved = acts["layers"][l][0]
+            weights = _lib.LayerWeights(*[t[n].data_ptr() for n in names])
+            out = _lib.LayerGrads(*[grads[n].data_ptr() for n in names])
+            shape.seed_attn, shape.seed_res1, shape.seed_res2 = seeds[1 + 3 * l: 4 + 3 * l]
+            _lib.check(lib.ptj_layer_bwd_ffn(shape, weights, saved, out, dx_p, dy_p, dh_pre, d_ln, dx_a, dy_a, ws, ws_bytes,
+                                             stream), "ptj_layer_bwd_ffn")
+            ready([f"l{l}.{n}" for n in ("b2f", "w2", "b1f", "w1", "g2", "b2")])
+            below = l > 0
+            _lib.check(lib.ptj_layer_bwd_attn(shape, weights, saved, out, dx_a, dy_a, d_attn, dqkv, d_ln, dx_b,
+                                              dy_b if below else 0, grads[f"l{l - 1}.b2f"].data_ptr() if below else 0,
+                                              seeds[3 * l] if below else 0, ks, ws, ws_bytes, stream), "ptj_layer_bwd_attn")
+            ready([f"l{l}.{n}" for n in ("w_o", "w_qkv", "g1", "b1")])
+            dx_p, dy_p = dx_b, dy_b
+        o = plan.grad_offsets[6]
+        return slab[o:o + plan.out_bytes].view(self.dtype).view(dx.shape)
 
     # -- backward --
     def backward(self, w: Weights, grads: dict, dlogits: torch.Tensor, acts: dict, ids_in: torch.Tensor, train: bool,
@@ -313,7 +441,10 @@ class Gpt2Step:
                               colsum_out=grads[f"l{cfg.layers - 1}.b2f"] if (fuse and cfg.layers > 0) else None)
         ready(["g_f", "b_f"])
 
-        for l in reversed(range(cfg.layers)):
+        native = bool(acts["layers"]) and not isinstance(acts["layers"][0], dict)  # as the forward pass went
+        if native:
+            dx = self._layers_bwd(self._plan(B, S, bool(train)), w, grads, acts, dx, dy, seeds, ready)
+        for l in reversed(range(0 if native else cfg.layers)):
             s_attn, s_res1, s_res2 = seeds[1 + 3 * l: 4 + 3 * l]
             a = acts["layers"][l]
             g = lambda n: w[f"l{l}.{n}"]

@@ -110,10 +110,10 @@ def layernorm_bwd(dloss_dx, layer_params, x, want_dx=True, want_dp=True, dx_add=
     dg = db = scratch = None
     n_scratch = 0
     if want_dp:
-        dg = dgamma_out if dgamma_out is not None else torch.empty(dim, device=x.device, dtype=torch.float32)
-        db = dbeta_out if dbeta_out is not None else torch.empty(dim, device=x.device, dtype=torch.float32)
+        dg = dgamma_out if dgamma_out is not None else x.new_empty(dim, dtype=torch.float32)
+        db = dbeta_out if dbeta_out is not None else x.new_empty(dim, dtype=torch.float32)
         n_scratch = _lib.lib().ptj_layernorm_bwd_scratch_floats(rows, dim)
-        scratch = torch.empty(max(n_scratch, 1), device=x.device, dtype=torch.float32)
+        scratch = x.new_empty(max(n_scratch, 1), dtype=torch.float32)
     if dx_add is not None:
         dx_add = _cuda(dx_add, "dx_add")
     if dropped is not None:
@@ -240,13 +240,13 @@ def gemm(a, b, *, a_kmajor=True, b_kmajor=True, M=None, N=None, K=None, lda=None
             if ws_n == 0:
                 split_k = 1  # this shape has no bad last round
             elif workspace is None or workspace.numel() < ws_n:
-                workspace = torch.empty(ws_n, device=a.device, dtype=torch.float32)
+                workspace = a.new_empty(ws_n, dtype=torch.float32)
     if dtype == torch.float32 and out.dtype == torch.float32:
         # bf16 planes of both operands (and K parts): with them the product runs on the tensor cores, at float32 accuracy
         ws_n = lib.ptj_gemm_f32_workspace_floats(M, N, K, int(a_kmajor), int(b_kmajor))
         if ws_n and (workspace is None or workspace.numel() < ws_n):
             try:
-                workspace = torch.empty(ws_n, device=a.device, dtype=torch.float32)
+                workspace = a.new_empty(ws_n, dtype=torch.float32)
             except torch.OutOfMemoryError:  # 6 bytes per operand element: a product that fits without them still runs
                 workspace = None
     dargs = None
@@ -285,7 +285,7 @@ def gemm_grouped2(problems, K, *, a_kmajor=True, b_kmajor=True):
         split = int(pr.get("split_k", 1))
         ws = pr.get("workspace")
         if split > 1 and (ws is None or ws.numel() < split * M * N):
-            ws = torch.empty(split * M * N, device=a.device, dtype=torch.float32)
+            ws = a.new_empty(split * M * N, dtype=torch.float32)
             pr["workspace"] = ws
         descs.append(_lib.GemmProblem(_ptr(a), _ptr(b), _ptr(out), M, N, pr["lda"], pr["ldb"], out.stride(0), _dt(out),
                                       _lib.EPI_ACCUM if pr.get("accumulate") else _lib.EPI_NONE, split, _ptr(ws),
@@ -349,7 +349,7 @@ def attn_keep_bits(q, k, v, out, seed, stream_id=0, p=None, bits=None):
     if need == 0:
         return None
     if bits is None or bits.numel() * bits.element_size() < need:
-        bits = torch.empty(need // 4, device=q.device, dtype=torch.int32)
+        bits = q.new_empty(need // 4, dtype=torch.int32)
     _lib.check(_lib.lib().ptj_attn_keep_bits(_ptr(bits), ctypes.byref(sh), p, _seed(seed), stream_id, _dt(q), _stream()),
                "ptj_attn_keep_bits")
     return bits
@@ -480,7 +480,7 @@ def t_scaled_dot_prod_attn_fwd3_t(qkv: torch.Tensor, mask: torch.Tensor = None, 
     times the block-diagonal document mask and the padding mask of the reference's collator; None = causal."""
     qkv = _cuda(qkv, "qkv")
     q, k, v = qkv.unbind(dim=2)
-    out = torch.empty(q.shape, device=qkv.device, dtype=qkv.dtype)
+    out = qkv.new_empty(q.shape, dtype=qkv.dtype)
     m, l = attn_fwd(q, k, v, out, train, p_gen_aux, row_kstart=_kstart_or_none(mask))
     return out, [m, l, out]
 
@@ -493,7 +493,7 @@ def t_scaled_dot_prod_attn_bkwd3_t(dloss_dx, acts, qkv: torch.Tensor, mask: torc
     m, l, out = acts
     d_o = _cuda(dloss_dx, "dloss_dx").to(qkv.dtype).reshape(out.shape)
     out = _cuda(out)
-    dq, dk, dv = (torch.empty(q.shape, device=qkv.device, dtype=qkv.dtype) for _ in range(3))
+    dq, dk, dv = (qkv.new_empty(q.shape, dtype=qkv.dtype) for _ in range(3))
     attn_bwd(d_o, q, k, v, out, _cuda(m), _cuda(l), dq, dk, dv, train, p_gen_aux, row_kstart=_kstart_or_none(mask))
     return dq, dk, dv
 
@@ -506,11 +506,11 @@ def cross_entropy(labels, logits, cols=None, want_grad=True, in_place=False, n_v
     cols = ld if cols is None else cols
     rows = logits.numel() // ld
     labels = _cuda(labels, "labels").reshape(-1).to(torch.int32)
-    row_stats = torch.empty(2 * rows, device=logits.device, dtype=torch.float32)
-    out3 = torch.empty(3, device=logits.device, dtype=torch.float32)
+    row_stats = logits.new_empty(2 * rows, dtype=torch.float32)
+    out3 = logits.new_empty(3, dtype=torch.float32)
     count = n_valid is None
     if count:
-        n_valid = torch.empty(1, device=logits.device, dtype=torch.float32)
+        n_valid = logits.new_empty(1, dtype=torch.float32)
     dlogits = None
     if want_grad:
         dlogits = logits if in_place else torch.empty_like(logits)
@@ -562,7 +562,7 @@ def argmax_rows(x: torch.Tensor, cols=None) -> torch.Tensor:
     assert x.dim() == 2 and x.stride(1) == 1, "rows may be strided, elements of a row must be contiguous"
     rows, ld = x.shape[0], x.stride(0)
     cols = x.shape[1] if cols is None else cols
-    out = torch.empty(rows, device=x.device, dtype=torch.int32)
+    out = x.new_empty(rows, dtype=torch.int32)
     _lib.check(_lib.lib().ptj_argmax_rows(_ptr(x), _ptr(out), rows, cols, ld, _dt(x), _stream()), "ptj_argmax_rows")
     return out
 
@@ -593,7 +593,7 @@ def embed_fwd(ids, w_emb, w_pos, train, seed, stream_id=0, out_dtype=None, p=Non
     V, D = w_emb.shape
     ids = _cuda(ids, "ids").to(torch.int32)
     out_dtype = out_dtype or w_emb.dtype
-    y = torch.empty((B, S, D), device=w_emb.device, dtype=out_dtype)
+    y = w_emb.new_empty((B, S, D), dtype=out_dtype)
     p = DROPOUT_RATE if p is None else p
     _lib.check(
         _lib.lib().ptj_embed_fwd(_ptr(ids), _ptr(w_emb), _ptr(w_pos), _ptr(y), B, S, D, V, p, int(bool(train)),
@@ -620,9 +620,9 @@ def colsum(x2d, cols=None, out=None):
     rows, ld = x2d.shape
     cols = ld if cols is None else cols
     if out is None:
-        out = torch.empty(cols, device=x2d.device, dtype=torch.float32)
+        out = x2d.new_empty(cols, dtype=torch.float32)
     n = _lib.lib().ptj_colsum_scratch_floats(rows, cols)
-    scratch = torch.empty(max(n, 1), device=x2d.device, dtype=torch.float32)
+    scratch = x2d.new_empty(max(n, 1), dtype=torch.float32)
     _lib.check(_lib.lib().ptj_colsum(_ptr(x2d), _ptr(out), _ptr(scratch), n, rows, cols, ld, _dt(x2d), _stream()),
                "ptj_colsum")
     return out
@@ -635,9 +635,9 @@ def gelu_bwd_colsum(dy2d, x_preact2d, colsum_out=None, in_place=False):
     assert dy.dim() == 2 and dy.shape == x.shape and dy.dtype == x.dtype
     rows, cols = dy.shape
     dx = dy if in_place else torch.empty_like(dy)
-    out = colsum_out if colsum_out is not None else torch.empty(cols, device=dy.device, dtype=torch.float32)
+    out = colsum_out if colsum_out is not None else dy.new_empty(cols, dtype=torch.float32)
     n = _lib.lib().ptj_colsum_scratch_floats(rows, cols)
-    scratch = torch.empty(max(n, 1), device=dy.device, dtype=torch.float32)
+    scratch = dy.new_empty(max(n, 1), dtype=torch.float32)
     _lib.check(_lib.lib().ptj_gelu_bwd_colsum(_ptr(dy), _ptr(x), _ptr(dx), _ptr(out), _ptr(scratch), n, rows, cols, cols,
                                               _dt(dy), _stream()), "ptj_gelu_bwd_colsum")
     return dx, out

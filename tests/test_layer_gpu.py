@@ -1,0 +1,43 @@
+"""A layer's launches issued by one library call against the same launches issued one by one: the same bits."""
+import pytest
+import torch
+
+from conftest import pkg
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype,dim,heads,ffn,layers,B,S,p,packed", [
+    (torch.bfloat16, 128, 4, 512, 2, 4, 128, 0.0, False),   # 32-wide heads, no dropout: no keep flags
+    (torch.bfloat16, 256, 4, 1000, 3, 2, 200, 0.1, True),   # ragged rows, documents, an FFN width that fills no tile
+    (torch.bfloat16, 768, 12, 3072, 1, 8, 1024, 0.1, False),  # tail splits, pairs of weight gradients, K parts
+    (torch.bfloat16, 64, 1, 192, 0, 1, 64, 0.1, False),     # no layer at all
+    (torch.float32, 256, 2, 512, 2, 2, 96, 0.1, True),
+    (torch.float32, 40, 5, 72, 1, 3, 17, 0.1, False),       # everything on the general kernels
+])
+@pytest.mark.parametrize("train", [True, False])
+def test_same_bits_as_single_launches(dtype, dim, heads, ffn, layers, B, S, p, packed, train):
+    ops, gpt2 = pkg("operators"), pkg("gpt2")
+    cfg = gpt2.GPT2Config(vocab=304, dim=dim, layers=layers, heads=heads, ffn=ffn, seq=S, dropout=p)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    flat = [0.05 * torch.randn(s, generator=g, device="cuda") + (1.0 if gpt2.base_name(n)[0] == "g" else 0.0)
+            for n, s in cfg.param_shapes()]
+    w = gpt2.Weights.from_pytree(gpt2.unflatten_like(flat, cfg), cfg, dtype)
+    y = torch.randint(1, 304, (B, S + 1), generator=g, device="cuda", dtype=torch.int32)
+    ks = ops.row_kstart_from_lengths([[max(1, S // 3), S // 2]] * B, S) if packed else None
+    seeds = list(range(5, 6 + 3 * layers))
+    results = []
+    try:
+        for single in (False, True):
+            ops.GEMM_PROFILE = [] if single else None
+            step, ready = gpt2.Gpt2Step(cfg, dtype), []
+            grads = {n: torch.full(s, 3.0, device="cuda") for n, s in cfg.param_shapes()}
+            stats = step.loss_and_grads(w, grads, y, train, seeds, row_kstart=ks, on_ready=ready.extend)
+            results.append([stats] + [grads[n] for n, _ in cfg.param_shapes()])
+            assert sorted(ready) == sorted(grads)
+            logits, _ = step.forward(w, y[:, :-1].contiguous(), train, seeds, row_kstart=ks)
+            results[-1].append(logits[:, :304])
+    finally:
+        ops.GEMM_PROFILE = None
+    assert ops.last_kernel_fault() == 0
+    assert all(torch.equal(a, b) for a, b in zip(*results))
