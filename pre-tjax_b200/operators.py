@@ -240,13 +240,13 @@ def gemm(a, b, *, a_kmajor=True, b_kmajor=True, M=None, N=None, K=None, lda=None
             if ws_n == 0:
                 split_k = 1  # this shape has no bad last round
             elif workspace is None or workspace.numel() < ws_n:
-                workspace = a.new_empty(ws_n, dtype=torch.float32)
+                workspace = torch.empty(ws_n, device=a.device, dtype=torch.float32)
     if dtype == torch.float32 and out.dtype == torch.float32:
         # bf16 planes of both operands (and K parts): with them the product runs on the tensor cores, at float32 accuracy
         ws_n = lib.ptj_gemm_f32_workspace_floats(M, N, K, int(a_kmajor), int(b_kmajor))
         if ws_n and (workspace is None or workspace.numel() < ws_n):
             try:
-                workspace = a.new_empty(ws_n, dtype=torch.float32)
+                workspace = torch.empty(ws_n, device=a.device, dtype=torch.float32)
             except torch.OutOfMemoryError:  # 6 bytes per operand element: a product that fits without them still runs
                 workspace = None
     dargs = None
@@ -285,7 +285,7 @@ def gemm_grouped2(problems, K, *, a_kmajor=True, b_kmajor=True):
         split = int(pr.get("split_k", 1))
         ws = pr.get("workspace")
         if split > 1 and (ws is None or ws.numel() < split * M * N):
-            ws = a.new_empty(split * M * N, dtype=torch.float32)
+            ws = torch.empty(split * M * N, device=a.device, dtype=torch.float32)
             pr["workspace"] = ws
         descs.append(_lib.GemmProblem(_ptr(a), _ptr(b), _ptr(out), M, N, pr["lda"], pr["ldb"], out.stride(0), _dt(out),
                                       _lib.EPI_ACCUM if pr.get("accumulate") else _lib.EPI_NONE, split, _ptr(ws),
