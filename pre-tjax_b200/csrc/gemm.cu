@@ -59,6 +59,7 @@ struct GemmParams {
   EpilogueParams ep;
   int64_t M, N, K;
   int num_m, num_n, num_kb, split_k;
+  int n_first;       // pair kernel: tiles along N follow one another (else along M)
   float* workspace;  // [split_k, M, N] partial sums when split_k > 1
   int out_bf16;
   int tma_store;  // outputs leave through tensor-map tile stores (bf16 output, 16-byte aligned rows, K not split)
@@ -511,7 +512,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         const int li = second ? item - items1 : item;
         const int tiles = q.num_m * q.num_n;
         const int split = li / tiles, tile = li - split * tiles;
-        const int m_blk = tile % q.num_m, n_blk = tile / q.num_m;
+        const int m_blk = q.n_first ? tile / q.num_n : tile % q.num_m, n_blk = q.n_first ? tile % q.num_n : tile / q.num_m;
         int kb0 = 0, kb1 = q.num_kb;  // (64-bit divisions only when K is split)
         if (q.split_k > 1) {
           kb0 = static_cast<int>(static_cast<int64_t>(split) * q.num_kb / q.split_k);
@@ -598,7 +599,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       const int li = second ? item - items1 : item;
       const int tiles = q.num_m * q.num_n;
       const int split = li / tiles, tile = li - split * tiles;
-      const int m_blk = tile % q.num_m, n_blk = tile / q.num_m;
+      const int m_blk = q.n_first ? tile / q.num_n : tile % q.num_m, n_blk = q.n_first ? tile % q.num_n : tile / q.num_m;
       const int buf = it & 1;
       const uint32_t aphase = (it >> 1) & 1u;
       float* wbias = bias_smem + (warp - kFirstEpilogueWarp) * (kChunks * 32);
@@ -828,7 +829,8 @@ splitk_finish_kernel(const float* __restrict__ ws, const EpilogueParams ep, int 
 
 // A product whose last round of 256 x 256 tiles would leave most of the 74 thread-block pairs idle (96 tiles: 74 + 22):
 // head rows that fill whole rounds, and the K parts for the remaining rows so that they fill one more round of short
-// work items. parts == 0: no split (the product does not go to the pair kernel, or its last round is >= 60 % full).
+// work items. parts == 0: no split (the product does not go to the pair kernel, or its last round is >= 60 % full). Half a
+// round of tiles or less (short batches: 36 tiles at [3072, 768]) is split over K whole.
 struct TailPlan { int64_t head_rows; int parts; };
 TailPlan tail_split_plan(int64_t M, int64_t N, int64_t K) {
   TailPlan none{0, 0};
@@ -836,7 +838,13 @@ TailPlan tail_split_plan(int64_t M, int64_t N, int64_t K) {
   const int64_t pairs = kNumSMs / 2;
   const int64_t num_m = ceil_div(M, 256), num_n = ceil_div(N, 256), tiles = num_m * num_n;
   const int64_t full = tiles / pairs, rest = tiles % pairs;
-  if (full < 1 || rest == 0 || rest > 44) return none;
+  if (full == 0) {  // fewer tiles than pairs: all rows, in as many parts as leave no pair without work
+    int64_t parts = pairs / tiles;
+    if (parts > 8) parts = 8;
+    if (parts > K / 64 / 4) parts = K / 64 / 4;
+    return parts >= 2 ? TailPlan{0, static_cast<int>(parts)} : none;
+  }
+  if (rest == 0 || rest > 44) return none;
   const int64_t head_mb = full * pairs / num_n, tail_tiles = (num_m - head_mb) * num_n;
   if (head_mb < 1 || tail_tiles < 1) return none;
   int64_t parts = (2 * pairs + tail_tiles) / (2 * tail_tiles);  // pairs / tail_tiles, rounded
@@ -1038,6 +1046,11 @@ extern "C" int ptj_gemm(const void* a, const void* b, void* c, const float* bias
   if (use_pair_kernel(M, N, K)) {
     p.num_m = static_cast<int>(ceil_div(M, 2 * BM));
     p.num_n = static_cast<int>(ceil_div(N, 256));
+    // Tiles along M run side by side and share their B rows, while A stays in the L2 for the next column of tiles. An A that
+    // does not fit there is read from memory once per column: then the tiles of a row of them run side by side. LM-head weight
+    // gradient [50257, 8192] x [8192, 768] (A 823 MB): 517 -> 442 us; weight gradients of a layer (A 13 to 50 MB) lose:
+    // 36.7 -> 45.4 us at [3072, 8192] x [8192, 768].
+    p.n_first = static_cast<double>(M) * static_cast<double>(K) * 2.0 > 126e6;
     CUtensorMap ta, tb;
     if (!make_pair_operand_maps(&ta, &tb, a, b, M, N, K, lda, ldb, a_kmajor != 0, b_kmajor != 0)) return PTJ_ERR_LAUNCH;
     // PTJ_SPLIT_TAIL: the rows of a mostly-empty last round of tiles become a second product of the same launch,
