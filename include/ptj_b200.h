@@ -223,12 +223,12 @@ size_t ptj_gemm_f32_workspace_floats(int64_t M, int64_t N, int64_t K, int a_kmaj
 
 /* split_k = PTJ_SPLIT_TAIL lets ptj_gemm even out a bad last round of tiles: a bf16 product on the 256 x 256-tile
  * thread-block-pair kernel whose tile count leaves most of the GPU idle in its last round (96 tiles on 74 pairs) runs
- * as head rows that fill whole rounds (none where half of the pairs or more would get no tile at all) plus, in the same
- * launch, the remaining rows split over K; a finishing kernel sums those parts in a fixed order and applies the epilogue. Epilogues PTJ_EPI_NONE (no bias) and
+ * as head rows that fill whole rounds plus, in the same launch, the remaining rows split over K; a finishing kernel
+ * sums those parts in a fixed order and applies the epilogue. Epilogues PTJ_EPI_NONE (no bias) and
  * PTJ_EPI_DROPOUT_RESID (K-major operands, 16-byte aligned bf16 rows); anything else, or a workspace smaller than
  * ptj_gemm_tail_split_floats(M, N, K) floats, runs unsplit. Head rows are bit-identical to the unsplit product, the
- * rest differs by the summation order. ptj_gemm_tail_split_rows: the first row of the split range (0 also where
- * ptj_gemm_tail_split_floats is 0 and there is none). */
+ * rest differs by the summation order. ptj_gemm_tail_split_rows: the first row of the split range (0: no split for
+ * this shape). */
 #define PTJ_SPLIT_TAIL (-1)
 size_t ptj_gemm_tail_split_floats(int64_t M, int64_t N, int64_t K);
 int64_t ptj_gemm_tail_split_rows(int64_t M, int64_t N, int64_t K);

@@ -829,8 +829,8 @@ splitk_finish_kernel(const float* __restrict__ ws, const EpilogueParams ep, int 
 
 // A product whose last round of 256 x 256 tiles would leave most of the 74 thread-block pairs idle (96 tiles: 74 + 22):
 // head rows that fill whole rounds, and the K parts for the remaining rows so that they fill one more round of short
-// work items. parts == 0: no split (the product does not go to the pair kernel, or its last round is >= 60 % full). Half a
-// round of tiles or less (short batches: 36 tiles at [3072, 768]) is split over K whole.
+// work items. parts == 0: no split (the product does not go to the pair kernel, or its last round is >= 60 % full). Fewer
+// tiles than pairs split over K whole (36 tiles at [3072, 768]) gained nothing over the finishing pass: forward pass 1.49 ms either way.
 struct TailPlan { int64_t head_rows; int parts; };
 TailPlan tail_split_plan(int64_t M, int64_t N, int64_t K) {
   TailPlan none{0, 0};
@@ -838,13 +838,7 @@ TailPlan tail_split_plan(int64_t M, int64_t N, int64_t K) {
   const int64_t pairs = kNumSMs / 2;
   const int64_t num_m = ceil_div(M, 256), num_n = ceil_div(N, 256), tiles = num_m * num_n;
   const int64_t full = tiles / pairs, rest = tiles % pairs;
-  if (full == 0) {  // fewer tiles than pairs: all rows, in as many parts as leave no pair without work
-    int64_t parts = pairs / tiles;
-    if (parts > 8) parts = 8;
-    if (parts > K / 64 / 4) parts = K / 64 / 4;
-    return parts >= 2 ? TailPlan{0, static_cast<int>(parts)} : none;
-  }
-  if (rest == 0 || rest > 44) return none;
+  if (full < 1 || rest == 0 || rest > 44) return none;
   const int64_t head_mb = full * pairs / num_n, tail_tiles = (num_m - head_mb) * num_n;
   if (head_mb < 1 || tail_tiles < 1) return none;
   int64_t parts = (2 * pairs + tail_tiles) / (2 * tail_tiles);  // pairs / tail_tiles, rounded
