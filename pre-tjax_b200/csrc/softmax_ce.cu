@@ -2,6 +2,8 @@
 // One thread block owns one row at a time. Pass 1 is an online max / sum-of-exponentials over 16-byte vectors
 // (Milakov & Gimelshein, "Online normalizer calculation for softmax"); pass 2 re-reads the row (it is still in
 // L2: a row of 50257 bf16 is 100 KB) and writes the result with plain vector stores. No atomics, no helper tensors.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace ptj {
@@ -316,6 +318,32 @@ struct Shifted {
   __device__ __forceinline__ float operator()(float x) const { return EXACT ? (x + c) * kLog2e : fmaf(x, kLog2e, c); }
 };
 
+// dlogits = 2^arg(x) k, as two factors where the shift is exact and in the exponent where it is not
+template <bool EXACT>
+struct Scaled {
+  Shifted<EXACT> arg;
+  float k, c3;
+  uint64_t k2, c32;
+  __device__ __forceinline__ Scaled(const Shifted<EXACT>& a, float k_)
+      : arg(a), k(k_), c3(EXACT ? a.c : a.c + log2f(k_)), k2(f2_pack(k_, k_)), c32(f2_pack(c3, c3)) {}
+  __device__ __forceinline__ uint4 operator()(const uint4& a) const {
+    const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+    uint32_t o[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float y0, y1;
+      f2_unpack(EXACT ? arg(bf2_as_f2(w[q])) : f2_fma(bf2_as_f2(w[q]), arg.l2e2, c32), y0, y1);
+      y0 = ex2_approx(y0);
+      y1 = ex2_approx(y1);
+      if (EXACT) f2_unpack(f2_mul(f2_pack(y0, y1), k2), y0, y1);
+      __nv_bfloat162 h = __floats2bfloat162_rn(y0, y1);
+      o[q] = *reinterpret_cast<uint32_t*>(&h);
+    }
+    return make_uint4(o[0], o[1], o[2], o[3]);
+  }
+  __device__ __forceinline__ float operator()(float x) const { return EXACT ? ex2_approx(arg(x)) * k : ex2_approx(fmaf(x, kLog2e, c3)); }
+};
+
 // sum over the row of 2^arg(x) (every thread gets it)
 template <bool EXACT>
 __device__ __forceinline__ float row_expsum_bf16(const __nv_bfloat16* xr, const RowEnds& re, const Shifted<EXACT>& arg,
@@ -340,9 +368,10 @@ __device__ __forceinline__ float row_expsum_bf16(const __nv_bfloat16* xr, const 
   return block_sum((s0 + s1) + (s2 + s3), red);
 }
 
+// Rows wider than the kernels below take.
 template <bool PHASED>
 __global__ void __launch_bounds__(kCeThreads, 3)
-cross_entropy_bf16_kernel(const int32_t* __restrict__ labels, const __nv_bfloat16* logits, __nv_bfloat16* dlogits,
+cross_entropy_bf16_wide_kernel(const int32_t* __restrict__ labels, const __nv_bfloat16* logits, __nv_bfloat16* dlogits,
                           float* __restrict__ row_stats, const float* __restrict__ n_valid, int64_t rows, int cols,
                           int64_t ld) {
   grid_dep_sync();
@@ -386,33 +415,263 @@ cross_entropy_bf16_kernel(const int32_t* __restrict__ labels, const __nv_bfloat1
     if (dr == nullptr) continue;
     // pass 3: dlogits = softmax / n_valid, the label's column minus 1 / n_valid
     const float k = inv_n / s;
-    const float c3 = PHASED ? arg.c : arg.c + log2f(k);
-    const uint64_t c32 = f2_pack(c3, c3), k2 = f2_pack(k, k);
+    const Scaled<PHASED> grad(arg, k);
     uint4* dv = reinterpret_cast<uint4*>(dr + re.head);
-    auto grad8 = [&](const uint4& a) {
-      const uint32_t w[4] = {a.x, a.y, a.z, a.w};
-      uint32_t o[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        float y0, y1;
-        f2_unpack(PHASED ? arg(bf2_as_f2(w[q])) : f2_fma(bf2_as_f2(w[q]), arg.l2e2, c32), y0, y1);
-        y0 = ex2_approx(y0);
-        y1 = ex2_approx(y1);
-        if (PHASED) f2_unpack(f2_mul(f2_pack(y0, y1), k2), y0, y1);
-        __nv_bfloat162 h = __floats2bfloat162_rn(y0, y1);
-        o[q] = *reinterpret_cast<uint32_t*>(&h);
-      }
-      return make_uint4(o[0], o[1], o[2], o[3]);
-    };
-    auto grad1 = [&](float x) { return PHASED ? ex2_approx(arg(x)) * k : ex2_approx(fmaf(x, kLog2e, c3)); };
-    for (int i = threadIdx.x; i < nvec; i += kCeThreads) dv[i] = grad8(xv[i]);
+    for (int i = threadIdx.x; i < nvec; i += kCeThreads) dv[i] = grad(xv[i]);
     for (int t = threadIdx.x; t < re.n; t += kCeThreads) {
       const int c = re.col(t);
-      dr[c] = __float2bfloat16_rn(grad1(__bfloat162float(xr[c])));
+      dr[c] = __float2bfloat16_rn(grad(__bfloat162float(xr[c])));
     }
     __syncthreads();  // the label's column has been written (by whichever thread owns it) before it is patched
-    if (threadIdx.x == 0) dr[label] = __float2bfloat16_rn(grad1(x_label) - inv_n);
+    if (threadIdx.x == 0) dr[label] = __float2bfloat16_rn(grad(x_label) - inv_n);
   }
+}
+
+// The same three passes over a row held in registers: kCeVecs vectors a thread, NT (256 or 512) threads a row, 1024 an SM. Every
+// thread copies the vectors it will need of the block's next row into shared memory while the current row is worked on, and
+// reads back only what it copied itself. Reading the row three times from L2 had the loads of each pass wait in turn. Device and
+// calls, before -> after: [8192, 8000] 105 -> 70 us, [8192, 14336] 131 -> 97, [8192, 1000] 57 -> 44, [4096, 20001] 92 -> 86.
+constexpr int kCeVecs = 7;
+template <int NT>
+__device__ __forceinline__ float rows_max(float v, float* red) {  // one barrier: every warp reduces the warps' values
+  v = warp_max(v);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  return warp_max((threadIdx.x & 31) < NT / 32 ? red[threadIdx.x & 31] : -INFINITY);
+}
+template <int NT>
+__device__ __forceinline__ float rows_sum(float v, float* red) {
+  v = warp_sum(v);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  return warp_sum((threadIdx.x & 31) < NT / 32 ? red[threadIdx.x & 31] : 0.f);
+}
+
+template <bool PHASED, int NT>
+__global__ void __launch_bounds__(NT, 1024 / NT)
+cross_entropy_bf16_kernel(const int32_t* __restrict__ labels, const __nv_bfloat16* logits, __nv_bfloat16* dlogits,
+                          float* __restrict__ row_stats, const float* __restrict__ n_valid, int64_t rows, int cols,
+                          int64_t ld) {
+  grid_dep_sync();
+  extern __shared__ uint4 next_s[];  // [kCeVecs][NT]
+  __shared__ float red[2][32];
+  const int tid = threadIdx.x;
+  const float inv_n = 1.f / *n_valid;
+  const uint32_t slot = static_cast<uint32_t>(__cvta_generic_to_shared(next_s + tid));
+  auto counts = [&](int label) { return label > 0 && label < cols; };
+  auto fetch = [&](int64_t row) {  // this thread's vectors of a row that counts
+    if (row < rows && counts(labels[row])) {
+      const __nv_bfloat16* xr = logits + row * ld;
+      const RowEnds re(cols, PHASED ? head_bf16(xr) : 0);
+      const uint4* xv = reinterpret_cast<const uint4*>(xr + re.head) + tid;
+#pragma unroll
+      for (int j = 0; j < kCeVecs; ++j)
+        if (tid + j * NT < re.nvec)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(slot + j * NT * 16), "l"(xv + j * NT) : "memory");
+    }
+  };
+  fetch(blockIdx.x);
+  for (int64_t row = blockIdx.x; row < rows; row += gridDim.x) {
+    const __nv_bfloat16* xr = logits + row * ld;
+    const RowEnds re(cols, PHASED ? head_bf16(xr) : 0);
+    const int nvec = re.nvec;
+    __nv_bfloat16* dr = dlogits != nullptr ? dlogits + row * ld : nullptr;
+    uint4* dv = dr != nullptr ? reinterpret_cast<uint4*>(dr + re.head) : nullptr;
+    const int label = labels[row];
+    if (!counts(label)) {  // padding (or an id outside the vocabulary): no contribution
+      fetch(row + gridDim.x);
+      if (tid == 0) {
+        row_stats[row] = 0.f;
+        row_stats[rows + row] = 0.f;
+      }
+      if (dr != nullptr) {
+        for (int i = tid; i < nvec; i += NT) dv[i] = make_uint4(0u, 0u, 0u, 0u);
+        for (int t = tid; t < re.n; t += NT) dr[re.col(t)] = __float2bfloat16_rn(0.f);
+      }
+      continue;
+    }
+    const float x_label = __bfloat162float(xr[label]);  // read before the row is overwritten in place
+    const bool ends = tid < re.n;                       // re.n <= 14: one element a thread
+    const int end_col = ends ? re.col(tid) : 0;
+    const float x_end = ends ? __bfloat162float(xr[end_col]) : -INFINITY;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    uint4 v[kCeVecs];
+    uint32_t pm = 0xff80ff80u;  // two packed -inf: what a vector beyond the row holds
+#pragma unroll
+    for (int j = 0; j < kCeVecs; ++j) {
+      v[j] = make_uint4(0xff80ff80u, 0xff80ff80u, 0xff80ff80u, 0xff80ff80u);
+      if (tid + j * NT < nvec) v[j] = next_s[tid + j * NT];
+    }
+    // pass 1: maximum
+#pragma unroll
+    for (int j = 0; j < kCeVecs; ++j) pm = bf2_max(pm, bf2_max(bf2_max(v[j].x, v[j].y), bf2_max(v[j].z, v[j].w)));
+    const float m = rows_max<NT>(fmaxf(fmaxf(__uint_as_float(pm << 16), __uint_as_float(pm & 0xffff0000u)), x_end), red[0]);
+    fetch(row + gridDim.x);  // (the vectors are in registers: the maximum was formed from them)
+    // is the label the first column that attains the maximum?
+    float hit = 0.f;
+    if (x_label == m) {  // (uniform over the block)
+      int earlier = 0;
+      for (int c = tid; c < label; c += NT) earlier |= (__bfloat162float(xr[c]) == m) ? 1 : 0;
+      hit = __syncthreads_or(earlier) ? 0.f : 1.f;
+    }
+    // pass 2: sum of exponentials
+    const Shifted<PHASED> arg(m);
+    float s0 = ends ? ex2_approx(arg(x_end)) : 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll
+    for (int j = 0; j < kCeVecs; ++j) {
+      if (j * NT >= nvec) break;
+      float e0, e1, e2, e3, e4, e5, e6, e7;
+      f2_unpack(arg(bf2_as_f2(v[j].x)), e0, e1);
+      f2_unpack(arg(bf2_as_f2(v[j].y)), e2, e3);
+      f2_unpack(arg(bf2_as_f2(v[j].z)), e4, e5);
+      f2_unpack(arg(bf2_as_f2(v[j].w)), e6, e7);
+      if (tid + j * NT < nvec) {  // (a row whose maximum is -inf must not take the filler for one of its elements)
+        s0 += ex2_approx(e0) + ex2_approx(e1);
+        s1 += ex2_approx(e2) + ex2_approx(e3);
+        s2 += ex2_approx(e4) + ex2_approx(e5);
+        s3 += ex2_approx(e6) + ex2_approx(e7);
+      }
+    }
+    const float s = rows_sum<NT>((s0 + s1) + (s2 + s3), red[1]);
+    if (tid == 0) {
+      row_stats[row] = -(x_label - m - logf(s));
+      row_stats[rows + row] = hit;
+    }
+    if (dr == nullptr) continue;
+    // pass 3: dlogits = softmax / n_valid, the label's column minus 1 / n_valid
+    const float k = inv_n / s;
+    const Scaled<PHASED> grad(arg, k);
+#pragma unroll
+    for (int j = 0; j < kCeVecs; ++j)
+      if (tid + j * NT < nvec) dv[tid + j * NT] = grad(v[j]);
+    if (ends) dr[end_col] = __float2bfloat16_rn(grad(x_end));
+    // the label's column, by the thread that has just written it
+    const int lv = label - re.head;
+    const bool in_vec = lv >= 0 && lv < nvec * 8;
+    if (in_vec ? (lv >> 3) % NT == tid : (ends && end_col == label)) dr[label] = __float2bfloat16_rn(grad(x_label) - inv_n);
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+// Rows too wide for the registers of half an SM's threads: the row stays in shared memory, two blocks of 512 threads an SM, so
+// that one block's barriers hide behind the other's arithmetic. A thread's vectors of the next row replace those of this
+// row as the last pass lets go of them. Before -> after: [8192, 50257] 376 -> 335 us, padded rows 363 -> 313, [8192, 35374]
+// 265 -> 257 (a whole SM's 1024 threads on one row in registers: 368, 333, 298). Two exponentials an element keep the
+// special-function unit busy for 177 us of it.
+constexpr int kCeRowThreads = 512;
+constexpr int kCeSmemCols = 57344;  // two rows of bf16 an SM
+template <bool PHASED>
+__global__ void __launch_bounds__(kCeRowThreads, 2)
+cross_entropy_bf16_smem_kernel(const int32_t* __restrict__ labels, const __nv_bfloat16* logits, __nv_bfloat16* dlogits,
+                               float* __restrict__ row_stats, const float* __restrict__ n_valid, int64_t rows, int cols,
+                               int64_t ld) {
+  grid_dep_sync();
+  constexpr int NT = kCeRowThreads;
+  extern __shared__ uint4 row_s[];  // this thread's vectors: row_s[tid + j * NT]
+  __shared__ float red[2][32];
+  const int tid = threadIdx.x;
+  const float inv_n = 1.f / *n_valid;
+  const uint32_t slot = static_cast<uint32_t>(__cvta_generic_to_shared(row_s));
+  auto counts = [&](int label) { return label > 0 && label < cols; };
+  struct Next {
+    const uint4* v;
+    int nvec;
+  };
+  auto find = [&](int64_t row) {  // the vectors of a row, none where it does not count
+    Next n{nullptr, 0};
+    if (row < rows && counts(labels[row])) {
+      const __nv_bfloat16* xr = logits + row * ld;
+      const RowEnds re(cols, PHASED ? head_bf16(xr) : 0);
+      n = Next{reinterpret_cast<const uint4*>(xr + re.head), re.nvec};
+    }
+    return n;
+  };
+  auto fetch = [&](const Next& n, int i) {
+    if (i < n.nvec) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(slot + i * 16), "l"(n.v + i) : "memory");
+  };
+  {
+    const Next first = find(blockIdx.x);
+    for (int i = tid; i < first.nvec; i += NT) fetch(first, i);
+  }
+  for (int64_t row = blockIdx.x; row < rows; row += gridDim.x) {
+    const __nv_bfloat16* xr = logits + row * ld;
+    const RowEnds re(cols, PHASED ? head_bf16(xr) : 0);
+    const int nvec = re.nvec;
+    __nv_bfloat16* dr = dlogits != nullptr ? dlogits + row * ld : nullptr;
+    uint4* dv = dr != nullptr ? reinterpret_cast<uint4*>(dr + re.head) : nullptr;
+    const Next next = find(row + gridDim.x);
+    const int label = labels[row];
+    if (!counts(label)) {  // padding (or an id outside the vocabulary): no contribution
+      for (int i = tid; i < next.nvec; i += NT) fetch(next, i);
+      if (tid == 0) {
+        row_stats[row] = 0.f;
+        row_stats[rows + row] = 0.f;
+      }
+      if (dr != nullptr) {
+        for (int i = tid; i < nvec; i += NT) dv[i] = make_uint4(0u, 0u, 0u, 0u);
+        for (int t = tid; t < re.n; t += NT) dr[re.col(t)] = __float2bfloat16_rn(0.f);
+      }
+      continue;
+    }
+    const float x_label = __bfloat162float(xr[label]);  // read before the row is overwritten in place
+    const bool ends = tid < re.n;                       // re.n <= 14: one element a thread
+    const int end_col = ends ? re.col(tid) : 0;
+    const float x_end = ends ? __bfloat162float(xr[end_col]) : -INFINITY;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    uint32_t pm = 0xff80ff80u;  // two packed -inf
+#pragma unroll 4
+    for (int i = tid; i < nvec; i += NT) {
+      const uint4 a = row_s[i];
+      pm = bf2_max(pm, bf2_max(bf2_max(a.x, a.y), bf2_max(a.z, a.w)));
+    }
+    const float m = rows_max<NT>(fmaxf(fmaxf(__uint_as_float(pm << 16), __uint_as_float(pm & 0xffff0000u)), x_end), red[0]);
+    // is the label the first column that attains the maximum?
+    float hit = 0.f;
+    if (x_label == m) {  // (uniform over the block)
+      int earlier = 0;
+      for (int c = tid; c < label; c += NT) earlier |= (__bfloat162float(xr[c]) == m) ? 1 : 0;
+      hit = __syncthreads_or(earlier) ? 0.f : 1.f;
+    }
+    const Shifted<PHASED> arg(m);
+    float s0 = ends ? ex2_approx(arg(x_end)) : 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll 2
+    for (int i = tid; i < nvec; i += NT) {
+      const uint4 a = row_s[i];
+      if (dr == nullptr) fetch(next, i);  // (the last pass over this vector)
+      float e0, e1, e2, e3, e4, e5, e6, e7;
+      f2_unpack(arg(bf2_as_f2(a.x)), e0, e1);
+      f2_unpack(arg(bf2_as_f2(a.y)), e2, e3);
+      f2_unpack(arg(bf2_as_f2(a.z)), e4, e5);
+      f2_unpack(arg(bf2_as_f2(a.w)), e6, e7);
+      s0 += ex2_approx(e0) + ex2_approx(e1);
+      s1 += ex2_approx(e2) + ex2_approx(e3);
+      s2 += ex2_approx(e4) + ex2_approx(e5);
+      s3 += ex2_approx(e6) + ex2_approx(e7);
+    }
+    const float s = rows_sum<NT>((s0 + s1) + (s2 + s3), red[1]);
+    if (tid == 0) {
+      row_stats[row] = -(x_label - m - logf(s));
+      row_stats[rows + row] = hit;
+    }
+    if (dr != nullptr) {
+      const float k = inv_n / s;
+      const Scaled<PHASED> grad(arg, k);
+#pragma unroll 2
+      for (int i = tid; i < nvec; i += NT) {
+        dv[i] = grad(row_s[i]);
+        fetch(next, i);
+      }
+      if (ends) dr[end_col] = __float2bfloat16_rn(grad(x_end));
+      // the label's column, by the thread that has just written it
+      const int lv = label - re.head;
+      const bool in_vec = lv >= 0 && lv < nvec * 8;
+      if (in_vec ? (lv >> 3) % NT == tid : (ends && end_col == label)) dr[label] = __float2bfloat16_rn(grad(x_label) - inv_n);
+    }
+    // rows may differ by a vector (the phase moves): one that only the next row has
+    const int j = tid + (nvec - tid + NT - 1) / NT * NT;
+    if (nvec >= 0 && j < next.nvec && j >= nvec) fetch(next, j);
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 // log-softmax forward / backward on the same three-pass scheme (bf16, every row on a 16-byte boundary)
@@ -614,11 +873,40 @@ extern "C" int ptj_cross_entropy(const int32_t* labels, const void* logits, void
     launch_k(cross_entropy_kernel<float>, row_grid(rows), kRowThreads, 0, st, 
         labels, static_cast<const float*>(logits), static_cast<float*>(dlogits), row_stats, n_valid, rows, cols, ld,
         same_phase<float>(logits, ld, dlogits, ld));
+  } else if (same_phase<__nv_bfloat16>(logits, ld, dlogits, ld) && cols <= 512 * kCeVecs * 8 &&
+             reinterpret_cast<uintptr_t>(logits) % 2 == 0) {
+    const bool aligned = aligned16(logits) && ld % 8 == 0;  // (the gradient is in the same phase)
+    auto launch = [&](auto nt) -> int {
+      constexpr int NT = decltype(nt)::value;
+      constexpr int kSmem = kCeVecs * NT * 16;
+      const auto kern = aligned ? cross_entropy_bf16_kernel<false, NT> : cross_entropy_bf16_kernel<true, NT>;
+      if (kSmem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return PTJ_ERR_LAUNCH;
+      }
+      const int64_t cap = static_cast<int64_t>(kNumSMs) * (1024 / NT);
+      launch_k(kern, static_cast<int>(rows < cap ? rows : cap), NT, kSmem, st, labels, static_cast<const __nv_bfloat16*>(logits),
+               static_cast<__nv_bfloat16*>(dlogits), row_stats, n_valid, rows, static_cast<int>(cols), ld);
+      return PTJ_OK;
+    };
+    const int rc = cols <= 256 * kCeVecs * 8 ? launch(std::integral_constant<int, 256>())
+                                             : launch(std::integral_constant<int, 512>());
+    if (rc != PTJ_OK) return rc;
+  } else if (same_phase<__nv_bfloat16>(logits, ld, dlogits, ld) && cols <= kCeSmemCols && reinterpret_cast<uintptr_t>(logits) % 2 == 0) {
+    const auto kern = aligned16(logits) && ld % 8 == 0 ? cross_entropy_bf16_smem_kernel<false> : cross_entropy_bf16_smem_kernel<true>;
+    const int smem = static_cast<int>(cols / 8 * 16);
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return PTJ_ERR_LAUNCH;
+    }
+    const int64_t cap = static_cast<int64_t>(kNumSMs) * 2;
+    launch_k(kern, static_cast<int>(rows < cap ? rows : cap), kCeRowThreads, smem, st, labels, static_cast<const __nv_bfloat16*>(logits),
+             static_cast<__nv_bfloat16*>(dlogits), row_stats, n_valid, rows, static_cast<int>(cols), ld);
   } else if (same_phase<__nv_bfloat16>(logits, ld, dlogits, ld) && cols <= 0x7fffffffLL &&
              reinterpret_cast<uintptr_t>(logits) % 2 == 0) {
     const int64_t cap = static_cast<int64_t>(kNumSMs) * 3;  // three resident 512-thread blocks per SM
     const bool aligned = aligned16(logits) && ld % 8 == 0;  // (the gradient is in the same phase)
-    launch_k(aligned ? cross_entropy_bf16_kernel<false> : cross_entropy_bf16_kernel<true>, static_cast<int>(rows < cap ? rows : cap), kCeThreads, 0, st, labels,
+    launch_k(aligned ? cross_entropy_bf16_wide_kernel<false> : cross_entropy_bf16_wide_kernel<true>, static_cast<int>(rows < cap ? rows : cap), kCeThreads, 0, st, labels,
              static_cast<const __nv_bfloat16*>(logits), static_cast<__nv_bfloat16*>(dlogits), row_stats, n_valid, rows,
              static_cast<int>(cols), ld);
   } else {
