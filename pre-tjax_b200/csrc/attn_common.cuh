@@ -43,6 +43,9 @@ int attn_keep_bits_tc(uint32_t* bits, const ptj_attn_shape& sh, const AttnDropou
 int attn_fwd_tc(const void* q, const void* k, const void* v, void* o, float* row_max, float* row_sum,
                 const uint32_t* keep_bits, const int32_t* row_kstart, const ptj_attn_shape& sh, const AttnDropout& dr,
                 cudaStream_t st);
+int attn_fwd_tc64(const void* q, const void* k, const void* v, void* o, float* row_max, float* row_sum,
+                  const uint32_t* keep_bits, const int32_t* row_kstart, const ptj_attn_shape& sh, const AttnDropout& dr,
+                  cudaStream_t st);  // the shapes of attn_bf16_probabilities
 // workspace: attn_bwd_tc_workspace_bytes(sh) bytes, 16-byte aligned (per-KV-tile dQ shares and per-row constants)
 size_t attn_bwd_tc_workspace_bytes(const ptj_attn_shape& sh);
 int attn_bwd_tc(const void* d_o, const void* q, const void* k, const void* v, const void* o, const float* row_max,

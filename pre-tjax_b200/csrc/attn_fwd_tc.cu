@@ -1,4 +1,5 @@
-// Causal flash attention forward on tcgen05 tensor cores (bf16 in, fp32 accumulate), heads up to 128 wide, any seq.
+// Causal flash attention forward on tcgen05 tensor cores (bf16 in, fp32 accumulate), heads up to 128 wide, any seq, float32
+// probabilities. (attn_fwd_tc64.cu: whole tiles of 64-wide heads, whose probabilities are rounded to bf16.)
 // Semantics: model_triton.py:608-611 / 510-517: softmax of the causally masked scaled scores, dropout on the
 // probabilities (no rescale), times V; the row maximum and row sum of exponentials are saved (acts0 / acts1, :699-700).
 //
@@ -12,23 +13,24 @@
 //               (group, block) has its own reference exponent, row sums and output accumulator, so the warps of a row never
 //               meet before the item ends; then the group that got the last tile merges the G NC states of each row
 //               (log-sum-exp merge in a fixed order) and writes it.
-// PARTS: what a probability is multiplied as. 1: rounded to bf16. 3: split exactly into three bf16 parts, three products
-// each, which keeps float32 probabilities; the operands of S are bf16 as they are.
+// A probability is split exactly into three bf16 parts, three products each; the operands of S are bf16 as they are.
 // Work items = (query tile, batch*head), heaviest first, dealt to the blocks in boustrophedon order; all tiles of a
 // block's items form one stream, so the next item's first tiles overlap the tail of the current one.
 // Tensor memory: two S buffers at columns [0,256), the G NC accumulators at [256,512).
 // Bound by the latencies a softmax warp meets in a row on its tile (tensor-memory loads, barriers, exponentials), not by a
 // pipe. Measured, dropout 0.1, flags drawn here: [4, 12, 500, 64] 22 us (the float32 FMA kernels 95), [8, 12, 1024, 32] 111
-// (338), [8, 12, 1024, 128] 136 (837); whole tiles of 64-wide heads, [8, 12, 1024, 64], flags given: 42 us, as a thread per
-// row of 128 columns took before (41); all 16 warps on one tile, 32 columns a thread: 65.
-#include "attn_tc_dev.cuh"
+// (338), [8, 12, 1024, 128] 136 (837). (With one bf16 part, [8, 12, 1024, 64]: 41.8 us with flags given, 74.6 with flags drawn
+// here, against 40.8 and 69 of attn_fwd_tc64.cu; all 16 warps on one tile, 32 columns a thread: 65.)
+#include "attn_fwd_sched.cuh"
 
 namespace ptj {
 namespace {
 
 using namespace attn_tc;
 
-template <int DHP, int PARTS>
+constexpr int kParts = 3;  // bf16 parts of a probability
+
+template <int DHP>
 struct Cfg {
   static constexpr int kG = DHP == 64 ? 2 : 1;     // groups
   static constexpr int kNC = 2;                    // column blocks of a tile
@@ -40,15 +42,14 @@ struct Cfg {
   static constexpr int kTB = T * DHP * 2;          // one operand tile
   // shared memory, in tiles: what fits beside the probabilities
   static constexpr int kQ = DHP == 64 ? 2 : 1;
-  static constexpr int kK = DHP == 64 ? (PARTS == 1 ? 3 : 2) : 1;
-  static constexpr int kV = DHP == 64 ? (PARTS == 1 ? 4 : 3) : 1;
-  static constexpr int kP = PARTS == 1 ? 2 : 1;    // probability buffers, PARTS tiles each
+  static constexpr int kK = DHP == 64 ? 2 : 1;
+  static constexpr int kV = DHP == 64 ? 3 : 1;
   static constexpr int kOffK = kQ * kTB;
   static constexpr int kOffV = kOffK + kK * kTB;
   static constexpr int kOffP = kOffV + kV * kTB;
-  static constexpr int kOffStats = kOffP + kP * PARTS * kPBytes;  // float [kAcc][3][128]
+  static constexpr int kOffStats = kOffP + kParts * kPBytes;  // float [kAcc][3][128]
   static constexpr int kOffBars = kOffStats + kAcc * 3 * T * 4;
-  static constexpr int kNumBars = 2 * (kQ + kK + kV) + 4 + kG + kP + 2;
+  static constexpr int kNumBars = 2 * (kQ + kK + kV) + 4 + kG + 1 + 2;
   static constexpr int kSmemBytes = kOffBars + kNumBars * 8 + 16 + 80 + 4 * 32 + 1024;  // (+ 32 first-tile entries)
   static_assert(kSmemBytes <= 227 * 1024, "shared memory of a block");
   // of 96 (640 threads) or 168 (384 threads) a thread at launch
@@ -57,47 +58,6 @@ struct Cfg {
 constexpr int kSBufs = 2;
 constexpr int kTmemCols = 512;
 constexpr uint32_t kColO = kSBufs * T;
-
-struct Sched {
-  int total, rounds, nq, BH;
-  uint32_t bh_magic;  // ceil(2^32 / BH): x / BH == umulhi(x, bh_magic) for every x the kernel meets (checked on the host)
-};
-
-// Position in the stream of (item, kv tile) pairs of one thread block; every role walks the same stream.
-// first_tile (row_kstart): per round of this block, the first KV tile its item needs (keys before the first key of every
-// row of the query tile are masked anyway: those tiles are skipped); nullptr = every item starts at tile 0.
-constexpr int kMaxRoundsTabled = 32;
-struct Cursor {
-  int n, ord, qt, bh, j, j0, g;
-  bool valid;
-  const int* first_tile;
-  __device__ __forceinline__ void next_item(const Sched& s) {
-    valid = false;
-    while (++n < s.rounds) {
-      const int pos = (n & 1) ? static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x);
-      const int sp = n * static_cast<int>(gridDim.x) + pos;
-      if (sp < s.total) {
-        const int t = s.BH == 1 ? sp : static_cast<int>(__umulhi(static_cast<uint32_t>(sp), s.bh_magic));  // sp / BH
-        qt = s.nq - 1 - t;
-        bh = sp - t * s.BH;
-        j0 = first_tile != nullptr ? first_tile[n] : 0;
-        j = j0;
-        ++ord;
-        valid = true;
-        return;
-      }
-    }
-  }
-  __device__ __forceinline__ void init(const Sched& s, const int* first = nullptr) {
-    n = -1; ord = -1; g = 0; qt = 0; bh = 0; j = 0; j0 = 0;
-    first_tile = first;
-    next_item(s);
-  }
-  __device__ __forceinline__ void advance(const Sched& s) {
-    ++g;
-    if (j == qt) next_item(s); else ++j;
-  }
-};
 
 // An item one of whose V tiles held an infinity or a NaN (replaced by zero before it was multiplied): the products of a
 // row's attended probabilities with those elements, columns [col0, col0 + 16). Slow and rare.
@@ -142,15 +102,14 @@ struct FwdViews {
 // p.kstart (optional): query row i attends keys [p.kstart[b, i], i] only (packed documents / padding, the block-diagonal x
 // causal x padding masks of the reference's collator, tokenized_dataset.py:110-131); a row whose range is empty gets a
 // zero output row and the statistics (row_max, row_sum) = (0, 1).
-template <int DHP, int PARTS, int MODE>
-__global__ void __launch_bounds__(Cfg<DHP, PARTS>::kThreads, 1)
+template <int DHP, int MODE>
+__global__ void __launch_bounds__(Cfg<DHP>::kThreads, 1)
 attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ FwdViews views,
                    float* __restrict__ row_max, float* __restrict__ row_sum, const __grid_constant__ AttnParams p,
                    const Sched sched) {
-  using C = Cfg<DHP, PARTS>;
+  using C = Cfg<DHP>;
   constexpr int kTB = C::kTB;
-  constexpr bool kExact = PARTS > 1;  // float32 probabilities, and an element that is not finite reaches what attends it only
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sm = align1024(smem_raw);
   uint8_t* q_s = sm;
@@ -168,8 +127,8 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   uint64_t* s_full = v_empty + C::kV;       // [2]
   uint64_t* o_full = s_full + kSBufs;       // [kG] per group: its tile's output MMAs, and all before, are done
   uint64_t* s_free = o_full + C::kG;        // [2] one arrival per warp of the tile's group from here on
-  uint64_t* p_ready = s_free + kSBufs;      // [kP]
-  uint64_t* stats_full = p_ready + C::kP;   // the item's row states are in shared memory (all softmax warps)
+  uint64_t* p_ready = s_free + kSBufs;
+  uint64_t* stats_full = p_ready + 1;   // the item's row states are in shared memory (all softmax warps)
   uint64_t* o_free = stats_full + 1;        // the item's accumulators and states have been read
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_free + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -319,17 +278,17 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     b.init(sched, first_tile);
     bool ok = true;
     while (b.valid && ok) {
-      const int st = b.g % C::kV, pb = b.g % C::kP;
+      const int st = b.g % C::kV;
       const bool first = b.j - b.j0 < C::kG;  // the group's first tile of the item: fresh accumulators ...
-      bool w = mbar_wait(&p_ready[pb], (b.g / C::kP) & 1, ctx, 0x1204u) &&
+      bool w = mbar_wait(p_ready, b.g & 1, ctx, 0x1204u) &&
                mbar_wait(&v_full[st], (b.g / C::kV) & 1, ctx, 0x1205u);
       if (w && first) w = mbar_wait(o_free, (b.ord & 1) ^ 1u, ctx, 0x1206u);  // ... once the previous item has been read out
       ok = __all_sync(0xffffffffu, w);
       if (!ok) break;
       tc_fence_after_sync();
-      const uint32_t pa = smem_u32(p_s + pb * PARTS * kPBytes), va = smem_u32(v_s + st * kTB);
+      const uint32_t pa = smem_u32(p_s), va = smem_u32(v_s + st * kTB);
 #pragma unroll
-      for (int part = 0; part < PARTS; ++part)
+      for (int part = 0; part < kParts; ++part)
 #pragma unroll
         for (int k16 = 0; k16 < T / 16; ++k16)
           mma_bf16_ss_elect(tmem + kColO + ((b.g % C::kG) * C::kNC + k16 / kPerBlock) * DHP,
@@ -356,7 +315,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     const int ntri = p.nq * (p.nq + 1) / 2;
     // float32 probabilities are kept at most 1 (the reference exponent is exceeded by less than 2^8, see below), so that a
     // sum with V overflows no earlier than one of the exact probabilities would
-    constexpr float kShift = kExact ? -8.f : 0.f;
+    constexpr float kShift = -8.f;
 
     Cursor c;
     c.init(sched, first_tile);
@@ -376,9 +335,8 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       const int first_key = p.kstart != nullptr && q_row < p.S
                                 ? __ldg(p.kstart + static_cast<int64_t>(c.bh / p.H) * p.S + q_row) : 0;
       if (mine) {
-        const int sb = c.g % kSBufs, pb = c.g % C::kP;
+        const int sb = c.g % kSBufs;
         const bool fresh = c.j - c.j0 < C::kG;
-        uint8_t* p_tile = p_s + pb * PARTS * kPBytes;
         // what does not wait for the scores: the keep flags of this thread's columns
         uint32_t keepw[kWords];
 #pragma unroll
@@ -436,10 +394,10 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           grow = (mloc - m_ref) * sc > 8.f;  // (both -inf: not a number, no growth)
           m_true = fmaxf(m_true, mloc);
         }
-        // The P buffer is free once the output MMAs of tile g - kP are done. (A wait can only tell a phase from the one before
-        // it: the group waits for every tile of its own, and with one buffer for two groups for every tile of the other.)
+        // The P buffer is free once the output MMAs of tile g - 1 are done. (A wait can only tell a phase from the one before
+        // it: the group waits for every tile of its own, and where there are two groups for every tile of the other.)
         ok = mbar_wait(&o_full[grp], ((c.g / C::kG) & 1) ^ 1u, ctx, 0x1302u);
-        if (C::kP < C::kG && ok && c.g > 0)
+        if (C::kG > 1 && ok && c.g > 0)
           ok = mbar_wait(&o_full[(c.g - 1) % C::kG], ((c.g - 1) / C::kG) & 1, ctx, 0x1302u);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
@@ -464,7 +422,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         // (a row that has met no key of its own yet carries m_ref = -inf; its scores are all -inf too and must give 0)
         const float ref = m_ref == -INFINITY ? 0.f : m_ref;
         const uint64_t sc2 = pack2(sc, sc), sh2 = pack2(kShift, kShift);
-        const uint64_t nm2 = kExact ? pack2(-ref, -ref) : pack2(-ref * sc, -ref * sc);
+        const uint64_t nm2 = pack2(-ref, -ref);
         uint64_t rp[2] = {0ull, 0ull};  // two packed running sums (four chains)
 #pragma unroll
         for (int w = 0; w < kWords; ++w) {
@@ -481,24 +439,24 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             for (int i = i8; i < i8 + 8; i += 2) {  // exp2(-inf) = 0 takes care of the masked columns
               const uint64_t x = pack2(s[i], s[i + 1]);
               float a, b;
-              unpack2(kExact ? fma2(add2(x, nm2), sc2, sh2) : fma2(x, sc2, nm2), a, b);
+              unpack2(fma2(add2(x, nm2), sc2, sh2), a, b);
               a = ex2_approx(a);
               b = ex2_approx(b);
               rp[(i >> 1) & 1] = add2(rp[(i >> 1) & 1], pack2(a, b));
               s[i] = a;
               s[i + 1] = b;
             }
-            uint32_t pw[PARTS][4];
-            split8<PARTS>(s + i8, pw);
+            uint32_t pw[kParts][4];
+            split8<kParts>(s + i8, pw);
             if (MODE != 0) {
 #pragma unroll
               for (int i = 0; i < 4; ++i) {
                 const uint32_t m = pair_mask(keepw[w], (i8 >> 1) + i);
 #pragma unroll
-                for (int part = 0; part < PARTS; ++part) pw[part][i] &= m;
+                for (int part = 0; part < kParts; ++part) pw[part][i] &= m;
               }
             }
-            store8<PARTS>(p_tile, row, (cb * kCW + 32 * w + i8) >> 3, pw);
+            store8<kParts>(p_s, row, (cb * kCW + 32 * w + i8) >> 3, pw);
           }
         }
         {
@@ -506,7 +464,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           unpack2(add2(rp[0], rp[1]), a, b);
           l += a + b;
         }
-        if (kExact) {  // this warp's share of the V tile: elements that are not finite must not meet masked probabilities
+        {  // this warp's share of the V tile: elements that are not finite must not meet masked probabilities
           const int st = c.g % C::kV;
           ok = mbar_wait(&v_full[st], (c.g / C::kV) & 1, ctx, 0x1307u);
           ok = __all_sync(0xffffffffu, ok);
@@ -520,7 +478,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         fence_proxy_async_smem();
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&p_ready[pb]);
+        if (lane == 0) mbar_arrive(p_ready);
       }
       if (last) {  // the item ends with this tile: its group merges the states of all and writes the rows
         ok = mbar_wait(o_free, (c.ord & 1) ^ 1u, ctx, 0x1306u);  // the previous item's states have been read
@@ -579,7 +537,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             if (lane == 0) mbar_arrive(o_free);  // the next item may overwrite the accumulators
           }
           if (q_row < p.S) {
-            if (kExact && *bad_v != 0 && !none) {
+            if (*bad_v != 0 && !none) {
               float t[16];
 #pragma unroll
               for (int i = 0; i < 16; ++i) t[i] = 0.f;
@@ -661,26 +619,21 @@ attn_keep_bits_kernel(uint32_t* __restrict__ bits, const AttnDropout dr, int S, 
   bits[tile * 512 + threadIdx.x] = word;
 }
 
-template <int DHP, int PARTS>
+template <int DHP>
 int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdViews& views, float* row_max,
                float* row_sum, const AttnParams& p, int mode, cudaStream_t st) {
-  using C = Cfg<DHP, PARTS>;
+  using C = Cfg<DHP>;
   using Kern = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const FwdViews, float*, float*,
                         const AttnParams, const Sched);
-  static const Kern kerns[3] = {attn_fwd_ws_kernel<DHP, PARTS, 0>, attn_fwd_ws_kernel<DHP, PARTS, 1>,
-                                attn_fwd_ws_kernel<DHP, PARTS, 2>};
+  static const Kern kerns[3] = {attn_fwd_ws_kernel<DHP, 0>, attn_fwd_ws_kernel<DHP, 1>,
+                                attn_fwd_ws_kernel<DHP, 2>};
   const Kern kern = kerns[mode];
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes) != cudaSuccess) {
     (void)cudaGetLastError();
     return PTJ_ERR_LAUNCH;
   }
   Sched s;
-  s.nq = p.nq;
-  s.BH = p.BH;
-  s.total = p.nq * p.BH;
-  const int grid = s.total < kNumSMs ? s.total : kNumSMs;
-  s.rounds = (s.total + grid - 1) / grid;
-  s.bh_magic = static_cast<uint32_t>(((1ull << 32) + s.BH - 1) / s.BH);
+  const int grid = make_sched(&s, p);
   launch_k(kern, grid, C::kThreads, C::kSmemBytes, st, tq, tk, tv, views, row_max, row_sum, p, s);
   PTJ_CHECK_LAUNCH();
   return PTJ_OK;
@@ -704,6 +657,7 @@ int attn_keep_bits_tc(uint32_t* bits, const ptj_attn_shape& sh, const AttnDropou
 int attn_fwd_tc(const void* q, const void* k, const void* v, void* o, float* row_max, float* row_sum,
                 const uint32_t* keep_bits, const int32_t* row_kstart, const ptj_attn_shape& sh, const AttnDropout& dr,
                 cudaStream_t st) {
+  if (attn_bf16_probabilities(sh)) return attn_fwd_tc64(q, k, v, o, row_max, row_sum, keep_bits, row_kstart, sh, dr, st);
   CUtensorMap tq, tk, tv;
   if (!make_map(&tq, q, sh, sh.q_strides) || !make_map(&tk, k, sh, sh.k_strides) || !make_map(&tv, v, sh, sh.v_strides))
     return PTJ_ERR_LAUNCH;
@@ -715,9 +669,8 @@ int attn_fwd_tc(const void* q, const void* k, const void* v, void* o, float* row
   const int mode = !masked ? 0 : (keep_bits != nullptr ? 2 : 1);
   const FwdViews views{make_view(q, sh.q_strides), make_view(k, sh.k_strides), make_view(v, sh.v_strides),
                        make_view(o, sh.o_strides)};
-  if (sh.d_head > 64) return launch_fwd<128, 3>(tq, tk, tv, views, row_max, row_sum, p, mode, st);
-  if (attn_bf16_probabilities(sh)) return launch_fwd<64, 1>(tq, tk, tv, views, row_max, row_sum, p, mode, st);
-  return launch_fwd<64, 3>(tq, tk, tv, views, row_max, row_sum, p, mode, st);
+  if (sh.d_head > 64) return launch_fwd<128>(tq, tk, tv, views, row_max, row_sum, p, mode, st);
+  return launch_fwd<64>(tq, tk, tv, views, row_max, row_sum, p, mode, st);
 }
 
 }  // namespace ptj
