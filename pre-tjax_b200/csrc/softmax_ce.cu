@@ -240,20 +240,20 @@ cross_entropy_kernel(const int32_t* __restrict__ labels, const T* logits, T* dlo
 // ---- bf16 cross entropy; logits and gradient rows start at the same distance from a 16-byte boundary -----------------
 // The kernel above spends about 25 instructions per logit (64-bit column arithmetic, arg-max bookkeeping and the
 // online rescale inside the inner loop, a compare per element for the label) and is issue-bound at half of the memory
-// roofline. This one walks the row three times with 16-byte vectors and does the least possible per element:
+// roofline. These walk the row three times with 16-byte vectors and do the least possible per element:
 //   1. maximum only, on packed bf16 pairs (half an instruction per element);
 //   2. sum of 2^((x - max) log2 e), two floats wide;
 //   3. dlogits = 2^(x log2 e + c), with c = -max log2 e + log2(1 / (n_valid * sum)) folding both scale factors into
 //      the exponent; the label's element is patched by one thread afterwards.
-// Passes 2 and 3 read the row from L2 (512-thread blocks, three per SM: the 444 rows in flight, 100 KB each at
-// GPT-2's vocabulary, stay well inside the L2). Accuracy: the label is the arg-max iff x[label] equals the maximum and no earlier column does (ties go to
+// A row is kept on chip between the passes, in registers or in shared memory; wider rows (beyond kCeSmemCols) are read again
+// from L2 (512-thread blocks, three per SM: the rows in flight stay well inside the L2). Accuracy: the label is the arg-max iff x[label] equals the maximum and no earlier column does (ties go to
 // the first index, as in torch.argmax); the second condition is only walked for rows where the first holds.
 // Rows of an odd vocabulary stored without padding (PHASED) start anywhere: up to seven elements before the first boundary
 // and seven after the last whole vector are walked one by one. They also keep the arithmetic of the generic kernel above:
 // the maximum is subtracted, exactly, before the product with log2 e, and the scale multiplies the exponential. (Folding
 // both into the exponent, as the aligned rows do, rounds max log2 e: an error of 2^-24 |max log2 e| in the loss, and an
 // overflow in rows that hold nothing but the type's lowest value.) [8192, 50257] contiguous: 507 us through the generic
-// kernel, 394 us here, calls and all; padded rows of the same size 340 us.
+// kernel, 376 us in three reads, 335 with the row in shared memory, calls and all; padded rows 363 and 313.
 constexpr int kCeThreads = 512;
 
 __device__ __forceinline__ uint32_t bf2_max(uint32_t a, uint32_t b) {
@@ -889,6 +889,7 @@ extern "C" int ptj_cross_entropy(const int32_t* labels, const void* logits, void
                static_cast<__nv_bfloat16*>(dlogits), row_stats, n_valid, rows, static_cast<int>(cols), ld);
       return PTJ_OK;
     };
+    // (a row on 256 threads while they can hold it: four blocks an SM, so that some are always between barriers)
     const int rc = cols <= 256 * kCeVecs * 8 ? launch(std::integral_constant<int, 256>())
                                              : launch(std::integral_constant<int, 512>());
     if (rc != PTJ_OK) return rc;
