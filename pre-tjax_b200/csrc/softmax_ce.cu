@@ -889,7 +889,7 @@ extern "C" int ptj_cross_entropy(const int32_t* labels, const void* logits, void
                static_cast<__nv_bfloat16*>(dlogits), row_stats, n_valid, rows, static_cast<int>(cols), ld);
       return PTJ_OK;
     };
-    // (a row on 256 threads while they can hold it: four blocks an SM, so that some are always between barriers)
+    // (256 threads, four blocks an SM, as long as their registers hold the row; then 512)
     const int rc = cols <= 256 * kCeVecs * 8 ? launch(std::integral_constant<int, 256>())
                                              : launch(std::integral_constant<int, 512>());
     if (rc != PTJ_OK) return rc;
