@@ -162,7 +162,7 @@ class _LayerPlan:
         self.shape = _lib.LayerShape(B, S, D, cfg.heads, F, _lib.PTJ_BF16 if es == 2 else _lib.PTJ_F32, int(train), cfg.dropout,
                                      0, 0, 0)
         ref = ctypes.byref(self.shape)
-        keep = int(lib.ptj_layer_keep_bits_bytes(ref))
+        self.keep_bytes = keep = int(lib.ptj_layer_keep_bits_bytes(ref))
         stats = 4 * B * cfg.heads * S
         # ln1, qkv, attn, row_max, row_sum, keep_bits, x_mid, ln2, h_pre, h_act (LayerActs after x), then the output
         self.act_offsets, self.act_bytes = self._place(
@@ -185,6 +185,55 @@ class _LayerPlan:
         return offsets, max(end, 1)
 
 
+class _SavedLayer:
+    """What a layer's forward call saved: its input (a tensor, or the layer below whose output it is), and everything else,
+    its output too, in one allocation at the plan's offsets."""
+    __slots__ = ("plan", "below", "slab")
+
+    def __init__(self, plan: _LayerPlan, below, slab: torch.Tensor):
+        self.plan, self.below, self.slab = plan, below, slab
+
+    def output_address(self) -> int:
+        return self.slab.data_ptr() + self.plan.out_offset
+
+    def addresses(self):
+        base = self.slab.data_ptr()
+        x = self.below.output_address() if isinstance(self.below, _SavedLayer) else self.below.data_ptr()
+        return _lib.LayerActs(x, *[base + o if o >= 0 else 0 for o in self.plan.act_offsets])
+
+    def _at(self, offset: int, dtype: torch.dtype, *shape):
+        return self.slab[offset:offset + math.prod(shape) * dtype.itemsize].view(dtype).view(shape)
+
+    def output(self, dtype: torch.dtype):
+        s = self.plan.shape
+        return self._at(self.plan.out_offset, dtype, s.batch * s.seq, s.dim)
+
+    def tensors(self, dtype: torch.dtype) -> dict:
+        """The same by name, as single launches save and take them."""
+        s, f32 = self.plan.shape, torch.float32
+        T, D = s.batch * s.seq, s.dim
+        ln1, qkv, attn, m, l, keep, x_mid, ln2, h_pre, h_act = self.plan.act_offsets
+        return {"x": self.below.output(dtype) if isinstance(self.below, _SavedLayer) else self.below,
+                "ln1": self._at(ln1, dtype, T, D), "qkv": self._at(qkv, dtype, T, 3 * D), "attn": self._at(attn, dtype, T, D),
+                "m": self._at(m, f32, s.batch, s.heads, s.seq), "l": self._at(l, f32, s.batch, s.heads, s.seq),
+                "keep": self._at(keep, torch.int32, self.plan.keep_bytes // 4) if keep >= 0 else None,
+                "x_mid": self._at(x_mid, dtype, T, D), "ln2": self._at(ln2, dtype, T, D),
+                "h_pre": self._at(h_pre, dtype, T, s.ffn), "h_act": self._at(h_act, dtype, T, s.ffn)}
+
+
+def _addresses(tensors, wanted, device: int):
+    """Addresses of the tensors that a library call reads and writes by the configuration's sizes, or None where one of them
+    is not what the call takes it for: `wanted` lists (name, shape, dtype), all contiguous and on one device. Looked at in
+    every pass, since tensors can be resized or replaced between two."""
+    out = []
+    for name, shape, dtype in wanted:
+        t = tensors[name]
+        if t.shape != shape or t.dtype is not dtype or not t.is_contiguous() or t.get_device() != device:
+            return None
+        out.append(t.data_ptr())
+    return out
+
+
 class Gpt2Step:
     """One forward + backward pass. Gradients are written into caller-provided float32 tensors (``grads[name]``),
     so a trainer can hand in views of one flat buffer and overlap their reduction with the rest of backward."""
@@ -204,7 +253,10 @@ class Gpt2Step:
         # input gradients whose last round of tiles is mostly empty: that round's rows split over K, same launch
         self.tail_split = True
         self._ws2 = [None, None]
-        self._layer_names = [[f"l{l}.{n}" for n in LAYER_TENSORS] for l in range(cfg.layers)]
+        # (name, shape, dtype) of each layer's weights and of their gradients
+        in_layer = [(n, torch.Size(s)) for n, s in cfg.param_shapes() if "." in n]
+        self._layer_weights = [(n, s, compute_dtype if base_name(n) in MATRIX_TENSORS else torch.float32) for n, s in in_layer]
+        self._layer_grads = [(n, s, torch.float32) for n, s in in_layer]
         self._plans = {}    # (batch, seq, train) -> _LayerPlan
         self._held = []     # workspaces that a recorded graph may still use
 
@@ -260,6 +312,14 @@ class Gpt2Step:
         product with events or has switched one of the variants above, which are sequences of their own."""
         return (ops.GEMM_PROFILE is None and not self.split_gelu_bwd and self.pair_wgrads and self.tail_split
                 and plan.fused)
+
+    @staticmethod
+    def _per_layer(struct, tensors, wanted, device: int):
+        """One struct of addresses per layer, or None where a tensor is not what the struct's reader takes it for: strided,
+        of another shape or type. Single launches (which take a stride and a type each, or refuse) do those."""
+        at = _addresses(tensors, wanted, device)
+        n = len(LAYER_TENSORS)
+        return None if at is None else [struct(*at[i:i + n]) for i in range(0, len(at), n)]
 
     def _wgrad2(self, first, second):
         """Two weight gradients (dy, x, out) in ONE launch of the thread-block-pair kernel when both qualify: their
@@ -330,10 +390,11 @@ class Gpt2Step:
         x = ops.embed_fwd(ids_in, w["w_emb"], w["w_pos"], train, seeds[0], out_dtype=self.dtype, p=p).view(T, D)
         acts = {"layers": [], "row_kstart": row_kstart}
         plan = self._plan(B, S, bool(train))
-        native = self._native(plan)
+        weights = self._per_layer(_lib.LayerWeights, w.t, self._layer_weights, x.get_device()) if self._native(plan) else None
+        native = weights is not None
         if native:
             row_kstart = ops._check_kstart(row_kstart, B, S, x.device)
-            x = self._layers_fwd(plan, w, x, seeds, row_kstart, acts)
+            x = self._layers_fwd(plan, weights, x, seeds, row_kstart, acts)
         tail = tail_split_for(T, D, cfg.ffn) if (self.tail_split and self.dtype == torch.bfloat16) else None
         for l in range(0 if native else cfg.layers):
             s_attn, s_res1, s_res2 = seeds[1 + 3 * l: 4 + 3 * l]
@@ -362,53 +423,45 @@ class Gpt2Step:
         ops.gemm(acts["x_f"], w["w_emb"], bias=w["b_head"], out=logits, N=cfg.vocab, ldc=self.vocab_ld)
         return logits, acts
 
-    def _layers_fwd(self, plan, w: Weights, x, seeds, row_kstart, acts):
+    def _layers_fwd(self, plan, weights, x, seeds, row_kstart, acts):
         """All layers through ptj_layer_fwd: the saved activations of each are one allocation."""
         lib, stream = _lib.lib(), ops._stream()
         ws, ws_bytes = self._layer_workspace(plan, False)
         ks = 0 if row_kstart is None else row_kstart.data_ptr()
-        t, seeds = w.t, [ops._seed(s_) for s_ in seeds]
-        at, shape, slab = x.data_ptr(), plan.shape, None
-        acts["row_kstart"] = row_kstart
-        for l, names in enumerate(self._layer_names):
-            slab = torch.empty(plan.act_bytes, device=x.device, dtype=torch.uint8)
-            base = slab.data_ptr()
-            weights = _lib.LayerWeights(*[t[n].data_ptr() for n in names])
-            saved = _lib.LayerActs(at, *[base + o if o >= 0 else 0 for o in plan.act_offsets])
+        seeds = [ops._seed(s_) for s_ in seeds]
+        shape = plan.shape
+        acts["row_kstart"], acts["plan"] = row_kstart, plan
+        at = x
+        for l in range(self.cfg.layers):
+            at = _SavedLayer(plan, at, torch.empty(plan.act_bytes, device=x.device, dtype=torch.uint8))
             shape.seed_attn, shape.seed_res1, shape.seed_res2 = seeds[1 + 3 * l: 4 + 3 * l]
-            out = base + plan.out_offset
-            _lib.check(lib.ptj_layer_fwd(shape, weights, saved, out, ks, ws, ws_bytes, stream), "ptj_layer_fwd")
-            acts["layers"].append((saved, slab, x))  # (the first layer's input is a tensor of its own)
-            at = out
-        if slab is None:
-            return x
-        return slab[plan.out_offset:plan.out_offset + plan.out_bytes].view(self.dtype).view(x.shape)
+            _lib.check(lib.ptj_layer_fwd(shape, weights[l], at.addresses(), at.output_address(), ks, ws, ws_bytes, stream),
+                       "ptj_layer_fwd")
+            acts["layers"].append(at)
+        return x if at is x else at.output(self.dtype)
 
-    def _layers_bwd(self, plan, w: Weights, grads, acts, dx, dy, seeds, ready):
+    def _layers_bwd(self, plan, weights, out, acts, dx, dy, seeds, ready):
         """All layers through ptj_layer_bwd_ffn and ptj_layer_bwd_attn; returns the gradient of the first one's input."""
         lib, stream = _lib.lib(), ops._stream()
         ws, ws_bytes = self._layer_workspace(plan, True)
         ks = acts.get("row_kstart")
         ks = 0 if ks is None else ks.data_ptr()
-        t, seeds = w.t, [ops._seed(s_) for s_ in seeds]
+        seeds = [ops._seed(s_) for s_ in seeds]
         shape = plan.shape
         # scratch shared by all layers, and the gradients of the residual stream in turn
         slab = torch.empty(plan.grad_bytes, device=dx.device, dtype=torch.uint8)
         base = slab.data_ptr()
         dh_pre, d_ln, d_attn, dqkv, dx_a, dy_a, dx_b, dy_b = [base + o for o in plan.grad_offsets]
         dx_p, dy_p = dx.data_ptr(), dy.data_ptr()
-        for l in range(len(self._layer_names) - 1, -1, -1):
-            names = self._layer_names[l]
-            saved = acts["layers"][l][0]
-            weights = _lib.LayerWeights(*[t[n].data_ptr() for n in names])
-            out = _lib.LayerGrads(*[grads[n].data_ptr() for n in names])
+        for l in range(self.cfg.layers - 1, -1, -1):
+            saved = acts["layers"][l].addresses()
             shape.seed_attn, shape.seed_res1, shape.seed_res2 = seeds[1 + 3 * l: 4 + 3 * l]
-            _lib.check(lib.ptj_layer_bwd_ffn(shape, weights, saved, out, dx_p, dy_p, dh_pre, d_ln, dx_a, dy_a, ws, ws_bytes,
-                                             stream), "ptj_layer_bwd_ffn")
+            _lib.check(lib.ptj_layer_bwd_ffn(shape, weights[l], saved, out[l], dx_p, dy_p, dh_pre, d_ln, dx_a, dy_a, ws,
+                                             ws_bytes, stream), "ptj_layer_bwd_ffn")
             ready([f"l{l}.{n}" for n in ("b2f", "w2", "b1f", "w1", "g2", "b2")])
             below = l > 0
-            _lib.check(lib.ptj_layer_bwd_attn(shape, weights, saved, out, dx_a, dy_a, d_attn, dqkv, d_ln, dx_b,
-                                              dy_b if below else 0, grads[f"l{l - 1}.b2f"].data_ptr() if below else 0,
+            _lib.check(lib.ptj_layer_bwd_attn(shape, weights[l], saved, out[l], dx_a, dy_a, d_attn, dqkv, d_ln, dx_b,
+                                              dy_b if below else 0, out[l - 1].b2f if below else 0,
                                               seeds[3 * l] if below else 0, ks, ws, ws_bytes, stream), "ptj_layer_bwd_attn")
             ready([f"l{l}.{n}" for n in ("w_o", "w_qkv", "g1", "b1")])
             dx_p, dy_p = dx_b, dy_b
@@ -441,12 +494,18 @@ class Gpt2Step:
                               colsum_out=grads[f"l{cfg.layers - 1}.b2f"] if (fuse and cfg.layers > 0) else None)
         ready(["g_f", "b_f"])
 
-        native = bool(acts["layers"]) and not isinstance(acts["layers"][0], dict)  # as the forward pass went
+        native = "plan" in acts and cfg.layers > 0  # as the forward pass went
         if native:
-            dx = self._layers_bwd(self._plan(B, S, bool(train)), w, grads, acts, dx, dy, seeds, ready)
+            weights = self._per_layer(_lib.LayerWeights, w.t, self._layer_weights, dx.get_device())
+            out = self._per_layer(_lib.LayerGrads, grads, self._layer_grads, dx.get_device())
+            native = weights is not None and out is not None
+        if native:
+            dx = self._layers_bwd(self._plan(B, S, bool(train)), weights, out, acts, dx, dy, seeds, ready)
         for l in reversed(range(0 if native else cfg.layers)):
             s_attn, s_res1, s_res2 = seeds[1 + 3 * l: 4 + 3 * l]
             a = acts["layers"][l]
+            if isinstance(a, _SavedLayer):
+                a = a.tensors(self.dtype)
             g = lambda n: w[f"l{l}.{n}"]
             G = lambda n: grads[f"l{l}.{n}"]
             # x_next = x_mid + dropout(W2 gelu(W1 ln2(x_mid) + b1f) + b2f)

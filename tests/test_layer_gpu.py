@@ -41,3 +41,38 @@ def test_same_bits_as_single_launches(dtype, dim, heads, ffn, layers, B, S, p, p
         ops.GEMM_PROFILE = None
     assert ops.last_kernel_fault() == 0
     assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_strided_weights_and_gradients(dtype):
+    """Matrices that are columns of wider ones: the same bits as contiguous ones, and nothing is written between the rows."""
+    ops, gpt2 = pkg("operators"), pkg("gpt2")
+    cfg = gpt2.GPT2Config(vocab=304, dim=256, layers=2, heads=4, ffn=512, seq=200, dropout=0.1)
+    g = torch.Generator(device="cuda").manual_seed(2)
+    flat = [0.05 * torch.randn(s, generator=g, device="cuda") + (1.0 if gpt2.base_name(n)[0] == "g" else 0.0)
+            for n, s in cfg.param_shapes()]
+    w = gpt2.Weights.from_pytree(gpt2.unflatten_like(flat, cfg), cfg, dtype)
+    y = torch.randint(1, 304, (2, 201), generator=g, device="cuda", dtype=torch.int32)
+    names = [n for n, s in cfg.param_shapes() if n.startswith("l") and len(s) == 2]  # (W_qkv is used as one matrix)
+
+    def wide(t):
+        buf = torch.full((t.shape[0], t.shape[1] + 24), 7.0, device="cuda", dtype=t.dtype)
+        buf[:, :t.shape[1]] = t
+        return buf, buf[:, :t.shape[1]]
+
+    def step(weights, grads):
+        stats = gpt2.Gpt2Step(cfg, dtype).loss_and_grads(gpt2.Weights(cfg, weights), grads, y, True, list(range(5, 12)))
+        torch.cuda.synchronize()
+        assert ops.last_kernel_fault() == 0
+        return [stats] + [grads[n] for n, _ in cfg.param_shapes()]
+
+    def fresh():
+        return {n: torch.full(s, 3.0, device="cuda") for n, s in cfg.param_shapes()}
+
+    want = step(w.t, fresh())
+    got = step({n: wide(t)[1] if n in names else t for n, t in w.t.items()}, fresh())
+    assert all(torch.equal(a, b) for a, b in zip(want, got))
+    buffers = {n: wide(t) for n, t in fresh().items() if n in names}
+    got = step(w.t, {**fresh(), **{n: view for n, (_, view) in buffers.items()}})
+    assert all(torch.equal(a, b) for a, b in zip(want, got))
+    assert all(bool((buf[:, view.shape[1]:] == 7.0).all()) for buf, view in buffers.values())
