@@ -516,7 +516,7 @@ cross_entropy_bf16_kernel(const int32_t* __restrict__ labels, const __nv_bfloat1
     }
     // pass 2: sum of exponentials
     const Shifted<PHASED> arg(m);
-    float s0 = ends ? ex2_approx(arg(x_end)) : 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+    float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
 #pragma unroll
     for (int j = 0; j < kCeVecs; ++j) {
       if (j * NT >= nvec) break;
@@ -532,6 +532,7 @@ cross_entropy_bf16_kernel(const int32_t* __restrict__ labels, const __nv_bfloat1
         s3 += ex2_approx(e6) + ex2_approx(e7);
       }
     }
+    if (ends) s0 += ex2_approx(arg(x_end));  // (last, the order of row_expsum_bf16: rows of 512 threads give its bits)
     const float s = rows_sum<NT>((s0 + s1) + (s2 + s3), red[1]);
     if (tid == 0) {
       row_stats[row] = -(x_label - m - logf(s));
@@ -633,7 +634,7 @@ cross_entropy_bf16_smem_kernel(const int32_t* __restrict__ labels, const __nv_bf
       hit = __syncthreads_or(earlier) ? 0.f : 1.f;
     }
     const Shifted<PHASED> arg(m);
-    float s0 = ends ? ex2_approx(arg(x_end)) : 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+    float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
 #pragma unroll 2
     for (int i = tid; i < nvec; i += NT) {
       const uint4 a = row_s[i];
@@ -648,6 +649,7 @@ cross_entropy_bf16_smem_kernel(const int32_t* __restrict__ labels, const __nv_bf
       s2 += ex2_approx(e4) + ex2_approx(e5);
       s3 += ex2_approx(e6) + ex2_approx(e7);
     }
+    if (ends) s0 += ex2_approx(arg(x_end));  // (last, the order of row_expsum_bf16: rows of 512 threads give its bits)
     const float s = rows_sum<NT>((s0 + s1) + (s2 + s3), red[1]);
     if (tid == 0) {
       row_stats[row] = -(x_label - m - logf(s));

@@ -42,3 +42,22 @@ def test_against_float64(cols, pad):
     assert float(err.max()) <= 0.0
     if pad and ld > cols:
         assert torch.equal(d[:, cols:], x[:, cols:]), "padding columns keep their values"
+
+
+@pytest.mark.parametrize("cols", [20001, 50257])  # held in registers, held in shared memory
+def test_bits_do_not_depend_on_where_a_row_is_held(cols):
+    """Every kernel adds up a row in the same order, the elements behind its last whole vector last: a row padded with -inf to
+    the width of the kernel that reads rows three times, its last element moved to that row's end, gives the same bits."""
+    ops = pkg("operators")
+    rows, wide, ld = 4096, 57345, 57352
+    g = torch.Generator(device="cuda").manual_seed(cols)
+    x = (2.0 * torch.randn(rows, (cols + 7) // 8 * 8, generator=g, device="cuda")).bfloat16()
+    x[:, [0, 1, 2, 3, 4, 5, 6, 7, 4096, 4097, cols - 1]] += 10.0  # elements of one thread that decide the sum
+    y = torch.randint(1, cols - 1, (rows,), generator=g, device="cuda", dtype=torch.int32)
+    z = torch.full((rows, ld), -float("inf"), device="cuda", dtype=torch.bfloat16)
+    z[:, :cols - 1] = x[:, :cols - 1]
+    z[:, wide - 1] = x[:, cols - 1]
+    _, _, d, loss = ops.cross_entropy(y, x, cols=cols, want_grad=True, want_rows=True)
+    _, _, e, want = ops.cross_entropy(y, z, cols=wide, want_grad=True, want_rows=True)
+    assert torch.equal(loss, want)
+    assert torch.equal(d[:, :cols - 1], e[:, :cols - 1]) and torch.equal(d[:, cols - 1], e[:, wide - 1])
