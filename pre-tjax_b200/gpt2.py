@@ -176,6 +176,10 @@ class _LayerPlan:
         # the LayerNorm backward that also writes the dropped gradient and its column sums takes these widths
         self.fused = D % 8 == 0 and D <= (2048 if es == 2 else 1024)
 
+    def call_shape(self):
+        """A copy for one pass to put its seeds into: another thread may be in a pass of the same shape."""
+        return _lib.LayerShape.from_buffer_copy(self.shape)
+
     @staticmethod
     def _place(sizes):
         offsets, end = [], 0
@@ -243,7 +247,8 @@ class Gpt2Step:
         self.dtype = compute_dtype
         # logits rows are padded so that every row starts on a 16-byte boundary
         self.vocab_ld = (cfg.vocab + 127) // 128 * 128
-        self._ws = None
+        self._ws = {}       # (device, stream, recording, slot) -> float32 workspace, see _workspace
+        self._held = []     # workspaces that a recorded graph may still use
         # FFN backward: gelu' inside the input-gradient GEMM's epilogue followed by a column-sum pass over its output
         # (measured 0.1 ms per GPT-2 small step faster), or, when set, a plain GEMM followed by ONE elementwise pass
         # that applies gelu' and sums the columns. Same results.
@@ -252,13 +257,11 @@ class Gpt2Step:
         self.pair_wgrads = True
         # input gradients whose last round of tiles is mostly empty: that round's rows split over K, same launch
         self.tail_split = True
-        self._ws2 = [None, None]
         # (name, shape, dtype) of each layer's weights and of their gradients
         in_layer = [(n, torch.Size(s)) for n, s in cfg.param_shapes() if "." in n]
         self._layer_weights = [(n, s, compute_dtype if base_name(n) in MATRIX_TENSORS else torch.float32) for n, s in in_layer]
         self._layer_grads = [(n, s, torch.float32) for n, s in in_layer]
         self._plans = {}    # (batch, seq, train) -> _LayerPlan
-        self._held = []     # workspaces that a recorded graph may still use
 
     # -- helpers --
     def _wgrad(self, dy2d, x2d, out, accumulate=False):
@@ -268,37 +271,44 @@ class Gpt2Step:
         split = 1
         if dy2d.dtype == torch.bfloat16:
             split = split_k_for(M, N, T)
-            need = split * M * N
-            if split > 1 and (self._ws is None or self._ws.numel() < need):
-                self._ws = torch.empty(need, device=out.device, dtype=torch.float32)
+        ws = self._workspace(split * M * N if split > 1 else 0, out.device)
         ops.gemm(dy2d, x2d, a_kmajor=False, b_kmajor=False, M=M, N=N, K=T, lda=dy2d.stride(0), ldb=x2d.stride(0),
                  out=out.view(M, N), epilogue=_lib.EPI_ACCUM if accumulate else _lib.EPI_NONE, split_k=split,
-                 workspace=self._ws)
+                 workspace=ws)
 
-    def _workspace(self, floats: int):
-        if self._ws is None or self._ws.numel() < floats:
-            self._ws = torch.empty(floats, device="cuda", dtype=torch.float32)
-        self._hold_recorded()
-        return self._ws
+    def _workspace(self, floats: int, device, least: int = None, slot: int = 0):
+        """A float32 tensor of at least `floats` elements (or, where that does not fit on the device, of `least`) for the
+        launches that the caller is about to issue on the current stream; None when nothing was needed so far.
 
-    def _hold_recorded(self):
-        """A recorded graph keeps the address of the workspace: it stays allocated when a larger one takes its place."""
-        if torch.cuda.is_current_stream_capturing() and not any(h is self._ws for h in self._held):
-            self._held.append(self._ws)
-
-    def _layer_workspace(self, plan, backward: bool):
-        """(address, bytes) of the workspace of a layer's launches; without the part that only makes products faster where
-        that does not fit (as for a single product, operators.gemm)."""
-        need = plan.ws_floats[backward]
-        if self._ws is None or self._ws.numel() < need:
+        One per stream: passes of one engine on two streams run side by side. Callers keep a reference until they have issued
+        their launches: another thread that needs more replaces the kept tensor. A recorded graph keeps the address, so what
+        it was recorded with stays allocated when a larger one takes its place, and serves no launch outside recordings."""
+        recording = torch.cuda.is_current_stream_capturing()
+        key = (device, ops._stream(), recording, slot)
+        ws = self._ws.get(key)
+        have = 0 if ws is None else ws.numel()
+        if have < floats:
             try:
-                self._ws = torch.empty(need, device="cuda", dtype=torch.float32)
+                ws = torch.empty(floats, device=device, dtype=torch.float32)
             except torch.OutOfMemoryError:
-                least = plan.ws_least[backward]
-                if self._ws is None or self._ws.numel() < least:
-                    self._ws = torch.empty(least, device="cuda", dtype=torch.float32)
-        self._hold_recorded()
-        return self._ws.data_ptr(), self._ws.numel() * 4
+                if least is None:
+                    raise
+                if have < least:
+                    ws = torch.empty(least, device=device, dtype=torch.float32)
+            if ws is not self._ws.get(key):
+                self._ws[key] = ws
+                if recording:
+                    self._held.append(ws)
+        return ws
+
+    def release_workspaces(self):
+        """Gives back the workspaces of launches outside recorded graphs; the next pass allocates what it needs."""
+        self._ws = {k: ws for k, ws in self._ws.items() if k[2]}
+
+    def _layer_workspace(self, plan, backward: bool, device):
+        """The workspace of a layer's launches; without the part that only makes products faster where that does not fit (as
+        for a single product, operators.gemm)."""
+        return self._workspace(max(1, plan.ws_floats[backward]), device, least=max(1, plan.ws_least[backward]))
 
     def _plan(self, B: int, S: int, train: bool):
         key = (B, S, train)
@@ -343,11 +353,7 @@ class Gpt2Step:
             probs = []
             for i, (dy, x, out) in enumerate(((dy0, x0, out0), (dy1, x1, out1))):
                 M, N = out.shape[0], x.shape[1]
-                ws = None
-                if best > 1:
-                    ws = self._ws2[i]
-                    if ws is None or ws.numel() < best * M * N:
-                        ws = self._ws2[i] = torch.empty(best * M * N, device=out.device, dtype=torch.float32)
+                ws = self._workspace(best * M * N, out.device, slot=1 + i) if best > 1 else None
                 probs.append(dict(a=dy, b=x, out=out.view(M, N), lda=dy.stride(0), ldb=x.stride(0), split_k=best,
                                   workspace=ws))
             ok = ops.gemm_grouped2(probs, T, a_kmajor=False, b_kmajor=False)
@@ -364,17 +370,17 @@ class Gpt2Step:
         # pairs a bad last round (96 tiles of 256 x 256 at GPT-2 small); parts of K even it out. Measured at
         # [8192, 768, 50257]: 543 us unsplit, 478 / 467 / 496 us in 2 / 3 / 4 parts; the K = 2304 and 3072 products of a
         # layer only lose (32 -> 40 us, 48 -> 56 us), hence the lower bound on K.
-        split = 1
+        split, floats = 1, 0
         if dy2d.dtype == torch.bfloat16 and not kw:
             tail = tail_split_for(T, N, K) if self.tail_split else None
             if tail is not None:
                 split = ops.SPLIT_TAIL  # the rows of the last, mostly empty round of tiles are split over K
-                self._workspace(tail[1])
+                floats = tail[1]
             elif K >= 16384:
                 split = split_k_for(T, N, K)
-                self._workspace(split * T * N)
+                floats = split * T * N
         return ops.gemm(dy2d, w2d, a_kmajor=True, b_kmajor=False, M=T, N=N, K=K, lda=dy2d.stride(0),
-                        ldb=w2d.stride(0), out_dtype=self.dtype, split_k=split, workspace=self._ws, **kw)
+                        ldb=w2d.stride(0), out_dtype=self.dtype, split_k=split, workspace=self._workspace(floats, dy2d.device), **kw)
 
     # -- forward --
     def forward(self, w: Weights, ids_in: torch.Tensor, train: bool, seeds: Sequence[int], row_kstart=None):
@@ -415,7 +421,7 @@ class Gpt2Step:
             a["h_act"] = ops.gemm(a["ln2"], g("w1"), bias=g("b1f"), epilogue=_lib.EPI_GELU, aux_out=a["h_pre"])
             x = ops.gemm(a["h_act"], g("w2"), bias=g("b2f"), epilogue=_lib.EPI_DROPOUT_RESID, aux=a["x_mid"],
                          dropout_args=(p, train, s_res2, 0), split_k=ops.SPLIT_TAIL if tail else 1,
-                         workspace=self._workspace(tail[1]) if tail else None)
+                         workspace=self._workspace(tail[1], x.device) if tail else None)
             acts["layers"].append(a)
         acts["x_last"] = x
         acts["x_f"] = ops.t_layernorm_fwd_t((w["g_f"], w["b_f"]), x)
@@ -426,16 +432,17 @@ class Gpt2Step:
     def _layers_fwd(self, plan, weights, x, seeds, row_kstart, acts):
         """All layers through ptj_layer_fwd: the saved activations of each are one allocation."""
         lib, stream = _lib.lib(), ops._stream()
-        ws, ws_bytes = self._layer_workspace(plan, False)
+        ws = self._layer_workspace(plan, False, x.device)
+        ws_p, ws_bytes = ws.data_ptr(), ws.numel() * 4
         ks = 0 if row_kstart is None else row_kstart.data_ptr()
         seeds = [ops._seed(s_) for s_ in seeds]
-        shape = plan.shape
+        shape = plan.call_shape()
         acts["row_kstart"], acts["plan"] = row_kstart, plan
         at = x
         for l in range(self.cfg.layers):
             at = _SavedLayer(plan, at, torch.empty(plan.act_bytes, device=x.device, dtype=torch.uint8))
             shape.seed_attn, shape.seed_res1, shape.seed_res2 = seeds[1 + 3 * l: 4 + 3 * l]
-            _lib.check(lib.ptj_layer_fwd(shape, weights[l], at.addresses(), at.output_address(), ks, ws, ws_bytes, stream),
+            _lib.check(lib.ptj_layer_fwd(shape, weights[l], at.addresses(), at.output_address(), ks, ws_p, ws_bytes, stream),
                        "ptj_layer_fwd")
             acts["layers"].append(at)
         return x if at is x else at.output(self.dtype)
@@ -443,11 +450,12 @@ class Gpt2Step:
     def _layers_bwd(self, plan, weights, out, acts, dx, dy, seeds, ready):
         """All layers through ptj_layer_bwd_ffn and ptj_layer_bwd_attn; returns the gradient of the first one's input."""
         lib, stream = _lib.lib(), ops._stream()
-        ws, ws_bytes = self._layer_workspace(plan, True)
+        ws = self._layer_workspace(plan, True, dx.device)
+        ws_p, ws_bytes = ws.data_ptr(), ws.numel() * 4
         ks = acts.get("row_kstart")
         ks = 0 if ks is None else ks.data_ptr()
         seeds = [ops._seed(s_) for s_ in seeds]
-        shape = plan.shape
+        shape = plan.call_shape()
         # scratch shared by all layers, and the gradients of the residual stream in turn
         slab = torch.empty(plan.grad_bytes, device=dx.device, dtype=torch.uint8)
         base = slab.data_ptr()
@@ -456,13 +464,13 @@ class Gpt2Step:
         for l in range(self.cfg.layers - 1, -1, -1):
             saved = acts["layers"][l].addresses()
             shape.seed_attn, shape.seed_res1, shape.seed_res2 = seeds[1 + 3 * l: 4 + 3 * l]
-            _lib.check(lib.ptj_layer_bwd_ffn(shape, weights[l], saved, out[l], dx_p, dy_p, dh_pre, d_ln, dx_a, dy_a, ws,
+            _lib.check(lib.ptj_layer_bwd_ffn(shape, weights[l], saved, out[l], dx_p, dy_p, dh_pre, d_ln, dx_a, dy_a, ws_p,
                                              ws_bytes, stream), "ptj_layer_bwd_ffn")
             ready([f"l{l}.{n}" for n in ("b2f", "w2", "b1f", "w1", "g2", "b2")])
             below = l > 0
             _lib.check(lib.ptj_layer_bwd_attn(shape, weights[l], saved, out[l], dx_a, dy_a, d_attn, dqkv, d_ln, dx_b,
                                               dy_b if below else 0, out[l - 1].b2f if below else 0,
-                                              seeds[3 * l] if below else 0, ks, ws, ws_bytes, stream), "ptj_layer_bwd_attn")
+                                              seeds[3 * l] if below else 0, ks, ws_p, ws_bytes, stream), "ptj_layer_bwd_attn")
             ready([f"l{l}.{n}" for n in ("w_o", "w_qkv", "g1", "b1")])
             dx_p, dy_p = dx_b, dy_b
         o = plan.grad_offsets[6]

@@ -320,6 +320,7 @@ class Trainer:
         self.use_graph = (bool(self.tc.cuda_graph) and self.device.type == "cuda"
                           and not (world > 1 and self.tc.global_token_norm))
         self._graph = None           # (batch shape, [graph | bucket index, ...], static ids, static stats)
+        self._record_stream = None   # the engine keeps one recorded workspace per stream that it was recorded on
         self._seed_words = None      # int64[1 + 3 L] on the device: this step's dropout seeds, read by the kernels
         self._seed_host = None
         self.graph_launches = 0      # kernels recorded in the graph (one replay launches that many)
@@ -404,6 +405,7 @@ class Trainer:
                         fwd_bwd()
                 torch.cuda.current_stream(self.device).wait_stream(side)
                 torch.cuda.synchronize(self.device)
+                self.engine.release_workspaces()  # (the warm-up stream's: nothing runs on it again)
                 graph = torch.cuda.CUDAGraph()
                 before = _lib.launch_count()
                 with torch.cuda.graph(graph):
@@ -438,8 +440,11 @@ class Trainer:
         stay valid in the later ones, and they are always replayed in this order."""
         dev = self.device
         torch.cuda.synchronize(dev)
+        self.engine.release_workspaces()  # (the unrecorded steps': the recording makes its own)
         pool = torch.cuda.graph_pool_handle()
-        stream = torch.cuda.Stream(dev)
+        if self._record_stream is None:
+            self._record_stream = torch.cuda.Stream(dev)
+        stream = self._record_stream
         stream.wait_stream(torch.cuda.current_stream(dev))
         parts: List[object] = []
         cur = [None]

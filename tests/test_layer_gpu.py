@@ -1,4 +1,6 @@
 """A layer's launches issued by one library call against the same launches issued one by one: the same bits."""
+import threading
+
 import pytest
 import torch
 
@@ -76,3 +78,42 @@ def test_strided_weights_and_gradients(dtype):
     got = step(w.t, {**fresh(), **{n: view for n, (_, view) in buffers.items()}})
     assert all(torch.equal(a, b) for a, b in zip(want, got))
     assert all(bool((buf[:, view.shape[1]:] == 7.0).all()) for buf, view in buffers.values())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_one_engine_on_two_streams_and_threads(dtype):
+    """Passes of one engine side by side, each on a stream and a thread of its own: the bits of passes one after the other."""
+    gpt2 = pkg("gpt2")
+    cfg = gpt2.GPT2Config(vocab=304, dim=256, layers=4, heads=4, ffn=1024, seq=256, dropout=0.1)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    flat = [0.05 * torch.randn(s, generator=g, device="cuda") + (1.0 if gpt2.base_name(n)[0] == "g" else 0.0)
+            for n, s in cfg.param_shapes()]
+    w = gpt2.Weights.from_pytree(gpt2.unflatten_like(flat, cfg), cfg, dtype)
+    ys = [torch.randint(1, 304, (4, 257), generator=g, device="cuda", dtype=torch.int32) for _ in range(2)]
+    step = gpt2.Gpt2Step(cfg, dtype)
+
+    def passes(i, out, n):
+        for _ in range(n):
+            grads = {name: torch.empty(s, device="cuda") for name, s in cfg.param_shapes()}
+            stats = step.loss_and_grads(w, grads, ys[i], True, list(range(100 * i, 100 * i + 13)))
+            out.append([stats] + list(grads.values()))
+
+    want = [[], []]
+    for i in range(2):
+        passes(i, want[i], 1)
+    torch.cuda.synchronize()
+    got, streams = [[], []], [torch.cuda.Stream() for _ in range(2)]
+
+    def work(i):
+        with torch.cuda.stream(streams[i]):
+            passes(i, got[i], 8)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    for i in range(2):
+        assert len(got[i]) == 8
+        assert all(torch.equal(a, b) for one in got[i] for a, b in zip(one, want[i][0]))

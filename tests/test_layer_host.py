@@ -1,5 +1,7 @@
 """What Gpt2Step hands to the library for a layer: the whole layer in one call where every tensor is what that call takes it
 for, single launches otherwise. The library is a stand-in that records its calls, so this runs without a GPU."""
+import threading
+
 import pytest
 import torch
 
@@ -42,7 +44,6 @@ def engine(dtype=torch.float32):
     g = pkg("gpt2")
     cfg = g.GPT2Config(vocab=64, dim=16, layers=2, heads=2, ffn=32, seq=S)
     step = g.Gpt2Step(cfg, dtype)
-    step._ws = torch.zeros(1 << 16)
     weights = {n: torch.zeros(s, dtype=dtype if g.base_name(n) in g.MATRIX_TENSORS else torch.float32)
                for n, s in cfg.param_shapes()}
     return cfg, step, weights, {n: torch.zeros(s) for n, s in cfg.param_shapes()}
@@ -95,3 +96,54 @@ def test_a_gradient_that_is_not_the_configurations_goes_to_single_launches(libra
     if other is not None:
         (product,) = [a for a in library.named("ptj_gemm") if a[2] == grads[name].data_ptr()]
         assert product[11] == grads[name].stride(0) and product[15] == pkg("_lib").PTJ_F32 + (other == "bf16")
+
+
+def test_threads_in_passes_of_one_shape_keep_their_seeds(library, monkeypatch):
+    """The library reads a layer's seeds during the call, while other threads run: here two passes of one engine are both in
+    their call before either reads."""
+    cfg, step, weights, _ = engine()
+    both, seen = threading.Barrier(2, timeout=20), {}
+
+    def layer_fwd(shape, *args):
+        both.wait()
+        seen.setdefault(threading.current_thread().name, []).append((shape.seed_attn, shape.seed_res1, shape.seed_res2))
+        both.wait()
+        return 0
+
+    library.ptj_layer_fwd = layer_fwd
+    ids = torch.ones(B, S, dtype=torch.int32)
+    seeds = {name: [base + i for i in range(1 + 3 * cfg.layers)] for name, base in (("one", 10), ("two", 50))}
+    threads = [threading.Thread(target=step.forward, name=name,
+                                args=(pkg("gpt2").Weights(cfg, weights), ids, True, seeds[name])) for name in seeds]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert seen == {name: [tuple(s[1 + 3 * l:4 + 3 * l]) for l in range(cfg.layers)] for name, s in seeds.items()}
+
+
+def test_each_stream_has_a_workspace_of_its_own(library, monkeypatch):
+    """... and a recorded graph one that serves nothing else, and that stays when a larger one takes its place."""
+    cfg, step, weights, _ = engine()
+    now = {"stream": 1, "recording": False, "bytes": 1 << 12}
+    monkeypatch.setattr(pkg("operators"), "_stream", lambda: now["stream"])
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: now["recording"])
+    library.ptj_layer_workspace_bytes = lambda *a: now["bytes"]
+
+    def workspace(**kw):
+        now.update(kw)
+        step._plans.clear()
+        library.calls.clear()
+        forward(cfg, step, weights)
+        used = {a[5:7] for a in library.named("ptj_layer_fwd")}
+        assert len(used) == 1
+        return used.pop()
+
+    first, second, recorded = workspace(), workspace(stream=2), workspace(recording=True)
+    assert len({first[0], second[0], recorded[0]}) == 3
+    assert workspace(stream=1, recording=False) == first and workspace(stream=2) == second
+    larger = workspace(recording=True, bytes=1 << 14)
+    assert larger[1] == 1 << 14 and larger[0] != recorded[0]
+    assert [t.data_ptr() for t in step._held] == [recorded[0], larger[0]]
+    step.release_workspaces()
+    assert workspace() == larger and workspace(recording=False)[0] not in (recorded[0], larger[0])
