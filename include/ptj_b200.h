@@ -316,7 +316,8 @@ int ptj_attn_bwd(const void* d_o, const void* q, const void* k, const void* v, c
  * library's other entry points on contiguous tensors [batch * seq, .] (the projection's columns ordered (head, q/k/v,
  * d_head)); a status other than PTJ_OK comes from the first of them that fails. Matrices and activations are `dtype`.
  * workspace: ptj_layer_workspace_bytes bytes, 16-byte aligned, contents irrelevant before and after; with `products` zero
- * the size without what K splits and float32 tensor-core products use (they then run without). */
+ * the size without what K splits, float32 tensor-core products and the attention backward of shapes that do not need one
+ * (ptj_attn_bwd) use: they then run without. acts->keep_bits may be NULL in any case: the kernels draw the flags. */
 typedef struct {
   int64_t batch, seq, dim, heads, ffn;
   int dtype, train;
@@ -336,7 +337,7 @@ typedef struct {             /* x is the layer's input; the rest is written by t
   const void* x;
   void *ln1, *qkv, *attn;
   float *row_max, *row_sum;  /* [batch, heads, seq] */
-  uint32_t* keep_bits;       /* ptj_layer_keep_bits_bytes bytes; NULL where that is 0 */
+  uint32_t* keep_bits;       /* ptj_layer_keep_bits_bytes bytes, or NULL */
   void *x_mid, *ln2, *h_pre, *h_act;
 } ptj_layer_acts;
 typedef struct {

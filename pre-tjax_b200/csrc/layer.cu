@@ -5,7 +5,7 @@
 // residual branch's gradient and its column sums in the LayerNorm backward (model_triton.py:2343-2410, 2545-2581).
 #include <math.h>
 
-#include "common.cuh"
+#include "attn_common.cuh"
 
 using namespace ptj;
 
@@ -132,7 +132,8 @@ extern "C" size_t ptj_layer_workspace_bytes(const ptj_layer_shape* s, int backwa
     need(ptj_layernorm_bwd_scratch_floats(T, D));
     need(ptj_colsum_scratch_floats(T, F));
     const ptj_attn_shape a = l.attn_shape();
-    need((ptj_attn_bwd_workspace_bytes(&a, s->dtype) + 3) / 4);
+    // (shapes with float32 probabilities run without it, on the general kernels)
+    if (products || attn_bf16_probabilities(a)) need((ptj_attn_bwd_workspace_bytes(&a, s->dtype) + 3) / 4);
   }
   if (!products) return most * sizeof(float);
   if (s->dtype == PTJ_F32) {

@@ -17,6 +17,7 @@ the logits with their gradient; nothing uses atomics, so results are bit-reprodu
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 from dataclasses import dataclass
 from typing import Callable, List, Optional, Sequence
@@ -154,15 +155,16 @@ def tail_split_for(M: int, N: int, K: int):
 
 class _LayerPlan:
     """Sizes of one layer's launches for a batch shape: where the saved activations lie in one allocation and the gradients in
-    another (each on a 256-byte boundary), and the workspace."""
+    another (each on a 256-byte boundary), and the workspace. flags: with room for the attention dropout's keep flags, which
+    the kernels draw for themselves otherwise."""
 
-    def __init__(self, cfg: GPT2Config, dtype: torch.dtype, B: int, S: int, train: bool):
+    def __init__(self, cfg: GPT2Config, dtype: torch.dtype, B: int, S: int, train: bool, flags: bool):
         lib = _lib.lib()
         T, D, F, es = B * S, cfg.dim, cfg.ffn, 2 if dtype == torch.bfloat16 else 4
         self.shape = _lib.LayerShape(B, S, D, cfg.heads, F, _lib.PTJ_BF16 if es == 2 else _lib.PTJ_F32, int(train), cfg.dropout,
                                      0, 0, 0)
         ref = ctypes.byref(self.shape)
-        self.keep_bytes = keep = int(lib.ptj_layer_keep_bits_bytes(ref))
+        self.keep_bytes = keep = int(lib.ptj_layer_keep_bits_bytes(ref)) if flags else 0
         stats = 4 * B * cfg.heads * S
         # ln1, qkv, attn, row_max, row_sum, keep_bits, x_mid, ln2, h_pre, h_act (LayerActs after x), then the output
         self.act_offsets, self.act_bytes = self._place(
@@ -191,19 +193,16 @@ class _LayerPlan:
 
 class _SavedLayer:
     """What a layer's forward call saved: its input (a tensor, or the layer below whose output it is), and everything else,
-    its output too, in one allocation at the plan's offsets."""
-    __slots__ = ("plan", "below", "slab")
+    its output too, in one allocation at the plan's offsets. `at` holds the addresses, all inside of these."""
+    __slots__ = ("plan", "below", "slab", "at", "output_at")
 
-    def __init__(self, plan: _LayerPlan, below, slab: torch.Tensor):
-        self.plan, self.below, self.slab = plan, below, slab
-
-    def output_address(self) -> int:
-        return self.slab.data_ptr() + self.plan.out_offset
-
-    def addresses(self):
+    def __init__(self, plan: _LayerPlan, below, device):
+        self.plan, self.below = plan, below
+        self.slab = torch.empty(plan.act_bytes, device=device, dtype=torch.uint8)
         base = self.slab.data_ptr()
-        x = self.below.output_address() if isinstance(self.below, _SavedLayer) else self.below.data_ptr()
-        return _lib.LayerActs(x, *[base + o if o >= 0 else 0 for o in self.plan.act_offsets])
+        self.output_at = base + plan.out_offset
+        self.at = _lib.LayerActs(below.output_at if isinstance(below, _SavedLayer) else below.data_ptr(),
+                                 *[base + o if o >= 0 else 0 for o in plan.act_offsets])
 
     def _at(self, offset: int, dtype: torch.dtype, *shape):
         return self.slab[offset:offset + math.prod(shape) * dtype.itemsize].view(dtype).view(shape)
@@ -225,17 +224,37 @@ class _SavedLayer:
                 "h_pre": self._at(h_pre, dtype, T, s.ffn), "h_act": self._at(h_act, dtype, T, s.ffn)}
 
 
-def _addresses(tensors, wanted, device: int):
-    """Addresses of the tensors that a library call reads and writes by the configuration's sizes, or None where one of them
-    is not what the call takes it for: `wanted` lists (name, shape, dtype), all contiguous and on one device. Looked at in
-    every pass, since tensors can be resized or replaced between two."""
-    out = []
-    for name, shape, dtype in wanted:
-        t = tensors[name]
-        if t.shape != shape or t.dtype is not dtype or not t.is_contiguous() or t.get_device() != device:
+class _Wanted:
+    """What a library call takes the tensors of every layer for, which it reads and writes by the configuration's sizes:
+    contiguous, of these shapes and types, on one device. Looked at in every pass, since tensors can be replaced or resized
+    between two; lists are compared whole, a third of a microsecond a tensor."""
+
+    def __init__(self, struct, cfg: GPT2Config, matrix_dtype: torch.dtype, only=LAYER_TENSORS):
+        self.struct, self.per_layer = struct, len(only)
+        self.fields = only
+        wanted = [(n, torch.Size(s)) for n, s in cfg.param_shapes() if "." in n and base_name(n) in only]
+        self.names, self.shapes = [n for n, _ in wanted], [s for _, s in wanted]
+        self.dtypes = [matrix_dtype if base_name(n) in MATRIX_TENSORS else torch.float32 for n in self.names]
+
+    def of(self, tensors, device: int):
+        """One struct of addresses per layer, or None where a tensor is something else: single launches, which take a stride
+        and a type each or refuse, do those."""
+        found = [tensors[n] for n in self.names]
+        if ([t.shape for t in found] != self.shapes or [t.dtype for t in found] != self.dtypes
+                or not all([t.is_contiguous() for t in found]) or any([t.get_device() != device for t in found])):
             return None
-        out.append(t.data_ptr())
-    return out
+        at, n = [t.data_ptr() for t in found], self.per_layer
+        if self.fields is LAYER_TENSORS:
+            return [self.struct(*at[i:i + n]) for i in range(0, len(at), n)]
+        return [self.struct(**dict(zip(self.fields, at[i:i + n]))) for i in range(0, len(at), n)]
+
+
+@functools.lru_cache(maxsize=64)  # (the pytree functions make an engine per call)
+def _wanted(cfg: GPT2Config, dtype: torch.dtype):
+    """What the forward call takes its weights for, the backward calls those that they read, and these the gradients."""
+    return (_Wanted(_lib.LayerWeights, cfg, dtype),
+            _Wanted(_lib.LayerWeights, cfg, dtype, ("g1", "w_qkv", "w_o", "g2", "w1", "w2")),
+            _Wanted(_lib.LayerGrads, cfg, torch.float32))
 
 
 class Gpt2Step:
@@ -257,11 +276,8 @@ class Gpt2Step:
         self.pair_wgrads = True
         # input gradients whose last round of tiles is mostly empty: that round's rows split over K, same launch
         self.tail_split = True
-        # (name, shape, dtype) of each layer's weights and of their gradients
-        in_layer = [(n, torch.Size(s)) for n, s in cfg.param_shapes() if "." in n]
-        self._layer_weights = [(n, s, compute_dtype if base_name(n) in MATRIX_TENSORS else torch.float32) for n, s in in_layer]
-        self._layer_grads = [(n, s, torch.float32) for n, s in in_layer]
-        self._plans = {}    # (batch, seq, train) -> _LayerPlan
+        self._fwd_weights, self._bwd_weights, self._grads = _wanted(cfg, compute_dtype)
+        self._plans = {}    # (batch, seq, train, flags) -> _LayerPlan
 
     # -- helpers --
     def _wgrad(self, dy2d, x2d, out, accumulate=False):
@@ -294,6 +310,9 @@ class Gpt2Step:
                 if least is None:
                     raise
                 if have < least:
+                    ws = None
+                    if not recording:
+                        self._ws.pop(key, None)  # (too small for either)
                     ws = torch.empty(least, device=device, dtype=torch.float32)
             if ws is not self._ws.get(key):
                 self._ws[key] = ws
@@ -306,15 +325,25 @@ class Gpt2Step:
         self._ws = {k: ws for k, ws in self._ws.items() if k[2]}
 
     def _layer_workspace(self, plan, backward: bool, device):
-        """The workspace of a layer's launches; without the part that only makes products faster where that does not fit (as
-        for a single product, operators.gemm)."""
+        """The workspace of a layer's launches; without the part that only makes them faster where that does not fit (as for
+        single launches, operators.gemm and operators.attn_bwd)."""
         return self._workspace(max(1, plan.ws_floats[backward]), device, least=max(1, plan.ws_least[backward]))
 
-    def _plan(self, B: int, S: int, train: bool):
-        key = (B, S, train)
+    def _with_room(self, launch):
+        """launch(), and once more without the kept workspaces where it finds no memory."""
+        try:
+            return launch()
+        except torch.OutOfMemoryError:
+            if torch.cuda.is_current_stream_capturing():
+                raise
+        self.release_workspaces()
+        return launch()
+
+    def _plan(self, B: int, S: int, train: bool, flags: bool = True):
+        key = (B, S, train, flags)
         plan = self._plans.get(key)
         if plan is None:
-            plan = self._plans[key] = _LayerPlan(self.cfg, self.dtype, B, S, train)
+            plan = self._plans[key] = _LayerPlan(self.cfg, self.dtype, B, S, train, flags)
         return plan
 
     def _native(self, plan) -> bool:
@@ -322,14 +351,6 @@ class Gpt2Step:
         product with events or has switched one of the variants above, which are sequences of their own."""
         return (ops.GEMM_PROFILE is None and not self.split_gelu_bwd and self.pair_wgrads and self.tail_split
                 and plan.fused)
-
-    @staticmethod
-    def _per_layer(struct, tensors, wanted, device: int):
-        """One struct of addresses per layer, or None where a tensor is not what the struct's reader takes it for: strided,
-        of another shape or type. Single launches (which take a stride and a type each, or refuse) do those."""
-        at = _addresses(tensors, wanted, device)
-        n = len(LAYER_TENSORS)
-        return None if at is None else [struct(*at[i:i + n]) for i in range(0, len(at), n)]
 
     def _wgrad2(self, first, second):
         """Two weight gradients (dy, x, out) in ONE launch of the thread-block-pair kernel when both qualify: their
@@ -380,13 +401,24 @@ class Gpt2Step:
                 split = split_k_for(T, N, K)
                 floats = split * T * N
         return ops.gemm(dy2d, w2d, a_kmajor=True, b_kmajor=False, M=T, N=N, K=K, lda=dy2d.stride(0),
-                        ldb=w2d.stride(0), out_dtype=self.dtype, split_k=split, workspace=self._workspace(floats, dy2d.device), **kw)
+                        ldb=w2d.stride(0), out_dtype=self.dtype, split_k=split,
+                        workspace=self._workspace(floats, dy2d.device) if floats else None, **kw)
 
     # -- forward --
     def forward(self, w: Weights, ids_in: torch.Tensor, train: bool, seeds: Sequence[int], row_kstart=None):
         """Returns (logits [B*S, vocab_ld] (first `vocab` columns valid), saved activations).
         row_kstart: optional int32 [B, S], first key each position attends to (packed documents / padding, see
         operators.row_kstart_from_mask); None = plain causal attention."""
+        try:
+            return self._forward(w, ids_in, train, seeds, row_kstart, True)
+        except torch.OutOfMemoryError:  # once more without what is kept only to be faster
+            if torch.cuda.is_current_stream_capturing():
+                raise
+        self.release_workspaces()
+        return self._forward(w, ids_in, train, seeds, row_kstart, False)
+
+    def _forward(self, w: Weights, ids_in: torch.Tensor, train: bool, seeds: Sequence[int], row_kstart, flags: bool):
+        """flags: the attention dropout's keep flags are drawn beforehand and saved, where the kernels take them."""
         cfg, p = self.cfg, self.cfg.dropout
         B, S = ids_in.shape
         assert S == cfg.seq, "the positional table is added without slicing: sequence length must equal cfg.seq"
@@ -395,8 +427,8 @@ class Gpt2Step:
             seeds = [0] * (1 + 3 * cfg.layers)
         x = ops.embed_fwd(ids_in, w["w_emb"], w["w_pos"], train, seeds[0], out_dtype=self.dtype, p=p).view(T, D)
         acts = {"layers": [], "row_kstart": row_kstart}
-        plan = self._plan(B, S, bool(train))
-        weights = self._per_layer(_lib.LayerWeights, w.t, self._layer_weights, x.get_device()) if self._native(plan) else None
+        plan = self._plan(B, S, bool(train), flags)
+        weights = self._fwd_weights.of(w.t, x.get_device()) if self._native(plan) else None
         native = weights is not None
         if native:
             row_kstart = ops._check_kstart(row_kstart, B, S, x.device)
@@ -412,7 +444,7 @@ class Gpt2Step:
             a["attn"] = x.new_empty((T, D))
             o4 = a["attn"].view(B, S, H, dh).transpose(1, 2)
             # the layer's attention-dropout keep flags are drawn once and shared by the forward and backward kernels
-            a["keep"] = ops.attn_keep_bits(q, k, v, o4, s_attn, p=p) if (train and p > 0.0) else None
+            a["keep"] = ops.attn_keep_bits(q, k, v, o4, s_attn, p=p) if (flags and train and p > 0.0) else None
             a["m"], a["l"] = ops.attn_fwd(q, k, v, o4, train, s_attn, p=p, keep_bits=a["keep"], row_kstart=row_kstart)
             a["x_mid"] = ops.gemm(a["attn"], g("w_o"), epilogue=_lib.EPI_DROPOUT_RESID, aux=x,
                                   dropout_args=(p, train, s_res1, 0))
@@ -440,9 +472,9 @@ class Gpt2Step:
         acts["row_kstart"], acts["plan"] = row_kstart, plan
         at = x
         for l in range(self.cfg.layers):
-            at = _SavedLayer(plan, at, torch.empty(plan.act_bytes, device=x.device, dtype=torch.uint8))
+            at = _SavedLayer(plan, at, x.device)
             shape.seed_attn, shape.seed_res1, shape.seed_res2 = seeds[1 + 3 * l: 4 + 3 * l]
-            _lib.check(lib.ptj_layer_fwd(shape, weights[l], at.addresses(), at.output_address(), ks, ws_p, ws_bytes, stream),
+            _lib.check(lib.ptj_layer_fwd(shape, weights[l], at.at, at.output_at, ks, ws_p, ws_bytes, stream),
                        "ptj_layer_fwd")
             acts["layers"].append(at)
         return x if at is x else at.output(self.dtype)
@@ -450,19 +482,19 @@ class Gpt2Step:
     def _layers_bwd(self, plan, weights, out, acts, dx, dy, seeds, ready):
         """All layers through ptj_layer_bwd_ffn and ptj_layer_bwd_attn; returns the gradient of the first one's input."""
         lib, stream = _lib.lib(), ops._stream()
+        # scratch shared by all layers, and the gradients of the residual stream in turn
+        slab = self._with_room(lambda: torch.empty(plan.grad_bytes, device=dx.device, dtype=torch.uint8))
         ws = self._layer_workspace(plan, True, dx.device)
         ws_p, ws_bytes = ws.data_ptr(), ws.numel() * 4
         ks = acts.get("row_kstart")
         ks = 0 if ks is None else ks.data_ptr()
         seeds = [ops._seed(s_) for s_ in seeds]
         shape = plan.call_shape()
-        # scratch shared by all layers, and the gradients of the residual stream in turn
-        slab = torch.empty(plan.grad_bytes, device=dx.device, dtype=torch.uint8)
         base = slab.data_ptr()
         dh_pre, d_ln, d_attn, dqkv, dx_a, dy_a, dx_b, dy_b = [base + o for o in plan.grad_offsets]
         dx_p, dy_p = dx.data_ptr(), dy.data_ptr()
         for l in range(self.cfg.layers - 1, -1, -1):
-            saved = acts["layers"][l].addresses()
+            saved = acts["layers"][l].at
             shape.seed_attn, shape.seed_res1, shape.seed_res2 = seeds[1 + 3 * l: 4 + 3 * l]
             _lib.check(lib.ptj_layer_bwd_ffn(shape, weights[l], saved, out[l], dx_p, dy_p, dh_pre, d_ln, dx_a, dy_a, ws_p,
                                              ws_bytes, stream), "ptj_layer_bwd_ffn")
@@ -492,7 +524,7 @@ class Gpt2Step:
         ops.colsum(dlogits, cols=V, out=grads["b_head"])
         self._head_wgrad(dlogits, acts["x_f"], grads["w_emb"])
         ready(["b_head"])
-        d = self._dgrad(dlogits, w["w_emb"], cols=V)
+        d = self._with_room(lambda: self._dgrad(dlogits, w["w_emb"], cols=V))
         # every LayerNorm backward also writes dropout(dx) for the residual branch that consumes it next
         fuse = D % 8 == 0 and D <= (2048 if self.dtype == torch.bfloat16 else 1024)
         s_next = seeds[3 * cfg.layers] if cfg.layers > 0 else 0  # last layer's second residual dropout
@@ -504,8 +536,7 @@ class Gpt2Step:
 
         native = "plan" in acts and cfg.layers > 0  # as the forward pass went
         if native:
-            weights = self._per_layer(_lib.LayerWeights, w.t, self._layer_weights, dx.get_device())
-            out = self._per_layer(_lib.LayerGrads, grads, self._layer_grads, dx.get_device())
+            weights, out = self._bwd_weights.of(w.t, dx.get_device()), self._grads.of(grads, dx.get_device())
             native = weights is not None and out is not None
         if native:
             dx = self._layers_bwd(self._plan(B, S, bool(train)), weights, out, acts, dx, dy, seeds, ready)

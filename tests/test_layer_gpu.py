@@ -1,4 +1,5 @@
 """A layer's launches issued by one library call against the same launches issued one by one: the same bits."""
+import ctypes
 import threading
 
 import pytest
@@ -117,3 +118,48 @@ def test_one_engine_on_two_streams_and_threads(dtype):
     for i in range(2):
         assert len(got[i]) == 8
         assert all(torch.equal(a, b) for one in got[i] for a, b in zip(one, want[i][0]))
+
+
+@pytest.mark.parametrize("dim,heads,S", [(256, 4, 200), (128, 4, 384)])  # ragged rows; 32-wide heads
+def test_a_step_without_room_for_flags_and_workspace(dim, heads, S, monkeypatch):
+    """bf16 attention off whole tiles of 64-wide heads needs neither keep flags nor a workspace: a step that finds no room for
+    them takes the flags from the kernels and the general backward kernels, and needs no more memory than that."""
+    ops, gpt2, lib = pkg("operators"), pkg("gpt2"), pkg("_lib")
+    cfg = gpt2.GPT2Config(vocab=304, dim=dim, layers=2, heads=heads, ffn=4 * dim, seq=S, dropout=0.1)
+    g = torch.Generator(device="cuda").manual_seed(4)
+    flat = [0.05 * torch.randn(s, generator=g, device="cuda") + (1.0 if gpt2.base_name(n)[0] == "g" else 0.0)
+            for n, s in cfg.param_shapes()]
+    w = gpt2.Weights.from_pytree(gpt2.unflatten_like(flat, cfg), cfg, torch.bfloat16)
+    B = 4
+    y = torch.randint(1, 304, (B, S + 1), generator=g, device="cuda", dtype=torch.int32)
+    plan = gpt2._LayerPlan(cfg, torch.bfloat16, B, S, True, True)
+    attention = lib.lib().ptj_attn_bwd_workspace_bytes(
+        ctypes.byref(lib.AttnShape(B, heads, S, dim // heads, *[(3 * S * dim, 3 * dim // heads, 3 * dim)] * 3,
+                                   (S * dim, dim // heads, dim))), lib.PTJ_BF16)
+    assert 0 < 4 * plan.ws_least[1] < attention <= 4 * plan.ws_floats[1] and plan.keep_bytes > 0
+    small = gpt2._LayerPlan(cfg, torch.bfloat16, B, S, True, False)
+    real, limit = torch.empty, [None]
+
+    def empty(*shape, **kw):
+        if limit[0] is not None and shape in limit[0]:
+            raise torch.OutOfMemoryError("no room")
+        return real(*shape, **kw)
+
+    monkeypatch.setattr(torch, "empty", empty)
+    results = []
+    for short in (False, True):
+        limit[0] = [(plan.act_bytes,), (plan.ws_floats[1],)] if short else None
+        step = gpt2.Gpt2Step(cfg, torch.bfloat16)
+        grads = {n: torch.zeros(s, device="cuda") for n, s in cfg.param_shapes()}
+        stats = step.loss_and_grads(w, grads, y, True, list(range(5, 12)))
+        torch.cuda.synchronize()
+        assert ops.last_kernel_fault() == 0
+        results.append((stats, grads))
+        kept = sum(t.numel() for t in step._ws.values())
+        assert kept <= max(small.ws_least[1], small.ws_floats[0]) if short else kept >= plan.ws_floats[1]
+    (want, a), (got, b) = results
+    assert torch.equal(want, got)  # the forward pass is the same: flags drawn beforehand or by the kernel
+    # The backward kernels differ by float32 errors, so that single values round to the next bf16 one, 2^-8 of it away. All of
+    # them would move a gradient by 2^-8; a hundredth part does, and each of the two layers adds its own.
+    for n in a:
+        assert float((a[n] - b[n]).norm()) <= 2.0 ** -8 * float(a[n].norm()), n

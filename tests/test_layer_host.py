@@ -147,3 +147,30 @@ def test_each_stream_has_a_workspace_of_its_own(library, monkeypatch):
     assert [t.data_ptr() for t in step._held] == [recorded[0], larger[0]]
     step.release_workspaces()
     assert workspace() == larger and workspace(recording=False)[0] not in (recorded[0], larger[0])
+
+
+def test_a_pass_that_finds_no_memory_runs_without_what_only_makes_it_faster(library, monkeypatch):
+    """Keep flags and the larger workspace are given up, in the forward pass wherever memory ran out, then in the backward
+    pass; the gradients' own buffer comes before the workspace."""
+    cfg, step, weights, grads = engine(torch.bfloat16)
+    big, limit, real = 1 << 30, [None], torch.empty
+
+    def empty(*shape, **kw):
+        t = real(*shape, **{**kw, "device": "meta"})
+        if limit[0] is not None and t.numel() * t.element_size() >= limit[0]:
+            raise torch.OutOfMemoryError("no room")
+        return t if t.numel() * t.element_size() >= big else real(*shape, **kw)
+
+    monkeypatch.setattr(torch, "empty", empty)
+    library.ptj_layer_keep_bits_bytes = lambda shape: big
+    library.ptj_layer_workspace_bytes = lambda shape, backward, products: big if products else 256
+    _, acts, _, _ = forward(cfg, step, weights)
+    calls = library.named("ptj_layer_fwd")
+    assert len(calls) == cfg.layers and all(a[2].keep_bits and a[6] == big for a in calls)
+    library.calls.clear()
+    limit[0] = big
+    logits, acts, ids, seeds = forward(cfg, step, weights)
+    calls = library.named("ptj_layer_fwd")
+    assert len(calls) == cfg.layers and all(not a[2].keep_bits and a[6] == 256 for a in calls)
+    step.backward(pkg("gpt2").Weights(cfg, weights), grads, logits, acts, ids, True, seeds)
+    assert [a[-2] for a in library.named("ptj_layer_bwd_attn")] == [256] * cfg.layers
