@@ -560,7 +560,8 @@ attn_bwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       tmem_ld_wait();
       arrive(&s_free[x]);  // dP may now overwrite the scores
       const uint64_t nl2 = pack2(-lse, -lse);
-      const bool odd = kExact && *bad_s != 0;
+      // (one answer for the warp: others may be raising the flag, and what follows is a warp's)
+      const bool odd = kExact && __any_sync(0xffffffffu, *bad_s != 0);
       // keys after the row (diagonal tile), before its document, rows beyond the sequence
       const bool edge = c.i == c.kt || p.kstart != nullptr || c.i * T + T > p.S || odd;
       uint8_t* w_tile = w_s + xw * PARTS * kPBytes;

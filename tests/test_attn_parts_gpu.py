@@ -1,5 +1,7 @@
 """Attention on the tensor cores with float32 probabilities in three bf16 parts (bf16 operands; every row length and head size
 but whole tiles of 64-wide heads) against float64: edges of tiles, narrow and wide heads, one to several tiles and items."""
+import math
+
 import pytest
 import torch
 
@@ -61,3 +63,50 @@ def test_keep_flags_and_a_missing_workspace(S, D):
     # two roundings to bf16 of values that differ by float32 errors: at most one unit in the last place (2^-7 of the value)
     for a, b in zip(res[0], res[2]):
         assert bool(((a.double() - b.double()).abs() <= 2.0 ** -7 * b.double().abs() + 1e-5).all())
+
+
+@pytest.mark.parametrize("S,D,p,flags,packed", [
+    (300, 128, 0.1, False, False),  # single buffers, three tiles: operands are looked at after the tile before is done
+    (300, 128, 0.1, True, True),
+    (500, 64, 0.2, True, False),    # four tiles, two groups, flags drawn beforehand
+    (260, 32, 0.0, False, True),
+])
+@pytest.mark.parametrize("what", ["one", "rows", "all"])
+def test_nonfinite_operands_give_what_the_general_kernels_give(S, D, p, flags, packed, what):
+    """Infinities and NaNs in Q, K, V or dO over several tiles: the same elements of every result are infinite or NaN as from
+    the general kernels, which rows on an odd stride run on, and the others agree."""
+    ops = pkg("operators")
+    B, H, seed = 3, 60, 5  # several items a block: what one meets does not reach the next
+    g = torch.Generator(device="cuda").manual_seed(S + D)
+    clean = [torch.randn(B, H, S, D, generator=g, device="cuda").bfloat16() for _ in range(4)]
+    ks = ops.row_kstart_from_lengths(documents(B, S, packed), S) if packed else None
+    bad = torch.tensor([math.nan, math.inf, -math.inf], device="cuda").bfloat16()
+    spread = lambda t: torch.nn.functional.pad(t, (0, 3))[..., :D]
+    for which in range(4):
+        x = [t.clone() for t in clean]
+        if what == "one":
+            x[which][0, 1, S // 2, D // 2] = bad[1]
+            x[which][1, 5, S - 3, 1] = bad[0]
+            x[which][2, 59, 0, D - 1] = bad[2]
+        elif what == "rows":
+            x[which][:, ::3, 5:S:37] = bad[torch.randint(0, 3, (B, H // 3, len(range(5, S, 37)), D), generator=g, device="cuda")]
+        else:
+            x[which][:, ::2] = bad[0]
+        q, k, v, do = x
+        o, dq, dk, dv = (torch.empty_like(q) for _ in range(4))
+        bits = ops.attn_keep_bits(q, k, v, o, seed, p=p) if flags else None
+        assert (bits is not None) == flags
+        m, l = ops.attn_fwd(q, k, v, o, True, seed, p=p, keep_bits=bits, row_kstart=ks)
+        ops.attn_bwd(do, q, k, v, o, m, l, dq, dk, dv, True, seed, p=p, keep_bits=bits, row_kstart=ks)
+        sq, sk, sv, sdo, so, go, gq, gk, gv = (spread(t) for t in (q, k, v, do, o, o, dq, dk, dv))
+        gm, _ = ops.attn_fwd(sq, sk, sv, go, True, seed, p=p, row_kstart=ks)
+        ops.attn_bwd(sdo, sq, sk, sv, so, m, l, gq, gk, gv, True, seed, p=p, row_kstart=ks)
+        torch.cuda.synchronize()
+        assert ops.last_kernel_fault() == 0
+        for name, got, want in (("O", o, go), ("maximum", m, gm), ("dQ", dq, gq), ("dK", dk, gk), ("dV", dv, gv)):
+            got, want = got.double(), want.double()
+            same = torch.where(torch.isfinite(want), torch.isfinite(got), (got == want) | (got.isnan() & want.isnan()))
+            assert bool(same.all()), (which, name, int((~same).sum()))
+            # two roundings to bf16, 2^-8 of the value each, and 2^-17 of sums of magnitudes (below 32) for float32 sums
+            err = (got - want).abs()[torch.isfinite(want)] - 2.0 ** -7 * want.abs()[torch.isfinite(want)]
+            assert err.numel() == 0 or float(err.max()) <= 2.0 ** -12, (which, name, float(err.max()))
