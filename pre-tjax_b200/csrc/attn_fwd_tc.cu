@@ -557,7 +557,8 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         if (cb == 0 && q_row < p.S) {
           const int64_t ri = static_cast<int64_t>(c.bh) * p.S + q_row;
           row_max[ri] = none ? 0.f : mt * p.scale;  // acts0: row maximum of the scaled scores
-          row_sum[ri] = none ? 1.f : lsum * ex2_approx((mx - mt) * sc - kShift);  // acts1: sum of exp(score - maximum)
+          // acts1: sum of exp(score - maximum); every score -inf: no reference to move from
+          row_sum[ri] = none ? 1.f : (mx == -INFINITY ? lsum : lsum * ex2_approx((mx - mt) * sc - kShift));
         }
       }
       c.advance(sched);

@@ -110,3 +110,17 @@ def test_nonfinite_operands_give_what_the_general_kernels_give(S, D, p, flags, p
             # two roundings to bf16, 2^-8 of the value each, and 2^-17 of sums of magnitudes (below 32) for float32 sums
             err = (got - want).abs()[torch.isfinite(want)] - 2.0 ** -7 * want.abs()[torch.isfinite(want)]
             assert err.numel() == 0 or float(err.max()) <= 2.0 ** -12, (which, name, float(err.max()))
+
+
+@pytest.mark.parametrize("S,D", [(300, 128), (200, 64)])
+def test_statistics_of_rows_whose_scores_are_all_minus_infinity(S, D):
+    """The maximum is -inf then, and the sum of exponentials 0, as from the general kernels."""
+    ops = pkg("operators")
+    q = torch.ones(1, 2, S, D, device="cuda", dtype=torch.bfloat16)
+    k, v = torch.full_like(q, 0.5), torch.ones_like(q)
+    k[:, :, :40, 3] = -math.inf  # rows up to 39 attend nothing else
+    o = torch.empty_like(q)
+    m, l = ops.attn_fwd(q, k, v, o, True, 1, p=0.0)
+    assert bool((m[..., :40] == -math.inf).all()) and bool((l[..., :40] == 0).all()) and bool(o[:, :, :40].isnan().all())
+    rows = torch.arange(1, S - 39, device="cuda", dtype=torch.float32)  # equal scores
+    assert bool(torch.isfinite(m[..., 40:]).all()) and bool(((l[..., 40:] - rows).abs() <= 2.0 ** -20 * rows).all())
