@@ -60,37 +60,71 @@ constexpr int kTmemCols = 512;
 constexpr uint32_t kColO = kSBufs * T;
 
 // An item one of whose V tiles held an infinity or a NaN (replaced by zero before it was multiplied): the products of a
-// row's attended probabilities with those elements, columns [col0, col0 + 16). Slow and rare.
+// row's attended probabilities with those elements, columns [col0, col0 + 16), added to o. A whole warp, a row a lane (`live`:
+// the row exists and attends keys). Each lane looks at one key's elements, so that keys without such elements cost a
+// thirty-second of a load; a key's probabilities are formed where they may change something: a column that is NaN stays NaN,
+// and with all of them the rest of the keys is left out. Forward passes of
+// [8, 12, 1024, 32] (117 us) and [8, 12, 1024, 128] (140) with one NaN in V: 138 and 199 us (a thread for itself, key by key, and
+// in all later items of the block: 4751 and 8352), with nothing else in V: 220 and 391 (24 and 246 ms).
 __device__ __noinline__ void add_nonfinite_v(float (&o)[16], const RowView& q, const RowView& k, const RowView& v, const AttnParams& p,
-                                             const uint32_t* rk_s, int mode, int bh, int q_row, int first_key, int col0,
+                                             const uint32_t* rk_s, int mode, int bh, int q_row, int first_key, bool live, int col0,
                                              float m_true) {
-  const int b = bh / p.H, h = bh % p.H;
-  const __nv_bfloat16* qr = q.row(b, h, q_row);
-  for (int j = max(first_key, 0); j <= q_row; ++j) {
-    const __nv_bfloat16* vr = v.row(b, h, j);
+  const int b = bh / p.H, h = bh % p.H, lane = threadIdx.x & 31;
+  const int vecs = min(2, (p.D - col0) / 8);
+  if (vecs <= 0) return;
+  const uint32_t all = (1u << (8 * vecs)) - 1u;
+  const int begin = __reduce_min_sync(0xffffffffu, live ? max(first_key, 0) : 0x7fffffff);
+  const int end = __reduce_max_sync(0xffffffffu, live ? q_row : -1);
+  uint32_t nan = 0u;  // columns of this lane's row that are NaN by now
+  for (int j0 = begin; j0 <= end; j0 += 32) {
     uint32_t bad = 0u;
-    for (int i = 0; i < 16 && col0 + i < p.D; ++i)
-      if (!isfinite(__bfloat162float(vr[col0 + i]))) bad |= 1u << i;
-    if (bad == 0u) continue;
-    const __nv_bfloat16* kr = k.row(b, h, j);
-    float s = 0.f;
-    for (int d = 0; d < p.D; ++d) s = fmaf(__bfloat162float(qr[d]), __bfloat162float(kr[d]), s);
-    float w = ex2_approx((s - m_true) * p.scale_log2);
-    if (mode != 0) {
-      const uint64_t idx = (static_cast<uint64_t>(bh) * p.S + q_row) * p.S + j;
-      uint32_t keep;
-      if (mode == 1) {
-        keep = keep_word(rk_s, idx, p.dr.stream_id, p.dr.thr16 << 16) & 1u;
-      } else {
-        const int qt = q_row / T, kt = j / T;
-        const uint32_t* words = reinterpret_cast<const uint32_t*>(p.keep_bits);
-        const int64_t tile = static_cast<int64_t>(bh) * (p.nq * (p.nq + 1) / 2) + qt * (qt + 1) / 2 + kt;
-        keep = (__ldg(words + (tile * T + q_row % T) * 4 + (j % T) / 32) >> (j & 31)) & 1u;
+    if (j0 + lane <= end) {
+      const uint4* vr = reinterpret_cast<const uint4*>(v.row(b, h, j0 + lane) + col0);
+      for (int x = 0; x < vecs; ++x) {
+        const uint4 e = vr[x];
+        const uint32_t w[4] = {e.x, e.y, e.z, e.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if ((w[i] & 0x7f80u) == 0x7f80u) bad |= 1u << (8 * x + 2 * i);
+          if ((w[i] & 0x7f800000u) == 0x7f800000u) bad |= 2u << (8 * x + 2 * i);
+        }
       }
-      if (keep == 0u) w = 0.f;
     }
-    for (int i = 0; i < 16; ++i)
-      if ((bad >> i) & 1u) o[i] += w * __bfloat162float(vr[col0 + i]);
+    for (uint32_t keys = __ballot_sync(0xffffffffu, bad != 0u); keys != 0u; keys &= keys - 1u) {
+      const int src = __ffs(keys) - 1, j = j0 + src;
+      const uint32_t cols = __shfl_sync(0xffffffffu, bad, src);
+      if (!live || j < first_key || j > q_row || (cols & ~nan) == 0u) continue;  // (each lane goes its own way to the next key)
+      const uint4 *qr = reinterpret_cast<const uint4*>(q.row(b, h, q_row)), *kr = reinterpret_cast<const uint4*>(k.row(b, h, j));
+      float s = 0.f;
+      for (int d = 0; d < p.D / 8; ++d) {
+        const uint4 x = qr[d], y = kr[d];
+        const uint32_t xw[4] = {x.x, x.y, x.z, x.w}, yw[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s = fmaf(bf16_hi(xw[i]), bf16_hi(yw[i]), fmaf(bf16_lo(xw[i]), bf16_lo(yw[i]), s));
+      }
+      float w = ex2_approx((s - m_true) * p.scale_log2);
+      if (mode != 0) {
+        const uint64_t idx = (static_cast<uint64_t>(bh) * p.S + q_row) * p.S + j;
+        uint32_t keep;
+        if (mode == 1) {
+          keep = keep_word(rk_s, idx, p.dr.stream_id, p.dr.thr16 << 16) & 1u;
+        } else {
+          const int qt = q_row / T, kt = j / T;
+          const uint32_t* words = reinterpret_cast<const uint32_t*>(p.keep_bits);
+          const int64_t tile = static_cast<int64_t>(bh) * (p.nq * (p.nq + 1) / 2) + qt * (qt + 1) / 2 + kt;
+          keep = (__ldg(words + (tile * T + q_row % T) * 4 + (j % T) / 32) >> (j & 31)) & 1u;
+        }
+        if (keep == 0u) w = 0.f;
+      }
+      const __nv_bfloat16* vr = v.row(b, h, j) + col0;
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        if ((cols >> i) & 1u) {
+          o[i] += w * __bfloat162float(vr[i]);
+          if (isnan(o[i])) nan |= 1u << i;
+        }
+    }
+    if (__all_sync(0xffffffffu, !live || nan == all)) break;
   }
 }
 
@@ -132,7 +166,9 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   uint64_t* o_free = stats_full + 1;        // the item's accumulators and states have been read
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_free + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  volatile int* bad_v = abort_flag + 1;  // a V tile of this block held an element that is not finite
+  // [2] ordinal + 1 of the last even / odd item of which a V tile held an element that is not finite. (An item's slot is
+  // written again two items on, and that one's tiles wait for this one's rows to be merged.)
+  volatile int* bad_v = abort_flag + 1;
   uint32_t* rk_s = tmem_slot + 4;        // Philox round keys (MODE 1)
   int* first_tab = reinterpret_cast<int*>(rk_s + 20);  // [kMaxRoundsTabled] first KV tile of this block's items
 
@@ -143,7 +179,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     for (uint64_t* b = bars; b < s_free; ++b) mbar_init(b, 1);  // TMA / MMA completions
     for (uint64_t* b = s_free; b < o_free + 1; ++b) mbar_init(b, b == stats_full ? C::kWarps : C::kGroupWarps);
     *abort_flag = 0;
-    *bad_v = 0;
+    bad_v[0] = bad_v[1] = 0;
     fence_barrier_init();
     prefetch_tensormap(&tm_q);
     prefetch_tensormap(&tm_k);
@@ -473,7 +509,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           bool bad = false;
 #pragma unroll
           for (int x = 0; x < kTB / C::kGroupWarps; x += 512) bad = zero_nonfinite(vt + x) || bad;
-          if (bad) *bad_v = 1;
+          if (bad) bad_v[c.ord & 1] = c.ord + 1;
         }
         fence_proxy_async_smem();
         tc_fence_before_sync();
@@ -499,6 +535,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after_sync();
+        const bool odd = __any_sync(0xffffffffu, bad_v[c.ord & 1] == c.ord + 1);  // (read before o_free lets the slot go)
         const bool single = c.j == c.j0;  // the other group had no tile of this item: its accumulators hold anything
         float mx = -INFINITY, mt = -INFINITY, f[C::kAcc], lsum = 0.f;
 #pragma unroll
@@ -536,15 +573,15 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             __syncwarp();
             if (lane == 0) mbar_arrive(o_free);  // the next item may overwrite the accumulators
           }
+          if (odd) {
+            float t[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) t[i] = 0.f;
+            add_nonfinite_v(t, views.q, views.k, views.v, p, rk_s, MODE, c.bh, q_row, first_key, q_row < p.S && !none, col, mt);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) o[i] += t[i];
+          }
           if (q_row < p.S) {
-            if (*bad_v != 0 && !none) {
-              float t[16];
-#pragma unroll
-              for (int i = 0; i < 16; ++i) t[i] = 0.f;
-              add_nonfinite_v(t, views.q, views.k, views.v, p, rk_s, MODE, c.bh, q_row, first_key, col, mt);
-#pragma unroll
-              for (int i = 0; i < 16; ++i) o[i] += t[i];
-            }
 #pragma unroll
             for (int c8 = 0; c8 < 2; ++c8) {
               float t[8];
