@@ -174,3 +174,33 @@ def test_a_pass_that_finds_no_memory_runs_without_what_only_makes_it_faster(libr
     assert len(calls) == cfg.layers and all(not a[2].keep_bits and a[6] == 256 for a in calls)
     step.backward(pkg("gpt2").Weights(cfg, weights), grads, logits, acts, ids, True, seeds)
     assert [a[-2] for a in library.named("ptj_layer_bwd_attn")] == [256] * cfg.layers
+
+
+def test_attention_backward_without_room_for_its_workspace(monkeypatch):
+    """Shapes that the general kernels can take run there; whole tiles of 64-wide heads say that memory ran out."""
+    ops, calls = pkg("operators"), []
+
+    class Library:
+        def ptj_attn_bwd_workspace_bytes(self, *a):
+            return 1 << 40
+
+        def ptj_attn_bwd(self, *a):
+            calls.append(a)
+            return 0
+
+    def empty(*a, **kw):
+        raise torch.OutOfMemoryError("no room")
+
+    monkeypatch.setattr(ops._lib, "lib", Library)
+    monkeypatch.setattr(ops, "_stream", lambda: 0)
+    monkeypatch.setattr(ops, "attn_bwd_workspace", empty)
+    for N, D, runs in ((100, 64, True), (128, 32, True), (128, 64, False)):
+        t = torch.ones(1, 1, N, D, dtype=torch.bfloat16)
+        m = torch.ones(1, 1, N)
+        calls.clear()
+        if not runs:
+            with pytest.raises(torch.OutOfMemoryError):
+                ops.attn_bwd(t, t, t, t, t, m, m, t, t, t, True, 1)
+        else:
+            ops.attn_bwd(t, t, t, t, t, m, m, t, t, t, True, 1)
+            assert [c[-4:-2] for c in calls] == [(None, 0)]
