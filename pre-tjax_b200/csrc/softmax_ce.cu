@@ -898,7 +898,9 @@ extern "C" int ptj_cross_entropy(const int32_t* labels, const void* logits, void
   } else if (same_phase<__nv_bfloat16>(logits, ld, dlogits, ld) && cols <= kCeSmemCols && reinterpret_cast<uintptr_t>(logits) % 2 == 0) {
     const auto kern = aligned16(logits) && ld % 8 == 0 ? cross_entropy_bf16_smem_kernel<false> : cross_entropy_bf16_smem_kernel<true>;
     const int smem = static_cast<int>(cols / 8 * 16);
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
+    // (the limit belongs to the kernel, not to this launch: always the widest row's, or a call of a narrower vocabulary on
+    // another thread would take it away between here and the launch)
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kCeSmemCols / 8 * 16) != cudaSuccess) {
       (void)cudaGetLastError();
       return PTJ_ERR_LAUNCH;
     }

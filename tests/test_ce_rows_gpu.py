@@ -1,5 +1,7 @@
 """The bf16 cross entropy that holds a row in registers, against float64: a few columns around the widths at which the threads
 per row change and at which the three-pass kernel takes over, more rows than blocks, padding rows among them, in place."""
+import threading
+
 import pytest
 import torch
 
@@ -61,3 +63,32 @@ def test_bits_do_not_depend_on_where_a_row_is_held(cols):
     _, _, e, want = ops.cross_entropy(y, z, cols=wide, want_grad=True, want_rows=True)
     assert torch.equal(loss, want)
     assert torch.equal(d[:, :cols - 1], e[:, :cols - 1]) and torch.equal(d[:, cols - 1], e[:, wide - 1])
+
+
+def test_vocabularies_of_several_threads():
+    """The shared memory that a kernel may use is a property of the kernel, not of a launch: a narrow call on one thread must
+    not lower it under a wide one on another."""
+    lib, failed, together = pkg("_lib").lib(), [], threading.Barrier(6)
+
+    def work(cols):
+        x = torch.zeros(1, cols, device="cuda", dtype=torch.bfloat16)
+        y = torch.ones(1, device="cuda", dtype=torch.int32)
+        out, n = torch.empty(5, device="cuda"), torch.ones(1, device="cuda")
+        stream = torch.cuda.Stream()
+        torch.cuda.synchronize()
+        args = (y.data_ptr(), x.data_ptr(), None, out.data_ptr(), n.data_ptr(), 0, out.data_ptr() + 8, 1, cols, cols,
+                pkg("_lib").PTJ_BF16, stream.cuda_stream)
+        together.wait()
+        for _ in range(2000):
+            rc = lib.ptj_cross_entropy(*args)
+            if rc != 0:
+                failed.append((cols, rc))
+                return
+
+    threads = [threading.Thread(target=work, args=(cols,)) for cols in (57344, 30000) * 3]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not failed
