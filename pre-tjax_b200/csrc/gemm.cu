@@ -830,7 +830,7 @@ splitk_finish_kernel(const float* __restrict__ ws, const EpilogueParams ep, int 
 // A product whose last round of 256 x 256 tiles would leave most of the 74 thread-block pairs idle (96 tiles: 74 + 22):
 // head rows that fill whole rounds, and the K parts for the remaining rows so that they fill one more round of short
 // work items. parts == 0: no split (the product does not go to the pair kernel, or its last round is >= 60 % full). Fewer
-// tiles than pairs split over K whole (36 tiles at [3072, 768]) gained nothing over the finishing pass: forward pass 1.49 ms either way.
+// tiles than pairs split over K whole (36 tiles at [3072, 768]) lost by the finishing pass: forward pass of GPT-2 small 1.47 -> 1.50 ms.
 struct TailPlan { int64_t head_rows; int parts; };
 TailPlan tail_split_plan(int64_t M, int64_t N, int64_t K) {
   TailPlan none{0, 0};
@@ -1041,9 +1041,11 @@ extern "C" int ptj_gemm(const void* a, const void* b, void* c, const float* bias
     p.num_m = static_cast<int>(ceil_div(M, 2 * BM));
     p.num_n = static_cast<int>(ceil_div(N, 256));
     // Tiles along M run side by side and share their B rows, while A stays in the L2 for the next column of tiles. An A that
-    // does not fit there is read from memory once per column: then the tiles of a row of them run side by side. LM-head weight
-    // gradient [50257, 8192] x [8192, 768] (A 823 MB): 517 -> 442 us; weight gradients of a layer (A 13 to 50 MB) lose:
-    // 36.7 -> 45.4 us at [3072, 8192] x [8192, 768].
+    // does not fit there (126 MB) is read from memory once per column: then the tiles of a row of them run side by side, whatever
+    // B is. Along M -> along N, [M, K] x [K, N]: LM-head weight gradient [50257, 8192] x [8192, 768] 498 -> 445 us, FFN products
+    // [16384, 4096] x [4096, 1024] 115 -> 102 and 110 -> 99, [32768, 3072] x [3072, 768] 137 -> 121 and 134 -> 116, weight gradients
+    // with K = 16384 and 32768 the same, as where B does not fit either ([8192, 8192] x [8192, 16384] 1724 and 1732). An A of 13
+    // to 50 MB loses: 36.7 -> 45.4 us at [3072, 8192] x [8192, 768].
     p.n_first = static_cast<double>(M) * static_cast<double>(K) * 2.0 > 126e6;
     CUtensorMap ta, tb;
     if (!make_pair_operand_maps(&ta, &tb, a, b, M, N, K, lda, ldb, a_kmajor != 0, b_kmajor != 0)) return PTJ_ERR_LAUNCH;
