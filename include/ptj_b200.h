@@ -266,8 +266,8 @@ int ptj_gemm_grouped2(const ptj_gemm_problem* p0, const ptj_gemm_problem* p1, in
  * acts1: running maximum of the scaled scores and sum of exp(score - max)).
  *   dtype PTJ_BF16 with d_head a multiple of 8 from 16 to 128 and 16-byte aligned rows runs the tcgen05 kernels. With
  *   d_head == 64 and seq % 128 == 0 they round probabilities and score gradients to bf16 before they are multiplied;
- *   otherwise they multiply them in three bf16 parts that hold all 24 bits of a float32. Everything else runs the SIMT
- *   kernels, float32 from the operands to the stored result.
+ *   otherwise they multiply them in three bf16 parts that hold all 24 bits of a float32, and sum in the tensor cores' float32
+ *   accumulators, which truncate. Everything else runs the SIMT kernels, float32 from the operands to the stored result.
  * Backward recomputes the probabilities; it is deterministic (no atomics).
  *
  * row_kstart (optional, int32[batch, seq]): the first key each query row may attend to, so that row i attends keys

@@ -33,7 +33,7 @@ int attn_bwd_simt(const void* d_o, const void* q, const void* k, const void* v, 
 
 // tcgen05 kernels: bf16, d_head a multiple of 8 from 16 to 128, any seq, 16-byte aligned strides.
 // attn_bf16_probabilities: d_head == 64 and seq % 128 == 0: probabilities and score gradients are rounded to bf16 before they
-// are multiplied; the other shapes multiply them in three bf16 parts (24 bits), as the general kernels do in float32.
+// are multiplied; the other shapes multiply them in three bf16 parts (24 bits; the general kernels in float32).
 inline bool attn_bf16_probabilities(const ptj_attn_shape& sh) { return sh.d_head == 64 && sh.seq % 128 == 0; }
 bool attn_tc_supported(const ptj_attn_shape& sh, const void* const* ptrs, int nptrs);
 // keep_bits (optional, both directions): the call's dropout keep flags from attn_keep_bits_tc; NULL = the kernels draw

@@ -13,7 +13,10 @@
 //               (group, block) has its own reference exponent, row sums and output accumulator, so the warps of a row never
 //               meet before the item ends; then the group that got the last tile merges the G NC states of each row
 //               (log-sum-exp merge in a fixed order) and writes it.
-// A probability is split exactly into three bf16 parts, three products each; the operands of S are bf16 as they are.
+// A probability is split exactly into three bf16 parts, three products each; the operands of S are bf16 as they are. Sums run in
+// the tensor cores' float32 accumulators, which truncate at every step: S over a head, O over a row's whole length. Errors
+// against float64 beside those of the float32 FMA kernels, [4, 12, 500, 64] and [2, 16, 1024, 128]: row maximum 7.0e-8 (3.8e-8) and
+// 1.5e-7 (5.5e-8), row sum 1.4e-7 (1.1e-7) and 2.6e-7 (1.7e-7); O, rounded to bf16, 1.592912e-3 and 1.607495e-3 on both.
 // Work items = (query tile, batch*head), heaviest first, dealt to the blocks in boustrophedon order; all tiles of a
 // block's items form one stream, so the next item's first tiles overlap the tail of the current one.
 // Tensor memory: two S buffers at columns [0,256), the G NC accumulators at [256,512).
