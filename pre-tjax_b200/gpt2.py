@@ -327,7 +327,7 @@ class Gpt2Step:
 
     def release_workspaces(self):
         """Gives back the workspaces of launches outside recorded graphs; the next pass allocates what it needs."""
-        self._ws = {k: ws for k, ws in self._ws.items() if k[2]}
+        self._ws = {k: ws for k, ws in list(self._ws.items()) if k[2]}  # (a copy: other threads add to it)
 
     def _layer_workspace(self, plan, backward: bool, device):
         """The workspace of a layer's launches; without the part that only makes them faster where that does not fit (as for
