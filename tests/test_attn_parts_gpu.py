@@ -1,5 +1,6 @@
 """Attention on the tensor cores with float32 probabilities in three bf16 parts (bf16 operands; every row length and head size
 but whole tiles of 64-wide heads) against float64: edges of tiles, narrow and wide heads, one to several tiles and items."""
+import ctypes
 import math
 
 import pytest
@@ -124,3 +125,32 @@ def test_statistics_of_rows_whose_scores_are_all_minus_infinity(S, D):
     assert bool((m[..., :40] == -math.inf).all()) and bool((l[..., :40] == 0).all()) and bool(o[:, :, :40].isnan().all())
     rows = torch.arange(1, S - 39, device="cuda", dtype=torch.float32)  # equal scores
     assert bool(torch.isfinite(m[..., 40:]).all()) and bool(((l[..., 40:] - rows).abs() <= 2.0 ** -20 * rows).all())
+
+
+def test_beyond_four_gigabytes_of_shares_the_general_kernels_run():
+    """dQ shares grow with the square of the row length: from 4 GiB on the call asks for no workspace, and each half of the
+    batch, which has its shares, gives the same up to two roundings."""
+    ops, lib = pkg("operators"), pkg("_lib")
+    B, H, S, D = 2, 64, 8065, 32
+    g = torch.Generator(device="cuda").manual_seed(1)
+    q, k, v, do = (torch.randn(B, H, S, D, generator=g, device="cuda").bfloat16() for _ in range(4))
+
+    def workspace(n):
+        sh = lib.AttnShape(n, H, S, D, *[q.stride()[:3]] * 4)
+        return lib.lib().ptj_attn_bwd_workspace_bytes(ctypes.byref(sh), lib.PTJ_BF16)
+
+    assert workspace(2) == 0 and 2 ** 31 < workspace(1) < 2 ** 32
+    o, *whole = (torch.empty_like(q) for _ in range(4))
+    m, l = ops.attn_fwd(q, k, v, o, True, 1, p=0.0)
+    ops.attn_bwd(do, q, k, v, o, m, l, *whole, True, 1, p=0.0)
+    halves = [torch.empty_like(q) for _ in range(3)]
+    for b in range(2):
+        one = lambda t: t[b:b + 1]
+        ops.attn_bwd(*map(one, (do, q, k, v, o, m, l, *halves)), True, 1, p=0.0)
+    torch.cuda.synchronize()
+    ops._ATTN_WORKSPACE.clear()
+    assert ops.last_kernel_fault() == 0
+    for name, a, b in zip(("dQ", "dK", "dV"), whole, halves):
+        # two roundings to bf16, and 2^-17 of sums of magnitudes (below 64) for float32 sums of up to 8065 terms
+        err = ((a.double() - b.double()).abs() - 2.0 ** -7 * a.double().abs()).max()
+        assert float(err) <= 2.0 ** -11, (name, float(err))
